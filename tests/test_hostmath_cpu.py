@@ -167,3 +167,16 @@ def test_device_form_transcript_matches_oracle(hm):
         assert val(ch) == want * R % o.R_MOD
         assert bytes(state) == bytes(t.strobe.state)
         assert (pos3[0], pos3[1]) == (t.strobe.pos, t.strobe.pos_begin)
+
+
+@pytest.mark.parametrize("name,p", [("fr", o.R_MOD), ("fq", o.Q_MOD)])
+def test_inverse_edges(hm, name, p):
+    """The inversion by division steps at the values where its limbs, signs and early end matter."""
+    rnd = random.Random(11)
+    out = (ctypes.c_uint32 * 8)()
+    rinv = pow(R, -1, p)
+    edge = [0, 1, 2, 3, p - 1, p - 2, (p - 1) // 2, (p + 1) // 2, R % p, pow(R, 2, p), 0xFFFFFFFF, (1 << 30) - 1, 1 << 30, 1 << 240,
+            (1 << 253) - 1] + [1 << (30 * i) for i in range(1, 9)] + [p >> i for i in range(1, 250, 31)]
+    for a in edge + [rnd.randrange(p) for _ in range(300)]:
+        getattr(hm, f"zkh_{name}_inv")(buf(a), out)
+        assert val(out) == (pow(a * rinv, -1, p) * R % p if a else 0)
