@@ -77,55 +77,6 @@ ZK_HD void madwide4(uint32_t* acc, uint32_t x0, uint32_t x1, uint32_t x2, uint32
 #endif
 }
 
-// acc[0..7] += t (single limb), ripple through all eight limbs; the caller has proved no carry out.
-ZK_HD void add_limb8(uint32_t* acc, uint32_t t) {
-#ifdef __CUDA_ARCH__
-  asm("add.cc.u32  %0, %0, %8;\n\t"
-      "addc.cc.u32 %1, %1, 0;\n\t"
-      "addc.cc.u32 %2, %2, 0;\n\t"
-      "addc.cc.u32 %3, %3, 0;\n\t"
-      "addc.cc.u32 %4, %4, 0;\n\t"
-      "addc.cc.u32 %5, %5, 0;\n\t"
-      "addc.cc.u32 %6, %6, 0;\n\t"
-      "addc.u32    %7, %7, 0;"
-      : "+r"(acc[0]), "+r"(acc[1]), "+r"(acc[2]), "+r"(acc[3]), "+r"(acc[4]), "+r"(acc[5]), "+r"(acc[6]),
-        "+r"(acc[7])
-      : "r"(t));
-#else
-  uint64_t c = t;
-  for (int k = 0; k < 8; k++) {
-    c += acc[k];
-    acc[k] = (uint32_t)c;
-    c >>= 32;
-  }
-#endif
-}
-
-// acc[0..8] += t (single limb) rippling through nine limbs; the caller has proved no carry out.
-ZK_HD void add_limb9(uint32_t* acc, uint32_t t) {
-#ifdef __CUDA_ARCH__
-  asm("add.cc.u32  %0, %0, %9;\n\t"
-      "addc.cc.u32 %1, %1, 0;\n\t"
-      "addc.cc.u32 %2, %2, 0;\n\t"
-      "addc.cc.u32 %3, %3, 0;\n\t"
-      "addc.cc.u32 %4, %4, 0;\n\t"
-      "addc.cc.u32 %5, %5, 0;\n\t"
-      "addc.cc.u32 %6, %6, 0;\n\t"
-      "addc.cc.u32 %7, %7, 0;\n\t"
-      "addc.u32    %8, %8, 0;"
-      : "+r"(acc[0]), "+r"(acc[1]), "+r"(acc[2]), "+r"(acc[3]), "+r"(acc[4]), "+r"(acc[5]), "+r"(acc[6]),
-        "+r"(acc[7]), "+r"(acc[8])
-      : "r"(t));
-#else
-  uint64_t c = t;
-  for (int k = 0; k < 9; k++) {
-    c += acc[k];
-    acc[k] = (uint32_t)c;
-    c >>= 32;
-  }
-#endif
-}
-
 // r = a + b over 8 limbs, returns the carry out.
 ZK_HD uint32_t add8(uint32_t* r, const uint32_t* a, const uint32_t* b) {
 #ifdef __CUDA_ARCH__
@@ -153,6 +104,39 @@ ZK_HD uint32_t add8(uint32_t* r, const uint32_t* a, const uint32_t* b) {
   }
   for (int k = 0; k < 8; k++) r[k] = t[k];
   return (uint32_t)c;
+#endif
+}
+
+// r += b over sixteen limbs as one chain; the caller has proved no carry out.
+ZK_HD void add16(uint32_t* r, const uint32_t* b) {
+#ifdef __CUDA_ARCH__
+  asm("add.cc.u32  %0, %0, %16;\n\t"
+      "addc.cc.u32 %1, %1, %17;\n\t"
+      "addc.cc.u32 %2, %2, %18;\n\t"
+      "addc.cc.u32 %3, %3, %19;\n\t"
+      "addc.cc.u32 %4, %4, %20;\n\t"
+      "addc.cc.u32 %5, %5, %21;\n\t"
+      "addc.cc.u32 %6, %6, %22;\n\t"
+      "addc.cc.u32 %7, %7, %23;\n\t"
+      "addc.cc.u32 %8, %8, %24;\n\t"
+      "addc.cc.u32 %9, %9, %25;\n\t"
+      "addc.cc.u32 %10, %10, %26;\n\t"
+      "addc.cc.u32 %11, %11, %27;\n\t"
+      "addc.cc.u32 %12, %12, %28;\n\t"
+      "addc.cc.u32 %13, %13, %29;\n\t"
+      "addc.cc.u32 %14, %14, %30;\n\t"
+      "addc.u32    %15, %15, %31;"
+      : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+        "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+      : "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]), "r"(b[6]), "r"(b[7]), "r"(b[8]), "r"(b[9]),
+        "r"(b[10]), "r"(b[11]), "r"(b[12]), "r"(b[13]), "r"(b[14]), "r"(b[15]));
+#else
+  uint64_t c = 0;
+  for (int k = 0; k < 16; k++) {
+    c += (uint64_t)r[k] + b[k];
+    r[k] = (uint32_t)c;
+    c >>= 32;
+  }
 #endif
 }
 
@@ -184,6 +168,85 @@ ZK_HD uint32_t sub8(uint32_t* r, const uint32_t* a, const uint32_t* b) {
   for (int k = 0; k < 8; k++) r[k] = t[k];
   return c ? 1u : 0u;
 #endif
+}
+
+// One row of a Montgomery product in the even / odd form (see mul): the carry out of the eight limbs of E belongs at limb
+// 8 of the running value, which is O[7]; the caller has proved that nothing is carried out of there.
+// E += (x0, x2, x4, x6) * y.
+ZK_HD void row_even(uint32_t* E, uint32_t& o7, uint32_t x0, uint32_t x2, uint32_t x4, uint32_t x6, uint32_t y) {
+#ifdef __CUDA_ARCH__
+  asm("mad.lo.cc.u32   %0, %9,  %13, %0;\n\t"
+      "madc.hi.cc.u32  %1, %9,  %13, %1;\n\t"
+      "madc.lo.cc.u32  %2, %10, %13, %2;\n\t"
+      "madc.hi.cc.u32  %3, %10, %13, %3;\n\t"
+      "madc.lo.cc.u32  %4, %11, %13, %4;\n\t"
+      "madc.hi.cc.u32  %5, %11, %13, %5;\n\t"
+      "madc.lo.cc.u32  %6, %12, %13, %6;\n\t"
+      "madc.hi.cc.u32  %7, %12, %13, %7;\n\t"
+      "addc.u32        %8, %8, 0;"
+      : "+r"(E[0]), "+r"(E[1]), "+r"(E[2]), "+r"(E[3]), "+r"(E[4]), "+r"(E[5]), "+r"(E[6]), "+r"(E[7]), "+r"(o7)
+      : "r"(x0), "r"(x2), "r"(x4), "r"(x6), "r"(y));
+#else
+  o7 += madwide4_c(E, x0, x2, x4, x6, y);
+#endif
+}
+
+// The division by 2^32 together with the next row's odd products: with E[0] = 0 the value (E + 2^32 O) / 2^32 has the
+// even part O + E[1] and the odd part E[2..7].  Only limb 0 of the even part is added here; its carry belongs at limb 1,
+// where the odd part begins, so it is the carry into the chain that adds (x1, x3, x5, x7) * y to the odd part.
+// On return O is the new even part and E the new odd part.
+// e8: the ninth limb of the old even part, for the callers that have one.
+ZK_HD void row_odd_shift(uint32_t* E, uint32_t* O, uint32_t x1, uint32_t x3, uint32_t x5, uint32_t x7, uint32_t y,
+                         uint32_t e8 = 0) {
+  uint32_t t[8];
+#ifdef __CUDA_ARCH__
+  asm("add.cc.u32      %8, %8, %9;\n\t"
+      "madc.lo.cc.u32  %0, %16, %20, %10;\n\t"
+      "madc.hi.cc.u32  %1, %16, %20, %11;\n\t"
+      "madc.lo.cc.u32  %2, %17, %20, %12;\n\t"
+      "madc.hi.cc.u32  %3, %17, %20, %13;\n\t"
+      "madc.lo.cc.u32  %4, %18, %20, %14;\n\t"
+      "madc.hi.cc.u32  %5, %18, %20, %15;\n\t"
+      "madc.lo.cc.u32  %6, %19, %20, %21;\n\t"
+      "madc.hi.u32     %7, %19, %20, 0;"
+      : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7]), "+r"(O[0])
+      : "r"(E[1]), "r"(E[2]), "r"(E[3]), "r"(E[4]), "r"(E[5]), "r"(E[6]), "r"(E[7]), "r"(x1), "r"(x3), "r"(x5), "r"(x7), "r"(y),
+        "r"(e8));
+#else
+  uint64_t c = (uint64_t)O[0] + E[1];
+  O[0] = (uint32_t)c;
+  c >>= 32;
+  const uint32_t x[4] = {x1, x3, x5, x7};
+  for (int k = 0; k < 4; k++) {
+    const uint64_t p = (uint64_t)x[k] * y;
+    c += (uint64_t)(uint32_t)p + (k < 3 ? E[2 * k + 2] : e8);
+    t[2 * k] = (uint32_t)c;
+    c >>= 32;
+    c += (p >> 32) + (k < 3 ? E[2 * k + 3] : 0u);
+    t[2 * k + 1] = (uint32_t)c;
+    c >>= 32;
+  }
+#endif
+#pragma unroll
+  for (int k = 0; k < 8; k++) E[k] = t[k];
+}
+
+// The same division when the next row's multiplier m = (new even limb 0) * inv depends on it (reduction rows without a
+// product): returns m.
+ZK_HD uint32_t redc_odd_shift(uint32_t* E, uint32_t* O, uint32_t x1, uint32_t x3, uint32_t x5, uint32_t x7, uint32_t inv,
+                              uint32_t e8 = 0) {
+  const uint32_t m = (O[0] + E[1]) * inv;
+  row_odd_shift(E, O, x1, x3, x5, x7, m, e8);
+  return m;
+}
+
+// Last division by 2^32: r = O + (E >> 32) with E[0] = 0; the caller has proved no carry out.
+ZK_HD void row_finish(uint32_t* r, const uint32_t* E, const uint32_t* O) {
+  uint32_t s[8];
+#pragma unroll
+  for (int k = 0; k < 7; k++) s[k] = E[k + 1];
+  s[7] = 0;
+  (void)add8(r, O, s);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -338,42 +401,34 @@ ZK_HD Fp<P> dbl(const Fp<P>& a) {
 // limbs, O the columns that start at odd limbs (O is offset by one limb), so every row of
 // partial products is a chain of non-overlapping 32x32+64 multiply-adds.  After the
 // reduction row the low limb of E is zero; dividing by 2^32 turns the odd columns into the
-// even ones and vice versa, so the two arrays swap roles instead of shifting.
-// Bounds: the running value E + 2^32*O stays below a + p, and below 2^32 (a + p) inside a
-// row, so O fits 8 limbs and E needs one extra limb (e8) only inside a row.
+// even ones and vice versa, so the two arrays swap roles instead of shifting, and the one limb
+// that has to move (E[1] onto O[0]) is the head of the next row's odd chain, which takes its carry.
+// What bounds it is the multiply pipe: 128 wide multiply-adds.  Moving E[1] by an eight-limb addition per row and
+// catching the carries in a ninth limb cost some 70 more instructions a product: 83 G products/s (two chains per thread,
+// 16 warps per SM) against 105 G/s as it is.
+// Bounds: the running value E + 2^32*O stays below a + p, and below 2^32 (a + p) < 2^288 inside a
+// row, so eight limbs of E and of O hold it, with E's carry put into O[7].
 template <class P>
 ZK_HD Fp<P> mul(const Fp<P>& a, const Fp<P>& b) {
-  uint32_t E[8], O[8];
+  uint32_t X[8], Y[8];
 #pragma unroll
-  for (int i = 0; i < 8; i++) E[i] = O[i] = 0;
+  for (int i = 0; i < 8; i++) X[i] = Y[i] = 0;
 #pragma unroll
   for (int i = 0; i < 8; i++) {
+    uint32_t* E = (i & 1) ? Y : X;  // the even columns of this row; the arrays swap roles from row to row
+    uint32_t* O = (i & 1) ? X : Y;
     const uint32_t bi = b.v[i];
-    uint32_t e8 = madwide4_c(E, a.v[0], a.v[2], a.v[4], a.v[6], bi);
-    madwide4(O, a.v[1], a.v[3], a.v[5], a.v[7], bi);
+    if (i == 0)
+      madwide4(O, a.v[1], a.v[3], a.v[5], a.v[7], bi);
+    else
+      row_odd_shift(O, E, a.v[1], a.v[3], a.v[5], a.v[7], bi);
+    row_even(E, O[7], a.v[0], a.v[2], a.v[4], a.v[6], bi);
     const uint32_t m = E[0] * P::inv;
-    e8 += madwide4_c(E, P::mod(0), P::mod(2), P::mod(4), P::mod(6), m);
     madwide4(O, P::mod(1), P::mod(3), P::mod(5), P::mod(7), m);
-    // divide by 2^32: new even = O + E[1]; new odd = E >> 64
-    add_limb8(O, E[1]);
-    uint32_t T[8];
-#pragma unroll
-    for (int k = 0; k < 6; k++) T[k] = E[k + 2];
-    T[6] = e8;
-    T[7] = 0;
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      E[k] = O[k];
-      O[k] = T[k];
-    }
+    row_even(E, O[7], P::mod(0), P::mod(2), P::mod(4), P::mod(6), m);
   }
-  // value = E + 2^32 * O  (< 2p < 2^256)
-  Fp<P> r;
-  uint32_t S[8];
-  S[0] = 0;
-#pragma unroll
-  for (int k = 1; k < 8; k++) S[k] = O[k - 1];
-  (void)add8(r.v, E, S);
+  Fp<P> r;  // after eight rows the even columns are in Y, the odd ones in X; the value is below 2p
+  row_finish(r.v, Y, X);
   final_sub<P>(r.v, 0);
   return r;
 }
@@ -407,6 +462,22 @@ ZK_HD FixedMul<P> make_fixed_mul(const Fp<P>& x_mont) {
   return t;
 }
 
+// The two Montgomery rounds: (E + 2^32 O) / 2^64 mod p for a sum below 3 * 2^289 held in nine even and nine odd limbs.
+// After the first division the value is below 2^260, so the second round stays below 2^288 and its odd part needs eight
+// limbs; the result before the subtraction is below 3 * 2^225 + p < 2p.
+template <class P>
+ZK_HD Fp<P> fixed_finish(uint32_t* E, uint32_t* O) {
+  uint32_t m = E[0] * P::inv;
+  row_even(O, O[8], P::mod(1), P::mod(3), P::mod(5), P::mod(7), m);
+  row_even(E, E[8], P::mod(0), P::mod(2), P::mod(4), P::mod(6), m);
+  m = redc_odd_shift(E, O, P::mod(1), P::mod(3), P::mod(5), P::mod(7), P::inv, E[8]);
+  row_even(O, O[8], P::mod(0), P::mod(2), P::mod(4), P::mod(6), m);
+  Fp<P> r;
+  (void)add8(r.v, O + 1, E);
+  final_sub<P>(r.v, 0);
+  return r;
+}
+
 template <class P>
 ZK_HD Fp<P> mul_fixed(const FixedMul<P>& t, const Fp<P>& d) {
   uint32_t E[9], O[9];
@@ -414,36 +485,10 @@ ZK_HD Fp<P> mul_fixed(const FixedMul<P>& t, const Fp<P>& d) {
   for (int i = 0; i < 9; i++) E[i] = O[i] = 0;
 #pragma unroll
   for (int j = 0; j < 8; j++) {
-    E[8] += madwide4_c(E, t.c[j][0], t.c[j][2], t.c[j][4], t.c[j][6], d.v[j]);
-    O[8] += madwide4_c(O, t.c[j][1], t.c[j][3], t.c[j][5], t.c[j][7], d.v[j]);
+    row_even(E, E[8], t.c[j][0], t.c[j][2], t.c[j][4], t.c[j][6], d.v[j]);
+    row_even(O, O[8], t.c[j][1], t.c[j][3], t.c[j][5], t.c[j][7], d.v[j]);
   }
-#pragma unroll
-  for (int round = 0; round < 2; round++) {
-    const uint32_t m = E[0] * P::inv;
-    E[8] += madwide4_c(E, P::mod(0), P::mod(2), P::mod(4), P::mod(6), m);
-    O[8] += madwide4_c(O, P::mod(1), P::mod(3), P::mod(5), P::mod(7), m);
-    // divide by 2^32: new even = O + E[1] (nine limbs), new odd = E >> 64
-    add_limb9(O, E[1]);
-    uint32_t T[9];
-#pragma unroll
-    for (int k = 0; k < 7; k++) T[k] = E[k + 2];
-    T[7] = 0;
-    T[8] = 0;
-#pragma unroll
-    for (int k = 0; k < 9; k++) {
-      E[k] = O[k];
-      O[k] = T[k];
-    }
-  }
-  // value = E + 2^32 * O < 2^227 + p
-  Fp<P> r;
-  uint32_t S[8];
-  S[0] = 0;
-#pragma unroll
-  for (int k = 1; k < 8; k++) S[k] = O[k - 1];
-  (void)add8(r.v, E, S);
-  final_sub<P>(r.v, 0);
-  return r;
+  return fixed_finish<P>(E, O);
 }
 
 // t0 * d0 + t1 * d1 + t2 * d2 for three launch-constant multipliers in one accumulation: the
@@ -457,39 +502,14 @@ ZK_HD Fp<P> mul_fixed3(const FixedMul<P>& t0, const uint32_t* d0, const FixedMul
   for (int i = 0; i < 9; i++) E[i] = O[i] = 0;
 #pragma unroll
   for (int j = 0; j < 8; j++) {
-    E[8] += madwide4_c(E, t0.c[j][0], t0.c[j][2], t0.c[j][4], t0.c[j][6], d0[j]);
-    O[8] += madwide4_c(O, t0.c[j][1], t0.c[j][3], t0.c[j][5], t0.c[j][7], d0[j]);
-    E[8] += madwide4_c(E, t1.c[j][0], t1.c[j][2], t1.c[j][4], t1.c[j][6], d1[j]);
-    O[8] += madwide4_c(O, t1.c[j][1], t1.c[j][3], t1.c[j][5], t1.c[j][7], d1[j]);
-    E[8] += madwide4_c(E, t2.c[j][0], t2.c[j][2], t2.c[j][4], t2.c[j][6], d2[j]);
-    O[8] += madwide4_c(O, t2.c[j][1], t2.c[j][3], t2.c[j][5], t2.c[j][7], d2[j]);
+    row_even(E, E[8], t0.c[j][0], t0.c[j][2], t0.c[j][4], t0.c[j][6], d0[j]);
+    row_even(O, O[8], t0.c[j][1], t0.c[j][3], t0.c[j][5], t0.c[j][7], d0[j]);
+    row_even(E, E[8], t1.c[j][0], t1.c[j][2], t1.c[j][4], t1.c[j][6], d1[j]);
+    row_even(O, O[8], t1.c[j][1], t1.c[j][3], t1.c[j][5], t1.c[j][7], d1[j]);
+    row_even(E, E[8], t2.c[j][0], t2.c[j][2], t2.c[j][4], t2.c[j][6], d2[j]);
+    row_even(O, O[8], t2.c[j][1], t2.c[j][3], t2.c[j][5], t2.c[j][7], d2[j]);
   }
-#pragma unroll
-  for (int round = 0; round < 2; round++) {
-    const uint32_t m = E[0] * P::inv;
-    E[8] += madwide4_c(E, P::mod(0), P::mod(2), P::mod(4), P::mod(6), m);
-    O[8] += madwide4_c(O, P::mod(1), P::mod(3), P::mod(5), P::mod(7), m);
-    add_limb9(O, E[1]);
-    uint32_t T[9];
-#pragma unroll
-    for (int k = 0; k < 7; k++) T[k] = E[k + 2];
-    T[7] = 0;
-    T[8] = 0;
-#pragma unroll
-    for (int k = 0; k < 9; k++) {
-      E[k] = O[k];
-      O[k] = T[k];
-    }
-  }
-  // value = E + 2^32 * O < 3 * 2^225 + p < 2p
-  Fp<P> r;
-  uint32_t S[8];
-  S[0] = 0;
-#pragma unroll
-  for (int k = 1; k < 8; k++) S[k] = O[k - 1];
-  (void)add8(r.v, E, S);
-  final_sub<P>(r.v, 0);
-  return r;
+  return fixed_finish<P>(E, O);
 }
 
 // a + p - b without the conditional correction: any value congruent to a - b below 2p.
@@ -529,33 +549,18 @@ ZK_HD void mul_wide(Wide& out, const uint32_t* a, const uint32_t* b) {
       madwide4(E + i + 1, a[1], a[3], a[5], a[7], b[i]);
     }
   }
-  // out = E + (O << 32)
-  uint32_t S[8];
+  // out = E + (O << 32); the product fits 512 bits
+  uint32_t S[16];
   S[0] = 0;
 #pragma unroll
-  for (int k = 1; k < 8; k++) S[k] = O[k - 1];
-  uint32_t c = add8(out.v, E, S);
-  // upper half with carry-in: fold the carry into the first addend limb chain
-  uint32_t S2[8];
+  for (int k = 0; k < 16; k++) out.v[k] = E[k];
 #pragma unroll
-  for (int k = 0; k < 8; k++) S2[k] = O[k + 7];
-  uint32_t hi[8];
-#pragma unroll
-  for (int k = 0; k < 8; k++) hi[k] = E[k + 8];
-  add_limb8(hi, c);  // E's upper half + carry cannot overflow: the product fits 512 bits
-  (void)add8(out.v + 8, hi, S2);
+  for (int k = 1; k < 16; k++) S[k] = O[k - 1];
+  add16(out.v, S);
 }
 
 // acc += w over 16 limbs (caller keeps acc below 2^512).
-ZK_HD void wide_add(Wide& acc, const Wide& w) {
-  uint32_t c = add8(acc.v, acc.v, w.v);
-  uint32_t hi[8];
-#pragma unroll
-  for (int k = 0; k < 8; k++) hi[k] = w.v[k + 8];
-  // hi + c cannot overflow 2^256 for the products used here (w < p^2 < 2^508)
-  add_limb8(hi, c);
-  (void)add8(acc.v + 8, acc.v + 8, hi);
-}
+ZK_HD void wide_add(Wide& acc, const Wide& w) { add16(acc.v, w.v); }
 
 // Keep acc < p * 2^256 by subtracting p from the upper half when it is >= p.
 // Valid while acc < 2 * p * 2^256, i.e. after adding at most 5 products of reduced operands
@@ -571,35 +576,28 @@ constexpr int kLazyProducts = 5;
 // upper half (< p) is added afterwards, so one conditional subtraction finishes.
 template <class P>
 ZK_HD Fp<P> redc(const Wide& t) {
-  uint32_t E[8], O[8];
+  uint32_t X[8], Y[8];
 #pragma unroll
   for (int i = 0; i < 8; i++) {
-    E[i] = t.v[i];
-    O[i] = 0;
+    X[i] = t.v[i];
+    Y[i] = 0;
   }
 #pragma unroll
   for (int i = 0; i < 8; i++) {
-    const uint32_t m = E[0] * P::inv;
-    uint32_t e8 = madwide4_c(E, P::mod(0), P::mod(2), P::mod(4), P::mod(6), m);
-    madwide4(O, P::mod(1), P::mod(3), P::mod(5), P::mod(7), m);
-    add_limb8(O, E[1]);
-    uint32_t T[8];
-#pragma unroll
-    for (int k = 0; k < 6; k++) T[k] = E[k + 2];
-    T[6] = e8;
-    T[7] = 0;
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      E[k] = O[k];
-      O[k] = T[k];
+    uint32_t* E = (i & 1) ? Y : X;
+    uint32_t* O = (i & 1) ? X : Y;
+    uint32_t m;
+    if (i == 0) {
+      m = E[0] * P::inv;
+      madwide4(O, P::mod(1), P::mod(3), P::mod(5), P::mod(7), m);
+    } else {
+      m = redc_odd_shift(O, E, P::mod(1), P::mod(3), P::mod(5), P::mod(7), P::inv);
     }
+    row_even(E, O[7], P::mod(0), P::mod(2), P::mod(4), P::mod(6), m);
   }
   Fp<P> r;
-  uint32_t S[8], lo[8];
-  S[0] = 0;
-#pragma unroll
-  for (int k = 1; k < 8; k++) S[k] = O[k - 1];
-  (void)add8(lo, E, S);                   // <= p
+  uint32_t lo[8];
+  row_finish(lo, Y, X);                   // <= p
   uint32_t c = add8(r.v, lo, t.v + 8);    // < 2p < 2^256
   final_sub<P>(r.v, c);
   return r;
