@@ -24,33 +24,54 @@ __device__ __forceinline__ void st_fr_plain(Fr* p, const Fr& x) {
   reinterpret_cast<uint4*>(p)[1] = hi;
 }
 
-// One level of the table: a[x + cur] = r * a[x]; a[x] -= a[x + cur], for x < cur.
-__global__ void __launch_bounds__(256) k_eq_level(Fr* a, uint64_t cur, const FixedMul<FrParams> r) {
-  for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < cur; x += (uint64_t)gridDim.x * blockDim.x) {
-    const Fr v = ld_fr_plain(a + x);
-    const Fr hi = mul_fixed(r, v);
-    st_fr_plain(a + x + cur, hi);
-    st_fr_plain(a + x, sub(v, hi));
+// The eq table in one launch.  A block makes the 2^kEqBits consecutive entries that share their high bits: the factor of the
+// high bits (a product over the variables above kEqBits, by one warp) seeds a doubling over the low variables in shared
+// memory, a[x + cur] = r a[x], a[x] -= a[x + cur], whose last level goes to global memory.  The same number of products as
+// level by level over the whole table, but one launch and one write of the table; launches and the multiplier tables that
+// the host made for every level were most of the time up to 2^20 entries (2^17 entries: a head launch of 11 us and seven
+// level launches of 2.5 us each, with some 4 us of host work before each).
+constexpr int kEqBits = 10;
+__global__ void __launch_bounds__(512) k_eq_table(Fr* out, const Fr* __restrict__ point, int k) {
+  __shared__ Fr sh[1 << (kEqBits - 1)];
+  const int low = k < kEqBits ? k : kEqBits, high = k - low;
+  Fr* dst = out + ((uint64_t)blockIdx.x << low);
+  if (threadIdx.x < 32) {
+    Fr f = Fr::one();
+    if ((int)threadIdx.x < high) {
+      const Fr r = ldg_fr(point + low + threadIdx.x);
+      f = ((blockIdx.x >> threadIdx.x) & 1u) ? r : sub(f, r);
+    }
+    int width = 1;
+    while (width < high) width <<= 1;
+#pragma unroll 1
+    for (int off = width >> 1; off > 0; off >>= 1) {
+      Fr o;
+#pragma unroll
+      for (int i = 0; i < 8; i++) o.v[i] = __shfl_down_sync(0xffffffffu, f.v[i], off);
+      f = mul(f, o);
+    }
+    if (threadIdx.x == 0) {
+      if (low == 0) st_fr_plain(dst, f); else sh[0] = f;
+    }
   }
-}
-
-// The first levels (table of at most 1024 entries) in one block.
-__global__ void __launch_bounds__(512) k_eq_head(Fr* a, const Fr* __restrict__ point, int levels) {
-  __shared__ Fr sh[1024];
-  if (threadIdx.x == 0) sh[0] = Fr::one();
   __syncthreads();
-  for (int i = 0; i < levels; i++) {
+#pragma unroll 1
+  for (int i = 0; i < low; i++) {
     const uint32_t cur = 1u << i;
-    const Fr r = point[i];
     if (threadIdx.x < cur) {
+      const Fr r = ldg_fr(point + i);
       const Fr v = sh[threadIdx.x];
-      const Fr hi = mul(r, v);
-      sh[threadIdx.x + cur] = hi;
-      sh[threadIdx.x] = sub(v, hi);
+      const Fr hi = mul(r, v), lo = sub(v, hi);
+      if (i == low - 1) {
+        st_fr_plain(dst + threadIdx.x + cur, hi);
+        st_fr_plain(dst + threadIdx.x, lo);
+      } else {
+        sh[threadIdx.x + cur] = hi;
+        sh[threadIdx.x] = lo;
+      }
     }
     __syncthreads();
   }
-  for (uint32_t x = threadIdx.x; x < (1u << levels); x += blockDim.x) a[x] = sh[x];
 }
 
 // Partial column sums: block (bx, by) covers 256 columns and the hi range of split by.
@@ -137,20 +158,11 @@ void launch_dot(const Fr* a, const Fr* b, uint64_t n, const RoundScratch& sc, cu
   k_dot<<<(unsigned)blocks, 256, 0, s>>>(a, b, n, sc.sink);
 }
 
-// out[0 .. 2^k) = eq(., point); point_dev holds the k coordinates on the device, point_host the
-// same values on the host (for the per-level multiplier tables).  Returns launches.
-int launch_eq_table(const Fr* point_dev, const Fr* point_host, uint32_t k, Fr* out, int sm_count, cudaStream_t s) {
-  const int head = k < 10 ? (int)k : 10;
-  k_eq_head<<<1, 512, 0, s>>>(out, point_dev, head);
-  int launches = 1;
-  for (uint32_t i = head; i < k; i++) {
-    const uint64_t cur = 1ull << i;
-    uint64_t blocks = (cur + 255) / 256;
-    if (blocks > (uint64_t)sm_count * 8) blocks = sm_count * 8;
-    k_eq_level<<<(unsigned)blocks, 256, 0, s>>>(out, cur, make_fixed_mul(point_host[i]));
-    launches++;
-  }
-  return launches;
+// out[0 .. 2^k) = eq(., point); point_dev holds the k coordinates on the device.  Returns launches.
+int launch_eq_table(const Fr* point_dev, uint32_t k, Fr* out, cudaStream_t s) {
+  const int low = k < (uint32_t)kEqBits ? (int)k : kEqBits;
+  k_eq_table<<<(unsigned)(1ull << (k - low)), 1 << (kEqBits - 1), 0, s>>>(out, point_dev, (int)k);
+  return 1;
 }
 
 uint32_t from_right_splits(uint64_t lo_n, uint64_t hi_n, int sm_count) {
