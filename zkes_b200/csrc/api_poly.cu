@@ -10,7 +10,7 @@ int eq_table_device(zk_ctx* ctx, const uint64_t* point_host, uint32_t k, Fr* poi
   cudaStream_t s = ctx->stream;
   if (k) ZK_CUDA(cudaMemcpyAsync(point_dev, point_host, (size_t)k * sizeof(Fr), cudaMemcpyHostToDevice, s));
   ctx->prof_begin(ZK_PROF_FROM_RIGHT, 32.0 * 3 * (double)(1ull << k), 1);
-  ctx->launches += launch_eq_table(point_dev, k, table, s);
+  ctx->launches += launch_eq_table(point_dev, k, table, ctx->sm_count, s);
   ctx->prof_end();
   return ZK_OK;
 }

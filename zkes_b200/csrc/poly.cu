@@ -24,37 +24,47 @@ __device__ __forceinline__ void st_fr_plain(Fr* p, const Fr& x) {
   reinterpret_cast<uint4*>(p)[1] = hi;
 }
 
-// The eq table in one launch.  A block makes the 2^kEqBits consecutive entries that share their high bits: the factor of the
-// high bits (a product over the variables above kEqBits, by one warp) seeds a doubling over the low variables in shared
-// memory, a[x + cur] = r a[x], a[x] -= a[x + cur], whose last level goes to global memory.  The same number of products as
-// level by level over the whole table, but one launch and one write of the table; launches and the multiplier tables that
-// the host made for every level were most of the time up to 2^20 entries (2^17 entries: a head launch of 11 us and seven
-// level launches of 2.5 us each, with some 4 us of host work before each).
-constexpr int kEqBits = 10;
-__global__ void __launch_bounds__(512) k_eq_table(Fr* out, const Fr* __restrict__ point, int k) {
-  __shared__ Fr sh[1 << (kEqBits - 1)];
+// The eq table in one launch, in stretches of 2^kEqBits consecutive entries that share their high bits; the factor of the
+// high bits is a product over the variables above kEqBits.  Launches and the multiplier tables that the host made for every
+// level were most of the time of a doubling level by level (2^17 entries: a head launch of 11 us and seven level launches of
+// 2.5 us each, with some 4 us of host work before each).
+//   One stretch a block (up to kEqWave blocks per SM): the factor seeds a doubling over the low variables in shared memory,
+//   a[x + cur] = r a[x], a[x] -= a[x + cur], whose last level goes to global memory; a chain of some twelve products.
+//   More: the doubling starts from one and makes the low table, and a block multiplies it by the factors of its stretches,
+//   one product an entry instead of a chain per stretch (2^21 entries: 54 us against 79 us with a chain for every stretch).
+constexpr int kEqBits = 10, kEqThreads = 512, kEqWave = 2;
+
+__device__ __forceinline__ Fr eq_factor(const Fr* __restrict__ point, uint64_t hi, int j) {
+  const Fr r = ldg_fr(point + j);
+  return ((hi >> j) & 1u) ? r : sub(Fr::one(), r);
+}
+
+__global__ void __launch_bounds__(kEqThreads) k_eq_table(Fr* out, const Fr* __restrict__ point, int k) {
+  __shared__ Fr sh[1 << kEqBits];
+  __shared__ Fr seeds[kEqThreads];
   const int low = k < kEqBits ? k : kEqBits, high = k - low;
-  Fr* dst = out + ((uint64_t)blockIdx.x << low);
+  const uint64_t n_hi = 1ull << high;
+  const bool seeded = n_hi <= gridDim.x;  // one stretch per block
   if (threadIdx.x < 32) {
     Fr f = Fr::one();
-    if ((int)threadIdx.x < high) {
-      const Fr r = ldg_fr(point + low + threadIdx.x);
-      f = ((blockIdx.x >> threadIdx.x) & 1u) ? r : sub(f, r);
-    }
-    int width = 1;
-    while (width < high) width <<= 1;
+    if (seeded) {
+      if ((int)threadIdx.x < high) f = eq_factor(point + low, blockIdx.x, threadIdx.x);
+      int width = 1;
+      while (width < high) width <<= 1;
 #pragma unroll 1
-    for (int off = width >> 1; off > 0; off >>= 1) {
-      Fr o;
+      for (int off = width >> 1; off > 0; off >>= 1) {
+        Fr o;
 #pragma unroll
-      for (int i = 0; i < 8; i++) o.v[i] = __shfl_down_sync(0xffffffffu, f.v[i], off);
-      f = mul(f, o);
+        for (int i = 0; i < 8; i++) o.v[i] = __shfl_down_sync(0xffffffffu, f.v[i], off);
+        f = mul(f, o);
+      }
     }
     if (threadIdx.x == 0) {
-      if (low == 0) st_fr_plain(dst, f); else sh[0] = f;
+      if (low == 0) st_fr_plain(out, f); else sh[0] = f;
     }
   }
   __syncthreads();
+  Fr* dst = out + ((uint64_t)blockIdx.x << low);
 #pragma unroll 1
   for (int i = 0; i < low; i++) {
     const uint32_t cur = 1u << i;
@@ -62,13 +72,33 @@ __global__ void __launch_bounds__(512) k_eq_table(Fr* out, const Fr* __restrict_
       const Fr r = ldg_fr(point + i);
       const Fr v = sh[threadIdx.x];
       const Fr hi = mul(r, v), lo = sub(v, hi);
-      if (i == low - 1) {
+      if (seeded && i == low - 1) {
         st_fr_plain(dst + threadIdx.x + cur, hi);
         st_fr_plain(dst + threadIdx.x, lo);
       } else {
         sh[threadIdx.x + cur] = hi;
         sh[threadIdx.x] = lo;
       }
+    }
+    __syncthreads();
+  }
+  if (seeded) return;
+  // this block's stretches are blockIdx.x, blockIdx.x + gridDim.x, ...: their factors kEqThreads at a time, then the products
+  for (uint64_t first = blockIdx.x; first < n_hi; first += (uint64_t)kEqThreads * gridDim.x) {
+    const uint64_t mine = first + (uint64_t)threadIdx.x * gridDim.x;
+    if (mine < n_hi) {
+      Fr f = eq_factor(point + low, mine, 0);
+#pragma unroll 1
+      for (int j = 1; j < high; j++) f = mul(f, eq_factor(point + low, mine, j));
+      seeds[threadIdx.x] = f;
+    }
+    __syncthreads();
+    for (uint32_t t = 0; t < kEqThreads; t++) {
+      const uint64_t hi = first + (uint64_t)t * gridDim.x;
+      if (hi >= n_hi) break;
+      const Fr f = seeds[t];
+#pragma unroll 1
+      for (uint32_t x = threadIdx.x; x < (1u << kEqBits); x += kEqThreads) st_fr_plain(out + (hi << kEqBits) + x, mul(f, sh[x]));
     }
     __syncthreads();
   }
@@ -159,9 +189,9 @@ void launch_dot(const Fr* a, const Fr* b, uint64_t n, const RoundScratch& sc, cu
 }
 
 // out[0 .. 2^k) = eq(., point); point_dev holds the k coordinates on the device.  Returns launches.
-int launch_eq_table(const Fr* point_dev, uint32_t k, Fr* out, cudaStream_t s) {
-  const int low = k < (uint32_t)kEqBits ? (int)k : kEqBits;
-  k_eq_table<<<(unsigned)(1ull << (k - low)), 1 << (kEqBits - 1), 0, s>>>(out, point_dev, (int)k);
+int launch_eq_table(const Fr* point_dev, uint32_t k, Fr* out, int sm_count, cudaStream_t s) {
+  const uint64_t stretches = k > (uint32_t)kEqBits ? 1ull << (k - kEqBits) : 1, wave = (uint64_t)sm_count * kEqWave;
+  k_eq_table<<<(unsigned)(stretches < wave ? stretches : wave), kEqThreads, 0, s>>>(out, point_dev, (int)k);
   return 1;
 }
 
