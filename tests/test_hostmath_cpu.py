@@ -180,3 +180,16 @@ def test_inverse_edges(hm, name, p):
     for a in edge + [rnd.randrange(p) for _ in range(300)]:
         getattr(hm, f"zkh_{name}_inv")(buf(a), out)
         assert val(out) == (pow(a * rinv, -1, p) * R % p if a else 0)
+
+
+@pytest.mark.parametrize("name,p", [("fr", o.R_MOD), ("fq", o.Q_MOD)])
+def test_device_rows(hm, name, p):
+    """The product rows that the device runs (the host has its own form of the product)."""
+    rnd = random.Random(12)
+    out = (ctypes.c_uint32 * 8)()
+    rinv = pow(R, -1, p)
+    edge = [0, 1, 2, p - 1, p - 2, (p - 1) // 2, R % p, 0xFFFFFFFF, (1 << 253) - 1] + [1 << (32 * i) for i in range(1, 8)]
+    for a in edge + [rnd.randrange(p) for _ in range(300)]:
+        for b in (R - 1, p, rnd.randrange(R), rnd.choice(edge)):
+            getattr(hm, f"zkh_{name}_mul_rows")(buf(a), buf(b), out)
+            assert val(out) == a * b * rinv % p

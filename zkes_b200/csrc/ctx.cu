@@ -28,6 +28,7 @@ int zk_ctx::setup() {
   ZK_CUDA(cudaMalloc(&resident_sh, 8192));
   ZK_CUDA(cudaMemsetAsync(resident_sh, 0, 8192, stream));
   ZK_CUDA(cudaMalloc(&tail_buf, sizeof(Fr) * 64 * kMaxPolys * 4));
+  ZK_CUDA(cudaHostAlloc(&host_points, kHostPointsBytes, cudaHostAllocDefault));
   ZK_CUDA(cudaHostAlloc(&host_small, 8192, cudaHostAllocDefault));
   ZK_CUDA(cudaStreamSynchronize(stream));
   return 0;
@@ -104,6 +105,7 @@ void zk_ctx::teardown() {
   cudaFree(aux);
   cudaFree(cmp);
   if (host_small) cudaFreeHost(host_small);
+  if (host_points) cudaFreeHost(host_points);
   for (auto& sp : prof_spans) {
     cudaEventDestroy(sp.e0);
     cudaEventDestroy(sp.e1);

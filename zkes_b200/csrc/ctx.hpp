@@ -54,6 +54,7 @@ struct MsmStatsPod {
 
 struct zk_comm;
 
+constexpr size_t kHostPointsBytes = 68 * 1024;  // zk_ctx::host_points
 constexpr size_t kFinalHostOffset = 7168;  // zk_ctx::host_small: where the final values land when they are read back with the rounds
 
 struct zk_ctx {
@@ -65,6 +66,7 @@ struct zk_ctx {
   zk::RoundScratch rs{};
   zk::Fr* final_out = nullptr;   // kMaxPolys + 1 elements
   void* tail_out = nullptr;      // device-resident rounds: messages, challenges, transcript state (8 KiB)
+  void* host_points = nullptr;   // pinned: window sums of a few rows and their combination (msm.cu)
   void* resident_sh = nullptr;   // zk::ResidentShared: hand-over area of the resident multi-round kernel (8 KiB)
   zk::Fr* tail_buf = nullptr;    // sharded proves: gathered values and the last log2(world) rounds' tables
   void* host_small = nullptr;    // pinned, 8 KiB: round messages and other tiny read-backs

@@ -681,6 +681,28 @@ static int windows_for(uint32_t max_mag, int w) {
   return k;
 }
 
+// Horner over the windows on the host, for one row or a few: a doubling is a chain of products, 0.3 us for a CPU core with
+// 64-bit limbs and 2.7 us for a warp, against which the two small copies and the synchronisation (some 20 us) count little
+// from a few dozen doublings on.
+constexpr uint32_t kHostCombineRows = 4, kHostCombineChain = 24;
+static int combine_on_host(zk_ctx* ctx, const Xyzz* window_sums, uint32_t rows, int w, int k_windows, Jacobian* out_dev) {
+  static_assert(kHostCombineRows * 128 * sizeof(Xyzz) + kHostCombineRows * sizeof(Jacobian) <= kHostPointsBytes, "128 windows of two bits at most");
+  Xyzz* ws = reinterpret_cast<Xyzz*>(ctx->host_points);
+  Jacobian* out = reinterpret_cast<Jacobian*>(ws + kHostCombineRows * 128);
+  ZK_CUDA(cudaMemcpyAsync(ws, window_sums, (size_t)rows * k_windows * sizeof(Xyzz), cudaMemcpyDeviceToHost, ctx->stream));
+  ZK_CUDA(cudaStreamSynchronize(ctx->stream));
+  for (uint32_t r = 0; r < rows; r++) {
+    Xyzz acc = Xyzz::inf();
+    for (int k = k_windows - 1; k >= 0; k--) {
+      for (int i = 0; i < w && !acc.is_inf(); i++) acc = dbl(acc);
+      acc = add(acc, ws[(size_t)r * k_windows + k]);
+    }
+    out[r] = to_jacobian(acc);
+  }
+  ZK_CUDA(cudaMemcpyAsync(out_dev, out, rows * sizeof(Jacobian), cudaMemcpyHostToDevice, ctx->stream));
+  return 0;
+}
+
 // row_ids == nullptr: `rows` dense rows of n scalars each over the same n bases.  Otherwise: n scalars in
 // all, scalar i contributes scalars[i] * bases[gather ? gather[i] : i] to output row row_ids[i] < rows.
 int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const uint32_t* row_ids, const Fr* scalars,
@@ -856,7 +878,12 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
     k_msm_bucket_reduce_rows<<<(n_items + 15) / 16, 128, 0, s>>>(bucket_sums, half, n_items, window_sums);
   else
     k_msm_bucket_reduce<<<n_items, threads, threads * sizeof(Xyzz), s>>>(bucket_sums, half, window_sums);
-  k_msm_combine<<<(rows + 63) / 64, 64, 0, s>>>(window_sums, rows, w, k_windows, out_dev);
+  if (rows <= kHostCombineRows && (uint32_t)w * (uint32_t)(k_windows - 1) >= kHostCombineChain) {
+    rc = combine_on_host(ctx, window_sums, rows, w, k_windows, out_dev);
+    if (rc) return rc;
+  } else {
+    k_msm_combine<<<(rows + 63) / 64, 64, 0, s>>>(window_sums, rows, w, k_windows, out_dev);
+  }
   ctx->launches += 2;
   ZK_CUDA(cudaGetLastError());
   ctx->msm_entries_sum += n_entries;
