@@ -1,0 +1,98 @@
+"""The routes of the MSM pipeline at the sizes where they change: long buckets, and the reduction of a window's buckets over
+several blocks.  The bases are known
+multiples of g, so that the expected point of any row is one multiple of g."""
+import ctypes
+import random
+
+import numpy as np
+import pytest
+
+import pyoracle as o
+from zkes_b200 import curve
+from zkes_b200._lib import ZK_MEM_DEVICE, ZK_MEM_HOST, check, lib
+from zkes_b200.field import to_mont_array
+
+pytestmark = pytest.mark.gpu
+vp = ctypes.c_void_p
+
+
+@pytest.fixture(scope="module")
+def multiples():
+    """k_i and k_i g; repeats, opposite points and infinity among them."""
+    rnd = random.Random(9)
+    ks = [rnd.randrange(1, 1 << 64) for _ in range(61)] + [0, 1, 1, 2, o.R_MOD - 1, o.R_MOD - 2, 3]
+    return ks, [o.g1_mul(o.G1_GEN, k) if k else None for k in ks]
+
+
+def of_g(k):
+    k %= o.R_MOD
+    return o.g1_mul(o.G1_GEN, k) if k else None
+
+
+def _device_msm(ctx, bases, scalars):
+    import torch
+
+    out = np.zeros((1, 12), dtype=np.uint64)
+    torch.cuda.synchronize()
+    check(lib.zk_msm_g1(ctx.handle, vp(bases.data_ptr()), ZK_MEM_DEVICE, vp(scalars.data_ptr()), ZK_MEM_DEVICE, bases.shape[0],
+                        vp(out.ctypes.data), ZK_MEM_HOST), "zk_msm_g1")
+    return curve.jacobian_to_affine_py(out)[0]
+
+
+def _repeated(pool, picks):
+    import torch
+
+    return torch.from_numpy(pool.view(np.int64)).cuda()[torch.from_numpy(picks).cuda()].contiguous()
+
+
+@pytest.mark.parametrize("n", [1 << 21, 10_000_003])
+@pytest.mark.parametrize("scalars", [[1, -1], [-128, 127, 5, 0, 1]])
+def test_long_buckets_of_repeated_points(ctx, multiples, n, scalars):
+    """Few buckets over millions of entries, and so few distinct points that equal, opposite and infinite operands meet at
+    every step of the running sums."""
+    ks, pts = multiples
+    rng = np.random.default_rng(n)
+    pick = rng.integers(0, len(ks), size=n)
+    sel = rng.integers(0, len(scalars), size=n)
+    counts = np.zeros((len(ks), len(scalars)), dtype=np.int64)
+    np.add.at(counts, (pick, sel), 1)
+    want = sum(int(counts[i, j]) * ks[i] * scalars[j] for i in range(len(ks)) for j in range(len(scalars)))
+    bases = _repeated(curve.affine_to_array(pts), pick)
+    sc = _repeated(to_mont_array([o.fr_from_int(v) for v in scalars]), sel)
+    assert _device_msm(ctx, bases, sc) == of_g(want)
+
+
+@pytest.mark.parametrize("n", [1 << 15, 100_003, (1 << 20) + 1])
+def test_full_width_windows(ctx, multiples, n):
+    """Full-width scalars: several blocks per window in the bucket reduction, a degenerate top window, and the
+    combination on the host."""
+    ks, pts = multiples
+    rng = np.random.default_rng(n)
+    rnd = random.Random(n)
+    scalars = [o.R_MOD - 1, (o.R_MOD - 1) // 2, (o.R_MOD + 1) // 2, 1, 0] + [rnd.randrange(o.R_MOD) for _ in range(2043)]
+    pick = rng.integers(0, len(ks), size=n)
+    sel = rng.integers(0, len(scalars), size=n)
+    per_scalar = [0] * len(scalars)
+    for i, j in zip(pick.tolist(), sel.tolist()):
+        per_scalar[j] += ks[i]
+    want = sum(t * s for t, s in zip(per_scalar, scalars))
+    assert _device_msm(ctx, _repeated(curve.affine_to_array(pts), pick), _repeated(to_mont_array(scalars), sel)) == of_g(want)
+
+
+@pytest.mark.parametrize("rows,n", [(2, 5000), (40, 700), (700, 300)])
+def test_full_width_rows(ctx, multiples, rows, n):
+    """The combination of the windows on the host, by a warp per row and by a thread per row."""
+    ks, pts = multiples
+    rng = np.random.default_rng(rows)
+    rnd = random.Random(rows)
+    scalars = [o.R_MOD - 1, 0, 1] + [rnd.randrange(o.R_MOD) for _ in range(509)]
+    pick = rng.integers(0, len(ks), size=n)
+    sel = rng.integers(0, len(scalars), size=(rows, n))
+    bases = np.ascontiguousarray(curve.affine_to_array(pts)[pick])
+    sc = np.ascontiguousarray(to_mont_array(scalars)[sel.reshape(-1)])
+    out = np.zeros((rows, 12), dtype=np.uint64)
+    check(lib.zk_msm_g1_batched(ctx.handle, vp(bases.ctypes.data), ZK_MEM_HOST, n, vp(sc.ctypes.data), ZK_MEM_HOST, rows,
+                                vp(out.ctypes.data), ZK_MEM_HOST), "zk_msm_g1_batched")
+    for r in sorted({0, 1, rows // 2, rows - 1}):
+        want = sum(ks[p] * scalars[s] for p, s in zip(pick.tolist(), sel[r].tolist()))
+        assert curve.jacobian_to_affine_py(out[r:r + 1])[0] == of_g(want), r

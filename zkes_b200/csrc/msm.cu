@@ -15,6 +15,7 @@
 // fold to a few bits, so they use one narrow window: no doublings, few buckets.
 #include "msm.hpp"
 #include "reduce.cuh"
+#include "quad.cuh"
 
 namespace zk {
 namespace {
@@ -249,6 +250,7 @@ __device__ __forceinline__ uint32_t bucket_of(const uint32_t* __restrict__ offse
 // few kilobytes instead of forty, which the instruction cache holds (measured 4 % faster on the
 // commit of 2^24 points; the inlined form stalled on instruction fetch).
 __device__ __noinline__ Fq fq_mul_call(const Fq a, const Fq b) { return mul(a, b); }
+__device__ __noinline__ Fq fq_sqr_call(const Fq a) { return sqr(a); }
 
 __device__ __forceinline__ Xyzz add_mixed_calls(const Xyzz& p, const Affine& q) {
   if (q.is_inf()) return p;
@@ -262,8 +264,8 @@ __device__ __forceinline__ Xyzz add_mixed_calls(const Xyzz& p, const Affine& q) 
     return d;
   }
   Xyzz r;
-  const Fq pp = fq_mul_call(pp_, pp_), ppp = fq_mul_call(pp_, pp), q_ = fq_mul_call(p.x, pp);
-  r.x = sub(sub(fq_mul_call(r_, r_), ppp), dbl(q_));
+  const Fq pp = fq_sqr_call(pp_), ppp = fq_mul_call(pp_, pp), q_ = fq_mul_call(p.x, pp);
+  r.x = sub(sub(fq_sqr_call(r_), ppp), dbl(q_));
   r.y = sub(fq_mul_call(r_, sub(q_, r.x)), fq_mul_call(p.y, ppp));
   r.zz = fq_mul_call(p.zz, pp);
   r.zzz = fq_mul_call(p.zzz, ppp);
@@ -329,34 +331,55 @@ __global__ void __launch_bounds__(256) k_msm_fixup_few(const uint32_t* __restric
   st_xyzz(bucket_sums + b, acc);
 }
 
-// One warp per listed bucket (those cut into many pieces).
-__global__ void __launch_bounds__(128) k_msm_fixup(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ many,
-                                                   const uint32_t* __restrict__ n_many, uint32_t seg,
-                                                   Xyzz* bucket_sums, const Xyzz* heads, const Xyzz* tails) {
-  __shared__ Xyzz sh[4][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t total = *n_many;
-  for (uint32_t item = blockIdx.x * 4 + warp; item < total; item += gridDim.x * 4) {
-  const uint32_t b = many[item];
-  const uint32_t s = offsets[b], e = offsets[b + 1];
-  const uint32_t c0 = s / seg, c1 = (e - 1) / seg;
-  // pieces: tail of chunk c0, heads of chunks c0+1 .. c1
-  Xyzz acc = Xyzz::inf();
-  for (uint32_t c = c0 + lane; c <= c1; c += 32) {
-    const Xyzz h = ld_xyzz(c == c0 ? tails + c : heads + c);
-    add_to(&acc, &h);
+// sh[0] = sh[0] + ... + sh[n - 1] for a power of two n of at most twice the block: a thread per addition while there are
+// enough of them, four lanes per addition for the last levels.  The whole block calls it after a barrier.
+__device__ __forceinline__ void tree_sum(Xyzz* sh, uint32_t n) {
+  uint32_t off = n >> 1;
+#pragma unroll 1
+  for (; off > blockDim.x / 4; off >>= 1) {
+    if (threadIdx.x < off) add_to(&sh[threadIdx.x], &sh[threadIdx.x + off]);
+    __syncthreads();
   }
-  sh[warp][lane] = acc;
-  __syncwarp();
-  for (int off = 16; off > 0; off >>= 1) {
-    if (lane < off) {
-      add_to(&acc, &sh[warp][lane + off]);
-      sh[warp][lane] = acc;
+#pragma unroll 1
+  for (; off > 0; off >>= 1) {
+    const uint32_t q = threadIdx.x >> 2, i = q < off ? q : 0;
+    if ((threadIdx.x & ~31u) < 4 * off) {  // whole warps
+      const int role = threadIdx.x & 3;
+      const QuadXyzz v = quad_add(quad_load(&sh[i], role), quad_load(&sh[i + off], role), role);
+      __syncwarp();
+      if (q < off) quad_store(&sh[q], v, role);
     }
-    __syncwarp();
+    __syncthreads();
   }
-  if (lane == 0) st_xyzz(bucket_sums + b, acc);
-  __syncwarp();
+}
+
+// A listed bucket (one cut into many pieces) per block and pass: the top window of full-width scalars has a handful of
+// buckets that between them take every point, a thousand pieces each.  The time is the longest chain of dependent
+// additions: 256 threads leave pieces / 256 of them plus eight levels of a tree, where a warp per bucket left
+// pieces / 32 plus five (100003 full-width scalars: 490 us against 131 us).
+constexpr int kFixupThreads = 256;
+__global__ void __launch_bounds__(kFixupThreads) k_msm_fixup(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ many,
+                                                             const uint32_t* __restrict__ n_many, uint32_t seg,
+                                                             Xyzz* bucket_sums, const Xyzz* heads, const Xyzz* tails) {
+  __shared__ Xyzz sh[kFixupThreads];
+  const uint32_t total = *n_many;
+  for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
+    const uint32_t b = many[item];
+    const uint32_t s = offsets[b], e = offsets[b + 1];
+    const uint32_t c0 = s / seg, c1 = (e - 1) / seg;
+    // pieces: tail of chunk c0, heads of chunks c0+1 .. c1
+    Xyzz acc = Xyzz::inf();
+    for (uint32_t c = c0 + threadIdx.x; c <= c1; c += kFixupThreads) {
+      const Xyzz h = ld_xyzz(c == c0 ? tails + c : heads + c);
+      add_to(&acc, &h);
+    }
+    sh[threadIdx.x] = acc;
+    __syncthreads();
+    uint32_t live = kFixupThreads;  // the shares beyond the number of pieces are infinity
+    while (live > 1 && live / 2 >= c1 - c0 + 1) live >>= 1;
+    tree_sum(sh, live);
+    if (threadIdx.x == 0) st_xyzz(bucket_sums + b, sh[0]);
+    __syncthreads();
   }
 }
 
@@ -438,53 +461,113 @@ __global__ void __launch_bounds__(32) k_msm_fixup_groups_final(const uint32_t* _
   if (threadIdx.x == 0) st_xyzz(bucket_sums + b, acc);
 }
 
-// One block per (row, window): sum_j (j + 1) * B_j over `half` buckets.
-__global__ void __launch_bounds__(256) k_msm_bucket_reduce(const Xyzz* __restrict__ bucket_sums, uint32_t half,
-                                                           Xyzz* window_sums) {
-  extern __shared__ unsigned char sh_raw[];
-  Xyzz* sh = reinterpret_cast<Xyzz*>(sh_raw);
-  const Xyzz* B = bucket_sums + (size_t)blockIdx.x * half;
-  const uint32_t per = (half + blockDim.x - 1) / blockDim.x;
-  const uint32_t lo = threadIdx.x * per;
-  const uint32_t hi = (lo + per < half) ? lo + per : half;
+// sum_j (j + 1) B_j over the `half` buckets of an item, one item per (row, window).  A run of len consecutive buckets is
+// carried as the pair A = sum_j (j - lo + 1) B_j, D = len * sum_j B_j, and two neighbouring runs of equal length join as
+// A = A1 + A2 + D2, D = 2 (D1 + D2): no multiples by an offset, and the two halves of a join are independent, so two threads
+// work on it.  A thread starts with a run of `per` buckets (running sums), a block joins its 128 runs, and a second launch
+// joins the blocks' runs of an item.  What bounds it is the chain of dependent additions (2 per + 2 per level of the tree),
+// so an item is spread over half / (128 per) blocks: 19 items of 8192 buckets take 224 + 24 us; one block per item with up to
+// 32 buckets a thread took 774 us and kept 19 of 148 SMs busy.
+constexpr uint32_t kReduceThreads = 128;
+
+// Joins n runs (a power of two, at most kReduceThreads) in A[], D[] (shared memory) into A[0], D[0].
+__device__ __forceinline__ void join_runs(Xyzz* A, Xyzz* D, uint32_t n) {
+  uint32_t pairs = n >> 1;
+#pragma unroll 1
+  for (; pairs > 16; pairs >>= 1) {  // a thread per half of a join, the D halves in warps of their own
+    const uint32_t t = threadIdx.x;
+    const bool is_a = t < pairs, is_d = t >= pairs && t < 2 * pairs;
+    const uint32_t i = is_a ? t : t - pairs;
+    Xyzz v;
+    if (is_a) {
+      v = A[2 * i];
+      add_to(&v, &A[2 * i + 1]);
+      add_to(&v, &D[2 * i + 1]);
+    } else if (is_d) {
+      v = D[2 * i];
+      add_to(&v, &D[2 * i + 1]);
+      dbl_in_place(&v);
+    }
+    __syncthreads();
+    if (is_a) A[i] = v;
+    if (is_d) D[i] = v;
+    __syncthreads();
+  }
+  // four lanes per half: the first two warps take the A halves, the others the D halves
+#pragma unroll 1
+  for (; pairs > 0; pairs >>= 1) {
+    const uint32_t q = (threadIdx.x & 63) >> 2, i = q < pairs ? q : 0;
+    const int role = threadIdx.x & 3;
+    const bool is_d = threadIdx.x >= 64;
+    Xyzz* R = is_d ? D : A;
+    QuadXyzz v = quad_add(quad_load(&R[2 * i], role), quad_load(&R[2 * i + 1], role), role);
+    if (is_d) v = quad_dbl(v, role); else v = quad_add(v, quad_load(&D[2 * i + 1], role), role);
+    __syncthreads();
+    if (q < pairs) quad_store(&R[q], v, role);
+    __syncthreads();
+  }
+}
+
+// runs[2 * block], runs[2 * block + 1] = A and D of the block's buckets; with one block per item A goes to window_sums.
+__global__ void __launch_bounds__(kReduceThreads) k_msm_bucket_reduce(const Xyzz* __restrict__ bucket_sums, uint32_t half,
+                                                                      uint32_t per, uint32_t blocks_per_item, Xyzz* runs,
+                                                                      Xyzz* window_sums) {
+  __shared__ Xyzz A[kReduceThreads], D[kReduceThreads];
+  const uint32_t item = blockIdx.x / blocks_per_item, part = blockIdx.x % blocks_per_item;
+  const Xyzz* B = bucket_sums + (size_t)item * half;
+  const uint32_t lo = (part * kReduceThreads + threadIdx.x) * per;
   Xyzz running = Xyzz::inf(), acc = Xyzz::inf();
-  if (lo < half) {
-    for (uint32_t j = hi; j-- > lo;) {
+  if (lo < half) {  // per divides half
+    for (uint32_t j = lo + per; j-- > lo;) {
       const Xyzz bj = ld_xyzz(B + j);
       add_to(&running, &bj);
       add_to(&acc, &running);
     }
-    if (lo) {
-      const Xyzz m = mul_small(running, lo);
-      add_to(&acc, &m);
-    }
+    for (uint32_t k = per; k > 1; k >>= 1) dbl_in_place(&running);
   }
-  sh[threadIdx.x] = acc;
+  A[threadIdx.x] = acc;
+  D[threadIdx.x] = running;
   __syncthreads();
-  for (uint32_t off = blockDim.x >> 1; off > 0; off >>= 1) {
-    if (threadIdx.x < off) {
-      add_to(&acc, &sh[threadIdx.x + off]);
-      sh[threadIdx.x] = acc;
+  uint32_t n = half / per;  // runs of the item
+  if (n > kReduceThreads) n = kReduceThreads;
+  join_runs(A, D, n);
+  if (threadIdx.x == 0) {
+    if (blocks_per_item == 1) {
+      st_xyzz(window_sums + item, A[0]);
+    } else {
+      st_xyzz(runs + 2 * (size_t)blockIdx.x, A[0]);
+      st_xyzz(runs + 2 * (size_t)blockIdx.x + 1, D[0]);
     }
-    __syncthreads();
   }
-  if (threadIdx.x == 0) st_xyzz(window_sums + blockIdx.x, acc);
 }
 
-// Many short rows (the d_x / d_y rows of a commitment: thousands of (row, window) items of at most
-// 256 buckets): a block per item leaves most of its additions to idle lanes.  Here eight lanes share
-// an item and four items a warp.  Lane l takes `per` consecutive buckets: running sums give its local
-// weighted sum A_l = sum_j (j - lo + 1) B_j and its plain sum R_l.  The item's result is
-// sum_l A_l + per * sum_{l >= 1} S_l with S_l = sum_{u >= l} R_u (a suffix scan over the eight lanes), so
-// every lane doubles its own S_l log2(per) times, adds A_l, and one three-level tree finishes.
-constexpr int kRowLanes = 8;
+__global__ void __launch_bounds__(kReduceThreads) k_msm_join_items(const Xyzz* __restrict__ runs, uint32_t blocks_per_item,
+                                                                   Xyzz* window_sums) {
+  __shared__ Xyzz A[kReduceThreads], D[kReduceThreads];
+  if (threadIdx.x < blocks_per_item) {
+    const size_t at = 2 * ((size_t)blockIdx.x * blocks_per_item + threadIdx.x);
+    A[threadIdx.x] = ld_xyzz(runs + at);
+    D[threadIdx.x] = ld_xyzz(runs + at + 1);
+  }
+  __syncthreads();
+  join_runs(A, D, blocks_per_item);
+  if (threadIdx.x == 0) st_xyzz(window_sums + blockIdx.x, A[0]);
+}
+
+// Many items (the d_x / d_y rows of a commitment: a thousand or more (row, window) items): a block per item leaves most of
+// its additions to idle lanes.  Here `lanes` lanes (a power of two, 8 to 32) share an item.  Lane l takes `per` consecutive
+// buckets: running sums give its local weighted sum A_l = sum_j (j - lo + 1) B_j and its plain sum R_l.  The item's result is
+// sum_l A_l + per * sum_{l >= 1} S_l with S_l = sum_{u >= l} R_u (a suffix scan over the item's lanes), so
+// every lane doubles its own S_l log2(per) times, adds A_l, and one tree over the lanes finishes.  The fewest lanes that still
+// fill the GPU are taken: 6 656 items of 512 buckets take 1.8 ms with eight lanes each.  The four reductions of a KZH3 commitment
+// and opening at 2^22 took 5.8 ms with a block per item everywhere (32 threads for these), and take 3.8 ms.
 __global__ void __launch_bounds__(128) k_msm_bucket_reduce_rows(const Xyzz* __restrict__ bucket_sums, uint32_t half,
-                                                               uint32_t n_items, Xyzz* window_sums) {
+                                                               uint32_t n_items, uint32_t lanes, Xyzz* window_sums) {
   __shared__ Xyzz sh[128];
-  const uint32_t t = threadIdx.x, l = t & (kRowLanes - 1);
-  const uint32_t item = blockIdx.x * (128 / kRowLanes) + t / kRowLanes;
+  const uint32_t t = threadIdx.x, l = t & (lanes - 1);
+  const uint32_t item = blockIdx.x * (128 / lanes) + t / lanes;
   const bool live = item < n_items;
-  const uint32_t per = half / kRowLanes;  // a power of two, at least 1
+  const uint32_t per = half / lanes;  // a power of two, at least 1
   const Xyzz* B = bucket_sums + (size_t)(live ? item : 0) * half;
   Xyzz running = Xyzz::inf(), acc = Xyzz::inf();
   if (live) {
@@ -498,10 +581,10 @@ __global__ void __launch_bounds__(128) k_msm_bucket_reduce_rows(const Xyzz* __re
   // inclusive suffix scan of the running sums over the item's lanes
   sh[t] = running;
   __syncwarp();
-#pragma unroll
-  for (uint32_t off = 1; off < kRowLanes; off <<= 1) {
+#pragma unroll 1
+  for (uint32_t off = 1; off < lanes; off <<= 1) {
     Xyzz other = Xyzz::inf();
-    if (l + off < kRowLanes) other = sh[t + off];
+    if (l + off < lanes) other = sh[t + off];
     __syncwarp();
     add_to(&running, &other);
     sh[t] = running;
@@ -513,8 +596,8 @@ __global__ void __launch_bounds__(128) k_msm_bucket_reduce_rows(const Xyzz* __re
   add_to(&acc, &running);
   sh[t] = acc;
   __syncwarp();
-#pragma unroll
-  for (uint32_t off = kRowLanes / 2; off > 0; off >>= 1) {
+#pragma unroll 1
+  for (uint32_t off = lanes / 2; off > 0; off >>= 1) {
     Xyzz other = Xyzz::inf();
     if (l < off) other = sh[t + off];
     __syncwarp();
@@ -535,6 +618,42 @@ __global__ void k_msm_combine(const Xyzz* __restrict__ window_sums, uint32_t row
     add_to(&acc, &ws);
   }
   out[row] = to_jacobian(acc);
+}
+
+// The same Horner sum for few rows, where the chain of W * K dependent doublings is the whole time (254 of them took a
+// thread 1.13 ms).  A warp takes a row and four lanes a point (quad.cuh).  The eight quads of a warp take an eighth of the
+// windows each, shift their sums up by their own number of doublings, and a tree over the quads finishes, so that the general
+// additions stay off the chain: 254 doublings and the additions take 560 us.
+__global__ void __launch_bounds__(32) k_msm_combine_quads(const Xyzz* __restrict__ window_sums, int w, int k_windows, Jacobian* out) {
+  __shared__ Xyzz sh[8];
+  const int lane = threadIdx.x, group = lane >> 2, role = lane & 3;
+  const Xyzz* ws = window_sums + (size_t)blockIdx.x * k_windows;
+  const int per = (k_windows + 7) >> 3, lo = group * per;
+  QuadXyzz p;
+  p.x = p.y = p.z = Fq::zero();
+  // the quad's windows: sum_k 2^(W (k - lo)) ws[k]; the last window by address stands in for those past the end
+#pragma unroll 1
+  for (int s = per - 1; s >= 0; s--) {
+    const int k = lo + s;
+    if (s != per - 1)
+#pragma unroll 1
+      for (int i = 0; i < w; i++) p = quad_dbl(p, role);
+    const QuadXyzz r = quad_add(p, quad_load(ws + (k < k_windows ? k : k_windows - 1), role), role);
+    if (k < k_windows) p = r;
+  }
+  // shifted up by W lo bits (a quad without windows holds infinity)
+  const int live = (k_windows + per - 1) / per;  // quads with windows
+  const int most = (live - 1) * per * w;
+#pragma unroll 1
+  for (int i = 0; i < most; i++) {
+    const QuadXyzz r = quad_dbl(p, role);
+    if (i < lo * w) p = r;
+  }
+  quad_store(sh + group, p, role);
+  __syncwarp();
+#pragma unroll 1
+  for (int off = 4; off > 0; off >>= 1) quad_add_to(&sh[group & (off - 1)], &sh[(group & (off - 1)) + off], group < off);
+  if (lane == 0) out[blockIdx.x] = to_jacobian(sh[0]);
 }
 
 // 64-bit total of the per-bucket counts (the 32-bit prefix sums would wrap silently past 2^32).
@@ -682,8 +801,8 @@ static int windows_for(uint32_t max_mag, int w) {
 }
 
 // Horner over the windows on the host, for one row or a few: a doubling is a chain of products, 0.3 us for a CPU core with
-// 64-bit limbs and 2.7 us for a warp, against which the two small copies and the synchronisation (some 20 us) count little
-// from a few dozen doublings on.
+// 64-bit limbs against 4.5 us for a GPU thread and 2.2 us for a warp, against which the two small copies and the
+// synchronisation (some 20 us) count little from a few dozen doublings on.
 constexpr uint32_t kHostCombineRows = 4, kHostCombineChain = 24;
 static int combine_on_host(zk_ctx* ctx, const Xyzz* window_sums, uint32_t rows, int w, int k_windows, Jacobian* out_dev) {
   static_assert(kHostCombineRows * 128 * sizeof(Xyzz) + kHostCombineRows * sizeof(Jacobian) <= kHostPointsBytes, "128 windows of two bits at most");
@@ -701,6 +820,29 @@ static int combine_on_host(zk_ctx* ctx, const Xyzz* window_sums, uint32_t rows, 
   }
   ZK_CUDA(cudaMemcpyAsync(out_dev, out, rows * sizeof(Jacobian), cudaMemcpyHostToDevice, ctx->stream));
   return 0;
+}
+
+// Lanes per item for k_msm_bucket_reduce_rows, 0 where an item is worth a block or more of its own.  More lanes shorten the
+// chain and add work (a scan and a tree over them), so they double only until half of the threads that fit the GPU (three
+// blocks of 128 per SM) have work: 4096 items of 128 buckets lost 2 % of their commitment with sixteen lanes instead of eight.
+static uint32_t reduce_lanes(uint32_t n_items, uint32_t half, int sm) {
+  if (n_items < 1024 || half < 8) return 0;
+  uint32_t lanes = 8;
+  while (lanes < 32 && lanes * 2 <= half && (uint64_t)n_items * lanes < (uint64_t)sm * 3 * 64) lanes *= 2;
+  return lanes;
+}
+
+// Buckets per thread and blocks per item of the bucket reduction.  Longer runs cost fewer additions in all (2 + 4 / per a
+// bucket), shorter ones a shorter chain: the runs double while the launch still fills the GPU with threads, and an item has at
+// most kReduceThreads blocks (the second launch joins them in one block).
+static void reduce_shape(uint32_t n_items, uint32_t half, uint32_t* per, uint32_t* parts) {
+  uint32_t p = 1;
+  while (p < half && (p < 32 && (uint64_t)n_items * (half / (2 * p)) >= 40000)) p *= 2;
+  if (p < 4) p = half < 4 ? half : 4;
+  while (half / p > kReduceThreads * kReduceThreads) p *= 2;
+  *per = p;
+  const uint32_t n = half / p;
+  *parts = n > kReduceThreads ? n / kReduceThreads : 1;
 }
 
 // row_ids == nullptr: `rows` dense rows of n scalars each over the same n bases.  Otherwise: n scalars in
@@ -769,7 +911,10 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
   // real total is checked after the count pass (entry slots are 32-bit)
   uint64_t max_entries = total * (uint64_t)k_windows;
   if (max_entries > 0xffffffffull) max_entries = 0xffffffffull;
-  size_t need = align256((n_buckets + 2) * 4ull) * 2 + align256(scan_scratch_elems(n_buckets + 1) * 4) +
+  uint32_t red_per, red_parts;
+  reduce_shape(rows * (uint32_t)k_windows, half, &red_per, &red_parts);
+  const uint64_t n_runs = red_parts > 1 ? 2ull * rows * k_windows * red_parts : 0;
+  size_t need = align256(n_runs * sizeof(Xyzz)) + align256((n_buckets + 2) * 4ull) * 2 + align256(scan_scratch_elems(n_buckets + 1) * 4) +
                 align256((size_t)n_buckets * sizeof(Xyzz)) + align256((size_t)rows * k_windows * sizeof(Xyzz)) + 4096;
   char* base = nullptr;
   // entries and chunk slots are sized after the count pass; reserve the worst case now
@@ -789,6 +934,7 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
   Xyzz* heads = (Xyzz*)take((chunk_guess + 1) * sizeof(Xyzz));
   Xyzz* tails = (Xyzz*)take((chunk_guess + 1) * sizeof(Xyzz));
   Xyzz* fix_part = (Xyzz*)take((size_t)kFixupPartials * sizeof(Xyzz));
+  Xyzz* runs = (Xyzz*)take(n_runs * sizeof(Xyzz));
 
   // ---- pass 2: count, scan, scatter
   ZK_CUDA(cudaMemsetAsync(offsets, 0, (n_buckets + 2) * 4ull, s));
@@ -860,30 +1006,33 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
       uint32_t* n_many = ctx->rs.sink.counter + 12;
       ZK_CUDA(cudaMemsetAsync(n_many, 0, 4, s));
       k_msm_fixup_few<<<(n_buckets + 255) / 256, 256, 0, s>>>(offsets, n_buckets, seg, bucket_sums, heads, tails, cursor, n_many);
-      k_msm_fixup<<<sm * 4, 128, 0, s>>>(offsets, cursor, n_many, seg, bucket_sums, heads, tails);
+      k_msm_fixup<<<sm * 2, kFixupThreads, 0, s>>>(offsets, cursor, n_many, seg, bucket_sums, heads, tails);
       ctx->launches++;
     }
     ctx->launches += 2;
   }
   // ---- reduce buckets, combine windows
-  // buckets per thread: the running sums cost 2 additions per bucket, the thread's offset multiple and
-  // the block tree are per-thread overhead, so threads take up to 32 buckets while enough threads remain
-  uint32_t per_thread = 4;
-  while (per_thread < 32 && (uint64_t)rows * k_windows * (half / (per_thread * 2)) >= 100000) per_thread *= 2;
-  uint32_t threads = half / per_thread;
-  if (threads < 32) threads = 32;
-  if (threads > 256) threads = 256;
   const uint32_t n_items = rows * (uint32_t)k_windows;
-  if (n_items >= 1024 && half >= kRowLanes && half <= 256)
-    k_msm_bucket_reduce_rows<<<(n_items + 15) / 16, 128, 0, s>>>(bucket_sums, half, n_items, window_sums);
-  else
-    k_msm_bucket_reduce<<<n_items, threads, threads * sizeof(Xyzz), s>>>(bucket_sums, half, window_sums);
-  if (rows <= kHostCombineRows && (uint32_t)w * (uint32_t)(k_windows - 1) >= kHostCombineChain) {
+  const uint32_t lanes = reduce_lanes(n_items, half, sm);
+  if (lanes) {
+    k_msm_bucket_reduce_rows<<<(n_items + 128 / lanes - 1) / (128 / lanes), 128, 0, s>>>(bucket_sums, half, n_items, lanes, window_sums);
+  } else {
+    k_msm_bucket_reduce<<<n_items * red_parts, kReduceThreads, 0, s>>>(bucket_sums, half, red_per, red_parts, runs, window_sums);
+    if (red_parts > 1) {
+      k_msm_join_items<<<n_items, kReduceThreads, 0, s>>>(runs, red_parts, window_sums);
+      ctx->launches++;
+    }
+  }
+  // up to a few rows per SM the combination is one chain of doublings, which the warp-per-row form shortens; with
+  // more rows the chains overlap and a thread per row does an eighth of the work
+  const uint32_t chain = (uint32_t)w * (uint32_t)(k_windows - 1);
+  if (rows <= kHostCombineRows && chain >= kHostCombineChain) {
     rc = combine_on_host(ctx, window_sums, rows, w, k_windows, out_dev);
     if (rc) return rc;
-  } else {
+  } else if (rows <= 4u * (uint32_t)sm)
+    k_msm_combine_quads<<<rows, 32, 0, s>>>(window_sums, w, k_windows, out_dev);
+  else
     k_msm_combine<<<(rows + 63) / 64, 64, 0, s>>>(window_sums, rows, w, k_windows, out_dev);
-  }
   ctx->launches += 2;
   ZK_CUDA(cudaGetLastError());
   ctx->msm_entries_sum += n_entries;
