@@ -707,6 +707,8 @@ __global__ void __launch_bounds__(128) k_select_sums(const Affine* __restrict__ 
   // warp-wide additions it issues, so the additions of a level are packed into as few warps as they fill: the row
   // sums' pairs take the first threads of the block, C's pairs the next, and whole warps sit a level out
   // (128, 64, 32 and 16 additions for the four levels, against two additions by every warp at every level).
+  // The last two levels of the rows and the levels of C across the rows have few additions: four lanes each (quad.cuh; this
+  // kernel 210 -> 187 us and the total of the blocks 62 -> 37 us at 2^18 entries).
   __shared__ Xyzz sh[2 * 128];  // [0, 128): shares of the rows' sums; [128, 256): shares of C
   sh[threadIdx.x] = acc_r;
   sh[128 + threadIdx.x] = acc_c;
@@ -715,31 +717,30 @@ __global__ void __launch_bounds__(128) k_select_sums(const Affine* __restrict__ 
 #pragma unroll 1
   for (int off = kSelLanes / 2; off > 0; off >>= 1) {
     const int per_kind = kRowsPerBlock * off;  // additions of this level for one of the two sums
-    if ((int)threadIdx.x < 2 * per_kind) {
-      const int kind = (int)threadIdx.x / per_kind, t = (int)threadIdx.x % per_kind;
-      Xyzz* at = sh + kind * 128 + (t / off) * kSelLanes + (t % off);
-      add_to(at, at + off);
+    if (2 * per_kind > 32) {
+      if ((int)threadIdx.x < 2 * per_kind) {
+        const int kind = (int)threadIdx.x / per_kind, t = (int)threadIdx.x % per_kind;
+        Xyzz* at = sh + kind * 128 + (t / off) * kSelLanes + (t % off);
+        add_to(at, at + off);
+      }
+    } else if ((threadIdx.x & ~31u) < 8u * per_kind) {
+      const int q = (int)threadIdx.x >> 2, kind = q / per_kind, t = q % per_kind;
+      Xyzz* at = sh + (kind & 1) * 128 + (t / off) * kSelLanes + (t % off);
+      quad_add_to(at, at + off, kind < 2);
     }
     __syncthreads();
   }
-  acc_r = sh[threadIdx.x];
+  if (group < rows && gl == 0) d_x[group] = to_jacobian(sh[threadIdx.x]);
+  // the shares of C of the block's rows
   Xyzz* sh_c = sh + 128;
-  if (group < rows && gl == 0) d_x[group] = to_jacobian(acc_r);
-  // the shares of C of the block's rows: one more tree, by the first lanes of the block
-  constexpr unsigned kRowMask = (1u << kRowsPerBlock) - 1u;
-  __syncthreads();  // sh_c[kSelLanes k] holds row k's share
-  if (threadIdx.x < kRowsPerBlock) {
-    Xyzz v = sh_c[kSelLanes * threadIdx.x];
-    __syncwarp(kRowMask);
 #pragma unroll 1
-    for (int off = kRowsPerBlock / 2; off > 0; off >>= 1) {
-      sh_c[threadIdx.x] = v;
-      __syncwarp(kRowMask);
-      if ((int)threadIdx.x < off) add_to(&v, &sh_c[threadIdx.x + off]);
-      __syncwarp(kRowMask);
+  for (int off = kRowsPerBlock / 2; off > 0; off >>= 1) {
+    if (threadIdx.x < 32) {
+      const int q = (int)threadIdx.x >> 2, i = q < off ? q : 0;
+      quad_add_to(&sh_c[kSelLanes * i], &sh_c[kSelLanes * (i + off)], q < off);
     }
-    if (threadIdx.x == 0) st_xyzz(c_partial + blockIdx.x, v);
   }
+  if (threadIdx.x == 0) st_xyzz(c_partial + blockIdx.x, sh_c[0]);
 }
 
 // C = the sum of the blocks' shares (one block).
@@ -752,16 +753,8 @@ __global__ void __launch_bounds__(256) k_select_total(const Xyzz* __restrict__ c
   }
   sh[threadIdx.x] = acc;
   __syncthreads();
-#pragma unroll 1
-  for (int off = 128; off > 0; off >>= 1) {
-    if ((int)threadIdx.x < off) {
-      const Xyzz v = sh[threadIdx.x + off];
-      add_to(&acc, &v);
-      sh[threadIdx.x] = acc;
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *c_out = to_jacobian(acc);
+  tree_sum(sh, 256);
+  if (threadIdx.x == 0) *c_out = to_jacobian(sh[0]);
 }
 
 }  // namespace
