@@ -49,6 +49,9 @@ __device__ __forceinline__ int bit_length(const uint32_t (&mag)[8]) {
   return bits;
 }
 
+// Blocks of 128 threads per SM of the kernels that add points in chains (108 registers; five spill).
+constexpr int kAccBlocks = 4;
+
 // Scalars whose folded magnitude is below 2^30 also have a compact form: a signed 32-bit integer.
 // When every scalar of a call has one (quantised weights and activations), the digit passes read
 // these 4 bytes instead of converting the 32-byte Montgomery value again.
@@ -272,7 +275,8 @@ __device__ __forceinline__ Xyzz add_mixed_calls(const Xyzz& p, const Affine& q) 
   return r;
 }
 
-__global__ void __launch_bounds__(128) k_msm_accumulate(const Affine* __restrict__ bases, const uint32_t* __restrict__ gather,
+__global__ void __launch_bounds__(128, kAccBlocks) k_msm_accumulate(const Affine* __restrict__ bases,
+                                                        const uint32_t* __restrict__ gather,
                                                         const uint32_t* __restrict__ entries,
                                                         const uint32_t* __restrict__ offsets, uint32_t n_buckets,
                                                         uint32_t n_entries, uint32_t seg, uint32_t n_chunks,
@@ -815,6 +819,23 @@ static int combine_on_host(zk_ctx* ctx, const Xyzz* window_sums, uint32_t rows, 
   return 0;
 }
 
+// Entries per chunk of the accumulation (a chunk is a thread's): whole waves of resident threads, of some 64 to 96 entries each
+// where there are that many.  Shorter chunks mean more pieces of buckets to join afterwards, a last wave that is nearly
+// empty costs as much as a full one: 2^24 entries in chunks of 32 left 2^19 pieces, whose sums took 286 us against 142 us for a
+// third of them; 1.9 M entries in one full wave instead of four fifths of one take 345 us against 436 us.
+constexpr uint32_t kChunkMin = 16, kChunkWaves = 12;
+static uint32_t chunk_entries(uint32_t n_entries, int sm) {
+  const uint64_t resident = (uint64_t)sm * kAccBlocks * 128;
+  uint64_t seg = (n_entries + resident - 1) / resident;
+  if (seg < kChunkMin) return kChunkMin;
+  if (seg > 96) {
+    uint64_t waves = seg / 64;
+    if (waves > kChunkWaves) waves = kChunkWaves;
+    seg = (n_entries + resident * waves - 1) / (resident * waves);
+  }
+  return (uint32_t)seg;
+}
+
 // Lanes per item for k_msm_bucket_reduce_rows, 0 where an item is worth a block or more of its own.  More lanes shorten the
 // chain and add work (a scan and a tree over them), so they double only until half of the threads that fit the GPU (three
 // blocks of 128 per SM) have work: 4096 items of 128 buckets lost 2 % of their commitment with sixteen lanes instead of eight.
@@ -911,8 +932,9 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
                 align256((size_t)n_buckets * sizeof(Xyzz)) + align256((size_t)rows * k_windows * sizeof(Xyzz)) + 4096;
   char* base = nullptr;
   // entries and chunk slots are sized after the count pass; reserve the worst case now
-  uint64_t chunk_guess = max_entries / 32 + 1;
-  if (chunk_guess > (1u << 20)) chunk_guess = 1u << 20;
+  uint64_t chunk_guess = max_entries / kChunkMin + 1;
+  const uint64_t chunk_cap = (uint64_t)sm * kAccBlocks * 128 * kChunkWaves;
+  if (chunk_guess > chunk_cap) chunk_guess = chunk_cap;
   need += align256(max_entries * 4) + 2 * align256((chunk_guess + 1) * sizeof(Xyzz)) + align256((size_t)kFixupPartials * sizeof(Xyzz));
   int rc = ctx->reserve_aux(need, (void**)&base);
   if (rc) return rc;
@@ -978,10 +1000,8 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
   // ---- accumulate
   ZK_CUDA(cudaMemsetAsync(bucket_sums, 0, (size_t)n_buckets * sizeof(Xyzz), s));
   if (n_entries) {
-    uint32_t n_chunks = n_entries / 32 + 1;
-    if (n_chunks > chunk_guess) n_chunks = (uint32_t)chunk_guess;
-    const uint32_t seg = (n_entries + n_chunks - 1) / n_chunks;
-    n_chunks = (n_entries + seg - 1) / seg;
+    const uint32_t seg = chunk_entries(n_entries, sm);
+    const uint32_t n_chunks = (n_entries + seg - 1) / seg;
     k_msm_accumulate<<<(n_chunks + 127) / 128, 128, 0, s>>>(bases, gather, entries, offsets, n_buckets, n_entries, seg,
                                                            n_chunks, bucket_sums, heads, tails);
     // pieces per bucket on average; from a few hundred on, one block per bucket is a long serial chain
