@@ -1,6 +1,6 @@
-"""The routes of the MSM pipeline at the sizes where they change: long buckets, and the reduction of a window's buckets over
-several blocks.  The bases are known
-multiples of g, so that the expected point of any row is one multiple of g."""
+"""The routes of the MSM pipeline at the sizes where they change: rows of small scalars by subset-sum tables, long buckets, and
+the reduction of a window's buckets over several blocks.  The bases are known multiples of g, so that the expected point of any
+row is one multiple of g."""
 import ctypes
 import random
 
@@ -27,6 +27,23 @@ def multiples():
 def of_g(k):
     k %= o.R_MOD
     return o.g1_mul(o.G1_GEN, k) if k else None
+
+
+def values(rnd, lo, hi):
+    return rnd.choice([lo, hi, 0, rnd.randint(lo, hi), rnd.randint(lo, hi)])
+
+
+@pytest.mark.parametrize("rows,n,lo,hi", [(2, 1, -128, 127), (300, 1, -1, 0), (64, 2, 0, 1), (40, 13, -128, 127), (700, 12, -128, 128),
+                                          (333, 25, -1, 1), (2050, 31, -32768, 32767), (97, 68, -(1 << 29), (1 << 29) - 1)])
+def test_rows_of_small_scalars(ctx, multiples, rows, n, lo, hi):
+    rnd = random.Random(rows * n)
+    ks, pts = multiples
+    mat = [[values(rnd, lo, hi) for _ in range(n)] for _ in range(rows)]
+    mat[0] = [lo] * n
+    mat[1] = [hi] * n
+    got = curve.msm_batched(ctx, curve.affine_to_array(pts[-n:]), [[o.fr_from_int(v) for v in r] for r in mat])
+    for r in list(range(0, rows, max(1, rows // 40))) + [1, rows - 1]:
+        assert got[r] == of_g(sum(v * k for v, k in zip(mat[r], ks[-n:]))), r
 
 
 def _device_msm(ctx, bases, scalars):

@@ -15,6 +15,7 @@
 // fold to a few bits, so they use one narrow window: no doublings, few buckets.
 #include "msm.hpp"
 #include "reduce.cuh"
+#include "batch_affine.cuh"
 #include "quad.cuh"
 
 namespace zk {
@@ -56,18 +57,24 @@ constexpr int kAccBlocks = 4;
 // When every scalar of a call has one (quantised weights and activations), the digit passes read
 // these 4 bytes instead of converting the 32-byte Montgomery value again.
 constexpr int kCompactBits = 30;
+constexpr int kRowsGroupMax = 12;  // bases a group of the subset-sum tables has at most (k_rows_*)
 constexpr int32_t kNotCompact = INT32_MIN;
 
-// max_out[0]: largest bit length; max_out[1]: largest magnitude among the scalars below 2^32.
+// max_out[0]: largest bit length; among the scalars below 2^32 max_out[1]: largest magnitude, max_out[2]: largest of v and
+// -v - 1, whose bit length is that of the two's complement form without its sign.
 __global__ void k_msm_bits(const Fr* __restrict__ scalars, uint64_t total, unsigned int* max_out, int32_t* compact) {
   int best = 0;
-  uint32_t best_mag = 0;
+  uint32_t best_mag = 0, best_span = 0;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
     uint32_t mag[8];
     const bool negv = fold_scalar(ld_scalar(scalars + i), mag);
     const int b = bit_length(mag);
     best = b > best ? b : best;
-    if (b <= 32) best_mag = mag[0] > best_mag ? mag[0] : best_mag;
+    if (b <= 32) {
+      best_mag = mag[0] > best_mag ? mag[0] : best_mag;
+      const uint32_t span = negv && mag[0] ? mag[0] - 1 : mag[0];
+      best_span = span > best_span ? span : best_span;
+    }
     if (compact) compact[i] = b <= kCompactBits ? (negv ? -(int32_t)mag[0] : (int32_t)mag[0]) : kNotCompact;
   }
 #pragma unroll
@@ -76,10 +83,13 @@ __global__ void k_msm_bits(const Fr* __restrict__ scalars, uint64_t total, unsig
     best = o > best ? o : best;
     const uint32_t m = __shfl_down_sync(0xffffffffu, best_mag, off);
     best_mag = m > best_mag ? m : best_mag;
+    const uint32_t p = __shfl_down_sync(0xffffffffu, best_span, off);
+    best_span = p > best_span ? p : best_span;
   }
   if ((threadIdx.x & 31) == 0 && best) {
     atomicMax(max_out, (unsigned int)best);
     atomicMax(max_out + 1, best_mag);
+    atomicMax(max_out + 2, best_span);
   }
 }
 
@@ -761,6 +771,151 @@ __global__ void __launch_bounds__(256) k_select_total(const Xyzz* __restrict__ c
   if (threadIdx.x == 0) *c_out = to_jacobian(sh[0]);
 }
 
+// ---- Many dense rows of small scalars over the same bases (the d_x rows of a quantised weight matrix, kzh2.rs:653-660),
+// by the method of the four Russians: the bases are taken in groups of `s`, all 2^s subset sums of a group are tabulated
+// once for all the rows, and a row adds, for every bit plane of its scalars (two's complement), one table entry per group.
+// That is planes * n / s additions a row and 2^s * n / s for the table, where buckets take n a row plus their reduction: for
+// 4096 rows of 4096 int8 values 11.2 M + 1.4 M additions against 16.8 M + 0.5 M, and nothing is sorted: the d_x rows of that
+// commitment take 2.4 ms (sums 1.82, tables 0.34, bits 0.07, joining 0.19) where counting, scattering, adding and reducing
+// the buckets took 3.9 ms.
+
+// idx[g][row * planes + k]: the bits of plane k of the scalars of group g.  A thread takes a (row, group).
+__global__ void __launch_bounds__(256) k_rows_bits(const int32_t* __restrict__ compact, uint32_t n, uint32_t rows, int planes, int s,
+                                                   uint32_t groups, uint16_t* idx) {
+  const uint64_t total = (uint64_t)rows * groups;
+  for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t row = (uint32_t)(t % rows), g = (uint32_t)(t / rows);
+    const int32_t* v = compact + (uint64_t)row * n + (uint64_t)g * s;
+    const int have = n - g * s < (uint32_t)s ? (int)(n - g * s) : s;
+    uint16_t* out = idx + (uint64_t)g * rows * planes + (uint64_t)row * planes;
+    int32_t w[kRowsGroupMax];
+#pragma unroll
+    for (int i = 0; i < kRowsGroupMax; i++) w[i] = i < have ? __ldg(v + i) : 0;
+    for (int k = 0; k < planes; k++) {
+      uint32_t bits = 0;
+#pragma unroll
+      for (int i = 0; i < kRowsGroupMax; i++) bits |= (((uint32_t)w[i] >> k) & 1u) << i;
+      out[k] = (uint16_t)bits;
+    }
+  }
+}
+
+// Subset sums of the low and of the high half of a group's bases, 2^lo_bits + 2^hi_bits affine points a group.
+__global__ void __launch_bounds__(128) k_rows_halves(const Affine* __restrict__ bases, uint32_t n, int s, int lo_bits, uint32_t groups,
+                                                     Affine* halves) {
+  const uint32_t per = (1u << lo_bits) + (1u << (s - lo_bits));
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= groups * per) return;
+  const uint32_t g = t / per, m = t % per;
+  const bool hi = m >= (1u << lo_bits);
+  const uint32_t mask = hi ? m - (1u << lo_bits) : m;
+  const uint32_t first = g * (uint32_t)s + (hi ? (uint32_t)lo_bits : 0u);
+  Xyzz acc = Xyzz::inf();
+#pragma unroll 1
+  for (int i = 0; (mask >> i) != 0; i++)
+    if (((mask >> i) & 1u) && first + i < n) acc = add_mixed_calls(acc, ld_affine(bases + first + i));
+  Affine r;
+  r.x = r.y = Fq::zero();
+  if (!acc.is_inf()) {
+    const Fq izzz = fq_inverse_fn(acc.zzz);
+    const Fq iz = fq_mul_fn(izzz, acc.zz);  // 1 / zz = (zz / zzz)^2
+    r.x = fq_mul_fn(acc.x, fq_mul_fn(iz, iz));
+    r.y = fq_mul_fn(acc.y, izzz);
+  }
+  halves[t] = r;
+}
+
+// table[g][m] = halves[g][low bits of m] + halves[g][high bits of m]: kBatchTable sums a thread share an inversion.
+constexpr int kBatchTable = 8;
+__global__ void __launch_bounds__(kBatchThreads, 4) k_rows_table(const Affine* __restrict__ halves, int s, int lo_bits, uint32_t groups,
+                                                                 Affine* table) {
+  __shared__ Fq sh[kBatchThreads];
+  const uint32_t per = (1u << lo_bits) + (1u << (s - lo_bits)), total = groups << s;
+  const uint32_t t0 = blockIdx.x * (kBatchThreads * kBatchTable) + threadIdx.x;
+  Fq pre[kBatchTable], run = Fq::one();
+#pragma unroll 1
+  for (int j = 0; j < kBatchTable; j++) {
+    const uint32_t t = t0 + j * kBatchThreads;
+    if (t >= total) continue;
+    const uint32_t g = t >> s, m = t & ((1u << s) - 1u);
+    const Affine p = ld_affine(halves + g * per + (m & ((1u << lo_bits) - 1u)));
+    const Affine q = ld_affine(halves + g * per + (1u << lo_bits) + (m >> lo_bits));
+    Fq den;
+    add_kind(p, q, &den);
+    pre[j] = run;
+    run = fq_mul_fn(run, den);
+  }
+  Fq inv = block_inverse(run, sh);
+#pragma unroll 1
+  for (int j = kBatchTable - 1; j >= 0; j--) {
+    const uint32_t t = t0 + j * kBatchThreads;
+    if (t >= total) continue;
+    const uint32_t g = t >> s, m = t & ((1u << s) - 1u);
+    const Affine p = ld_affine(halves + g * per + (m & ((1u << lo_bits) - 1u)));
+    const Affine q = ld_affine(halves + g * per + (1u << lo_bits) + (m >> lo_bits));
+    Fq den;
+    const AddKind kind = add_kind(p, q, &den);
+    const Fq mine = fq_mul_fn(inv, pre[j]);
+    inv = fq_mul_fn(inv, den);
+    table[t] = add_with_inverse(p, q, kind, mine);
+  }
+}
+
+// pieces[q][u]: unit u = (row, plane) over the groups [q seg, (q + 1) seg).  The lanes of a warp are neighbouring units at the
+// same group, so their table reads fall into one group's 2^s entries and their idx reads are consecutive.
+__global__ void __launch_bounds__(128, kAccBlocks) k_rows_sums(const Affine* __restrict__ table, const uint16_t* __restrict__ idx, uint32_t units,
+                                                   int s, uint32_t groups, uint32_t seg, uint32_t n_pieces, Xyzz* pieces) {
+  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n_pieces) return;
+  const uint32_t q = c / units, u = c % units;
+  const uint32_t g1 = (q + 1) * seg < groups ? (q + 1) * seg : groups;
+  Xyzz acc = Xyzz::inf();
+  for (uint32_t g = q * seg; g < g1; g++) {
+    const uint32_t m = idx[(uint64_t)g * units + u];
+    if (m) acc = add_mixed_calls(acc, ld_affine(table + ((uint64_t)g << s) + m));
+  }
+  st_xyzz(pieces + c, acc);
+}
+
+// The sum of a unit's pieces: four lanes a unit, lane l of a unit takes the pieces l, l + 4, ...; written over piece 0.
+__global__ void __launch_bounds__(128) k_rows_units(Xyzz* pieces, uint32_t units, uint32_t parts) {
+  __shared__ Xyzz sh[128];
+  // thread = lane-of-unit * 32 + unit-in-block: the lanes of a warp read neighbouring units
+  const uint32_t l = threadIdx.x >> 5, u = blockIdx.x * 32 + (threadIdx.x & 31);
+  Xyzz acc = Xyzz::inf();
+  if (u < units)
+    for (uint32_t q = l; q < parts; q += 4) {
+      const Xyzz v = ld_xyzz(pieces + (uint64_t)q * units + u);
+      add_to(&acc, &v);
+    }
+  sh[threadIdx.x] = acc;
+  __syncthreads();
+  if (l < 2) {
+    add_to(&acc, &sh[threadIdx.x + 64]);
+    sh[threadIdx.x] = acc;
+  }
+  __syncthreads();
+  if (l == 0) {
+    add_to(&acc, &sh[threadIdx.x + 32]);
+    if (u < units) st_xyzz(pieces + u, acc);
+  }
+}
+
+// A row's result: sum_k 2^k (plane k), the top plane (the sign bits) subtracted.
+__global__ void __launch_bounds__(64) k_rows_planes(const Xyzz* __restrict__ unit_sums, uint32_t rows, int planes, Jacobian* out) {
+  const uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
+  if (row >= rows) return;
+  Xyzz acc = Xyzz::inf();
+#pragma unroll 1
+  for (int k = planes - 1; k >= 0; k--) {
+    Xyzz v = ld_xyzz(unit_sums + (uint64_t)row * planes + k);
+    if (k == planes - 1) v = neg(v);
+    dbl_in_place(&acc);
+    add_to(&acc, &v);
+  }
+  out[row] = to_jacobian(acc);
+}
+
 }  // namespace
 
 // Window width for n points per row whose scalars have at most max_bits magnitude bits.
@@ -859,6 +1014,97 @@ static void reduce_shape(uint32_t n_items, uint32_t half, uint32_t* per, uint32_
   *parts = n > kReduceThreads ? n / kReduceThreads : 1;
 }
 
+// Shape of the subset-sum method for `rows` dense rows of n small scalars, group = 0 when buckets take fewer additions.
+struct RowsPlan {
+  int group = 0;  // bases per group
+  int planes = 0;
+  uint32_t groups = 0;
+};
+
+static RowsPlan rows_plan(uint64_t n, uint32_t rows, uint32_t max_span, int k_windows, uint32_t half) {
+  RowsPlan best;
+  int planes = 1;
+  while (planes < 32 && (max_span >> (planes - 1))) planes++;
+  // additions a row by buckets: one an entry, and two per bucket in general coordinates (14 products to 10)
+  double least = (double)rows * k_windows * ((double)n + 2.8 * half);
+  if ((uint64_t)rows * planes >= (1ull << 31)) return best;
+  for (int s = 2; s <= kRowsGroupMax; s++) {
+    const uint64_t groups = (n + s - 1) / s;
+    if ((groups << s) >= (1ull << 31) || (uint64_t)rows * planes * groups >= (1ull << 40)) continue;
+    const double cost = (double)rows * planes * groups + (double)(groups << s);
+    if (cost < least) {
+      least = cost;
+      best.group = s;
+      best.planes = planes;
+      best.groups = (uint32_t)groups;
+    }
+  }
+  return best;
+}
+
+static int rows_run(zk_ctx* ctx, const Affine* bases, const int32_t* compact, uint32_t n, uint32_t rows, const RowsPlan& plan,
+                    Jacobian* out_dev, MsmStats* stats, int max_bits) {
+  cudaStream_t st = ctx->stream;
+  const int sm = ctx->sm_count, s = plan.group, lo_bits = (s + 1) / 2;
+  const uint32_t groups = plan.groups;
+  const uint64_t units = (uint64_t)rows * plan.planes;
+  // A unit's groups are cut into `parts` chains, a thread each.  The time is the waves of threads that takes times a
+  // chain's length, plus the additions that join the chains (14 products to 10, at half the efficiency): 32768 units of 342 groups
+  // in three parts are 1.3 waves, which cost two, and took 2.17 ms; nine parts are 3.9.
+  const uint64_t resident = (uint64_t)sm * kAccBlocks * 128;
+  uint64_t parts = 1;
+  double least = 1e300;
+  for (uint64_t p = 1; p <= 64 && p <= groups; p++) {
+    const uint64_t waves = (units * p + resident - 1) / resident;
+    const double cost = (double)waves * (double)((groups + p - 1) / p) + 2.8 * (double)(units * p) / (double)resident;
+    if (cost < least) {
+      least = cost;
+      parts = p;
+    }
+  }
+  const uint32_t seg = (uint32_t)((groups + parts - 1) / parts);
+  parts = (groups + seg - 1) / seg;
+  const uint64_t n_pieces = parts * units;
+  if (n_pieces >= (1ull << 31)) return fail(-1, "msm: %llu partial sums exceed 2^31 - 1; split the rows", (unsigned long long)n_pieces);
+  const uint32_t half_points = groups * ((1u << lo_bits) + (1u << (s - lo_bits)));
+  const uint64_t table_points = (uint64_t)groups << s;
+  char* base = nullptr;
+  int rc = ctx->reserve_aux(align256(units * groups * 2) + align256((uint64_t)half_points * sizeof(Affine)) +
+                                align256(table_points * sizeof(Affine)) + align256(n_pieces * sizeof(Xyzz)) + 1024, (void**)&base);
+  if (rc) return rc;
+  size_t off = 0;
+  auto take = [&](size_t bytes) { char* p = base + off; off += align256(bytes); return p; };
+  uint16_t* idx = (uint16_t*)take(units * groups * 2);
+  Affine* halves = (Affine*)take((uint64_t)half_points * sizeof(Affine));
+  Affine* table = (Affine*)take(table_points * sizeof(Affine));
+  Xyzz* pieces = (Xyzz*)take(n_pieces * sizeof(Xyzz));
+  const uint64_t cells = (uint64_t)rows * groups;
+  const uint64_t bit_blocks = (cells + 255) / 256;
+  k_rows_bits<<<(unsigned)(bit_blocks < (uint64_t)sm * 32 ? bit_blocks : (uint64_t)sm * 32), 256, 0, st>>>(compact, n, rows, plan.planes, s, groups, idx);
+  k_rows_halves<<<(half_points + 127) / 128, 128, 0, st>>>(bases, n, s, lo_bits, groups, halves);
+  const uint64_t per_block = kBatchThreads * kBatchTable;
+  k_rows_table<<<(unsigned)((table_points + per_block - 1) / per_block), kBatchThreads, 0, st>>>(halves, s, lo_bits, groups, table);
+  k_rows_sums<<<(unsigned)((n_pieces + 127) / 128), 128, 0, st>>>(table, idx, (uint32_t)units, s, groups, seg, (uint32_t)n_pieces, pieces);
+  if (parts > 1) {
+    k_rows_units<<<(unsigned)((units + 31) / 32), 128, 0, st>>>(pieces, (uint32_t)units, (uint32_t)parts);
+    ctx->launches++;
+  }
+  k_rows_planes<<<(rows + 63) / 64, 64, 0, st>>>(pieces, rows, plan.planes, out_dev);
+  ctx->launches += 5;
+  ZK_CUDA(cudaGetLastError());
+  const uint64_t additions = units * groups + table_points;
+  ctx->msm_entries_sum += additions;
+  ctx->msm_calls++;
+  if (stats) {
+    stats->window_bits = 1;
+    stats->windows = plan.planes;
+    stats->entries = additions;
+    stats->buckets = 0;
+    stats->max_bits = max_bits;
+  }
+  return 0;
+}
+
 // row_ids == nullptr: `rows` dense rows of n scalars each over the same n bases.  Otherwise: n scalars in
 // all, scalar i contributes scalars[i] * bases[gather ? gather[i] : i] to output row row_ids[i] < rows.
 int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const uint32_t* row_ids, const Fr* scalars,
@@ -876,26 +1122,28 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
   // ---- pass 1: scalar magnitude (and the compact form of small scalars); a caller that runs several
   // MSMs over the same scalars passes `prep` and the pass runs once
   unsigned int max_bits = 0;
-  uint32_t max_mag = 0;
+  uint32_t max_mag = 0, max_span = 0;
   const int32_t* compact = nullptr;
   if (prep && prep->valid && prep->scalars == scalars && prep->total == total) {
     max_bits = prep->max_bits;
     max_mag = prep->max_mag;
+    max_span = prep->max_span;
     compact = prep->compact;
   } else {
     unsigned int* d_bits = ctx->rs.sink.counter + 8;  // spare words of the context's counter block
     int32_t* cbuf = nullptr;
     int crc = ctx->reserve_cmp(total * 4 + 256, (void**)&cbuf);
     if (crc) return crc;
-    ZK_CUDA(cudaMemsetAsync(d_bits, 0, 8, s));
+    ZK_CUDA(cudaMemsetAsync(d_bits, 0, 12, s));
     k_msm_bits<<<sm * 8, 256, 0, s>>>(scalars, total, d_bits, cbuf);
     ctx->launches++;
-    ZK_CUDA(cudaMemcpyAsync(ctx->host_small, d_bits, 8, cudaMemcpyDeviceToHost, s));
+    ZK_CUDA(cudaMemcpyAsync(ctx->host_small, d_bits, 12, cudaMemcpyDeviceToHost, s));
     ZK_CUDA(cudaStreamSynchronize(s));
-    unsigned int two[2];
-    memcpy(two, ctx->host_small, 8);
-    max_bits = two[0];
-    max_mag = two[1];
+    unsigned int found[3];
+    memcpy(found, ctx->host_small, 12);
+    max_bits = found[0];
+    max_mag = found[1];
+    max_span = found[2];
     if (max_bits <= (unsigned)kCompactBits) compact = cbuf;
     if (prep) {
       prep->valid = true;
@@ -903,6 +1151,7 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
       prep->total = total;
       prep->max_bits = max_bits;
       prep->max_mag = max_mag;
+      prep->max_span = max_span;
       prep->compact = compact;
     }
   }
@@ -917,6 +1166,10 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
   const int k_windows = compact ? windows_for(max_mag, w) : ((int)max_bits + 1 + w - 1) / w;
   const uint32_t half = 1u << (w - 1);
   const uint64_t n_buckets64 = (uint64_t)rows * k_windows * half;
+  if (compact && rows > 1 && !row_ids && !gather) {
+    const RowsPlan plan = rows_plan(n, rows, max_span, k_windows, half);
+    if (plan.group) return rows_run(ctx, bases, compact, (uint32_t)n, rows, plan, out_dev, stats, (int)max_bits);
+  }
   if (n_buckets64 >= (1ull << 31)) return fail(-1, "msm: %llu buckets exceed the 32-bit key space; split the rows", (unsigned long long)n_buckets64);
   const uint32_t n_buckets = (uint32_t)n_buckets64;
 

@@ -21,6 +21,7 @@ struct MsmPrep {
   uint64_t total = 0;
   unsigned max_bits = 0;
   uint32_t max_mag = 0;            // exact largest magnitude when max_bits <= 32
+  uint32_t max_span = 0;           // then also the largest of v and -v - 1
   const int32_t* compact = nullptr;  // signed 32-bit form of every scalar, or NULL when some do not fit
 };
 
