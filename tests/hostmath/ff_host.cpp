@@ -12,6 +12,8 @@ template <class P> static void ld(Fp<P>& x, const uint32_t* p) { memcpy(x.v, p, 
     Fp<P> x, y; ld(x, a); ld(y, b); Fp<P> z = mul(x, y); memcpy(r, z.v, 32); }               \
   extern "C" void zkh_##name##_mul_rows(const uint32_t* a, const uint32_t* b, uint32_t* r) {  \
     Fp<P> x, y; ld(x, a); ld(y, b); Fp<P> z = mul_rows(x, y); memcpy(r, z.v, 32); }          \
+  extern "C" void zkh_##name##_sqr_rows(const uint32_t* a, uint32_t* r) {                     \
+    Fp<P> x; ld(x, a); Wide t; sqr_wide(t, x.v); Fp<P> z = redc<P>(t); memcpy(r, z.v, 32); } \
   extern "C" void zkh_##name##_add(const uint32_t* a, const uint32_t* b, uint32_t* r) {      \
     Fp<P> x, y; ld(x, a); ld(y, b); Fp<P> z = add(x, y); memcpy(r, z.v, 32); }               \
   extern "C" void zkh_##name##_sub(const uint32_t* a, const uint32_t* b, uint32_t* r) {      \

@@ -184,7 +184,7 @@ def test_inverse_edges(hm, name, p):
 
 @pytest.mark.parametrize("name,p", [("fr", o.R_MOD), ("fq", o.Q_MOD)])
 def test_device_rows(hm, name, p):
-    """The product rows that the device runs (the host has its own form of the product)."""
+    """The product rows and the square that the device runs (the host has its own form of the product)."""
     rnd = random.Random(12)
     out = (ctypes.c_uint32 * 8)()
     rinv = pow(R, -1, p)
@@ -193,3 +193,5 @@ def test_device_rows(hm, name, p):
         for b in (R - 1, p, rnd.randrange(R), rnd.choice(edge)):
             getattr(hm, f"zkh_{name}_mul_rows")(buf(a), buf(b), out)
             assert val(out) == a * b * rinv % p
+        getattr(hm, f"zkh_{name}_sqr_rows")(buf(a), out)
+        assert val(out) == a * a * rinv % p
