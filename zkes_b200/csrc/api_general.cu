@@ -99,18 +99,18 @@ int sbool_prove(zk_ctx* ctx, zk_comm* comm, uint32_t num_var, uint32_t n_terms, 
   for (uint32_t round = 0; round < num_var; round++) {
     const uint32_t vars_left = num_var - round;
     const uint64_t S = 1ull << vars_left;
-    // every value is one in the first round (the fill above); later rounds read the eq factors from records
-    if (round) {
-      launch_eq_records(eq_cur, S / 2, eq_rec, ctx->sm_count, s);
-      ctx->launches++;
-    }
+    // every value is one in the first round (the fill above); later rounds read the eq factors from the records that the
+    // round before left
     launch_sbool_msg(e_key[e], e_val[e], counts + e, k_upper, round ? eq_rec : eq_cur, d_w, vars_left, round == 0,
                      ctx->next_msg_scratch(comm != nullptr), s);
     ctx->launches++;
     rc = fs_round(ctx, comm, 4, round, fs, fs_user, tr, round_msgs, challenges, &challenge);
     if (rc) return rc;
     Fr* eq_next = (round & 1) ? eq0 : eq1;  // eq0 holds 2^n, eq1 2^(n-1); later rounds fit either
-    launch_fold(eq_cur, eq_next, challenge, S / 2, ctx->rs.max_blocks, s);
+    if (S >= 4)
+      launch_eq_fold_records(eq_cur, S / 4, challenge, eq_next, eq_rec, ctx->sm_count, s);
+    else
+      launch_fold(eq_cur, eq_next, challenge, S / 2, ctx->rs.max_blocks, s);
     eq_cur = eq_next;
     ctx->launches += 1 + launch_sparse_fold(e_key[e], e_val[e], counts + e, k_upper, challenge, block_counts, e_key[e ^ 1],
                                             e_val[e ^ 1], counts + (e ^ 1), s);
