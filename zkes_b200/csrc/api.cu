@@ -295,18 +295,16 @@ int linear_rounds(zk_ctx* ctx, zk_comm* comm, int L, uint32_t rounds, const Fr**
   // (rounds round_offset + first ...), the transcript state and the resident kernel's error word.
   // The first `canonical` of them are the multi-round kernel's, which writes canonical integers, not Montgomery form.
   auto collect_device_rounds = [&](uint32_t first, uint32_t left, bool resident, uint32_t canonical) -> int {
-    ResidentShared* sh = reinterpret_cast<ResidentShared*>(ctx->resident_sh);
     const size_t bytes = ((size_t)left * (L + 2)) * sizeof(Fr) + sizeof(StrobeState);
-    unsigned int* h_flags = reinterpret_cast<unsigned int*>(reinterpret_cast<char*>(ctx->host_small) + 8192 - 16);
-    ZK_CUDA(cudaMemcpyAsync(ctx->host_small, ctx->tail_out, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    if (resident) ZK_CUDA(cudaMemcpyAsync(h_flags, sh, 16, cudaMemcpyDeviceToHost, ctx->stream));
-    // the final values come back in the same synchronisation (the kernels before this point have written them)
-    const bool with_final = bytes <= kFinalHostOffset;  // (always, for tables that fit a GPU)
-    if (with_final)
-      ZK_CUDA(cudaMemcpyAsync(reinterpret_cast<char*>(ctx->host_small) + kFinalHostOffset, ctx->final_out,
-                              (kMaxPolys + 1) * sizeof(Fr), cudaMemcpyDeviceToHost, ctx->stream));
+    static_assert(34 * (kMaxPolys + 2) * sizeof(Fr) + sizeof(StrobeState) <= kFinalHostOffset, "34 rounds fit before the final values");
+    const unsigned int* h_flags = reinterpret_cast<const unsigned int*>(reinterpret_cast<const char*>(ctx->host_small) + kFlagsHostOffset);
+    // the final values and the error word come back in the same copy (the kernels before this point have written them): three
+    // copies of some 3 us each were most of what a small prove spent outside its kernel
+    if (bytes > kFinalHostOffset) return fail(ZK_ERR_ARG, "device rounds: too many rounds");
+    ZK_CUDA(cudaMemcpyAsync(ctx->host_small, ctx->tail_out, resident ? kFlagsHostOffset + 16 : kFinalHostOffset + (kMaxPolys + 1) * sizeof(Fr),
+                            cudaMemcpyDeviceToHost, ctx->stream));
     ZK_CUDA(cudaStreamSynchronize(ctx->stream));
-    ctx->final_on_host = with_final;
+    ctx->final_on_host = true;
     if (resident && h_flags[2] >= 2) return fail(ZK_ERR_TIMEOUT, "sharded rounds: another rank's partial sums or table chunk did not arrive");
     if (resident && h_flags[2] != 0) return fail(ZK_ERR_TIMEOUT, "resident round kernel: a wait for a challenge ran out");
     Fr* h_msgs = reinterpret_cast<Fr*>(ctx->host_small);
@@ -358,7 +356,7 @@ int linear_rounds(zk_ctx* ctx, zk_comm* comm, int L, uint32_t rounds, const Fr**
     const uint32_t R = rounds + 1 + logw - gathered_log;  // messages of the sharded launch
     const uint32_t left = rounds + logw;                   // messages until the end of the protocol
     const size_t bytes = ((size_t)left * (L + 2)) * sizeof(Fr) + sizeof(StrobeState);
-    if (R >= 1 && R <= rounds && bytes <= 8192 - 16) {
+    if (R >= 1 && R <= rounds && bytes <= kFinalHostOffset) {
       const StrobeState st = strobe_now();
       Fr* d_msgs = reinterpret_cast<Fr*>(ctx->tail_out);
       Fr* d_chal = d_msgs + (size_t)left * (L + 1);
@@ -423,7 +421,7 @@ int linear_rounds(zk_ctx* ctx, zk_comm* comm, int L, uint32_t rounds, const Fr**
       ResidentShared* sh = reinterpret_cast<ResidentShared*>(ctx->resident_sh);
       bool resident = false;
       if (round == 0 && rounds >= 2 && L <= 3 && ctx->ahead_log >= 2 &&
-          (size_t)left * (L + 2) * sizeof(Fr) + sizeof(StrobeState) <= 8192 - 16) {
+          (size_t)left * (L + 2) * sizeof(Fr) + sizeof(StrobeState) <= kFinalHostOffset) {
         // All rounds in one cooperative launch: in step while the tables are large, prepared ahead of their
         // challenges once they are small, final values included.
         uint32_t ahead_from = 0;

@@ -23,13 +23,14 @@ int zk_ctx::setup() {
   rs.sink.pub_msg = reinterpret_cast<Fr*>(dev_view);
   rs.sink.pub_flag = reinterpret_cast<unsigned int*>(reinterpret_cast<char*>(dev_view) + 16 * sizeof(Fr));
   rs.sink.seq = 0;
-  ZK_CUDA(cudaMalloc(&final_out, sizeof(Fr) * 16));
-  ZK_CUDA(cudaMalloc(&tail_out, 8192));
-  ZK_CUDA(cudaMalloc(&resident_sh, 8192));
+  // one block, laid out as host_small mirrors it, so that a prove's results come back in one copy
+  ZK_CUDA(cudaMalloc(&tail_out, 8192 + 8192));
+  final_out = reinterpret_cast<Fr*>(reinterpret_cast<char*>(tail_out) + kFinalHostOffset);
+  resident_sh = reinterpret_cast<char*>(tail_out) + kFlagsHostOffset;
   ZK_CUDA(cudaMemsetAsync(resident_sh, 0, 8192, stream));
   ZK_CUDA(cudaMalloc(&tail_buf, sizeof(Fr) * 64 * kMaxPolys * 4));
   ZK_CUDA(cudaHostAlloc(&host_points, kHostPointsBytes, cudaHostAllocDefault));
-  ZK_CUDA(cudaHostAlloc(&host_small, 8192, cudaHostAllocDefault));
+  ZK_CUDA(cudaHostAlloc(&host_small, kFlagsHostOffset + 256, cudaHostAllocDefault));
   ZK_CUDA(cudaStreamSynchronize(stream));
   return 0;
 }
@@ -97,10 +98,8 @@ void zk_ctx::teardown() {
   cudaFree(rs.sink.counter);
   cudaFree(rs.sink.msg);
   if (mailbox) cudaFreeHost(mailbox);
-  cudaFree(final_out);
   cudaFree(tail_buf);
   cudaFree(tail_out);
-  cudaFree(resident_sh);
   cudaFree(work);
   cudaFree(aux);
   cudaFree(cmp);

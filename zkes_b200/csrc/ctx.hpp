@@ -54,8 +54,11 @@ struct MsmStatsPod {
 
 struct zk_comm;
 
+// zk_ctx::tail_out and its mirror zk_ctx::host_small: messages, challenges and transcript state from 0, then the final
+// values, then the hand-over area of the resident kernel (host_small mirrors its first 16 bytes, the error word among them)
+constexpr size_t kFinalHostOffset = 7168;
+constexpr size_t kFlagsHostOffset = 8192;
 constexpr size_t kHostPointsBytes = 68 * 1024;  // zk_ctx::host_points
-constexpr size_t kFinalHostOffset = 7168;  // zk_ctx::host_small: where the final values land when they are read back with the rounds
 
 struct zk_ctx {
   int device = 0;
@@ -64,10 +67,10 @@ struct zk_ctx {
   cudaStream_t side_stream = nullptr;  // a bandwidth-bound pass that may run beside latency-bound launches
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   zk::RoundScratch rs{};
-  zk::Fr* final_out = nullptr;   // kMaxPolys + 1 elements
+  zk::Fr* final_out = nullptr;   // kMaxPolys + 1 elements, inside tail_out's block
   void* tail_out = nullptr;      // device-resident rounds: messages, challenges, transcript state (8 KiB)
   void* host_points = nullptr;   // pinned: window sums of a few rows and their combination (msm.cu)
-  void* resident_sh = nullptr;   // zk::ResidentShared: hand-over area of the resident multi-round kernel (8 KiB)
+  void* resident_sh = nullptr;   // zk::ResidentShared: hand-over area of the resident multi-round kernel (8 KiB, inside tail_out's block)
   zk::Fr* tail_buf = nullptr;    // sharded proves: gathered values and the last log2(world) rounds' tables
   void* host_small = nullptr;    // pinned, 8 KiB: round messages and other tiny read-backs
   void* mailbox = nullptr;       // pinned + mapped: message kernels publish here, the host polls
