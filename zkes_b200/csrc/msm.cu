@@ -259,9 +259,10 @@ __device__ __forceinline__ uint32_t bucket_of(const uint32_t* __restrict__ offse
   return lo;
 }
 
-// The mixed addition with its ten products as calls of one shared routine: the loop body is then a
-// few kilobytes instead of forty, which the instruction cache holds (measured 4 % faster on the
-// commit of 2^24 points; the inlined form stalled on instruction fetch).
+// The mixed addition with its ten products as calls of one shared routine, for the kernels that hold other additions
+// besides.  The kernels whose loop is the addition alone (k_msm_accumulate, k_rows_sums) inline it: with the product at some
+// 185 instructions the loop body fits the instruction cache, and the calls' register moves cost 2.5 to 4 % (2 809 us against
+// 2 739 us for 2^24 entries, 1 820 against 1 740 us for 11.2 M table additions).
 __device__ __noinline__ Fq fq_mul_call(const Fq a, const Fq b) { return mul(a, b); }
 __device__ __noinline__ Fq fq_sqr_call(const Fq a) { return sqr(a); }
 
@@ -310,7 +311,7 @@ __global__ void __launch_bounds__(128, kAccBlocks) k_msm_accumulate(const Affine
     const uint32_t col = ent & 0x7fffffffu;
     Affine pt = ld_affine(bases + (gather ? gather[col] : col));
     if (ent & 0x80000000u) pt = neg(pt);
-    acc = add_mixed_calls(acc, pt);
+    acc = add_mixed(acc, pt);
   }
   // the bucket in progress at the end of the chunk
   const bool continues = b_end > end;
@@ -872,7 +873,7 @@ __global__ void __launch_bounds__(128, kAccBlocks) k_rows_sums(const Affine* __r
   Xyzz acc = Xyzz::inf();
   for (uint32_t g = q * seg; g < g1; g++) {
     const uint32_t m = idx[(uint64_t)g * units + u];
-    if (m) acc = add_mixed_calls(acc, ld_affine(table + ((uint64_t)g << s) + m));
+    if (m) acc = add_mixed(acc, ld_affine(table + ((uint64_t)g << s) + m));
   }
   st_xyzz(pieces + c, acc);
 }
