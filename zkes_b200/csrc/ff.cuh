@@ -468,12 +468,19 @@ inline Fp<P> mul_host(const Fp<P>& a, const Fp<P>& b) {
     t[3] = (uint64_t)c;
     t[4] = t[5] + (uint64_t)(c >> 64);
   }
-  Fp<P> r;  // below 2p < 2^256
+  uint64_t d[4], borrow = 0;  // the value is below 2p < 2^256: subtract p unless that borrows
   for (int i = 0; i < 4; i++) {
-    r.v[2 * i] = (uint32_t)t[i];
-    r.v[2 * i + 1] = (uint32_t)(t[i] >> 32);
+    const u128 v = (u128)t[i] - p[i] - borrow;
+    d[i] = (uint64_t)v;
+    borrow = (uint64_t)(v >> 64) & 1;
   }
-  final_sub<P>(r.v, 0);
+  const uint64_t keep = 0 - borrow;
+  Fp<P> r;
+  for (int i = 0; i < 4; i++) {
+    const uint64_t v = (t[i] & keep) | (d[i] & ~keep);
+    r.v[2 * i] = (uint32_t)v;
+    r.v[2 * i + 1] = (uint32_t)(v >> 32);
+  }
   return r;
 }
 
