@@ -1,0 +1,31 @@
+// Host build of the MSM's shape rules (csrc/msm_plan.hpp) for the CPU unit tests.
+#include "../../zkes_b200/csrc/msm_plan.hpp"
+using namespace zk;
+
+// out: buckets, scratch bytes
+extern "C" void zkp_buckets(uint64_t total, uint32_t rows, int w, int k_windows, int sm, uint64_t* out) {
+  const BucketPlan b = bucket_plan(total, rows, w, k_windows, sm);
+  out[0] = b.n_buckets;
+  out[1] = b.scratch;
+}
+// out: window bits, windows (of scalars below 2^30 with the largest magnitude max_mag)
+extern "C" void zkp_windows(uint64_t n, uint32_t rows, uint32_t max_mag, uint64_t* out) {
+  int bits = 0;
+  while (max_mag >> bits) bits++;
+  const int w = pick_window(n, rows, bits);
+  out[0] = (uint64_t)w;
+  out[1] = (uint64_t)windows_for(max_mag, w);
+}
+// out: group, planes, groups, seg, parts, scratch bytes, partial sums, chains held at a time
+extern "C" void zkp_rows(uint64_t n, uint32_t rows, uint32_t max_span, int k_windows, uint32_t half, int sm, uint64_t max_scratch,
+                         uint64_t* out) {
+  const RowsPlan p = rows_plan(n, rows, max_span, k_windows, half, sm, max_scratch);
+  out[0] = (uint64_t)p.group;
+  out[1] = (uint64_t)p.planes;
+  out[2] = p.groups;
+  out[3] = p.seg;
+  out[4] = p.parts;
+  out[5] = p.scratch();
+  out[6] = (uint64_t)p.parts * rows * p.planes;
+  out[7] = p.slab;
+}

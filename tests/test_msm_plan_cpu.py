@@ -1,0 +1,68 @@
+"""The rules by which the MSM pipeline picks its route and cuts its work (zkes_b200/csrc/msm_plan.hpp), on the CPU."""
+import ctypes
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+SM = 148
+FREE_SCRATCH = 256 << 20  # what the tables may take whatever the buckets would
+# largest magnitude, largest of v and -v - 1
+KINDS = {"bit": (1, 1), "minus": (1, 0), "sign": (1, 1), "int8": (128, 127), "int16": (32768, 32767), "int30": ((1 << 30) - 1, (1 << 30) - 1)}
+
+
+@pytest.fixture(scope="module")
+def plan(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("plan") / "libmsmplan.so")
+    subprocess.run(["g++", "-O2", "-shared", "-fPIC", "-std=c++17", os.path.join(HERE, "hostmath", "msm_plan_host.cpp"), "-o", so], check=True)
+    lib = ctypes.CDLL(so)
+    u64, u32, i = ctypes.c_uint64, ctypes.c_uint32, ctypes.c_int
+    lib.zkp_buckets.argtypes = [u64, u32, i, i, i, ctypes.c_void_p]
+    lib.zkp_windows.argtypes = [u64, u32, u32, ctypes.c_void_p]
+    lib.zkp_rows.argtypes = [u64, u32, u32, i, u32, i, u64, ctypes.c_void_p]
+
+    def call(name, n_out, *args):
+        out = (u64 * n_out)()
+        getattr(lib, name)(*args, out)
+        return list(out)
+
+    return call
+
+
+def shapes(plan, rows, n, kind):
+    mag, span = KINDS[kind]
+    w, k = plan("zkp_windows", 2, n, rows, mag)
+    buckets, scratch = plan("zkp_buckets", 2, n * rows, rows, w, k, SM)
+    return span, w, k, buckets, scratch
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("rows,n", [(1024, 1 << 20), (320, 1 << 18), (4096, 1 << 17), (1 << 14, 1 << 14), (1 << 22, 300), (2, 1 << 28), (1 << 24, 7)])
+def test_subset_tables_take_no_more_scratch_than_buckets(plan, rows, n, kind):
+    """A call whose buckets fit the memory is not refused for the tables' sake."""
+    span, w, k, buckets, scratch = shapes(plan, rows, n, kind)
+    if buckets >= 1 << 31:
+        scratch = (1 << 64) - 1
+    group, _, _, _, parts, need, pieces, slab = plan("zkp_rows", 8, n, rows, span, k, 1 << (w - 1), SM, scratch)
+    assert need <= max(scratch, FREE_SCRATCH) or not group
+    assert pieces < 1 << 31
+    assert 1 <= slab <= parts or not group
+
+
+def test_tables_by_slabs(plan):
+    """2^20 columns in 1024 rows of int8 values: 9 GB of tables at once, made in slabs that fit the buckets' 4.6 GB."""
+    span, w, k, _, scratch = shapes(plan, 1024, 1 << 20, "int8")
+    at_once = plan("zkp_rows", 8, 1 << 20, 1024, span, k, 1 << (w - 1), SM, 1 << 60)
+    held = plan("zkp_rows", 8, 1 << 20, 1024, span, k, 1 << (w - 1), SM, scratch)
+    assert at_once[7] == at_once[4] and at_once[5] > scratch
+    assert held[:5] == at_once[:5] and 1 <= held[7] < held[4] and held[5] <= scratch
+
+
+def test_chains_cover_every_group(plan):
+    for rows, n, kind in [(4096, 4096, "int8"), (1024, 1024, "int8"), (3000, 777, "int16"), (100, 5000, "bit"), (5, 6, "int8")]:
+        span, w, k, _, _ = shapes(plan, rows, n, kind)
+        group, planes, groups, seg, parts = plan("zkp_rows", 8, n, rows, span, k, 1 << (w - 1), SM, 1 << 60)[:5]
+        if group:
+            assert (groups - 1) * group < n <= groups * group
+            assert (parts - 1) * seg < groups <= parts * seg

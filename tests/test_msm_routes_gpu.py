@@ -62,6 +62,35 @@ def _repeated(pool, picks):
     return torch.from_numpy(pool.view(np.int64)).cuda()[torch.from_numpy(picks).cuda()].contiguous()
 
 
+def test_rows_within_the_scratch_of_buckets(multiples):
+    """256 rows of 2^18 four-bit values: the tables (0.65 GB at once) are made in slabs that take no more than the buckets' 0.5 GB."""
+    import torch
+
+    from zkes_b200 import Context
+
+    ks, pts = multiples
+    rows, n = 256, 1 << 18
+    rng = np.random.default_rng(4)
+    pick = rng.integers(0, len(ks), size=n)
+    bases = _repeated(curve.affine_to_array(pts), pick)
+    vals = torch.randint(-8, 8, (rows, n), dtype=torch.int8, device="cuda", generator=torch.Generator(device="cuda").manual_seed(4))
+    f = torch.from_numpy(to_mont_array([o.fr_from_int(v) for v in range(-8, 8)]).view(np.int64)).cuda()[(vals.reshape(-1).int() + 8)]
+    out = np.zeros((rows, 12), dtype=np.uint64)
+    torch.cuda.synchronize()
+    c = Context(0)
+    before = torch.cuda.mem_get_info()[0]
+    check(lib.zk_msm_g1_batched(c.handle, vp(bases.data_ptr()), ZK_MEM_DEVICE, n, vp(f.data_ptr()), ZK_MEM_DEVICE, rows,
+                                vp(out.ctypes.data), ZK_MEM_HOST), "zk_msm_g1_batched")
+    taken = before - torch.cuda.mem_get_info()[0]
+    c.close()
+    buckets = 4 * rows * n + (rows * 8 + 2 * 148 * 4 * 128 * 12) * 128  # entries, bucket sums, pieces of chunks
+    compact = 4 * rows * n
+    assert taken <= buckets + compact + (64 << 20), taken  # with allocation granularity and the code loaded by the call
+    for r in (0, 1, 131, rows - 1):
+        per_base = np.bincount(pick, weights=vals[r].cpu().numpy(), minlength=len(ks))
+        assert curve.jacobian_to_affine_py(out[r:r + 1])[0] == of_g(sum(int(v) * k for v, k in zip(per_base, ks))), r
+
+
 @pytest.mark.parametrize("n", [1 << 21, 10_000_003])
 @pytest.mark.parametrize("scalars", [[1, -1], [-128, 127, 5, 0, 1]])
 def test_long_buckets_of_repeated_points(ctx, multiples, n, scalars):

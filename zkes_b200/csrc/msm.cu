@@ -14,8 +14,8 @@
 // Small scalars (quantised int8 / int16 weights and activations, negatives stored as r - |v|)
 // fold to a few bits, so they use one narrow window: no doublings, few buckets.
 #include "msm.hpp"
+#include "msm_plan.hpp"
 
-#include <algorithm>
 #include "reduce.cuh"
 #include "batch_affine.cuh"
 #include "quad.cuh"
@@ -52,14 +52,9 @@ __device__ __forceinline__ int bit_length(const uint32_t (&mag)[8]) {
   return bits;
 }
 
-// Blocks of 128 threads per SM of the kernels that add points in chains (108 registers; five spill).
-constexpr int kAccBlocks = 4;
-
 // Scalars whose folded magnitude is below 2^30 also have a compact form: a signed 32-bit integer.
 // When every scalar of a call has one (quantised weights and activations), the digit passes read
 // these 4 bytes instead of converting the 32-byte Montgomery value again.
-constexpr int kCompactBits = 30;
-constexpr int kRowsGroupMax = 12;  // bases a group of the subset-sum tables has at most (k_rows_*)
 constexpr int32_t kNotCompact = INT32_MIN;
 
 // max_out[0]: largest bit length; among the scalars below 2^32 max_out[1]: largest magnitude, max_out[2]: largest of v and
@@ -326,7 +321,6 @@ __global__ void __launch_bounds__(128, kAccBlocks) k_msm_accumulate(const Affine
 }
 
 constexpr uint32_t kFewPieces = 8;
-constexpr uint32_t kFixupPartials = 4096;  // partial sums of the grouped fix-up (buckets x groups)
 
 // One thread per bucket: buckets cut into at most kFewPieces pieces are summed in place; longer
 // ones are left to the warp-per-bucket kernel below (found through the `many` list).
@@ -485,7 +479,6 @@ __global__ void __launch_bounds__(32) k_msm_fixup_groups_final(const uint32_t* _
 // joins the blocks' runs of an item.  What bounds it is the chain of dependent additions (2 per + 2 per level of the tree),
 // so an item is spread over half / (128 per) blocks: 19 items of 8192 buckets take 224 + 24 us; one block per item with up to
 // 32 buckets a thread took 774 us and kept 19 of 148 SMs busy.
-constexpr uint32_t kReduceThreads = 128;
 
 // Joins n runs (a power of two, at most kReduceThreads) in A[], D[] (shared memory) into A[0], D[0].
 __device__ __forceinline__ void join_runs(Xyzz* A, Xyzz* D, uint32_t n) {
@@ -782,13 +775,14 @@ __global__ void __launch_bounds__(256) k_select_total(const Xyzz* __restrict__ c
 // commitment take 2.4 ms (sums 1.82, tables 0.34, bits 0.07, joining 0.19) where counting, scattering, adding and reducing
 // the buckets took 3.9 ms.
 
-// idx[g][row * planes + k]: the bits of plane k of the scalars of group g.  A thread takes a (row, group).
-__global__ void __launch_bounds__(256) k_rows_bits(const int32_t* __restrict__ compact, uint32_t n, uint32_t rows, int planes, int s,
-                                                   uint32_t groups, uint16_t* idx) {
+// idx[g][row * planes + k]: the bits of plane k of the scalars of group g.  A thread takes a (row, group).  n of the scalars of a
+// row, which are `stride` apart from the next row's.
+__global__ void __launch_bounds__(256) k_rows_bits(const int32_t* __restrict__ compact, uint64_t stride, uint32_t n, uint32_t rows, int planes,
+                                                   int s, uint32_t groups, uint16_t* idx) {
   const uint64_t total = (uint64_t)rows * groups;
   for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t row = (uint32_t)(t % rows), g = (uint32_t)(t / rows);
-    const int32_t* v = compact + (uint64_t)row * n + (uint64_t)g * s;
+    const int32_t* v = compact + row * stride + (uint64_t)g * s;
     const int have = n - g * s < (uint32_t)s ? (int)(n - g * s) : s;
     uint16_t* out = idx + (uint64_t)g * rows * planes + (uint64_t)row * planes;
     int32_t w[kRowsGroupMax];
@@ -921,44 +915,9 @@ __global__ void __launch_bounds__(64) k_rows_planes(const Xyzz* __restrict__ uni
 
 }  // namespace
 
-// Window width for n points per row whose scalars have at most max_bits magnitude bits.
-static int pick_window(uint64_t n, uint32_t rows, int max_bits) {
-  int lg = 0;
-  while ((1ull << (lg + 1)) <= n) lg++;
-  // a row costs windows * (n + 2 * 2^(w-1)) additions; with many rows the buckets (128 bytes each, per
-  // row and window) also have to fit in memory, so rows use a narrower window
-  int w = rows > 1 ? lg - 4 : lg - 2;
-  if (w > 16) w = 16;
-  if (w < 3) w = 3;
-  if (w > max_bits + 1) w = max_bits + 1;
-  if (w < 2) w = 2;
-  // A top window of two or three bits has a handful of buckets that between them take every point, and joining their pieces is
-  // a chain of its own: from 2^16 points on one bit less per window is cheaper (full-width scalars, 14 bits leave two for the
-  // nineteenth window, 13 leave seven for the twentieth: 100003 points 1 140 us against 941 us; 15 and 16 bits leave fourteen,
-  // and 262143 points take 1 623 us with 15 against 1 872 us with 14).  With fewer points the wider window stays the better one
-  // (12000 points: 548 us with 11 bits, 583 us with 10).
-  if (rows == 1 && w >= 14 && max_bits > kCompactBits && (max_bits + 1) - w * ((max_bits + w) / w - 1) < 4) w--;
-  return w;
-}
-
-size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
-
 int msm_run(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const Fr* scalars, uint64_t n, uint32_t rows,
             Jacobian* out_dev, MsmStats* stats, MsmPrep* prep) {
   return msm_run_rows(ctx, bases, gather, nullptr, scalars, n, rows, out_dev, stats, prep);
-}
-
-// Signed-digit windows needed for magnitudes up to max_mag: k digits in (-half, half] reach
-// half * (1 + 2^w + ... + 2^(w (k - 1))).
-static int windows_for(uint32_t max_mag, int w) {
-  const uint64_t half = 1ull << (w - 1);
-  uint64_t reach = 0;
-  int k = 0;
-  do {
-    reach = (reach << w) + half;
-    k++;
-  } while (reach < max_mag);
-  return k;
 }
 
 // Horner over the windows on the host, for one row or a few: a doubling is a chain of products, 0.3 us for a CPU core with
@@ -983,123 +942,41 @@ static int combine_on_host(zk_ctx* ctx, const Xyzz* window_sums, uint32_t rows, 
   return 0;
 }
 
-// Entries per chunk of the accumulation (a chunk is a thread's): whole waves of resident threads, of some 64 to 96 entries each
-// where there are that many.  Shorter chunks mean more pieces of buckets to join afterwards, a last wave that is nearly
-// empty costs as much as a full one: 2^24 entries in chunks of 32 left 2^19 pieces, whose sums took 286 us against 142 us for a
-// third of them; 1.9 M entries in one full wave instead of four fifths of one take 345 us against 436 us.
-constexpr uint32_t kChunkMin = 16, kChunkWaves = 12;
-static uint32_t chunk_entries(uint32_t n_entries, int sm) {
-  const uint64_t resident = (uint64_t)sm * kAccBlocks * 128;
-  uint64_t seg = (n_entries + resident - 1) / resident;
-  if (seg < kChunkMin) return kChunkMin;
-  if (seg > 96) {
-    uint64_t waves = seg / 64;
-    if (waves > kChunkWaves) waves = kChunkWaves;
-    seg = (n_entries + resident * waves - 1) / (resident * waves);
-  }
-  return (uint32_t)seg;
-}
-
-// Lanes per item for k_msm_bucket_reduce_rows, 0 where an item is worth a block or more of its own.  More lanes shorten the
-// chain and add work (a scan and a tree over them), so they double only until half of the threads that fit the GPU (three
-// blocks of 128 per SM) have work: 4096 items of 128 buckets lost 2 % of their commitment with sixteen lanes instead of eight.
-static uint32_t reduce_lanes(uint32_t n_items, uint32_t half, int sm) {
-  if (n_items < 1024 || half < 8) return 0;
-  uint32_t lanes = 8;
-  while (lanes < 32 && lanes * 2 <= half && (uint64_t)n_items * lanes < (uint64_t)sm * 3 * 64) lanes *= 2;
-  return lanes;
-}
-
-// Buckets per thread and blocks per item of the bucket reduction.  Longer runs cost fewer additions in all (2 + 4 / per a
-// bucket), shorter ones a shorter chain: the runs double while the launch still fills the GPU with threads, and an item has at
-// most kReduceThreads blocks (the second launch joins them in one block).
-static void reduce_shape(uint32_t n_items, uint32_t half, uint32_t* per, uint32_t* parts) {
-  uint32_t p = 1;
-  while (p < half && (p < 32 && (uint64_t)n_items * (half / (2 * p)) >= 40000)) p *= 2;
-  if (p < 4) p = half < 4 ? half : 4;
-  while (half / p > kReduceThreads * kReduceThreads) p *= 2;
-  *per = p;
-  const uint32_t n = half / p;
-  *parts = n > kReduceThreads ? n / kReduceThreads : 1;
-}
-
-// Shape of the subset-sum method for `rows` dense rows of n small scalars, group = 0 when buckets take fewer additions.
-struct RowsPlan {
-  int group = 0;  // bases per group
-  int planes = 0;
-  uint32_t groups = 0;
-};
-
-static RowsPlan rows_plan(uint64_t n, uint32_t rows, uint32_t max_span, int k_windows, uint32_t half) {
-  RowsPlan best;
-  int planes = 1;
-  while (planes < 32 && (max_span >> (planes - 1))) planes++;
-  // additions a row by buckets: one an entry, and two per bucket in general coordinates (14 products to 10)
-  double least = (double)rows * k_windows * ((double)n + 2.8 * half);
-  if ((uint64_t)rows * planes >= (1ull << 31)) return best;
-  for (int s = 2; s <= kRowsGroupMax; s++) {
-    const uint64_t groups = (n + s - 1) / s;
-    if ((groups << s) >= (1ull << 31) || (uint64_t)rows * planes * groups >= (1ull << 40)) continue;
-    const double cost = (double)rows * planes * groups + (double)(groups << s);
-    if (cost < least) {
-      least = cost;
-      best.group = s;
-      best.planes = planes;
-      best.groups = (uint32_t)groups;
-    }
-  }
-  return best;
-}
-
 static int rows_run(zk_ctx* ctx, const Affine* bases, const int32_t* compact, uint32_t n, uint32_t rows, const RowsPlan& plan,
                     Jacobian* out_dev, MsmStats* stats, int max_bits) {
   cudaStream_t st = ctx->stream;
   const int sm = ctx->sm_count, s = plan.group, lo_bits = (s + 1) / 2;
-  const uint32_t groups = plan.groups;
+  const uint32_t groups = plan.groups, seg = plan.seg, parts = plan.parts;
   const uint64_t units = (uint64_t)rows * plan.planes;
-  // A unit's groups are cut into `parts` chains, a thread each.  The time is the waves of threads that takes times a
-  // chain's length, plus the additions that join the chains (14 products to 10, at half the efficiency): 32768 units of 342 groups
-  // in three parts are 1.3 waves, which cost two, and took 2.17 ms; nine parts are 3.9.
-  const uint64_t resident = (uint64_t)sm * kAccBlocks * 128;
-  uint64_t parts = 1;
-  double least = 1e300;
-  for (uint64_t p = 1; p <= 64 && p <= groups; p++) {
-    const uint64_t waves = (units * p + resident - 1) / resident;
-    const double cost = (double)waves * (double)((groups + p - 1) / p) + 2.8 * (double)(units * p) / (double)resident;
-    if (cost < least) {
-      least = cost;
-      parts = p;
-    }
-  }
-  const uint32_t seg = (uint32_t)((groups + parts - 1) / parts);
-  parts = (groups + seg - 1) / seg;
-  const uint64_t n_pieces = parts * units;
-  if (n_pieces >= (1ull << 31)) return fail(-1, "msm: %llu partial sums exceed 2^31 - 1; split the rows", (unsigned long long)n_pieces);
-  const uint32_t half_points = groups * ((1u << lo_bits) + (1u << (s - lo_bits)));
   const uint64_t table_points = (uint64_t)groups << s;
   char* base = nullptr;
-  int rc = ctx->reserve_aux(align256(units * groups * 2) + align256((uint64_t)half_points * sizeof(Affine)) +
-                                align256(table_points * sizeof(Affine)) + align256(n_pieces * sizeof(Xyzz)) + 1024, (void**)&base);
+  int rc = ctx->reserve_aux(plan.scratch(), (void**)&base);
   if (rc) return rc;
   size_t off = 0;
   auto take = [&](size_t bytes) { char* p = base + off; off += align256(bytes); return p; };
-  uint16_t* idx = (uint16_t*)take(units * groups * 2);
-  Affine* halves = (Affine*)take((uint64_t)half_points * sizeof(Affine));
-  Affine* table = (Affine*)take(table_points * sizeof(Affine));
-  Xyzz* pieces = (Xyzz*)take(n_pieces * sizeof(Xyzz));
-  const uint64_t cells = (uint64_t)rows * groups;
-  const uint64_t bit_blocks = (cells + 255) / 256;
-  k_rows_bits<<<(unsigned)(bit_blocks < (uint64_t)sm * 32 ? bit_blocks : (uint64_t)sm * 32), 256, 0, st>>>(compact, n, rows, plan.planes, s, groups, idx);
-  k_rows_halves<<<(half_points + 127) / 128, 128, 0, st>>>(bases, n, s, lo_bits, groups, halves);
-  const uint64_t per_block = kBatchThreads * kBatchTable;
-  k_rows_table<<<(unsigned)((table_points + per_block - 1) / per_block), kBatchThreads, 0, st>>>(halves, s, lo_bits, groups, table);
-  k_rows_sums<<<(unsigned)((n_pieces + 127) / 128), 128, 0, st>>>(table, idx, (uint32_t)units, s, groups, seg, (uint32_t)n_pieces, pieces);
+  uint16_t* idx = (uint16_t*)take(plan.idx_bytes);
+  Affine* halves = (Affine*)take(plan.halves_bytes);
+  Affine* table = (Affine*)take(plan.table_bytes);
+  Xyzz* pieces = (Xyzz*)take(plan.pieces_bytes);
+  for (uint32_t q0 = 0; q0 < parts; q0 += plan.slab) {  // the chains [q0, q0 + chains) and their groups [g0, g0 + held)
+    const uint32_t chains = std::min(plan.slab, parts - q0), g0 = q0 * seg, held = std::min(groups - g0, chains * seg);
+    const uint32_t first = g0 * (uint32_t)s, left = n - first;
+    const uint32_t half_points = held * ((1u << lo_bits) + (1u << (s - lo_bits)));
+    const uint64_t bit_blocks = ((uint64_t)rows * held + 255) / 256;
+    const uint64_t per_block = kBatchThreads * kBatchTable, table_blocks = (((uint64_t)held << s) + per_block - 1) / per_block;
+    const uint32_t sums = chains * (uint32_t)units;
+    k_rows_bits<<<(unsigned)std::min<uint64_t>(bit_blocks, (uint64_t)sm * 32), 256, 0, st>>>(compact + first, n, left, rows, plan.planes, s, held, idx);
+    k_rows_halves<<<(half_points + 127) / 128, 128, 0, st>>>(bases + first, left, s, lo_bits, held, halves);
+    k_rows_table<<<(unsigned)table_blocks, kBatchThreads, 0, st>>>(halves, s, lo_bits, held, table);
+    k_rows_sums<<<(sums + 127) / 128, 128, 0, st>>>(table, idx, (uint32_t)units, s, held, seg, sums, pieces + (uint64_t)q0 * units);
+    ctx->launches += 4;
+  }
   if (parts > 1) {
-    k_rows_units<<<(unsigned)((units + 31) / 32), 128, 0, st>>>(pieces, (uint32_t)units, (uint32_t)parts);
+    k_rows_units<<<(unsigned)((units + 31) / 32), 128, 0, st>>>(pieces, (uint32_t)units, parts);
     ctx->launches++;
   }
   k_rows_planes<<<(rows + 63) / 64, 64, 0, st>>>(pieces, rows, plan.planes, out_dev);
-  ctx->launches += 5;
+  ctx->launches++;
   ZK_CUDA(cudaGetLastError());
   const uint64_t additions = units * groups + table_points;
   ctx->msm_entries_sum += additions;
@@ -1173,45 +1050,36 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
   // small scalars: the exact largest magnitude is known, which can save the window that would only
   // hold carries (int8 values reach 128 = one 8-bit signed digit)
   const int k_windows = compact ? windows_for(max_mag, w) : ((int)max_bits + 1 + w - 1) / w;
-  const uint32_t half = 1u << (w - 1);
-  const uint64_t n_buckets64 = (uint64_t)rows * k_windows * half;
+  const BucketPlan plan = bucket_plan(total, rows, w, k_windows, sm);
+  const uint32_t half = plan.half;
+  const bool too_many = plan.n_buckets >= (1ull << 31);
+  const uint32_t n_buckets = (uint32_t)plan.n_buckets;
+  const size_t scan_bytes = too_many ? 0 : align256(scan_scratch_elems(n_buckets + 1) * 4);
   if (compact && rows > 1 && !row_ids && !gather) {
-    const RowsPlan plan = rows_plan(n, rows, max_span, k_windows, half);
-    if (plan.group) return rows_run(ctx, bases, compact, (uint32_t)n, rows, plan, out_dev, stats, (int)max_bits);
+    const RowsPlan by_sums = rows_plan(n, rows, max_span, k_windows, half, sm, too_many ? ~(size_t)0 : plan.scratch + scan_bytes);
+    if (by_sums.group) {
+      const int rc = rows_run(ctx, bases, compact, (uint32_t)n, rows, by_sums, out_dev, stats, (int)max_bits);
+      if (rc != -2 /*ZK_ERR_OOM*/) return rc;  // no room for the tables: the buckets of a small call may still have it
+    }
   }
-  if (n_buckets64 >= (1ull << 31)) return fail(-1, "msm: %llu buckets exceed the 32-bit key space; split the rows", (unsigned long long)n_buckets64);
-  const uint32_t n_buckets = (uint32_t)n_buckets64;
+  if (too_many) return fail(-1, "msm: %llu buckets exceed the 32-bit key space; split the rows", (unsigned long long)plan.n_buckets);
 
   // ---- scratch layout (second scratch region of the context; the first holds caller data)
-  // worst case: every scalar has a non-zero digit in every window; small scalars have fewer, and the
-  // real total is checked after the count pass (entry slots are 32-bit)
-  uint64_t max_entries = total * (uint64_t)k_windows;
-  if (max_entries > 0xffffffffull) max_entries = 0xffffffffull;
-  uint32_t red_per, red_parts;
-  reduce_shape(rows * (uint32_t)k_windows, half, &red_per, &red_parts);
-  const uint64_t n_runs = red_parts > 1 ? 2ull * rows * k_windows * red_parts : 0;
-  size_t need = align256(n_runs * sizeof(Xyzz)) + align256((n_buckets + 2) * 4ull) * 2 + align256(scan_scratch_elems(n_buckets + 1) * 4) +
-                align256((size_t)n_buckets * sizeof(Xyzz)) + align256((size_t)rows * k_windows * sizeof(Xyzz)) + 4096;
   char* base = nullptr;
-  // entries and chunk slots are sized after the count pass; reserve the worst case now
-  uint64_t chunk_guess = max_entries / kChunkMin + 1;
-  const uint64_t chunk_cap = (uint64_t)sm * kAccBlocks * 128 * kChunkWaves;
-  if (chunk_guess > chunk_cap) chunk_guess = chunk_cap;
-  need += align256(max_entries * 4) + 2 * align256((chunk_guess + 1) * sizeof(Xyzz)) + align256((size_t)kFixupPartials * sizeof(Xyzz));
-  int rc = ctx->reserve_aux(need, (void**)&base);
+  int rc = ctx->reserve_aux(plan.scratch + scan_bytes, (void**)&base);
   if (rc) return rc;
   size_t off = 0;
   auto take = [&](size_t bytes) { char* p = base + off; off += align256(bytes); return p; };
   uint32_t* offsets = (uint32_t*)take((n_buckets + 2) * 4ull);
   uint32_t* cursor = (uint32_t*)take((n_buckets + 2) * 4ull);
-  uint32_t* scan_tmp = (uint32_t*)take(scan_scratch_elems(n_buckets + 1) * 4);
+  uint32_t* scan_tmp = (uint32_t*)take(scan_bytes);
   Xyzz* bucket_sums = (Xyzz*)take((size_t)n_buckets * sizeof(Xyzz));
   Xyzz* window_sums = (Xyzz*)take((size_t)rows * k_windows * sizeof(Xyzz));
-  uint32_t* entries = (uint32_t*)take(max_entries * 4);
-  Xyzz* heads = (Xyzz*)take((chunk_guess + 1) * sizeof(Xyzz));
-  Xyzz* tails = (Xyzz*)take((chunk_guess + 1) * sizeof(Xyzz));
+  uint32_t* entries = (uint32_t*)take(plan.max_entries * 4);
+  Xyzz* heads = (Xyzz*)take((plan.chunks + 1) * sizeof(Xyzz));
+  Xyzz* tails = (Xyzz*)take((plan.chunks + 1) * sizeof(Xyzz));
   Xyzz* fix_part = (Xyzz*)take((size_t)kFixupPartials * sizeof(Xyzz));
-  Xyzz* runs = (Xyzz*)take(n_runs * sizeof(Xyzz));
+  Xyzz* runs = (Xyzz*)take(plan.n_runs * sizeof(Xyzz));
 
   // ---- pass 2: count, scan, scatter
   ZK_CUDA(cudaMemsetAsync(offsets, 0, (n_buckets + 2) * 4ull, s));
@@ -1293,9 +1161,9 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
   if (lanes) {
     k_msm_bucket_reduce_rows<<<(n_items + 128 / lanes - 1) / (128 / lanes), 128, 0, s>>>(bucket_sums, half, n_items, lanes, window_sums);
   } else {
-    k_msm_bucket_reduce<<<n_items * red_parts, kReduceThreads, 0, s>>>(bucket_sums, half, red_per, red_parts, runs, window_sums);
-    if (red_parts > 1) {
-      k_msm_join_items<<<n_items, kReduceThreads, 0, s>>>(runs, red_parts, window_sums);
+    k_msm_bucket_reduce<<<n_items * plan.red_parts, kReduceThreads, 0, s>>>(bucket_sums, half, plan.red_per, plan.red_parts, runs, window_sums);
+    if (plan.red_parts > 1) {
+      k_msm_join_items<<<n_items, kReduceThreads, 0, s>>>(runs, plan.red_parts, window_sums);
       ctx->launches++;
     }
   }

@@ -1,0 +1,201 @@
+// Shapes of the MSM pipeline (msm.cu): which route a call takes, how its work is cut, and the scratch that this needs.  Host
+// arithmetic on sizes alone, without CUDA, so that it can be checked on a machine without a GPU.
+#pragma once
+#include <algorithm>
+#include <cstddef>
+#include <cstdint>
+
+namespace zk {
+
+constexpr int kCompactBits = 30;  // magnitudes below 2^30 have a compact form (k_msm_bits)
+constexpr int kAccBlocks = 4;     // blocks of 128 threads per SM of the kernels that add points in chains (126 and 122 registers)
+constexpr uint32_t kReduceThreads = 128;   // threads of a block of the bucket reduction
+constexpr uint32_t kFixupPartials = 4096;  // partial sums of the grouped fix-up (buckets x groups)
+constexpr int kRowsGroupMax = 12;          // bases a group of the subset-sum tables has at most (k_rows_*)
+constexpr size_t kAffineBytes = 64, kXyzzBytes = 128;
+
+inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
+
+// Window width for n points per row whose scalars have at most max_bits magnitude bits.
+inline int pick_window(uint64_t n, uint32_t rows, int max_bits) {
+  int lg = 0;
+  while ((1ull << (lg + 1)) <= n) lg++;
+  // a row costs windows * (n + 2 * 2^(w-1)) additions; with many rows the buckets (128 bytes each, per
+  // row and window) also have to fit in memory, so rows use a narrower window
+  int w = rows > 1 ? lg - 4 : lg - 2;
+  if (w > 16) w = 16;
+  if (w < 3) w = 3;
+  if (w > max_bits + 1) w = max_bits + 1;
+  if (w < 2) w = 2;
+  // A top window of two or three bits has a handful of buckets that between them take every point, and joining their pieces is
+  // a chain of its own: from 2^16 points on one bit less per window is cheaper (full-width scalars, 14 bits leave two for the
+  // nineteenth window, 13 leave seven for the twentieth: 100003 points 1 140 us against 941 us; 15 and 16 bits leave fourteen,
+  // and 262143 points take 1 623 us with 15 against 1 872 us with 14).  With fewer points the wider window stays the better one
+  // (12000 points: 548 us with 11 bits, 583 us with 10).
+  if (rows == 1 && w >= 14 && max_bits > kCompactBits && (max_bits + 1) - w * ((max_bits + w) / w - 1) < 4) w--;
+  return w;
+}
+
+// Signed-digit windows needed for magnitudes up to max_mag: k digits in (-half, half] reach
+// half * (1 + 2^w + ... + 2^(w (k - 1))).
+inline int windows_for(uint32_t max_mag, int w) {
+  const uint64_t half = 1ull << (w - 1);
+  uint64_t reach = 0;
+  int k = 0;
+  do {
+    reach = (reach << w) + half;
+    k++;
+  } while (reach < max_mag);
+  return k;
+}
+
+// Entries per chunk of the accumulation (a chunk is a thread's): whole waves of resident threads, of some 64 to 96 entries each
+// where there are that many.  Shorter chunks mean more pieces of buckets to join afterwards, a last wave that is nearly
+// empty costs as much as a full one: 2^24 entries in chunks of 32 left 2^19 pieces, whose sums took 286 us against 142 us for a
+// third of them; 1.9 M entries in one full wave instead of four fifths of one take 345 us against 436 us.
+constexpr uint32_t kChunkMin = 16, kChunkWaves = 12;
+inline uint32_t chunk_entries(uint32_t n_entries, int sm) {
+  const uint64_t resident = (uint64_t)sm * kAccBlocks * 128;
+  uint64_t seg = (n_entries + resident - 1) / resident;
+  if (seg < kChunkMin) return kChunkMin;
+  if (seg > 96) {
+    uint64_t waves = seg / 64;
+    if (waves > kChunkWaves) waves = kChunkWaves;
+    seg = (n_entries + resident * waves - 1) / (resident * waves);
+  }
+  return (uint32_t)seg;
+}
+
+// Lanes per item for k_msm_bucket_reduce_rows, 0 where an item is worth a block or more of its own.  More lanes shorten the
+// chain and add work (a scan and a tree over them), so they double only until half of the threads that fit the GPU (three
+// blocks of 128 per SM) have work: 4096 items of 128 buckets lost 2 % of their commitment with sixteen lanes instead of eight.
+inline uint32_t reduce_lanes(uint32_t n_items, uint32_t half, int sm) {
+  if (n_items < 1024 || half < 8) return 0;
+  uint32_t lanes = 8;
+  while (lanes < 32 && lanes * 2 <= half && (uint64_t)n_items * lanes < (uint64_t)sm * 3 * 64) lanes *= 2;
+  return lanes;
+}
+
+// Buckets per thread and blocks per item of the bucket reduction.  Longer runs cost fewer additions in all (2 + 4 / per a
+// bucket), shorter ones a shorter chain: the runs double while the launch still fills the GPU with threads, and an item has at
+// most kReduceThreads blocks (the second launch joins them in one block).
+inline void reduce_shape(uint32_t n_items, uint32_t half, uint32_t* per, uint32_t* parts) {
+  uint32_t p = 1;
+  while (p < half && (p < 32 && (uint64_t)n_items * (half / (2 * p)) >= 40000)) p *= 2;
+  if (p < 4) p = half < 4 ? half : 4;
+  while (half / p > kReduceThreads * kReduceThreads) p *= 2;
+  *per = p;
+  const uint32_t n = half / p;
+  *parts = n > kReduceThreads ? n / kReduceThreads : 1;
+}
+
+// Buckets of a call and the scratch of their route, laid out for the worst case: every scalar has a non-zero digit in every
+// window.  Small scalars have fewer, and the real total is checked after the count pass (entry slots are 32-bit).
+struct BucketPlan {
+  int w = 0, k_windows = 0;
+  uint32_t half = 0;            // buckets per (row, window)
+  uint64_t n_buckets = 0;       // 2^31 or more: not representable, nothing below is set
+  uint64_t max_entries = 0;
+  uint64_t chunks = 0;          // of the accumulation, at most
+  uint32_t red_per = 0, red_parts = 0;
+  uint64_t n_runs = 0;
+  size_t scratch = 0;           // bytes, without the scan's own
+};
+
+inline BucketPlan bucket_plan(uint64_t total, uint32_t rows, int w, int k_windows, int sm) {
+  BucketPlan b;
+  b.w = w;
+  b.k_windows = k_windows;
+  b.half = 1u << (w - 1);
+  b.n_buckets = (uint64_t)rows * k_windows * b.half;
+  if (b.n_buckets >= (1ull << 31)) return b;
+  b.max_entries = std::min<uint64_t>(total * (uint64_t)k_windows, 0xffffffffull);
+  b.chunks = std::min<uint64_t>(b.max_entries / kChunkMin + 1, (uint64_t)sm * kAccBlocks * 128 * kChunkWaves);
+  reduce_shape(rows * (uint32_t)k_windows, b.half, &b.red_per, &b.red_parts);
+  b.n_runs = b.red_parts > 1 ? 2ull * rows * k_windows * b.red_parts : 0;
+  b.scratch = align256(b.n_runs * kXyzzBytes) + 2 * align256((b.n_buckets + 2) * 4) + align256(b.n_buckets * kXyzzBytes) +
+              align256((size_t)rows * k_windows * kXyzzBytes) + align256(b.max_entries * 4) + 2 * align256((b.chunks + 1) * kXyzzBytes) +
+              align256((size_t)kFixupPartials * kXyzzBytes) + 4096;
+  return b;
+}
+
+// Shape of the subset-sum method for `rows` dense rows of n small scalars, group = 0 when buckets are taken instead.
+struct RowsPlan {
+  int group = 0;  // bases per group
+  int planes = 0;
+  uint32_t groups = 0;
+  uint32_t seg = 0, parts = 0;  // a unit's groups are cut into `parts` chains of `seg`, a thread each
+  uint32_t slab = 0;            // chains whose tables are held at a time
+  size_t idx_bytes = 0, halves_bytes = 0, table_bytes = 0, pieces_bytes = 0;
+  uint32_t slab_groups() const { return (uint32_t)std::min<uint64_t>(groups, (uint64_t)slab * seg); }
+  size_t scratch() const { return align256(idx_bytes) + align256(halves_bytes) + align256(table_bytes) + align256(pieces_bytes) + 1024; }
+};
+
+// The time is the waves of threads that the chains take times a chain's length, plus the additions that join the chains
+// (14 products to 10, at half the efficiency): 32768 units of 342 groups in three parts are 1.3 waves, which cost two, and took
+// 2.17 ms; nine parts are 3.9.
+inline void rows_chains(RowsPlan* p, uint32_t rows, int sm) {
+  const uint64_t units = (uint64_t)rows * p->planes, resident = (uint64_t)sm * kAccBlocks * 128;
+  uint64_t parts = 1;
+  double least = 1e300;
+  for (uint64_t c = 1; c <= 64 && c <= p->groups; c++) {
+    const uint64_t waves = (units * c + resident - 1) / resident;
+    const double cost = (double)waves * (double)((p->groups + c - 1) / c) + 2.8 * (double)(units * c) / (double)resident;
+    if (cost < least) {
+      least = cost;
+      parts = c;
+    }
+  }
+  p->seg = (uint32_t)((p->groups + parts - 1) / parts);
+  p->parts = (p->groups + p->seg - 1) / p->seg;
+}
+
+// Sizes with the tables of `slab` chains held at a time.
+inline void rows_sizes(RowsPlan* p, uint32_t rows, uint32_t slab) {
+  const uint64_t units = (uint64_t)rows * p->planes;
+  const int s = p->group, lo_bits = (s + 1) / 2;
+  p->slab = slab;
+  const uint64_t held = p->slab_groups();
+  p->idx_bytes = units * held * 2;
+  p->halves_bytes = held * ((1u << lo_bits) + (1u << (s - lo_bits))) * kAffineBytes;
+  p->table_bytes = (held << s) * kAffineBytes;
+  p->pieces_bytes = p->parts * units * kXyzzBytes;
+}
+
+// max_scratch: what the buckets' route would take.  Above kRowsScratch the tables never take more than that: they are made for
+// as many chains at a time as fit (2^20 columns in 1024 rows of int8 values: 9 GB at once, 4.6 GB of buckets).
+constexpr size_t kRowsScratch = 256ull << 20;
+inline RowsPlan rows_plan(uint64_t n, uint32_t rows, uint32_t max_span, int k_windows, uint32_t half, int sm, size_t max_scratch) {
+  RowsPlan best;
+  int planes = 1;
+  while (planes < 32 && (max_span >> (planes - 1))) planes++;
+  // additions a row by buckets: one an entry, and two per bucket in general coordinates (14 products to 10)
+  double least = (double)rows * k_windows * ((double)n + 2.8 * half);
+  const uint64_t units = (uint64_t)rows * planes;
+  if (units >= (1ull << 31)) return best;
+  for (int s = 2; s <= kRowsGroupMax; s++) {
+    const uint64_t groups = (n + s - 1) / s;
+    if ((groups << s) >= (1ull << 31) || units * groups >= (1ull << 40)) continue;
+    const double cost = (double)(units * groups) + (double)(groups << s);
+    if (cost >= least) continue;
+    RowsPlan p;
+    p.group = s;
+    p.planes = planes;
+    p.groups = (uint32_t)groups;
+    rows_chains(&p, rows, sm);
+    if (p.parts * units >= (1ull << 31)) continue;
+    const size_t limit = std::max(max_scratch, kRowsScratch);
+    uint32_t slab = p.parts;
+    rows_sizes(&p, rows, slab);
+    while (p.scratch() > limit && slab > 1) {
+      slab = (slab + 1) / 2;
+      rows_sizes(&p, rows, slab);
+    }
+    if (p.scratch() > limit) continue;
+    least = cost;
+    best = p;
+  }
+  return best;
+}
+
+}  // namespace zk
