@@ -29,3 +29,4 @@ extern "C" void zkp_rows(uint64_t n, uint32_t rows, uint32_t max_span, int k_win
   out[6] = (uint64_t)p.parts * rows * p.planes;
   out[7] = p.slab;
 }
+extern "C" uint32_t zkp_reduce_lanes(uint32_t n_items, uint32_t half, int sm) { return reduce_lanes(n_items, half, sm); }

@@ -22,7 +22,12 @@ def plan(tmp_path_factory):
     lib.zkp_windows.argtypes = [u64, u32, u32, ctypes.c_void_p]
     lib.zkp_rows.argtypes = [u64, u32, u32, i, u32, i, u64, ctypes.c_void_p]
 
+    lib.zkp_reduce_lanes.argtypes = [u32, u32, i]
+    lib.zkp_reduce_lanes.restype = u32
+
     def call(name, n_out, *args):
+        if n_out == 0:
+            return getattr(lib, name)(*args)
         out = (u64 * n_out)()
         getattr(lib, name)(*args, out)
         return list(out)
@@ -66,3 +71,17 @@ def test_chains_cover_every_group(plan):
         if group:
             assert (groups - 1) * group < n <= groups * group
             assert (parts - 1) * seg < groups <= parts * seg
+
+
+@pytest.mark.parametrize("half", [2, 4])
+@pytest.mark.parametrize("items", [1, 85, 1024, 174080])
+def test_few_buckets_an_item_get_a_thread(plan, items, half):
+    """A block per item would keep one thread of 128 busy."""
+    assert plan("zkp_reduce_lanes", 0, items, half, SM) == 1
+
+
+@pytest.mark.parametrize("half", [8, 16, 128, 512, 32768])
+@pytest.mark.parametrize("items", [1, 1023, 1024, 2000, 30000])
+def test_lanes_divide_the_buckets(plan, items, half):
+    lanes = plan("zkp_reduce_lanes", 0, items, half, SM)
+    assert lanes in ((0,) if items < 1024 else (8, 16, 32)) and lanes <= half

@@ -142,3 +142,9 @@ def test_full_width_rows(ctx, multiples, rows, n):
     for r in sorted({0, 1, rows // 2, rows - 1}):
         want = sum(ks[p] * scalars[s] for p, s in zip(pick.tolist(), sel[r].tolist()))
         assert curve.jacobian_to_affine_py(out[r:r + 1])[0] == of_g(want), r
+
+
+@pytest.mark.parametrize("rows,n", [(2, 30), (3, 100), (300, 130), (650, 255)])
+def test_full_width_rows_of_few_buckets(ctx, multiples, rows, n):
+    """Fewer than 256 bases a row: windows of three bits, whose four buckets are one thread's."""
+    test_full_width_rows(ctx, multiples, rows, n)

@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_msm_join_items(const Xyzz* _
 }
 
 // Many items (the d_x / d_y rows of a commitment: a thousand or more (row, window) items): a block per item leaves most of
-// its additions to idle lanes.  Here `lanes` lanes (a power of two, 8 to 32) share an item.  Lane l takes `per` consecutive
+// its additions to idle lanes.  Here `lanes` lanes (a power of two, 1 to 32) share an item.  Lane l takes `per` consecutive
 // buckets: running sums give its local weighted sum A_l = sum_j (j - lo + 1) B_j and its plain sum R_l.  The item's result is
 // sum_l A_l + per * sum_{l >= 1} S_l with S_l = sum_{u >= l} R_u (a suffix scan over the item's lanes), so
 // every lane doubles its own S_l log2(per) times, adds A_l, and one tree over the lanes finishes.  The fewest lanes that still
