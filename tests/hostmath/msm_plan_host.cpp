@@ -30,3 +30,4 @@ extern "C" void zkp_rows(uint64_t n, uint32_t rows, uint32_t max_span, int k_win
   out[7] = p.slab;
 }
 extern "C" uint32_t zkp_reduce_lanes(uint32_t n_items, uint32_t half, int sm) { return reduce_lanes(n_items, half, sm); }
+extern "C" int zkp_combine_by(uint32_t rows, int w, int k_windows, int sm) { return (int)combine_by(rows, w, k_windows, sm); }

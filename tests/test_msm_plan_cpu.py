@@ -24,6 +24,7 @@ def plan(tmp_path_factory):
 
     lib.zkp_reduce_lanes.argtypes = [u32, u32, i]
     lib.zkp_reduce_lanes.restype = u32
+    lib.zkp_combine_by.argtypes = [u32, i, i, i]
 
     def call(name, n_out, *args):
         if n_out == 0:
@@ -85,3 +86,13 @@ def test_few_buckets_an_item_get_a_thread(plan, items, half):
 def test_lanes_divide_the_buckets(plan, items, half):
     lanes = plan("zkp_reduce_lanes", 0, items, half, SM)
     assert lanes in ((0,) if items < 1024 else (8, 16, 32)) and lanes <= half
+
+
+def test_who_combines_the_windows(plan):
+    host, warps, threads = 0, 1, 2
+    by = lambda rows, w, k: plan("zkp_combine_by", 0, rows, w, k, SM)  # noqa: E731
+    for rows in (1, 4, 5, 592, 593):
+        assert by(rows, 9, 1) == threads  # one window: nothing to combine
+    assert by(1, 14, 19) == by(4, 8, 4) == host
+    assert by(5, 8, 4) == by(1, 3, 2) == by(592, 3, 85) == warps
+    assert by(593, 3, 85) == threads

@@ -920,10 +920,7 @@ int msm_run(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const Fr* 
   return msm_run_rows(ctx, bases, gather, nullptr, scalars, n, rows, out_dev, stats, prep);
 }
 
-// Horner over the windows on the host, for one row or a few: a doubling is a chain of products, 0.3 us for a CPU core with
-// 64-bit limbs against 4.5 us for a GPU thread and 2.2 us for a warp, against which the two small copies and the
-// synchronisation (some 20 us) count little from a few dozen doublings on.
-constexpr uint32_t kHostCombineRows = 4, kHostCombineChain = 24;
+// Horner over the windows on the host, for one row or a few (combine_by).
 static int combine_on_host(zk_ctx* ctx, const Xyzz* window_sums, uint32_t rows, int w, int k_windows, Jacobian* out_dev) {
   static_assert(kHostCombineRows * 128 * sizeof(Xyzz) + kHostCombineRows * sizeof(Jacobian) <= kHostPointsBytes, "128 windows of two bits at most");
   Xyzz* ws = reinterpret_cast<Xyzz*>(ctx->host_points);
@@ -1167,16 +1164,18 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
       ctx->launches++;
     }
   }
-  // up to a few rows per SM the combination is one chain of doublings, which the warp-per-row form shortens; with
-  // more rows the chains overlap and a thread per row does an eighth of the work
-  const uint32_t chain = (uint32_t)w * (uint32_t)(k_windows - 1);
-  if (rows <= kHostCombineRows && chain >= kHostCombineChain) {
-    rc = combine_on_host(ctx, window_sums, rows, w, k_windows, out_dev);
-    if (rc) return rc;
-  } else if (rows <= 4u * (uint32_t)sm)
-    k_msm_combine_quads<<<rows, 32, 0, s>>>(window_sums, w, k_windows, out_dev);
-  else
-    k_msm_combine<<<(rows + 63) / 64, 64, 0, s>>>(window_sums, rows, w, k_windows, out_dev);
+  switch (combine_by(rows, w, k_windows, sm)) {
+    case Combine::kHost:
+      rc = combine_on_host(ctx, window_sums, rows, w, k_windows, out_dev);
+      if (rc) return rc;
+      break;
+    case Combine::kWarps:
+      k_msm_combine_quads<<<rows, 32, 0, s>>>(window_sums, w, k_windows, out_dev);
+      break;
+    case Combine::kThreads:
+      k_msm_combine<<<(rows + 63) / 64, 64, 0, s>>>(window_sums, rows, w, k_windows, out_dev);
+      break;
+  }
   ctx->launches += 2;
   ZK_CUDA(cudaGetLastError());
   ctx->msm_entries_sum += n_entries;

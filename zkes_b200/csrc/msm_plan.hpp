@@ -93,6 +93,21 @@ inline void reduce_shape(uint32_t n_items, uint32_t half, uint32_t* per, uint32_
   *parts = n > kReduceThreads ? n / kReduceThreads : 1;
 }
 
+// Who combines the windows of a row (sum_k 2^(W k) window k, a chain of W (windows - 1) dependent doublings).
+//   the host: up to four rows, from a few dozen doublings on.  A doubling takes a CPU core 0.3 us with 64-bit limbs, a GPU thread
+//   4.5 us and a warp 2.2 us, against which the two small copies and the synchronisation (some 20 us) count little.
+//   a warp per row: up to a few rows per SM, where the combination is one such chain (40 rows of two windows of three bits: 284 us
+//   by threads, 275 by warps; of 16 bits in six windows: 361 and 308).
+//   a thread per row: more rows, whose chains overlap while a thread does an eighth of a warp's work; and a single window, where
+//   there is no chain and a warp's tree only adds to the time (one row 169 us by a warp, 156 by a thread; 592 rows 268 and 257).
+enum class Combine { kHost, kWarps, kThreads };
+constexpr uint32_t kHostCombineRows = 4, kHostCombineChain = 24;
+inline Combine combine_by(uint32_t rows, int w, int k_windows, int sm) {
+  const uint32_t chain = (uint32_t)w * (uint32_t)(k_windows - 1);
+  if (chain == 0 || rows > 4u * (uint32_t)sm) return Combine::kThreads;
+  return rows <= kHostCombineRows && chain >= kHostCombineChain ? Combine::kHost : Combine::kWarps;
+}
+
 // Buckets of a call and the scratch of their route, laid out for the worst case: every scalar has a non-zero digit in every
 // window.  Small scalars have fewer, and the real total is checked after the count pass (entry slots are 32-bit).
 struct BucketPlan {
