@@ -31,3 +31,7 @@ extern "C" void zkp_rows(uint64_t n, uint32_t rows, uint32_t max_span, int k_win
 }
 extern "C" uint32_t zkp_reduce_lanes(uint32_t n_items, uint32_t half, int sm) { return reduce_lanes(n_items, half, sm); }
 extern "C" int zkp_combine_by(uint32_t rows, int w, int k_windows, int sm) { return (int)combine_by(rows, w, k_windows, sm); }
+extern "C" uint32_t zkp_fixup_groups(uint32_t n_buckets, uint32_t n_chunks, uint64_t longest, uint32_t seg) {
+  return fixup_groups(n_buckets, n_chunks, longest, seg);
+}
+extern "C" uint32_t zkp_chunk_entries(uint32_t n_entries, int sm) { return chunk_entries(n_entries, sm); }

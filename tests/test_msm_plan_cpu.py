@@ -24,6 +24,8 @@ def plan(tmp_path_factory):
 
     lib.zkp_reduce_lanes.argtypes = [u32, u32, i]
     lib.zkp_reduce_lanes.restype = u32
+    lib.zkp_fixup_groups.argtypes = [u32, u32, u64, u32]
+    lib.zkp_chunk_entries.argtypes = [u32, i]
     lib.zkp_combine_by.argtypes = [u32, i, i, i]
 
     def call(name, n_out, *args):
@@ -96,3 +98,16 @@ def test_who_combines_the_windows(plan):
     assert by(1, 14, 19) == by(4, 8, 4) == host
     assert by(5, 8, 4) == by(1, 3, 2) == by(592, 3, 85) == warps
     assert by(593, 3, 85) == threads
+
+
+@pytest.mark.parametrize("buckets", [1, 128, 4096, 8192])
+@pytest.mark.parametrize("n", [1, 4095, 1 << 16, 1 << 18, 3_000_000, 1 << 24])
+def test_equal_digits_are_no_long_chain(plan, buckets, n):
+    """One window of n digits that all fall into one bucket: a thread adds 64 pieces at most, as with 2^18 digits in chunks of 32
+    and a block of 128 threads, or the bucket has all the blocks that there are."""
+    seg = plan("zkp_chunk_entries", 0, n, SM)
+    chunks = (n + seg - 1) // seg
+    groups = plan("zkp_fixup_groups", 0, buckets, chunks, n, seg)
+    most = min(32, 16384 // buckets)
+    assert 1 <= groups <= most
+    assert (chunks + 1) / (128 * groups) <= 64 or groups == most

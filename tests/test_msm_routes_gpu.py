@@ -148,3 +148,17 @@ def test_full_width_rows(ctx, multiples, rows, n):
 def test_full_width_rows_of_few_buckets(ctx, multiples, rows, n):
     """Fewer than 256 bases a row: windows of three bits, whose four buckets are one thread's."""
     test_full_width_rows(ctx, multiples, rows, n)
+
+
+@pytest.mark.parametrize("n", [70_001, 1 << 18, 3_000_000])
+@pytest.mark.parametrize("top", [100, 3000])
+def test_one_hot_bucket_among_many(ctx, multiples, n, top):
+    """Digits of which nearly all are the same: the pieces of that bucket are shared by several blocks, the others' are not."""
+    ks, pts = multiples
+    rng = np.random.default_rng(n + top)
+    pick = rng.integers(0, len(ks), size=n)
+    vals = np.where(rng.random(n) < 0.99, top - 1, rng.integers(-top, top + 1, size=n))
+    per_base = np.bincount(pick, weights=vals, minlength=len(ks))
+    sc = _repeated(to_mont_array([o.fr_from_int(v) for v in range(-top, top + 1)]), vals + top)
+    got = _device_msm(ctx, _repeated(curve.affine_to_array(pts), pick), sc)
+    assert got == of_g(sum(int(v) * k for v, k in zip(per_base, ks)))

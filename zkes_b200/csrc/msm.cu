@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(128, kAccBlocks) k_msm_accumulate(const Affine
 constexpr uint32_t kFewPieces = 8;
 
 // One thread per bucket: buckets cut into at most kFewPieces pieces are summed in place; longer
-// ones are left to the warp-per-bucket kernel below (found through the `many` list).
+// ones are left to the block-per-bucket kernel below (found through the `many` list).
 __global__ void __launch_bounds__(256) k_msm_fixup_few(const uint32_t* __restrict__ offsets, uint32_t n_buckets, uint32_t seg,
                                                        Xyzz* bucket_sums, const Xyzz* heads, const Xyzz* tails,
                                                        uint32_t* many, uint32_t* n_many) {
@@ -394,82 +394,59 @@ __global__ void __launch_bounds__(kFixupThreads) k_msm_fixup(const uint32_t* __r
   }
 }
 
-// Few, long buckets (one narrow window over millions of points): one block per bucket.
-__global__ void __launch_bounds__(128) k_msm_fixup_block(const uint32_t* __restrict__ offsets, uint32_t seg,
-                                                         Xyzz* bucket_sums, const Xyzz* heads, const Xyzz* tails) {
+// Few buckets, cut into many pieces: `groups` blocks per bucket, of which those that a bucket's pieces keep busy stay (one per
+// kFixupShare pieces: uniform digits give every bucket the same, but all of them may as well lie in one bucket), each leaving a
+// partial sum; the block that finishes a bucket last adds the partial sums.
+// turn[b] == offsets[b + 1] on entry (the cursor of the scatter) counts the blocks that are through.  2^18 int8 scalars, 99 % of
+// them equal: 1299 us with a block per bucket, 412 us with up to 32 (uniform ones: 400 and 366 us).
+__device__ __forceinline__ Xyzz ld_partial(const Xyzz* p) {  // written by another block of this launch: past the L1 cache
+  const uint4* q = reinterpret_cast<const uint4*>(p);
+  Xyzz v;
+  Fq* f[4] = {&v.x, &v.y, &v.zz, &v.zzz};
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const uint4 a = __ldcg(q + 2 * i), b = __ldcg(q + 2 * i + 1);
+    f[i]->v[0] = a.x; f[i]->v[1] = a.y; f[i]->v[2] = a.z; f[i]->v[3] = a.w;
+    f[i]->v[4] = b.x; f[i]->v[5] = b.y; f[i]->v[6] = b.z; f[i]->v[7] = b.w;
+  }
+  return v;
+}
+__global__ void __launch_bounds__(128) k_msm_fixup_block(const uint32_t* __restrict__ offsets, uint32_t seg, uint32_t groups, uint32_t* turn,
+                                                         Xyzz* bucket_sums, const Xyzz* heads, const Xyzz* tails, Xyzz* partial) {
   __shared__ Xyzz sh[128];
-  const uint32_t b = blockIdx.x;
+  __shared__ bool last;
+  const uint32_t b = blockIdx.x, g = blockIdx.y;
   const uint32_t s = offsets[b], e = offsets[b + 1];
   if (e <= s) return;
   const uint32_t c0 = s / seg, c1 = (e - 1) / seg;
-  if (c0 == c1) return;
+  if (c0 == c1) return;  // the accumulation wrote this bucket directly
+  const uint32_t want = (c1 - c0) / kFixupShare + 1, share = want < groups ? want : groups;
+  if (g >= share) return;
+  // pieces: tail of chunk c0, heads of chunks c0+1 .. c1
   Xyzz acc = Xyzz::inf();
-  for (uint32_t c = c0 + threadIdx.x; c <= c1; c += blockDim.x) {
+  for (uint32_t c = c0 + g + share * threadIdx.x; c <= c1; c += share * blockDim.x) {
     const Xyzz h = ld_xyzz(c == c0 ? tails + c : heads + c);
     add_to(&acc, &h);
   }
   sh[threadIdx.x] = acc;
   __syncthreads();
-  for (uint32_t off = blockDim.x >> 1; off > 0; off >>= 1) {
-    if (threadIdx.x < off) {
-      add_to(&acc, &sh[threadIdx.x + off]);
-      sh[threadIdx.x] = acc;
+  uint32_t live = 128;  // the shares beyond the number of pieces are infinity
+  while (live > 1 && live / 2 >= (c1 - c0) / share + 1) live >>= 1;
+  tree_sum(sh, live);
+  if (share > 1) {
+    if (threadIdx.x == 0) {
+      st_xyzz(partial + (size_t)b * groups + g, sh[0]);
+      __threadfence();
+      last = atomicAdd(turn + b, 1u) == e + share - 1;
     }
     __syncthreads();
-  }
-  if (threadIdx.x == 0) st_xyzz(bucket_sums + b, acc);
-}
-
-// Very long buckets (a narrow window over millions of points, or the single bucket of an all-ones MSM): the
-// pieces of a bucket are shared by `groups` blocks, each leaving a partial sum, and a second small launch adds
-// the partial sums of every bucket.
-__global__ void __launch_bounds__(128) k_msm_fixup_groups(const uint32_t* __restrict__ offsets, uint32_t seg, uint32_t groups,
-                                                          const Xyzz* heads, const Xyzz* tails, Xyzz* partial) {
-  __shared__ Xyzz sh[128];
-  const uint32_t b = blockIdx.x, g = blockIdx.y;
-  const uint32_t s = offsets[b], e = offsets[b + 1];
-  Xyzz acc = Xyzz::inf();
-  if (e > s) {
-    const uint32_t c0 = s / seg, c1 = (e - 1) / seg;
-    if (c0 != c1)
-      for (uint32_t c = c0 + g + groups * threadIdx.x; c <= c1; c += groups * blockDim.x) {
-        const Xyzz h = ld_xyzz(c == c0 ? tails + c : heads + c);
-        add_to(&acc, &h);
-      }
-  }
-  sh[threadIdx.x] = acc;
-  __syncthreads();
-  for (uint32_t off = blockDim.x >> 1; off > 0; off >>= 1) {
-    if (threadIdx.x < off) {
-      add_to(&acc, &sh[threadIdx.x + off]);
-      sh[threadIdx.x] = acc;
-    }
+    if (!last) return;
+    __threadfence();
+    if (threadIdx.x < kFixupGroups) sh[threadIdx.x] = threadIdx.x < share ? ld_partial(partial + (size_t)b * groups + threadIdx.x) : Xyzz::inf();
     __syncthreads();
+    tree_sum(sh, kFixupGroups);
   }
-  if (threadIdx.x == 0) st_xyzz(partial + (size_t)b * groups + g, acc);
-}
-
-__global__ void __launch_bounds__(32) k_msm_fixup_groups_final(const uint32_t* __restrict__ offsets, uint32_t seg, uint32_t groups,
-                                                               const Xyzz* partial, Xyzz* bucket_sums) {
-  __shared__ Xyzz sh[32];
-  const uint32_t b = blockIdx.x;
-  const uint32_t s = offsets[b], e = offsets[b + 1];
-  if (e <= s || s / seg == (e - 1) / seg) return;  // the accumulation wrote this bucket directly
-  Xyzz acc = Xyzz::inf();
-  for (uint32_t g = threadIdx.x; g < groups; g += 32) {
-    const Xyzz h = ld_xyzz(partial + (size_t)b * groups + g);
-    add_to(&acc, &h);
-  }
-  sh[threadIdx.x] = acc;
-  __syncwarp();
-  for (int off = 16; off > 0; off >>= 1) {
-    if (threadIdx.x < (unsigned)off) {
-      add_to(&acc, &sh[threadIdx.x + off]);
-      sh[threadIdx.x] = acc;
-    }
-    __syncwarp();
-  }
-  if (threadIdx.x == 0) st_xyzz(bucket_sums + b, acc);
+  if (threadIdx.x == 0) st_xyzz(bucket_sums + b, sh[0]);
 }
 
 // sum_j (j + 1) B_j over the `half` buckets of an item, one item per (row, window).  A run of len consecutive buckets is
@@ -1132,21 +1109,14 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
     const uint32_t n_chunks = (n_entries + seg - 1) / seg;
     k_msm_accumulate<<<(n_chunks + 127) / 128, 128, 0, s>>>(bases, gather, entries, offsets, n_buckets, n_entries, seg,
                                                            n_chunks, bucket_sums, heads, tails);
-    // pieces per bucket on average; from a few hundred on, one block per bucket is a long serial chain
-    const uint32_t avg_pieces = n_chunks / n_buckets;
-    uint32_t groups = (avg_pieces + 255) / 256;
-    if (n_buckets <= kFixupPartials && groups > kFixupPartials / n_buckets) groups = kFixupPartials / n_buckets;
-    if (n_buckets <= 8192 && n_buckets <= kFixupPartials && groups >= 2) {
-      k_msm_fixup_groups<<<dim3(n_buckets, groups), 128, 0, s>>>(offsets, seg, groups, heads, tails, fix_part);
-      k_msm_fixup_groups_final<<<n_buckets, 32, 0, s>>>(offsets, seg, groups, fix_part, bucket_sums);
-      ctx->launches++;
-    } else if (n_buckets <= 8192) {
-      k_msm_fixup_block<<<n_buckets, 128, 0, s>>>(offsets, seg, bucket_sums, heads, tails);
+    // cursor[] is free again after the scatter: it stands at the ends of the buckets
+    if (n_buckets <= kFixupBuckets) {
+      const uint32_t groups = fixup_groups(n_buckets, n_chunks, row_ids ? n_entries : n, seg);
+      k_msm_fixup_block<<<dim3(n_buckets, groups), 128, 0, s>>>(offsets, seg, groups, cursor, bucket_sums, heads, tails, fix_part);
     } else {
-      // cursor[] is free again after the scatter: reuse it as the list of long buckets
       uint32_t* n_many = ctx->rs.sink.counter + 12;
       ZK_CUDA(cudaMemsetAsync(n_many, 0, 4, s));
-      k_msm_fixup_few<<<(n_buckets + 255) / 256, 256, 0, s>>>(offsets, n_buckets, seg, bucket_sums, heads, tails, cursor, n_many);
+      k_msm_fixup_few<<<(n_buckets + 255) / 256, 256, 0, s>>>(offsets, n_buckets, seg, bucket_sums, heads, tails, cursor /* the list of long buckets */, n_many);
       k_msm_fixup<<<sm * 2, kFixupThreads, 0, s>>>(offsets, cursor, n_many, seg, bucket_sums, heads, tails);
       ctx->launches++;
     }

@@ -10,7 +10,6 @@ namespace zk {
 constexpr int kCompactBits = 30;  // magnitudes below 2^30 have a compact form (k_msm_bits)
 constexpr int kAccBlocks = 4;     // blocks of 128 threads per SM of the kernels that add points in chains (126 and 122 registers)
 constexpr uint32_t kReduceThreads = 128;   // threads of a block of the bucket reduction
-constexpr uint32_t kFixupPartials = 4096;  // partial sums of the grouped fix-up (buckets x groups)
 constexpr int kRowsGroupMax = 12;          // bases a group of the subset-sum tables has at most (k_rows_*)
 constexpr size_t kAffineBytes = 64, kXyzzBytes = 128;
 
@@ -64,6 +63,16 @@ inline uint32_t chunk_entries(uint32_t n_entries, int sm) {
     seg = (n_entries + resident * waves - 1) / (resident * waves);
   }
   return (uint32_t)seg;
+}
+
+// Up to kFixupBuckets buckets, the pieces of a bucket that was cut by the chunks are added by up to kFixupGroups blocks, one per
+// kFixupShare pieces (k_msm_fixup_block).  How many a bucket can keep busy is bounded by the digits that a (row, window) has:
+// `longest` of them may all be the same one, and then a single block adds its pieces one after the other.
+constexpr uint32_t kFixupBuckets = 8192, kFixupGroups = 32, kFixupShare = 256;
+constexpr uint32_t kFixupPartials = 16384;  // partial sums (buckets x blocks)
+inline uint32_t fixup_groups(uint32_t n_buckets, uint32_t n_chunks, uint64_t longest, uint32_t seg) {
+  const uint64_t pieces = std::min<uint64_t>(n_chunks, longest / seg + 2);
+  return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>({(pieces + kFixupShare - 1) / kFixupShare, kFixupGroups, kFixupPartials / n_buckets}));
 }
 
 // Lanes per item for k_msm_bucket_reduce_rows, 0 where an item is worth a block or more of its own.  More lanes shorten the
