@@ -162,3 +162,19 @@ def test_one_hot_bucket_among_many(ctx, multiples, n, top):
     sc = _repeated(to_mont_array([o.fr_from_int(v) for v in range(-top, top + 1)]), vals + top)
     got = _device_msm(ctx, _repeated(curve.affine_to_array(pts), pick), sc)
     assert got == of_g(sum(int(v) * k for v, k in zip(per_base, ks)))
+
+
+@pytest.mark.parametrize("n,hot,share", [(3_000_000, 5000, 1.0), (3_000_000, 1500, 0.3), (3_000_000, 1200, 1.0), (200_000, 600, 0.9), (1_500_000, 40, 0.5)])
+def test_buckets_of_some_pieces(ctx, multiples, n, hot, share):
+    """Thousands of buckets of nine to twenty-four pieces (a thread each), hundreds of them (a warp each), longer ones (a block
+    each), and all kinds at once."""
+    ks, pts = multiples
+    rng = np.random.default_rng(n + hot)
+    pick = rng.integers(0, len(ks), size=n)
+    values = rng.choice(np.arange(1, 32769), size=hot, replace=False)
+    vals = np.where(rng.random(n) < share, values[rng.integers(0, hot, size=n)], rng.integers(-32768, 32769, size=n))
+    vals[0] = 32768
+    per_base = np.bincount(pick, weights=vals, minlength=len(ks))
+    sc = _repeated(to_mont_array([o.fr_from_int(v) for v in range(-32768, 32769)]), vals + 32768)
+    got = _device_msm(ctx, _repeated(curve.affine_to_array(pts), pick), sc)
+    assert got == of_g(sum(int(v) * k for v, k in zip(per_base, ks)))

@@ -320,21 +320,24 @@ __global__ void __launch_bounds__(128, kAccBlocks) k_msm_accumulate(const Affine
     st_xyzz(bucket_sums + b, acc);
 }
 
-constexpr uint32_t kFewPieces = 8;
+constexpr uint32_t kManyPieces = 24;
 
-// One thread per bucket: buckets cut into at most kFewPieces pieces are summed in place; longer
-// ones are left to the block-per-bucket kernel below (found through the `many` list).
-__global__ void __launch_bounds__(256) k_msm_fixup_few(const uint32_t* __restrict__ offsets, uint32_t n_buckets, uint32_t seg,
+// One thread per bucket: buckets cut into at most `few` pieces are summed in place.  Longer ones are listed for k_msm_fixup,
+// those of more than kManyPieces from the front of `list`, the others from its end (listed[0] and listed[1] of them).
+__global__ void __launch_bounds__(256) k_msm_fixup_few(const uint32_t* __restrict__ offsets, uint32_t n_buckets, uint32_t seg, uint32_t few,
                                                        Xyzz* bucket_sums, const Xyzz* heads, const Xyzz* tails,
-                                                       uint32_t* many, uint32_t* n_many) {
+                                                       uint32_t* list, uint32_t* listed) {
   const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n_buckets) return;
   const uint32_t s = offsets[b], e = offsets[b + 1];
   if (e <= s) return;
   const uint32_t c0 = s / seg, c1 = (e - 1) / seg;
   if (c0 == c1) return;
-  if (c1 - c0 >= kFewPieces) {
-    many[atomicAdd(n_many, 1u)] = b;
+  if (c1 - c0 >= few) {
+    if (c1 - c0 >= kManyPieces)
+      list[atomicAdd(listed, 1u)] = b;
+    else
+      list[n_buckets - 1 - atomicAdd(listed + 1, 1u)] = b;
     return;
   }
   Xyzz acc = ld_xyzz(tails + c0);
@@ -364,27 +367,63 @@ __device__ __forceinline__ void tree_sum(Xyzz* sh, uint32_t n) {
   }
 }
 
-// A listed bucket (one cut into many pieces) per block and pass: the top window of full-width scalars has a handful of
-// buckets that between them take every point, a thousand pieces each.  The time is the longest chain of dependent
-// additions: 256 threads leave pieces / 256 of them plus eight levels of a tree, where a warp per bucket left
-// pieces / 32 plus five (100003 full-width scalars: 490 us against 131 us).
+// The listed buckets.  The time is the longest chain of dependent additions.
+//   Many pieces: a bucket per block and pass.  The top window of full-width scalars has a handful of buckets that between them
+//   take every point, a thousand pieces each: 256 threads leave pieces / 256 additions plus eight levels of a tree, where a warp
+//   per bucket left pieces / 32 plus five (100003 full-width scalars: 490 us against 131 us).
+//   Up to kManyPieces: a warp each, four or five levels of a tree, while there are no more of them than warps; a thread each, a chain of
+//   up to kManyPieces additions, where uniform digits make them thousands (64 rows of 16384 int8 values: 8192 buckets of eight
+//   or nine pieces: 1089 us with a block each, 588 us).
 constexpr int kFixupThreads = 256;
-__global__ void __launch_bounds__(kFixupThreads) k_msm_fixup(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ many,
-                                                             const uint32_t* __restrict__ n_many, uint32_t seg,
+__global__ void __launch_bounds__(kFixupThreads) k_msm_fixup(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ list,
+                                                             const uint32_t* __restrict__ listed, uint32_t n_buckets, uint32_t seg,
                                                              Xyzz* bucket_sums, const Xyzz* heads, const Xyzz* tails) {
   __shared__ Xyzz sh[kFixupThreads];
-  const uint32_t total = *n_many;
-  for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
-    const uint32_t b = many[item];
+  // pieces of a bucket: tail of chunk c0, heads of chunks c0+1 .. c1; the sum of every `step`-th of them from `first` on
+  auto pieces_of = [&](uint32_t b, uint32_t* c0, uint32_t* c1) {
     const uint32_t s = offsets[b], e = offsets[b + 1];
-    const uint32_t c0 = s / seg, c1 = (e - 1) / seg;
-    // pieces: tail of chunk c0, heads of chunks c0+1 .. c1
+    *c0 = s / seg;
+    *c1 = (e - 1) / seg;
+  };
+  auto share = [&](uint32_t c0, uint32_t c1, uint32_t first, uint32_t step) {
     Xyzz acc = Xyzz::inf();
-    for (uint32_t c = c0 + threadIdx.x; c <= c1; c += kFixupThreads) {
+    for (uint32_t c = c0 + first; c <= c1; c += step) {
       const Xyzz h = ld_xyzz(c == c0 ? tails + c : heads + c);
       add_to(&acc, &h);
     }
-    sh[threadIdx.x] = acc;
+    return acc;
+  };
+  const uint32_t n_long = listed[0], n_mid = listed[1], warps = gridDim.x * (kFixupThreads / 32);
+  uint32_t c0, c1;
+  if (n_mid > warps) {
+    for (uint32_t item = threadIdx.x * gridDim.x + blockIdx.x; item < n_mid; item += gridDim.x * kFixupThreads) {
+      const uint32_t b = list[n_buckets - 1 - item];
+      pieces_of(b, &c0, &c1);
+      st_xyzz(bucket_sums + b, share(c0, c1, 0, 1));
+    }
+  } else {
+    const uint32_t item = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, lane = threadIdx.x & 31;
+    if (item < n_mid) {
+      const uint32_t b = list[n_buckets - 1 - item];
+      pieces_of(b, &c0, &c1);
+      Xyzz* mine = sh + (threadIdx.x & ~31u);
+      mine[lane] = share(c0, c1, lane, 32);
+      __syncwarp();
+      if (c1 - c0 >= 16 && lane < 16) add_to(&mine[lane], &mine[lane + 16]);
+      __syncwarp();
+#pragma unroll 1
+      for (uint32_t off = 8; off > 0; off >>= 1) {
+        const uint32_t q = lane >> 2, i = q < off ? q : 0;
+        quad_add_to(&mine[i], &mine[i + off], q < off);
+      }
+      if (lane == 0) st_xyzz(bucket_sums + b, mine[0]);
+    }
+  }
+  __syncthreads();
+  for (uint32_t item = blockIdx.x; item < n_long; item += gridDim.x) {
+    const uint32_t b = list[item];
+    pieces_of(b, &c0, &c1);
+    sh[threadIdx.x] = share(c0, c1, threadIdx.x, kFixupThreads);
     __syncthreads();
     uint32_t live = kFixupThreads;  // the shares beyond the number of pieces are infinity
     while (live > 1 && live / 2 >= c1 - c0 + 1) live >>= 1;
@@ -1114,10 +1153,10 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
       const uint32_t groups = fixup_groups(n_buckets, n_chunks, row_ids ? n_entries : n, seg);
       k_msm_fixup_block<<<dim3(n_buckets, groups), 128, 0, s>>>(offsets, seg, groups, cursor, bucket_sums, heads, tails, fix_part);
     } else {
-      uint32_t* n_many = ctx->rs.sink.counter + 12;
-      ZK_CUDA(cudaMemsetAsync(n_many, 0, 4, s));
-      k_msm_fixup_few<<<(n_buckets + 255) / 256, 256, 0, s>>>(offsets, n_buckets, seg, bucket_sums, heads, tails, cursor /* the list of long buckets */, n_many);
-      k_msm_fixup<<<sm * 2, kFixupThreads, 0, s>>>(offsets, cursor, n_many, seg, bucket_sums, heads, tails);
+      uint32_t* listed = ctx->rs.sink.counter + 12;
+      ZK_CUDA(cudaMemsetAsync(listed, 0, 8, s));
+      k_msm_fixup_few<<<(n_buckets + 255) / 256, 256, 0, s>>>(offsets, n_buckets, seg, fixup_few(seg), bucket_sums, heads, tails, cursor /* the list of long buckets */, listed);
+      k_msm_fixup<<<sm * 2, kFixupThreads, 0, s>>>(offsets, cursor, listed, n_buckets, seg, bucket_sums, heads, tails);
       ctx->launches++;
     }
     ctx->launches += 2;

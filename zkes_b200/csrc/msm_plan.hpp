@@ -75,6 +75,9 @@ inline uint32_t fixup_groups(uint32_t n_buckets, uint32_t n_chunks, uint64_t lon
   return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>({(pieces + kFixupShare - 1) / kFixupShare, kFixupGroups, kFixupPartials / n_buckets}));
 }
 
+// More buckets: a thread each adds up to this many pieces (k_msm_fixup_few): 256 entries, in pieces of the chunk's length.
+inline uint32_t fixup_few(uint32_t seg) { return std::max(8u, 256 / seg); }
+
 // Lanes per item for k_msm_bucket_reduce_rows, 0 where an item is worth a block or more of its own.  More lanes shorten the
 // chain and add work (a scan and a tree over them), so they double only until half of the threads that fit the GPU (three
 // blocks of 128 per SM) have work: 4096 items of 128 buckets lost 2 % of their commitment with sixteen lanes instead of eight.
