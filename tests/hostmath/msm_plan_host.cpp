@@ -35,4 +35,3 @@ extern "C" uint32_t zkp_fixup_groups(uint32_t n_buckets, uint32_t n_chunks, uint
   return fixup_groups(n_buckets, n_chunks, longest, seg);
 }
 extern "C" uint32_t zkp_chunk_entries(uint32_t n_entries, int sm) { return chunk_entries(n_entries, sm); }
-extern "C" uint32_t zkp_fixup_few(uint32_t seg) { return fixup_few(seg); }

@@ -25,7 +25,6 @@ def plan(tmp_path_factory):
     lib.zkp_reduce_lanes.argtypes = [u32, u32, i]
     lib.zkp_reduce_lanes.restype = u32
     lib.zkp_fixup_groups.argtypes = [u32, u32, u64, u32]
-    lib.zkp_fixup_few.argtypes = [u32]
     lib.zkp_chunk_entries.argtypes = [u32, i]
     lib.zkp_combine_by.argtypes = [u32, i, i, i]
 
@@ -109,13 +108,6 @@ def test_equal_digits_are_no_long_chain(plan, buckets, n):
     seg = plan("zkp_chunk_entries", 0, n, SM)
     chunks = (n + seg - 1) // seg
     groups = plan("zkp_fixup_groups", 0, buckets, chunks, n, seg)
-    most = min(32, 16384 // buckets)
+    most = min(128, 16384 // buckets)
     assert 1 <= groups <= most
     assert (chunks + 1) / (128 * groups) <= 64 or groups == most
-
-
-@pytest.mark.parametrize("n", [1000, 300_000, 1_000_000, 3_000_000, 1 << 24, 1 << 31])
-def test_buckets_of_256_entries_are_no_listed_ones(plan, n):
-    """The length up to which a thread adds up a bucket counts entries, not pieces, whose length follows the call's size."""
-    seg = plan("zkp_chunk_entries", 0, n, SM)
-    assert plan("zkp_fixup_few", 0, seg) >= max(8, 256 // seg)

@@ -320,24 +320,34 @@ __global__ void __launch_bounds__(128, kAccBlocks) k_msm_accumulate(const Affine
     st_xyzz(bucket_sums + b, acc);
 }
 
-constexpr uint32_t kManyPieces = 24;
+constexpr uint32_t kFewPieces = 8, kManyPieces = 24, kCrowd = 4;
 
-// One thread per bucket: buckets cut into at most `few` pieces are summed in place.  Longer ones are listed for k_msm_fixup,
-// those of more than kManyPieces from the front of `list`, the others from its end (listed[0] and listed[1] of them).
-__global__ void __launch_bounds__(256) k_msm_fixup_few(const uint32_t* __restrict__ offsets, uint32_t n_buckets, uint32_t seg, uint32_t few,
+// One thread per bucket: buckets cut into at most kFewPieces pieces are summed in place, and up to kManyPieces where kCrowd lanes
+// of a warp have such a bucket: uniform digits make them thousands, for which a chain of up to kManyPieces additions a thread is
+// the least work, while for a few of them it is the longest chain of the call (32 rows of 16384 int16 values: 104 us against
+// 38).  The others are listed for k_msm_fixup, those of more than kManyPieces from the front of `list`, the rest from its end
+// (listed[0] and listed[1] of them).
+__global__ void __launch_bounds__(256) k_msm_fixup_few(const uint32_t* __restrict__ offsets, uint32_t n_buckets, uint32_t seg,
                                                        Xyzz* bucket_sums, const Xyzz* heads, const Xyzz* tails,
                                                        uint32_t* list, uint32_t* listed) {
   const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n_buckets) return;
-  const uint32_t s = offsets[b], e = offsets[b + 1];
-  if (e <= s) return;
-  const uint32_t c0 = s / seg, c1 = (e - 1) / seg;
-  if (c0 == c1) return;
-  if (c1 - c0 >= few) {
-    if (c1 - c0 >= kManyPieces)
-      list[atomicAdd(listed, 1u)] = b;
-    else
+  uint32_t c0 = 0, c1 = 0;
+  if (b < n_buckets) {
+    const uint32_t s = offsets[b], e = offsets[b + 1];
+    if (e > s) {
+      c0 = s / seg;
+      c1 = (e - 1) / seg;
+    }
+  }
+  const uint32_t cuts = c1 - c0;
+  const bool some = cuts >= kFewPieces && cuts < kManyPieces;
+  const bool crowd = __popc(__ballot_sync(0xffffffffu, some)) >= kCrowd;
+  if (cuts == 0) return;
+  if (cuts >= kFewPieces && !(some && crowd)) {
+    if (some)
       list[n_buckets - 1 - atomicAdd(listed + 1, 1u)] = b;
+    else
+      list[atomicAdd(listed, 1u)] = b;
     return;
   }
   Xyzz acc = ld_xyzz(tails + c0);
@@ -371,9 +381,8 @@ __device__ __forceinline__ void tree_sum(Xyzz* sh, uint32_t n) {
 //   Many pieces: a bucket per block and pass.  The top window of full-width scalars has a handful of buckets that between them
 //   take every point, a thousand pieces each: 256 threads leave pieces / 256 additions plus eight levels of a tree, where a warp
 //   per bucket left pieces / 32 plus five (100003 full-width scalars: 490 us against 131 us).
-//   Up to kManyPieces: a warp each, four or five levels of a tree, while there are no more of them than warps; a thread each, a chain of
-//   up to kManyPieces additions, where uniform digits make them thousands (64 rows of 16384 int8 values: 8192 buckets of eight
-//   or nine pieces: 1089 us with a block each, 588 us).
+//   Up to kManyPieces: a warp each, four or five levels of a tree (64 rows of 16384 int8 values, 8192 buckets of eight or nine
+//   pieces: 1089 us with a block each, 579 us with what k_msm_fixup_few keeps and a warp for the rest).
 constexpr int kFixupThreads = 256;
 __global__ void __launch_bounds__(kFixupThreads) k_msm_fixup(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ list,
                                                              const uint32_t* __restrict__ listed, uint32_t n_buckets, uint32_t seg,
@@ -393,31 +402,23 @@ __global__ void __launch_bounds__(kFixupThreads) k_msm_fixup(const uint32_t* __r
     }
     return acc;
   };
-  const uint32_t n_long = listed[0], n_mid = listed[1], warps = gridDim.x * (kFixupThreads / 32);
+  const uint32_t n_long = listed[0], n_mid = listed[1], lane = threadIdx.x & 31;
   uint32_t c0, c1;
-  if (n_mid > warps) {
-    for (uint32_t item = threadIdx.x * gridDim.x + blockIdx.x; item < n_mid; item += gridDim.x * kFixupThreads) {
-      const uint32_t b = list[n_buckets - 1 - item];
-      pieces_of(b, &c0, &c1);
-      st_xyzz(bucket_sums + b, share(c0, c1, 0, 1));
-    }
-  } else {
-    const uint32_t item = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, lane = threadIdx.x & 31;
-    if (item < n_mid) {
-      const uint32_t b = list[n_buckets - 1 - item];
-      pieces_of(b, &c0, &c1);
-      Xyzz* mine = sh + (threadIdx.x & ~31u);
-      mine[lane] = share(c0, c1, lane, 32);
-      __syncwarp();
-      if (c1 - c0 >= 16 && lane < 16) add_to(&mine[lane], &mine[lane + 16]);
-      __syncwarp();
+  Xyzz* mine = sh + (threadIdx.x & ~31u);
+  for (uint32_t item = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; item < n_mid; item += gridDim.x * (kFixupThreads / 32)) {
+    const uint32_t b = list[n_buckets - 1 - item];
+    pieces_of(b, &c0, &c1);
+    mine[lane] = share(c0, c1, lane, 32);
+    __syncwarp();
+    if (c1 - c0 >= 16 && lane < 16) add_to(&mine[lane], &mine[lane + 16]);
+    __syncwarp();
 #pragma unroll 1
-      for (uint32_t off = 8; off > 0; off >>= 1) {
-        const uint32_t q = lane >> 2, i = q < off ? q : 0;
-        quad_add_to(&mine[i], &mine[i + off], q < off);
-      }
-      if (lane == 0) st_xyzz(bucket_sums + b, mine[0]);
+    for (uint32_t off = 8; off > 0; off >>= 1) {
+      const uint32_t q = lane >> 2, i = q < off ? q : 0;
+      quad_add_to(&mine[i], &mine[i + off], q < off);
     }
+    if (lane == 0) st_xyzz(bucket_sums + b, mine[0]);
+    __syncwarp();
   }
   __syncthreads();
   for (uint32_t item = blockIdx.x; item < n_long; item += gridDim.x) {
@@ -437,7 +438,7 @@ __global__ void __launch_bounds__(kFixupThreads) k_msm_fixup(const uint32_t* __r
 // kFixupShare pieces: uniform digits give every bucket the same, but all of them may as well lie in one bucket), each leaving a
 // partial sum; the block that finishes a bucket last adds the partial sums.
 // turn[b] == offsets[b + 1] on entry (the cursor of the scatter) counts the blocks that are through.  2^18 int8 scalars, 99 % of
-// them equal: 1299 us with a block per bucket, 412 us with up to 32 (uniform ones: 400 and 366 us).
+// them equal: 1299 us with a block per bucket, 408 us with up to 128 (uniform ones: 404 and 377 us).
 __device__ __forceinline__ Xyzz ld_partial(const Xyzz* p) {  // written by another block of this launch: past the L1 cache
   const uint4* q = reinterpret_cast<const uint4*>(p);
   Xyzz v;
@@ -1155,7 +1156,7 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
     } else {
       uint32_t* listed = ctx->rs.sink.counter + 12;
       ZK_CUDA(cudaMemsetAsync(listed, 0, 8, s));
-      k_msm_fixup_few<<<(n_buckets + 255) / 256, 256, 0, s>>>(offsets, n_buckets, seg, fixup_few(seg), bucket_sums, heads, tails, cursor /* the list of long buckets */, listed);
+      k_msm_fixup_few<<<(n_buckets + 255) / 256, 256, 0, s>>>(offsets, n_buckets, seg, bucket_sums, heads, tails, cursor /* the list of long buckets */, listed);
       k_msm_fixup<<<sm * 2, kFixupThreads, 0, s>>>(offsets, cursor, listed, n_buckets, seg, bucket_sums, heads, tails);
       ctx->launches++;
     }

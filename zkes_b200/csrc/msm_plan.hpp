@@ -68,15 +68,12 @@ inline uint32_t chunk_entries(uint32_t n_entries, int sm) {
 // Up to kFixupBuckets buckets, the pieces of a bucket that was cut by the chunks are added by up to kFixupGroups blocks, one per
 // kFixupShare pieces (k_msm_fixup_block).  How many a bucket can keep busy is bounded by the digits that a (row, window) has:
 // `longest` of them may all be the same one, and then a single block adds its pieces one after the other.
-constexpr uint32_t kFixupBuckets = 8192, kFixupGroups = 32, kFixupShare = 256;
+constexpr uint32_t kFixupBuckets = 8192, kFixupGroups = 128, kFixupShare = 256;
 constexpr uint32_t kFixupPartials = 16384;  // partial sums (buckets x blocks)
 inline uint32_t fixup_groups(uint32_t n_buckets, uint32_t n_chunks, uint64_t longest, uint32_t seg) {
   const uint64_t pieces = std::min<uint64_t>(n_chunks, longest / seg + 2);
   return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>({(pieces + kFixupShare - 1) / kFixupShare, kFixupGroups, kFixupPartials / n_buckets}));
 }
-
-// More buckets: a thread each adds up to this many pieces (k_msm_fixup_few): 256 entries, in pieces of the chunk's length.
-inline uint32_t fixup_few(uint32_t seg) { return std::max(8u, 256 / seg); }
 
 // Lanes per item for k_msm_bucket_reduce_rows, 0 where an item is worth a block or more of its own.  More lanes shorten the
 // chain and add work (a scan and a tree over them), so they double only until half of the threads that fit the GPU (three
