@@ -320,14 +320,15 @@ __global__ void __launch_bounds__(128, kAccBlocks) k_msm_accumulate(const Affine
     st_xyzz(bucket_sums + b, acc);
 }
 
-constexpr uint32_t kFewPieces = 8, kManyPieces = 24, kCrowd = 4;
+constexpr uint32_t kFewPieces = 8, kManyPieces = 24;
+constexpr int kFixupThreads = 256;
 
-// One thread per bucket: buckets cut into at most kFewPieces pieces are summed in place, and up to kManyPieces where kCrowd lanes
-// of a warp have such a bucket: uniform digits make them thousands, for which a chain of up to kManyPieces additions a thread is
-// the least work, while for a few of them it is the longest chain of the call (32 rows of 16384 int16 values: 104 us against
-// 38).  The others are listed for k_msm_fixup, those of more than kManyPieces from the front of `list`, the rest from its end
+// One thread per bucket: buckets cut into at most kFewPieces pieces are summed in place, and up to kManyPieces where `crowd` lanes
+// of a warp have such a bucket: uniform digits can make them thousands, for which a chain of up to kManyPieces additions a thread
+// is the least work, while for a few of them it is the longest chain of the call (32 rows of 16384 int16 values: 104 us against
+// 38).  crowd is 4 where the chunks are enough for more such buckets than k_msm_fixup has warps, else beyond reach.  The others are listed for k_msm_fixup, those of more than kManyPieces from the front of `list`, the rest from its end
 // (listed[0] and listed[1] of them).
-__global__ void __launch_bounds__(256) k_msm_fixup_few(const uint32_t* __restrict__ offsets, uint32_t n_buckets, uint32_t seg,
+__global__ void __launch_bounds__(256) k_msm_fixup_few(const uint32_t* __restrict__ offsets, uint32_t n_buckets, uint32_t seg, int crowd,
                                                        Xyzz* bucket_sums, const Xyzz* heads, const Xyzz* tails,
                                                        uint32_t* list, uint32_t* listed) {
   const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -341,9 +342,9 @@ __global__ void __launch_bounds__(256) k_msm_fixup_few(const uint32_t* __restric
   }
   const uint32_t cuts = c1 - c0;
   const bool some = cuts >= kFewPieces && cuts < kManyPieces;
-  const bool crowd = __popc(__ballot_sync(0xffffffffu, some)) >= kCrowd;
+  const bool crowded = __popc(__ballot_sync(0xffffffffu, some)) >= crowd;
   if (cuts == 0) return;
-  if (cuts >= kFewPieces && !(some && crowd)) {
+  if (cuts >= kFewPieces && !(some && crowded)) {
     if (some)
       list[n_buckets - 1 - atomicAdd(listed + 1, 1u)] = b;
     else
@@ -383,8 +384,7 @@ __device__ __forceinline__ void tree_sum(Xyzz* sh, uint32_t n) {
 //   per bucket left pieces / 32 plus five (100003 full-width scalars: 490 us against 131 us).
 //   Up to kManyPieces: a warp each, four or five levels of a tree (64 rows of 16384 int8 values, 8192 buckets of eight or nine
 //   pieces: 1089 us with a block each, 579 us with what k_msm_fixup_few keeps and a warp for the rest).
-constexpr int kFixupThreads = 256;
-__global__ void __launch_bounds__(kFixupThreads) k_msm_fixup(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ list,
+__global__ void __launch_bounds__(kFixupThreads, 2) k_msm_fixup(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ list,
                                                              const uint32_t* __restrict__ listed, uint32_t n_buckets, uint32_t seg,
                                                              Xyzz* bucket_sums, const Xyzz* heads, const Xyzz* tails) {
   __shared__ Xyzz sh[kFixupThreads];
@@ -1156,7 +1156,8 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
     } else {
       uint32_t* listed = ctx->rs.sink.counter + 12;
       ZK_CUDA(cudaMemsetAsync(listed, 0, 8, s));
-      k_msm_fixup_few<<<(n_buckets + 255) / 256, 256, 0, s>>>(offsets, n_buckets, seg, bucket_sums, heads, tails, cursor /* the list of long buckets */, listed);
+      const int crowd = n_chunks > kFewPieces * 2u * (uint32_t)sm * (kFixupThreads / 32) ? 4 : 33;
+      k_msm_fixup_few<<<(n_buckets + 255) / 256, 256, 0, s>>>(offsets, n_buckets, seg, crowd, bucket_sums, heads, tails, cursor /* the list of long buckets */, listed);
       k_msm_fixup<<<sm * 2, kFixupThreads, 0, s>>>(offsets, cursor, listed, n_buckets, seg, bucket_sums, heads, tails);
       ctx->launches++;
     }
