@@ -17,9 +17,9 @@ extern "C" void zkp_windows(uint64_t n, uint32_t rows, uint32_t max_mag, uint64_
   out[1] = (uint64_t)windows_for(max_mag, w);
 }
 // out: group, planes, groups, seg, parts, scratch bytes, partial sums, chains held at a time
-extern "C" void zkp_rows(uint64_t n, uint32_t rows, uint32_t max_span, int k_windows, uint32_t half, int sm, uint64_t max_scratch,
+extern "C" void zkp_rows(uint64_t n, uint32_t rows, uint32_t max_span, uint64_t nonzero, int w, int k_windows, int sm, uint64_t max_scratch,
                          uint64_t* out) {
-  const RowsPlan p = rows_plan(n, rows, max_span, k_windows, half, sm, max_scratch);
+  const RowsPlan p = rows_plan(n, rows, max_span, nonzero, bucket_plan(n * rows, rows, w, k_windows, sm), sm, max_scratch);
   out[0] = (uint64_t)p.group;
   out[1] = (uint64_t)p.planes;
   out[2] = p.groups;

@@ -20,7 +20,7 @@ def plan(tmp_path_factory):
     u64, u32, i = ctypes.c_uint64, ctypes.c_uint32, ctypes.c_int
     lib.zkp_buckets.argtypes = [u64, u32, i, i, i, ctypes.c_void_p]
     lib.zkp_windows.argtypes = [u64, u32, u32, ctypes.c_void_p]
-    lib.zkp_rows.argtypes = [u64, u32, u32, i, u32, i, u64, ctypes.c_void_p]
+    lib.zkp_rows.argtypes = [u64, u32, u32, u64, i, i, i, u64, ctypes.c_void_p]
 
     lib.zkp_reduce_lanes.argtypes = [u32, u32, i]
     lib.zkp_reduce_lanes.restype = u32
@@ -52,7 +52,7 @@ def test_subset_tables_take_no_more_scratch_than_buckets(plan, rows, n, kind):
     span, w, k, buckets, scratch = shapes(plan, rows, n, kind)
     if buckets >= 1 << 31:
         scratch = (1 << 64) - 1
-    group, _, _, _, parts, need, pieces, slab = plan("zkp_rows", 8, n, rows, span, k, 1 << (w - 1), SM, scratch)
+    group, _, _, _, parts, need, pieces, slab = plan("zkp_rows", 8, n, rows, span, n * rows, w, k, SM, scratch)
     assert need <= max(scratch, FREE_SCRATCH) or not group
     assert pieces < 1 << 31
     assert 1 <= slab <= parts or not group
@@ -61,19 +61,43 @@ def test_subset_tables_take_no_more_scratch_than_buckets(plan, rows, n, kind):
 def test_tables_by_slabs(plan):
     """2^20 columns in 1024 rows of int8 values: 9 GB of tables at once, made in slabs that fit the buckets' 4.6 GB."""
     span, w, k, _, scratch = shapes(plan, 1024, 1 << 20, "int8")
-    at_once = plan("zkp_rows", 8, 1 << 20, 1024, span, k, 1 << (w - 1), SM, 1 << 60)
-    held = plan("zkp_rows", 8, 1 << 20, 1024, span, k, 1 << (w - 1), SM, scratch)
+    at_once = plan("zkp_rows", 8, 1 << 20, 1024, span, 1 << 30, w, k, SM, 1 << 60)
+    held = plan("zkp_rows", 8, 1 << 20, 1024, span, 1 << 30, w, k, SM, scratch)
     assert at_once[7] == at_once[4] and at_once[5] > scratch
     assert held[:5] == at_once[:5] and 1 <= held[7] < held[4] and held[5] <= scratch
 
 
 def test_chains_cover_every_group(plan):
-    for rows, n, kind in [(4096, 4096, "int8"), (1024, 1024, "int8"), (3000, 777, "int16"), (100, 5000, "bit"), (5, 6, "int8")]:
+    for rows, n, kind in [(4096, 4096, "int8"), (1024, 1024, "int8"), (3000, 777, "int16"), (1000, 5000, "bit"), (50, 6, "int8")]:
         span, w, k, _, _ = shapes(plan, rows, n, kind)
-        group, planes, groups, seg, parts = plan("zkp_rows", 8, n, rows, span, k, 1 << (w - 1), SM, 1 << 60)[:5]
-        if group:
-            assert (groups - 1) * group < n <= groups * group
-            assert (parts - 1) * seg < groups <= parts * seg
+        group, planes, groups, seg, parts = plan("zkp_rows", 8, n, rows, span, n * rows, w, k, SM, 1 << 60)[:5]
+        assert group
+        assert (groups - 1) * group < n <= groups * group
+        assert (parts - 1) * seg < groups <= parts * seg
+
+
+# rows, columns, kind, share of zeros, subset sums: measured, both ways at least a tenth apart
+ROUTES = [
+    (4096, 4096, "int8", 0, True),     # 2.63 ms by sums, 4.06 by buckets
+    (4096, 4096, "int8", .9, False),   # 2.61, 1.79
+    (4096, 4096, "int16", .9, False),  # 4.27, 3.09
+    (4096, 4096, "bit", 0, True),      # 1.11, 2.75
+    (1024, 512, "int8", 0, True),      # 0.38, 0.59
+    (4096, 8, "int16", 0, True),       # 0.33, 0.41
+    (4096, 8, "int16", .995, True),    # 0.32, 2.26: hundreds of empty buckets between two entries
+    (16, 16384, "bit", 0, False),      # 0.62, 0.29
+    (16, 16384, "sign", .75, False),
+    (4, 65536, "minus", .9, False),    # 2.71, 0.26
+    (2, 65536, "int8", 0, False),
+    (16, 16384, "int8", 0, False),     # 0.67, 0.43
+]
+
+
+@pytest.mark.parametrize("rows,n,kind,zeros,sums", ROUTES)
+def test_rows_take_the_faster_route(plan, rows, n, kind, zeros, sums):
+    span, w, k, _, scratch = shapes(plan, rows, n, kind)
+    nonzero = int(rows * n * (1 - zeros) * {"bit": .5, "minus": .5, "sign": 2 / 3}.get(kind, 1))
+    assert (plan("zkp_rows", 8, n, rows, span, nonzero, w, k, SM, scratch)[0] > 0) == sums
 
 
 @pytest.mark.parametrize("half", [2, 4])

@@ -57,16 +57,25 @@ __device__ __forceinline__ int bit_length(const uint32_t (&mag)[8]) {
 // these 4 bytes instead of converting the 32-byte Montgomery value again.
 constexpr int32_t kNotCompact = INT32_MIN;
 
-// max_out[0]: largest bit length; among the scalars below 2^32 max_out[1]: largest magnitude, max_out[2]: largest of v and
-// -v - 1, whose bit length is that of the two's complement form without its sign.
-__global__ void k_msm_bits(const Fr* __restrict__ scalars, uint64_t total, unsigned int* max_out, int32_t* compact) {
+// bits: largest bit length; among the scalars below 2^32 mag: largest magnitude, span: largest of v and
+// -v - 1, whose bit length is that of the two's complement form without its sign.  nonzero: how many are not zero.
+struct MsmBits {
+  unsigned int bits, mag, span, pad;
+  unsigned long long nonzero;
+};
+__global__ void k_msm_bits(const Fr* __restrict__ scalars, uint64_t total, MsmBits* found, int32_t* compact) {
+  __shared__ unsigned int s_found[4];
+  if (threadIdx.x < 4) s_found[threadIdx.x] = 0;
+  __syncthreads();
   int best = 0;
+  uint32_t nonzero = 0;
   uint32_t best_mag = 0, best_span = 0;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
     uint32_t mag[8];
     const bool negv = fold_scalar(ld_scalar(scalars + i), mag);
     const int b = bit_length(mag);
     best = b > best ? b : best;
+    nonzero += b != 0;
     if (b <= 32) {
       best_mag = mag[0] > best_mag ? mag[0] : best_mag;
       const uint32_t span = negv && mag[0] ? mag[0] - 1 : mag[0];
@@ -82,11 +91,21 @@ __global__ void k_msm_bits(const Fr* __restrict__ scalars, uint64_t total, unsig
     best_mag = m > best_mag ? m : best_mag;
     const uint32_t p = __shfl_down_sync(0xffffffffu, best_span, off);
     best_span = p > best_span ? p : best_span;
+    nonzero += __shfl_down_sync(0xffffffffu, nonzero, off);
   }
+  // one set of global atomics a block: with one a warp they were a third of the time of a small call's pass
   if ((threadIdx.x & 31) == 0 && best) {
-    atomicMax(max_out, (unsigned int)best);
-    atomicMax(max_out + 1, best_mag);
-    atomicMax(max_out + 2, best_span);
+    atomicMax(&s_found[0], (unsigned int)best);
+    atomicMax(&s_found[1], best_mag);
+    atomicMax(&s_found[2], best_span);
+    atomicAdd(&s_found[3], nonzero);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && s_found[0]) {
+    atomicMax(&found->bits, s_found[0]);
+    atomicMax(&found->mag, s_found[1]);
+    atomicMax(&found->span, s_found[2]);
+    atomicAdd(&found->nonzero, (unsigned long long)s_found[3]);
   }
 }
 
@@ -1021,40 +1040,31 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
   if (n >= (1ull << 31)) return fail(-1, "msm: at most 2^31 - 1 points per row");
   // ---- pass 1: scalar magnitude (and the compact form of small scalars); a caller that runs several
   // MSMs over the same scalars passes `prep` and the pass runs once
-  unsigned int max_bits = 0;
-  uint32_t max_mag = 0, max_span = 0;
-  const int32_t* compact = nullptr;
-  if (prep && prep->valid && prep->scalars == scalars && prep->total == total) {
-    max_bits = prep->max_bits;
-    max_mag = prep->max_mag;
-    max_span = prep->max_span;
-    compact = prep->compact;
-  } else {
-    unsigned int* d_bits = ctx->rs.sink.counter + 8;  // spare words of the context's counter block
+  MsmPrep own;
+  if (!prep) prep = &own;
+  if (!(prep->valid && prep->scalars == scalars && prep->total == total)) {
+    MsmBits* d_found = reinterpret_cast<MsmBits*>(ctx->rs.sink.counter + 8);  // spare words of the context's counter block
     int32_t* cbuf = nullptr;
     int crc = ctx->reserve_cmp(total * 4 + 256, (void**)&cbuf);
     if (crc) return crc;
-    ZK_CUDA(cudaMemsetAsync(d_bits, 0, 12, s));
-    k_msm_bits<<<sm * 8, 256, 0, s>>>(scalars, total, d_bits, cbuf);
+    ZK_CUDA(cudaMemsetAsync(d_found, 0, sizeof(MsmBits), s));
+    k_msm_bits<<<sm * 8, 256, 0, s>>>(scalars, total, d_found, cbuf);
     ctx->launches++;
-    ZK_CUDA(cudaMemcpyAsync(ctx->host_small, d_bits, 12, cudaMemcpyDeviceToHost, s));
+    ZK_CUDA(cudaMemcpyAsync(ctx->host_small, d_found, sizeof(MsmBits), cudaMemcpyDeviceToHost, s));
     ZK_CUDA(cudaStreamSynchronize(s));
-    unsigned int found[3];
-    memcpy(found, ctx->host_small, 12);
-    max_bits = found[0];
-    max_mag = found[1];
-    max_span = found[2];
-    if (max_bits <= (unsigned)kCompactBits) compact = cbuf;
-    if (prep) {
-      prep->valid = true;
-      prep->scalars = scalars;
-      prep->total = total;
-      prep->max_bits = max_bits;
-      prep->max_mag = max_mag;
-      prep->max_span = max_span;
-      prep->compact = compact;
-    }
+    MsmBits found;
+    memcpy(&found, ctx->host_small, sizeof(found));
+    prep->valid = true;
+    prep->scalars = scalars;
+    prep->total = total;
+    prep->max_bits = found.bits;
+    prep->max_mag = found.mag;
+    prep->max_span = found.span;
+    prep->nonzero = found.nonzero;
+    prep->compact = found.bits <= (unsigned)kCompactBits ? cbuf : nullptr;
   }
+  const unsigned int max_bits = prep->max_bits;
+  const int32_t* compact = prep->compact;
   if (max_bits == 0) {
     k_set_infinity<<<(rows + 127) / 128, 128, 0, s>>>(out_dev, rows);
     ctx->launches++;
@@ -1063,14 +1073,14 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
   const int w = pick_window(row_ids ? (n / rows ? n / rows : 1) : n, rows, (int)max_bits);
   // small scalars: the exact largest magnitude is known, which can save the window that would only
   // hold carries (int8 values reach 128 = one 8-bit signed digit)
-  const int k_windows = compact ? windows_for(max_mag, w) : ((int)max_bits + 1 + w - 1) / w;
+  const int k_windows = compact ? windows_for(prep->max_mag, w) : ((int)max_bits + 1 + w - 1) / w;
   const BucketPlan plan = bucket_plan(total, rows, w, k_windows, sm);
   const uint32_t half = plan.half;
   const bool too_many = plan.n_buckets >= (1ull << 31);
   const uint32_t n_buckets = (uint32_t)plan.n_buckets;
   const size_t scan_bytes = too_many ? 0 : align256(scan_scratch_elems(n_buckets + 1) * 4);
   if (compact && rows > 1 && !row_ids && !gather) {
-    const RowsPlan by_sums = rows_plan(n, rows, max_span, k_windows, half, sm, too_many ? ~(size_t)0 : plan.scratch + scan_bytes);
+    const RowsPlan by_sums = rows_plan(n, rows, prep->max_span, prep->nonzero, plan, sm, too_many ? ~(size_t)0 : plan.scratch + scan_bytes);
     if (by_sums.group) {
       const int rc = rows_run(ctx, bases, compact, (uint32_t)n, rows, by_sums, out_dev, stats, (int)max_bits);
       if (rc != -2 /*ZK_ERR_OOM*/) return rc;  // no room for the tables: the buckets of a small call may still have it

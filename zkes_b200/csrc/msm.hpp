@@ -22,6 +22,7 @@ struct MsmPrep {
   unsigned max_bits = 0;
   uint32_t max_mag = 0;            // exact largest magnitude when max_bits <= 32
   uint32_t max_span = 0;           // then also the largest of v and -v - 1
+  uint64_t nonzero = 0;            // scalars that are not zero
   const int32_t* compact = nullptr;  // signed 32-bit form of every scalar, or NULL when some do not fit
 };
 

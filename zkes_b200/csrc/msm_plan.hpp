@@ -2,6 +2,7 @@
 // arithmetic on sizes alone, without CUDA, so that it can be checked on a machine without a GPU.
 #pragma once
 #include <algorithm>
+#include <cmath>
 #include <cstddef>
 #include <cstdint>
 
@@ -193,12 +194,52 @@ inline void rows_sizes(RowsPlan* p, uint32_t rows, uint32_t slab) {
 // max_scratch: what the buckets' route would take.  Above kRowsScratch the tables never take more than that: they are made for
 // as many chains at a time as fit (2^20 columns in 1024 rows of int8 values: 9 GB at once, 4.6 GB of buckets).
 constexpr size_t kRowsScratch = 256ull << 20;
-inline RowsPlan rows_plan(uint64_t n, uint32_t rows, uint32_t max_span, int k_windows, uint32_t half, int sm, size_t max_scratch) {
+
+// Microseconds of the two routes beyond what they share (the pass over the scalars and its read-back), from the times of their
+// kernels at 148 SMs.  Both have parts that are rates and parts that are chains of dependent additions, 4.8 us each, which small
+// calls and few rows never get below: counting additions alone sent 16 rows of 16384 bits to the sums (613 us, 385 by buckets)
+// and took no account of zeros, which have no digits (4096 rows of 4096 int8 values, nine in ten of them zero: 2609 and 1786 us).
+// Over 4366 shapes (2 to 16384 rows of 8 to 65536 values of 1 to 24 bits, none to 99.5 % of them zero) the route taken is 0.7 %
+// slower than the better one on average (geometric mean), where the count of additions was 12 % slower and up to ten times.
+inline double buckets_us(const BucketPlan& b, uint32_t rows, uint64_t nonzero, uint64_t total, int sm) {
+  const double resident = (double)sm * kAccBlocks * 128, items = (double)rows * b.k_windows, nb = (double)b.n_buckets;
+  const double entries = std::max(1.0, (double)nonzero * b.k_windows), seg = std::max((double)kChunkMin, entries / resident);
+  double t = 60 + 24e-6 * (double)total * b.k_windows;  // counting, scan, scatter, a second read-back
+  // accumulation: chains of seg entries, on which a thread also passes over the empty buckets between its entries
+  const double chunks = std::max(1.0, entries / kChunkMin);
+  const double walk = nb > entries ? 0.15 * nb / chunks * (1 + std::log(std::min(32.0, chunks))) : 0;
+  t += std::max(4.8 * std::min(seg, entries) + walk, 0.166e-3 * entries);
+  t += b.n_buckets <= kFixupBuckets ? 6 + 0.014 * std::min(nb, entries / 8) : 30 + 0.5e-3 * std::min(nb, 8 * entries / seg);
+  const uint32_t lanes = reduce_lanes((uint32_t)items, b.half, sm);
+  if (lanes) {
+    const double per = (double)b.half / lanes, steps = 2 * per + 2 * std::log2(lanes) + (lanes > 1 ? std::log2(per) + 1 : 0);
+    t += steps * std::max(lanes > 1 ? 5.0 : 8.0, 0.3e-3 * items * lanes);
+  } else {
+    t += std::max(60 + 0.1 * items + 4 * std::log2(b.half), 0.75e-3 * nb);
+  }
+  const double chain = b.w * (b.k_windows - 1);
+  if (chain > 0) t += rows <= 4u * (uint32_t)sm ? 20 + 1.6 * chain + 0.03 * rows : 15 + 5 * chain;
+  return t;
+}
+
+inline double sums_us(const RowsPlan& p, uint32_t rows, uint64_t nonzero, uint64_t total) {
+  const int s = p.group;
+  const double units = (double)rows * p.planes, groups = p.groups, table = std::ldexp(groups, s);
+  const double halves = groups * (std::ldexp(1.0, (s + 1) / 2) + std::ldexp(1.0, s / 2));
+  // a warp adds where any of the rows that its 32 units belong to has a scalar that is not zero
+  const double busy = 1 - std::pow(1 - (double)nonzero / (double)total, s * std::max(1.0, 32.0 / p.planes));
+  double t = 0.004e-3 * (double)total + std::max(21 + 2.2 * s, 1.4e-3 * halves) + std::max(50.0, 0.174e-3 * table);
+  t += std::max(4.8 * p.seg * busy, 0.156e-3 * units * groups * busy) + 0.004e-3 * units * groups;
+  if (p.parts > 1) t += std::max(8 + 1.85 * p.parts, 0.3e-3 * p.parts * units);
+  return t + 11.3 * (p.planes - 1);
+}
+
+// The shape with the fewest additions whose scratch fits, if it is faster than the buckets b.
+inline RowsPlan rows_plan(uint64_t n, uint32_t rows, uint32_t max_span, uint64_t nonzero, const BucketPlan& b, int sm, size_t max_scratch) {
   RowsPlan best;
   int planes = 1;
   while (planes < 32 && (max_span >> (planes - 1))) planes++;
-  // additions a row by buckets: one an entry, and two per bucket in general coordinates (14 products to 10)
-  double least = (double)rows * k_windows * ((double)n + 2.8 * half);
+  double least = 1e300;
   const uint64_t units = (uint64_t)rows * planes;
   if (units >= (1ull << 31)) return best;
   for (int s = 2; s <= kRowsGroupMax; s++) {
@@ -223,6 +264,8 @@ inline RowsPlan rows_plan(uint64_t n, uint32_t rows, uint32_t max_span, int k_wi
     least = cost;
     best = p;
   }
+  if (best.group && b.n_buckets < (1ull << 31) && sums_us(best, rows, nonzero, n * rows) >= buckets_us(b, rows, nonzero, n * rows, sm))
+    return RowsPlan();
   return best;
 }
 
