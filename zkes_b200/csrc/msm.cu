@@ -16,6 +16,7 @@
 #include "msm.hpp"
 #include "msm_plan.hpp"
 
+#include <algorithm>
 #include "reduce.cuh"
 #include "batch_affine.cuh"
 #include "quad.cuh"
@@ -342,32 +343,25 @@ __global__ void __launch_bounds__(128, kAccBlocks) k_msm_accumulate(const Affine
 constexpr uint32_t kFewPieces = 8, kManyPieces = 24;
 constexpr int kFixupThreads = 256;
 
-// One thread per bucket: buckets cut into at most kFewPieces pieces are summed in place, and up to kManyPieces where `crowd` lanes
-// of a warp have such a bucket: uniform digits can make them thousands, for which a chain of up to kManyPieces additions a thread
-// is the least work, while for a few of them it is the longest chain of the call (32 rows of 16384 int16 values: 104 us against
-// 38).  crowd is 4 where the chunks are enough for more such buckets than k_msm_fixup has warps, else beyond reach.  The others are listed for k_msm_fixup, those of more than kManyPieces from the front of `list`, the rest from its end
-// (listed[0] and listed[1] of them).
-__global__ void __launch_bounds__(256) k_msm_fixup_few(const uint32_t* __restrict__ offsets, uint32_t n_buckets, uint32_t seg, int crowd,
+// One thread per bucket: buckets cut into at most `few` pieces are summed in place.  The others are listed for k_msm_fixup, those of
+// more than kManyPieces from the front of `list`, the rest from its end (listed[0] and listed[1] of them).
+// few is kManyPieces where there are more buckets of that kind than k_msm_fixup has warps (k_total64 counts them): a chain of that
+// many additions a thread is then the least work.  Else it is kFewPieces: for some of them it would be the longest chain of the
+// call (65536 scalars of 64 bits, whose top window has 256 buckets of sixteen pieces: 681 us against 537).
+__global__ void __launch_bounds__(256) k_msm_fixup_few(const uint32_t* __restrict__ offsets, uint32_t n_buckets, uint32_t seg, uint32_t few,
                                                        Xyzz* bucket_sums, const Xyzz* heads, const Xyzz* tails,
                                                        uint32_t* list, uint32_t* listed) {
   const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t c0 = 0, c1 = 0;
-  if (b < n_buckets) {
-    const uint32_t s = offsets[b], e = offsets[b + 1];
-    if (e > s) {
-      c0 = s / seg;
-      c1 = (e - 1) / seg;
-    }
-  }
-  const uint32_t cuts = c1 - c0;
-  const bool some = cuts >= kFewPieces && cuts < kManyPieces;
-  const bool crowded = __popc(__ballot_sync(0xffffffffu, some)) >= crowd;
-  if (cuts == 0) return;
-  if (cuts >= kFewPieces && !(some && crowded)) {
-    if (some)
-      list[n_buckets - 1 - atomicAdd(listed + 1, 1u)] = b;
-    else
+  if (b >= n_buckets) return;
+  const uint32_t s = offsets[b], e = offsets[b + 1];
+  if (e <= s) return;
+  const uint32_t c0 = s / seg, c1 = (e - 1) / seg;
+  if (c0 == c1) return;
+  if (c1 - c0 >= few) {
+    if (c1 - c0 >= kManyPieces)
       list[atomicAdd(listed, 1u)] = b;
+    else
+      list[n_buckets - 1 - atomicAdd(listed + 1, 1u)] = b;
     return;
   }
   Xyzz acc = ld_xyzz(tails + c0);
@@ -702,13 +696,29 @@ __global__ void __launch_bounds__(32) k_msm_combine_quads(const Xyzz* __restrict
   if (lane == 0) out[blockIdx.x] = to_jacobian(sh[0]);
 }
 
-// 64-bit total of the per-bucket counts (the 32-bit prefix sums would wrap silently past 2^32).
-__global__ void k_total64(const uint32_t* __restrict__ counts, uint32_t n, unsigned long long* total) {
+// 64-bit total of the per-bucket counts (the 32-bit prefix sums would wrap silently past 2^32), and how many of them lie in
+// [from, to).
+struct BucketCounts {
+  unsigned long long total;
+  unsigned int within;
+};
+__global__ void k_total64(const uint32_t* __restrict__ counts, uint32_t n, uint32_t from, uint32_t to, BucketCounts* found) {
   unsigned long long s = 0;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s += counts[i];
+  uint32_t within = 0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t c = counts[i];
+    s += c;
+    within += c >= from && c < to;
+  }
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-  if ((threadIdx.x & 31) == 0 && s) atomicAdd(total, s);
+  for (int off = 16; off > 0; off >>= 1) {
+    s += __shfl_down_sync(0xffffffffu, s, off);
+    within += __shfl_down_sync(0xffffffffu, within, off);
+  }
+  if ((threadIdx.x & 31) == 0 && s) {
+    atomicAdd(&found->total, s);
+    if (within) atomicAdd(&found->within, within);
+  }
 }
 
 __global__ void k_set_infinity(Jacobian* out, uint32_t rows) {
@@ -1124,14 +1134,16 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
       k_msm_digits<0, false><<<sm * 8, 256, 0, s>>>(scalars, compact, row_ids, n, rows, w, k_windows, offsets, nullptr);
   }
   ctx->launches++;
-  unsigned long long* d_total = reinterpret_cast<unsigned long long*>(ctx->rs.sink.counter + 10);
-  ZK_CUDA(cudaMemsetAsync(d_total, 0, 8, s));
-  k_total64<<<sm * 4, 256, 0, s>>>(offsets, n_buckets, d_total);
+  BucketCounts* d_counts = reinterpret_cast<BucketCounts*>(ctx->rs.sink.counter + 10);
+  ZK_CUDA(cudaMemsetAsync(d_counts, 0, sizeof(BucketCounts), s));
+  const uint32_t chunk = chunk_entries((uint32_t)std::min<uint64_t>(prep->nonzero * (uint64_t)k_windows, 0xffffffffull), sm);  // or a little less
+  k_total64<<<sm * 4, 256, 0, s>>>(offsets, n_buckets, kFewPieces * chunk, kManyPieces * chunk, d_counts);
   ctx->launches++;
-  ZK_CUDA(cudaMemcpyAsync(ctx->host_small, d_total, 8, cudaMemcpyDeviceToHost, s));
+  ZK_CUDA(cudaMemcpyAsync(ctx->host_small, d_counts, sizeof(BucketCounts), cudaMemcpyDeviceToHost, s));
   ZK_CUDA(cudaStreamSynchronize(s));
-  unsigned long long total64 = 0;
-  memcpy(&total64, ctx->host_small, 8);
+  BucketCounts counts;
+  memcpy(&counts, ctx->host_small, sizeof(counts));
+  const unsigned long long total64 = counts.total;
   if (total64 > 0xffffffffull) return fail(-1, "msm: %llu digit entries exceed 2^32 - 1; split the call", total64);
   ctx->launches += exclusive_scan_u32(offsets, n_buckets, scan_tmp, true, s);
   ZK_CUDA(cudaMemcpyAsync(cursor, offsets, (n_buckets + 1) * 4ull, cudaMemcpyDeviceToDevice, s));
@@ -1166,8 +1178,8 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
     } else {
       uint32_t* listed = ctx->rs.sink.counter + 12;
       ZK_CUDA(cudaMemsetAsync(listed, 0, 8, s));
-      const int crowd = n_chunks > kFewPieces * 2u * (uint32_t)sm * (kFixupThreads / 32) ? 4 : 33;
-      k_msm_fixup_few<<<(n_buckets + 255) / 256, 256, 0, s>>>(offsets, n_buckets, seg, crowd, bucket_sums, heads, tails, cursor /* the list of long buckets */, listed);
+      const uint32_t few = counts.within > 2u * (uint32_t)sm * (kFixupThreads / 32) ? kManyPieces : kFewPieces;
+      k_msm_fixup_few<<<(n_buckets + 255) / 256, 256, 0, s>>>(offsets, n_buckets, seg, few, bucket_sums, heads, tails, cursor /* the list of long buckets */, listed);
       k_msm_fixup<<<sm * 2, kFixupThreads, 0, s>>>(offsets, cursor, listed, n_buckets, seg, bucket_sums, heads, tails);
       ctx->launches++;
     }
