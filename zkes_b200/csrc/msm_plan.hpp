@@ -81,9 +81,11 @@ inline uint32_t fixup_groups(uint32_t n_buckets, uint32_t n_chunks, uint64_t lon
 // blocks of 128 per SM) have work: 4096 items of 128 buckets lost 2 % of their commitment with sixteen lanes instead of eight.
 // An item of two or four buckets (rows of fewer than 256 bases, scalars of one bit) is one thread's: a block has nothing to
 // share out (2048 rows of 128 full-width scalars, 174080 items: 28.8 ms with a block each, 5.6 with a thread, 5.9 with two and
-// 6.4 with four lanes; 4 rows, 340 items: 0.87 and 0.85 ms).
+// 6.4 with four lanes; 16 rows, 1360 items: 1.22 and 1.05 ms; 4 rows, 340 items: 0.87 and 0.85 ms).  With fewer items the blocks
+// cost nothing, and most buckets may be empty, which a thread skips, but not a warp that has 32 items (one point, 85 items: 407 us
+// with a thread each, 337 with a block).
 inline uint32_t reduce_lanes(uint32_t n_items, uint32_t half, int sm) {
-  if (half < 8) return 1;
+  if (half < 8) return n_items < 512 ? 0 : 1;
   if (n_items < 1024) return 0;
   uint32_t lanes = 8;
   while (lanes < 32 && lanes * 2 <= half && (uint64_t)n_items * lanes < (uint64_t)sm * 3 * 64) lanes *= 2;
