@@ -395,8 +395,10 @@ __device__ __forceinline__ void tree_sum(Xyzz* sh, uint32_t n) {
 //   Many pieces: a bucket per block and pass.  The top window of full-width scalars has a handful of buckets that between them
 //   take every point, a thousand pieces each: 256 threads leave pieces / 256 additions plus eight levels of a tree, where a warp
 //   per bucket left pieces / 32 plus five (100003 full-width scalars: 490 us against 131 us).
-//   Up to kManyPieces: a warp each, four or five levels of a tree (64 rows of 16384 int8 values, 8192 buckets of eight or nine
-//   pieces: 1089 us with a block each, 579 us with what k_msm_fixup_few keeps and a warp for the rest).
+//   Up to kManyPieces: a block each too while there are blocks for them, whose quads are quicker (4096 full-width scalars, with a
+//   handful of them: 21 us of this kernel, 45 us with a warp each); else a warp each (64 rows of 16384 int8 values, 8192 buckets
+//   of eight or nine pieces: the call took 1089 us with a block each, and takes 579 us with a warp or with what
+//   k_msm_fixup_few keeps).
 __global__ void __launch_bounds__(kFixupThreads, 2) k_msm_fixup(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ list,
                                                              const uint32_t* __restrict__ listed, uint32_t n_buckets, uint32_t seg,
                                                              Xyzz* bucket_sums, const Xyzz* heads, const Xyzz* tails) {
@@ -416,9 +418,10 @@ __global__ void __launch_bounds__(kFixupThreads, 2) k_msm_fixup(const uint32_t* 
     return acc;
   };
   const uint32_t n_long = listed[0], n_mid = listed[1], lane = threadIdx.x & 31;
+  const uint32_t by_warps = n_mid > gridDim.x ? n_mid : 0, by_blocks = n_long + n_mid - by_warps;
   uint32_t c0, c1;
   Xyzz* mine = sh + (threadIdx.x & ~31u);
-  for (uint32_t item = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; item < n_mid; item += gridDim.x * (kFixupThreads / 32)) {
+  for (uint32_t item = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; item < by_warps; item += gridDim.x * (kFixupThreads / 32)) {
     const uint32_t b = list[n_buckets - 1 - item];
     pieces_of(b, &c0, &c1);
     mine[lane] = share(c0, c1, lane, 32);
@@ -434,8 +437,8 @@ __global__ void __launch_bounds__(kFixupThreads, 2) k_msm_fixup(const uint32_t* 
     __syncwarp();
   }
   __syncthreads();
-  for (uint32_t item = blockIdx.x; item < n_long; item += gridDim.x) {
-    const uint32_t b = list[item];
+  for (uint32_t item = blockIdx.x; item < by_blocks; item += gridDim.x) {
+    const uint32_t b = item < n_long ? list[item] : list[n_buckets - 1 - (item - n_long)];
     pieces_of(b, &c0, &c1);
     sh[threadIdx.x] = share(c0, c1, threadIdx.x, kFixupThreads);
     __syncthreads();
