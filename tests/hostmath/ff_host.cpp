@@ -2,6 +2,7 @@
 // The carry chains compile to their portable C form here, so the algorithms (not the PTX)
 // are what these symbols exercise.
 #include "../../zkes_b200/csrc/ff.cuh"
+#include <chrono>
 #include <cstring>
 using namespace zk;
 
@@ -24,6 +25,18 @@ template <class P> static void ld(Fp<P>& x, const uint32_t* p) { memcpy(x.v, p, 
     Fp<P> x; ld(x, a); Fp<P> z = to_mont(x); memcpy(r, z.v, 32); }                           \
   extern "C" void zkh_##name##_from_mont(const uint32_t* a, uint32_t* r) {                   \
     Fp<P> x; ld(x, a); Fp<P> z = from_mont(x); memcpy(r, z.v, 32); }                         \
+  extern "C" void zkh_##name##_from_mont_rows(const uint32_t* a, uint32_t* r) {               \
+    Wide t; memset(&t, 0, sizeof t); memcpy(t.v, a, 32); Fp<P> z = redc<P>(t); memcpy(r, z.v, 32); } \
+  /* nanoseconds of a chain of n conversions (kind 0) or products (kind 1), the shorter of eight */ \
+  extern "C" double zkh_##name##_chain_ns(uint32_t* a, int kind, int n) {                      \
+    Fp<P> x; ld(x, a); double least = 1e30;                                                    \
+    for (int rep = 0; rep < 8; rep++) {                                                        \
+      const auto t0 = std::chrono::steady_clock::now();                                        \
+      for (int i = 0; i < n; i++) x = kind ? mul(x, x) : from_mont(x);                         \
+      const std::chrono::duration<double, std::nano> d = std::chrono::steady_clock::now() - t0; \
+      if (d.count() < least) least = d.count();                                                \
+    }                                                                                          \
+    memcpy(a, x.v, 32); return least / n; }                                                    \
   extern "C" void zkh_##name##_mul_fixed(const uint32_t* x, const uint32_t* d, uint32_t* r) {  \
     Fp<P> a, b; ld(a, x); ld(b, d); FixedMul<P> t = make_fixed_mul(a);                        \
     Fp<P> z = mul_fixed(t, b); memcpy(r, z.v, 32); }                                         \

@@ -195,3 +195,25 @@ def test_device_rows(hm, name, p):
             assert val(out) == a * b * rinv % p
         getattr(hm, f"zkh_{name}_sqr_rows")(buf(a), out)
         assert val(out) == a * a * rinv % p
+
+
+@pytest.mark.parametrize("name,p", [("fr", o.R_MOD), ("fq", o.Q_MOD)])
+def test_out_of_montgomery_form(hm, name, p):
+    """The host's form and the reduction alone, which the device runs, over every value of eight limbs."""
+    rnd = random.Random(13)
+    out = (ctypes.c_uint32 * 8)()
+    rinv = pow(R, -1, p)
+    for a in [0, 1, p - 1, p, R - 1, R % p, 0xFFFFFFFF] + [rnd.randrange(R) for _ in range(300)]:
+        for form in ("from_mont", "from_mont_rows"):
+            getattr(hm, f"zkh_{name}_{form}")(buf(a), out)
+            assert val(out) == a * rinv % p, form
+
+
+@pytest.mark.parametrize("name,p", [("fr", o.R_MOD), ("fq", o.Q_MOD)])
+def test_out_of_montgomery_form_costs_the_host_a_product(hm, name, p):
+    """Every message of a round that the host steps is converted: with 32-bit rows it took 2.7 products' time."""
+    fn = getattr(hm, f"zkh_{name}_chain_ns")
+    fn.restype = ctypes.c_double
+    x = buf(random.Random(14).randrange(p))
+    best = min(fn(x, 0, 20000) / fn(x, 1, 20000) for _ in range(5))
+    assert best < 1.7

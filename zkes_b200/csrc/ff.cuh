@@ -798,14 +798,20 @@ ZK_HD Fp<P> to_mont(const Fp<P>& canonical) {
   return mul(Fp<P>::r2(), canonical);
 }
 template <class P>
-ZK_HD Fp<P> from_mont(const Fp<P>& a) {  // the reduction alone: half the multiply-adds of a product by one (k_msm_bits: 297 -> 208 us)
-  Wide t;
+ZK_HD Fp<P> from_mont(const Fp<P>& a) {
+#ifdef __CUDA_ARCH__
+  Wide t;  // the reduction alone: half the multiply-adds of a product by one (k_msm_bits: 297 -> 208 us)
 #pragma unroll
   for (int i = 0; i < 8; i++) {
     t.v[i] = a.v[i];
     t.v[i + 8] = 0;
   }
   return redc<P>(t);
+#else
+  Fp<P> one = Fp<P>::zero();  // four 64-bit limbs beat the 32-bit reduction: 25 ns against 68
+  one.v[0] = 1;
+  return mul_host(a, one);
+#endif
 }
 
 // Small unsigned integer as a field element (Montgomery form).
