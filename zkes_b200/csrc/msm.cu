@@ -566,7 +566,9 @@ __global__ void __launch_bounds__(kReduceThreads) k_msm_bucket_reduce(const Xyzz
       add_to(&running, &bj);
       add_to(&acc, &running);
     }
-    for (uint32_t k = per; k > 1; k >>= 1) dbl_in_place(&running);
+    // D is for joining: an item that is one run has no use for it (half of the kernel's 12 us for two buckets)
+    if (per < half)
+      for (uint32_t k = per; k > 1; k >>= 1) dbl_in_place(&running);
   }
   A[threadIdx.x] = acc;
   D[threadIdx.x] = running;
