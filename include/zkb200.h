@@ -328,11 +328,12 @@ int zk_g1_compress(zk_ctx* ctx, const uint64_t* affine, zk_mem affine_mem, uint6
 int zk_g1_decompress(zk_ctx* ctx, const uint8_t* in, zk_mem in_mem, uint64_t n, uint64_t* affine_out, zk_mem out_mem);
 
 /* Shape the last MSM on this context chose (window width, windows, largest scalar magnitude in
- * bits, digit entries, buckets): used to report algorithmic work. */
+ * bits, digit entries, buckets): used to report algorithmic work.  Rows of small scalars that are added up from tables of
+ * subset sums have windows of one bit, one per bit plane, table entries in the place of digit entries, and no buckets. */
 int zk_msm_last_stats(zk_ctx* ctx, int* window_bits, int* windows, int* max_bits, uint64_t* entries, uint64_t* buckets);
 /* Work of all the MSMs this context ran since the last reset (a KZH commit runs two, an opening several): the
- * number of MSM pipelines, their non-zero signed digits (each is one mixed addition into a bucket) and the
- * buckets they reduced.  reset != 0 clears the counters after reading.  No counterpart in the reference. */
+ * number of MSM pipelines, their non-zero signed digits and looked-up table entries (each is one mixed addition into a
+ * bucket or onto a row's sum, but for the entries of empty subsets; the sums that make the tables are not counted) and the buckets they reduced.  reset != 0 clears the counters after reading.  No counterpart in the reference. */
 int zk_msm_work(zk_ctx* ctx, uint64_t* calls, uint64_t* entries, uint64_t* buckets, int reset);
 
 /* ---- KZH2 / KZH3 polynomial commitments, G1 side ------------------------------------------ */

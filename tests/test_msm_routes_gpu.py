@@ -178,3 +178,46 @@ def test_buckets_of_some_pieces(ctx, multiples, n, hot, share):
     sc = _repeated(to_mont_array([o.fr_from_int(v) for v in range(-32768, 32769)]), vals + 32768)
     got = _device_msm(ctx, _repeated(curve.affine_to_array(pts), pick), sc)
     assert got == of_g(sum(int(v) * k for v, k in zip(per_base, ks)))
+
+
+@pytest.mark.parametrize("rows,n", [(1024, 1024), (1024, 1003), (4096, 1000)])
+def test_rows_in_several_chains(ctx, multiples, rows, n):
+    """Hundreds of groups in a few chains of several groups each, the last one shorter."""
+    import torch
+
+    ks, pts = multiples
+    rng = np.random.default_rng(rows + n)
+    pick = rng.integers(0, len(ks), size=n)
+    vals = rng.integers(-128, 128, size=(rows, n))
+    vals[1], vals[2] = -128, 127
+    f = _repeated(to_mont_array([o.fr_from_int(v) for v in range(-128, 128)]), vals.reshape(-1) + 128)
+    bases = _repeated(curve.affine_to_array(pts), pick)
+    out = np.zeros((rows, 12), dtype=np.uint64)
+    torch.cuda.synchronize()
+    check(lib.zk_msm_g1_batched(ctx.handle, vp(bases.data_ptr()), ZK_MEM_DEVICE, n, vp(f.data_ptr()), ZK_MEM_DEVICE, rows,
+                                vp(out.ctypes.data), ZK_MEM_HOST), "zk_msm_g1_batched")
+    for r in sorted({0, 1, 2, rows // 3, rows - 2, rows - 1}):
+        per_base = np.bincount(pick, weights=vals[r], minlength=len(ks))
+        assert curve.jacobian_to_affine_py(out[r:r + 1])[0] == of_g(sum(int(v) * k for v, k in zip(per_base, ks))), r
+
+
+def test_full_width_rows_with_32_lanes(ctx, multiples):
+    """1720 items of 32 buckets: 32 lanes an item."""
+    test_full_width_rows(ctx, multiples, 40, 2000)
+
+
+def test_work_of_rows_by_subset_sums(ctx, multiples):
+    """The reported entries are table look-ups, one per row, bit plane and group; the sums that make the tables are not among them."""
+    _, pts = multiples
+    rows, n = 700, 12
+    rnd = random.Random(3)
+    mat = [[o.fr_from_int(rnd.randint(-128, 127)) for _ in range(n)] for _ in range(rows)]
+    mat[0][0] = o.fr_from_int(-128)
+    calls, entries, buckets = ctypes.c_uint64(), ctypes.c_uint64(), ctypes.c_uint64()
+    args = (ctypes.byref(calls), ctypes.byref(entries), ctypes.byref(buckets), 1)
+    check(lib.zk_msm_work(ctx.handle, *args), "zk_msm_work")
+    curve.msm_batched(ctx, curve.affine_to_array(pts[-n:]), mat)
+    check(lib.zk_msm_work(ctx.handle, *args), "zk_msm_work")
+    planes = 8
+    assert calls.value == 1 and buckets.value == 0
+    assert entries.value % (rows * planes) == 0 and 1 <= entries.value // (rows * planes) <= n // 2

@@ -49,7 +49,8 @@ inline Fr transcript_challenge_scalar(MerlinTranscript& t, const uint8_t* label,
 
 struct MsmStatsPod {
   int window_bits = 0, windows = 0, max_bits = 0;
-  uint32_t entries = 0, buckets = 0;
+  uint64_t entries = 0;
+  uint32_t buckets = 0;
 };
 
 struct zk_comm;
@@ -72,7 +73,7 @@ struct zk_ctx {
   void* host_points = nullptr;   // pinned: window sums of a few rows and their combination (msm.cu)
   void* resident_sh = nullptr;   // zk::ResidentShared: hand-over area of the resident multi-round kernel (8 KiB, inside tail_out's block)
   zk::Fr* tail_buf = nullptr;    // sharded proves: gathered values and the last log2(world) rounds' tables
-  void* host_small = nullptr;    // pinned, 8 KiB: round messages and other tiny read-backs
+  void* host_small = nullptr;    // pinned, kFlagsHostOffset + 256 bytes: round messages and other tiny read-backs
   void* mailbox = nullptr;       // pinned + mapped: message kernels publish here, the host polls
   void* work = nullptr;          // grow-only device scratch (copies of caller data, round buffers)
   size_t work_bytes = 0;
@@ -98,7 +99,7 @@ struct zk_ctx {
     round_times.push_back(std::chrono::duration<double, std::micro>(now - round_t0).count());
   }
   MsmStatsPod last_msm;          // shape of the most recent MSM (window width, windows, entries)
-  uint64_t msm_entries_sum = 0;  // digit entries (= bucket additions) of every MSM since the last zk_msm_work reset
+  uint64_t msm_entries_sum = 0;  // mixed additions into buckets or of table entries of every MSM since the last zk_msm_work reset
   uint64_t msm_bucket_sum = 0;   // buckets reduced by those MSMs
   uint64_t msm_calls = 0;
   std::atomic<uint64_t> launches{0};

@@ -996,7 +996,6 @@ static int rows_run(zk_ctx* ctx, const Affine* bases, const int32_t* compact, ui
   const int sm = ctx->sm_count, s = plan.group, lo_bits = (s + 1) / 2;
   const uint32_t groups = plan.groups, seg = plan.seg, parts = plan.parts;
   const uint64_t units = (uint64_t)rows * plan.planes;
-  const uint64_t table_points = (uint64_t)groups << s;
   char* base = nullptr;
   int rc = ctx->reserve_aux(plan.scratch(), (void**)&base);
   if (rc) return rc;
@@ -1026,13 +1025,13 @@ static int rows_run(zk_ctx* ctx, const Affine* bases, const int32_t* compact, ui
   k_rows_planes<<<(rows + 63) / 64, 64, 0, st>>>(pieces, rows, plan.planes, out_dev);
   ctx->launches++;
   ZK_CUDA(cudaGetLastError());
-  const uint64_t additions = units * groups + table_points;
-  ctx->msm_entries_sum += additions;
+  const uint64_t lookups = units * groups;  // one mixed addition each, but for the empty subsets
+  ctx->msm_entries_sum += lookups;
   ctx->msm_calls++;
   if (stats) {
     stats->window_bits = 1;
     stats->windows = plan.planes;
-    stats->entries = additions;
+    stats->entries = lookups;
     stats->buckets = 0;
     stats->max_bits = max_bits;
   }
@@ -1209,12 +1208,14 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
       break;
     case Combine::kWarps:
       k_msm_combine_quads<<<rows, 32, 0, s>>>(window_sums, w, k_windows, out_dev);
+      ctx->launches++;
       break;
     case Combine::kThreads:
       k_msm_combine<<<(rows + 63) / 64, 64, 0, s>>>(window_sums, rows, w, k_windows, out_dev);
+      ctx->launches++;
       break;
   }
-  ctx->launches += 2;
+  ctx->launches++;  // the bucket reduction
   ZK_CUDA(cudaGetLastError());
   ctx->msm_entries_sum += n_entries;
   ctx->msm_bucket_sum += n_buckets;
