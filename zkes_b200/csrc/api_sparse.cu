@@ -176,9 +176,8 @@ static int sparse_dense_impl(zk_ctx* ctx, zk_comm* comm, uint32_t total_var, uin
     // the few values it needs on the fly, so this fold waits and is done together with the next
     // one in a single pass over the table (k_fold2).
     const bool next_sparse = round + 1 < num_var && (!K_rule || (S / 2) > dense_cap);
-    // The table fold (bandwidth-bound, long) and the entry fold (three short launches) touch disjoint
-    // buffers: the table fold goes to the side stream and the two run side by side.  With the
-    // per-kernel profiler on they stay in line so that each span times one kernel alone.
+    // The table fold goes to the side stream, which the next message waits for.  Nothing runs beside it since the message kernel
+    // binds the entries itself.  With the per-kernel profiler on it stays in line so that each span times one kernel alone.
     const bool fold_now = pending || !next_sparse;
     const bool beside = fold_now && !ctx->prof_on;
     cudaStream_t fs_stream = beside ? ctx->side_stream : s;

@@ -823,7 +823,8 @@ ZK_HD Fp<P> from_u32(uint32_t x) {
 }
 
 // Multiplicative inverse (0 maps to 0) by the division steps of Bernstein and Yang, "Fast constant-time gcd computation
-// and modular inversion" (2019), with the counter delta started at 1/2.  Fermat's power is a chain of some 380 dependent
+// and modular inversion" (2019), with the counter delta started at 1/2 as P. Wuille and G. Maxwell proposed ("Bounds on
+// divsteps iterations in safegcd", 2021: 590 steps suffice for 256-bit inputs, 741 as in the paper).  Fermat's power is a chain of some 380 dependent
 // products; here the low words alone decide thirty steps, which are collected in a 2x2 matrix and then applied to the
 // whole numbers, so an inversion is about 18 batches of thirty 32-bit steps and two matrix products over nine limbs.
 // k_normalize on 4096 points (an inversion per thread): 22 us against 173 us.
@@ -831,8 +832,8 @@ ZK_HD Fp<P> from_u32(uint32_t x) {
 // Numbers are nine limbs of 30 bits, the lower eight in [0, 2^30), the top one signed.  f and g stay within (-p, p].
 // d and e satisfy d a = f and e a = g (mod p); a batch takes each to (u d + v e + m p) / 2^30 with |u| + |v| <= 2^30 and
 // m in [-2^29, 2^29) chosen to make the division exact, so they grow by at most p/2 a batch and stay below 13 p in
-// absolute value: no reduction is needed before the end.  25 batches (750 steps) are more than the 590 that suffice for
-// 256-bit inputs; the loop ends as soon as g is zero.
+// absolute value: no reduction is needed before the end.  25 batches (750 steps) are more than either bound;
+// the loop ends as soon as g is zero.
 template <class P>
 ZK_HD int32_t mod30(int i) {  // limb i of p in base 2^30; a constant after unrolling
   const int bit = 30 * i, k = bit >> 5, sh = bit & 31;

@@ -39,14 +39,14 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
 int msm_select_sums(zk_ctx* ctx, const Affine* full, const Affine* mid, const uint32_t* idx_dev, uint32_t n, uint32_t low_bits,
                     uint32_t rows, Jacobian* out_dev, void* scratch);
 
-// ---- Host-side inversion: the division steps of inverse() take a CPU core 6 us (0 maps to 0).
+// ---- Host-side inversion (0 maps to 0): the division steps of inverse(), 1.6 us of a CPU core.
 template <class P>
 inline Fp<P> inverse_host(const Fp<P>& a) {
   return inverse(a);
 }
 
 // CurveGroup::into_affine of one point on the host: the point is read back anyway, and a launch for one thread's inversion
-// (some 20 us) costs more than the 6 us it takes here.
+// (some 20 us) costs more than the 2 us it takes here.
 inline Affine jacobian_to_affine_host(const Jacobian& j) {
   Affine a;
   if (j.z.is_zero()) {

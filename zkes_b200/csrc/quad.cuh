@@ -96,17 +96,10 @@ __device__ __forceinline__ QuadXyzz quad_add(const QuadXyzz& p, const QuadXyzz& 
   return r;
 }
 
-// a += b and a = 2 (a + b) for points in shared memory, one copy of the code each.
+// a += b for points in shared memory, one copy of the code.
 static __device__ __noinline__ void quad_add_to(Xyzz* a, const Xyzz* b, bool on) {
   const int role = threadIdx.x & 3;
   const QuadXyzz r = quad_add(quad_load(a, role), quad_load(b, role), role);
-  __syncwarp();
-  if (on) quad_store(a, r, role);
-  __syncwarp();
-}
-static __device__ __noinline__ void quad_dbl_in_place(Xyzz* a, bool on) {
-  const int role = threadIdx.x & 3;
-  const QuadXyzz r = quad_dbl(quad_load(a, role), role);
   __syncwarp();
   if (on) quad_store(a, r, role);
   __syncwarp();
