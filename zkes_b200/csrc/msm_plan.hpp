@@ -28,11 +28,11 @@ inline int pick_window(uint64_t n, uint32_t rows, int max_bits) {
   if (w > max_bits + 1) w = max_bits + 1;
   if (w < 2) w = 2;
   // A top window of one to three bits has a handful of buckets that between them take every point, and joining their pieces is
-  // a chain of its own; one bit less per window then costs at most one window more.  Of full-width scalars this is the width 14,
-  // 2^16 to 2^17 - 1 points: it leaves three bits with the sign for the nineteenth window, 13 leaves eight for the twentieth
-  // (100003 points: 1 140 us against 941).  15 and 16 bits leave fifteen (262143 points: 1 623 us with 15, 1 872 us with 14).  The
-  // narrower windows stay as they are: 12 bits (2^14 points on) would leave two bits for three, and 11 bits take 12000 points
-  // in 548 us where 10, with five bits for two, take 583.
+  // a chain of its own; one bit less per window then costs at most one window more.  Of full-width scalars (254 bits with the
+  // sign) this is the width 14, 2^16 to 2^17 - 1 points: it leaves two bits for the nineteenth window, 13 leaves seven for the
+  // twentieth (100003 points: 1 140 us against 941).  15 and 16 bits leave fourteen (262143 points: 1 623 us with 15, 1 872 us
+  // with 14).  Narrower windows stay as they are: 12 bits (2^14 points on) leave two bits, but 11 would leave one; and 11 bits
+  // take 12000 points in 548 us where 10, which leave four, take 583.
   if (rows == 1 && w >= 14 && max_bits > kCompactBits && (max_bits + 1) - w * ((max_bits + w) / w - 1) < 4) w--;
   return w;
 }
