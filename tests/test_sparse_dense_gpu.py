@@ -62,6 +62,21 @@ def test_adjacent_runs(ctx):
     assert proof.round_messages == oproof.round_messages and proof.final_eval == oproof.final_eval
 
 
+@pytest.mark.parametrize("n", [3, 4, 6, 7, 9])
+@pytest.mark.parametrize("kind", ["largest", "mixed"])
+def test_double_folds_of_extreme_tables(ctx, n, kind):
+    """One entry keeps the prover in entry form, so the table is folded two variables at a time down to two elements: tiles of 32
+    outputs whole and in part, with elements whose bytes make the largest sums (p - 1 in memory) beside zeros."""
+    rnd = random.Random(n)
+    largest = (o.R_MOD - 1) * pow(1 << 256, -1, o.R_MOD) % o.R_MOD  # its Montgomery form is p - 1
+    dense = [largest if kind == "largest" else rnd.choice([0, largest, rnd.randrange(o.R_MOD)]) for _ in range(1 << n)]
+    idx, vals = [rnd.randrange(1 << n)], [rnd.randrange(1, o.R_MOD)]
+    t, ot = Transcript(b"sd"), o.Transcript(b"sd")
+    proof = SparseDenseSumcheckProver(n, t).prove(ctx, idx, vals, DenseMLPoly.from_evaluations(dense), t)
+    _, oproof = o.sparse_dense_prove(n, idx, vals, dense, ot)
+    assert proof.round_messages == oproof.round_messages and proof.final_eval == oproof.final_eval
+
+
 def test_rejects_unsorted_or_out_of_range(ctx):
     dense = DenseMLPoly.from_evaluations([1] * 16)
     for bad in ([3, 2], [1, 1], [5, 16]):
