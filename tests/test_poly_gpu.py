@@ -1,11 +1,15 @@
 """eq tables and fix_variables_from_right on the GPU against the oracle, with the closed forms of
 tests/test_lagrange_basis.rs and tests/test_fix_variables.rs:278-307."""
+import ctypes
 import random
 
+import numpy as np
 import pytest
 
 import pyoracle as o
 from zkes_b200 import DenseMLPoly, evaluate_lagrange_basis, fix_variables_from_right
+from zkes_b200._lib import ZK_MEM_HOST, check, lib
+from zkes_b200.field import from_mont_array, to_mont_array
 
 pytestmark = pytest.mark.gpu
 M = o.R_MOD
@@ -47,6 +51,22 @@ def test_from_right_random(ctx, n, k):
     if n <= 12:
         lowpt = [rnd.randrange(M) for _ in range(n - k)]
         assert o.evaluate_multilinear_extension(got, lowpt) == o.evaluate_multilinear_extension(f, lowpt + pt)
+
+
+@pytest.mark.parametrize("lo,hi", [(0, 4), (0, 5), (0, 11), (1, 5), (3, 6), (4, 5), (5, 8), (5, 9), (2, 10), (6, 4)])
+@pytest.mark.parametrize("kind", ["largest", "random"])
+def test_weighted_fold_edges(ctx, lo, hi, kind):
+    """2^hi rows of 2^lo columns around the sizes where the byte products begin (32 rows), a block's columns (16) and the rows that
+    its weights are held for (256) end, with the largest bytes that an element can have (p - 1 in memory) and random ones."""
+    rnd = random.Random(100 * lo + hi)
+    largest = (M - 1) * pow(1 << 256, -1, M) % M
+    f = [largest if kind == "largest" else rnd.randrange(M) for _ in range(1 << (lo + hi))]
+    w = [largest if kind == "largest" else rnd.choice([0, rnd.randrange(M)]) for _ in range(1 << hi)]
+    fm, wm, out = to_mont_array(f), to_mont_array(w), np.zeros((1 << lo, 4), dtype=np.uint64)
+    vp = ctypes.c_void_p
+    check(lib.zk_weighted_fold_from_right(ctx.handle, lo + hi, vp(fm.ctypes.data), ZK_MEM_HOST, hi, vp(wm.ctypes.data), ZK_MEM_HOST,
+                                          vp(out.ctypes.data), ZK_MEM_HOST), "zk_weighted_fold_from_right")
+    assert list(from_mont_array(out)) == [sum(w[h] * f[(h << lo) + c] for h in range(1 << hi)) % M for c in range(1 << lo)]
 
 
 @pytest.mark.parametrize("n", [0, 1, 3, 8, 11, 15])

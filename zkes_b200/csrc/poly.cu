@@ -3,6 +3,7 @@
 //   fix from right   out[lo] = sum_hi eq[hi] * f[hi * 2^rem + lo]   (poly.rs:705-758)
 #include "internal.hpp"
 #include "reduce.cuh"
+#include "byte_mma.cuh"
 
 namespace zk {
 namespace {
@@ -130,6 +131,197 @@ __global__ void __launch_bounds__(256) k_from_right(const Fr* __restrict__ f, co
   st_fr_plain(partial + (uint64_t)blockIdx.y * lo_n + lo, redc<FrParams>(acc));
 }
 
+// The same sums on the tensor cores (byte_mma.cuh): for a column, D[j][i] = sum_hi (byte j of eq[hi]) (byte i of f[hi][lo]) is a
+// product of matrices of bytes, 32 x hi_n by hi_n x 32, and the column's sum is sum_ij 2^(8 (i + j)) D[i][j].
+// A warp takes two columns and 32 rows a step: 2 KiB of f, streamed through kCtStages slots of its own in shared memory, which the
+// lanes read back as eight bytes of eight rows each and transpose to four rows of a byte in a word, as the instruction wants its
+// second operand.  The 2 x 32 x 32 sums stay in registers from step to step.  eq is brought into the order of the first operand once
+// per kCtChunk rows for the block's eight warps.
+// The steps of all columns form one line that is cut into equal pieces, one for each block that fits the GPU, so that no place idles
+// whatever the shape; where a piece ends inside a column, or a column inside a piece, the block puts its sums together (some ten
+// steps' worth) and leaves them in a slot of the column's own, and k_sum_splits adds the slots.
+// 2^12 rows of 2^12 columns take 102 us (5.3 TB/s of the table's bytes), where the integer pipe took 171 with 64 multiply-adds an
+// element; cut by columns alone, 256 blocks for 296 places, it was 112 us.  What bounds it now is issue: some 100 instructions a warp
+// and step beside 16 of the tensor cores.
+constexpr int kCtThreads = 256, kCtWarps = kCtThreads / 32, kCtStages = 4, kCtChunk = 256, kCtStep = 32, kCtCols = 2 * kCtWarps;
+constexpr size_t kCtShared = (size_t)kCtWarps * kCtStages * 2048 + (size_t)kCtChunk * 32;
+
+// out[b] = bytes b of a0, a1, a2, a3
+__device__ __forceinline__ void transpose_bytes(uint32_t (&out)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
+  const uint32_t l0 = __byte_perm(a0, a1, 0x5140), h0 = __byte_perm(a0, a1, 0x7362);
+  const uint32_t l1 = __byte_perm(a2, a3, 0x5140), h1 = __byte_perm(a2, a3, 0x7362);
+  out[0] = __byte_perm(l0, l1, 0x5410);
+  out[1] = __byte_perm(l0, l1, 0x7632);
+  out[2] = __byte_perm(h0, h1, 0x5410);
+  out[3] = __byte_perm(h0, h1, 0x7632);
+}
+
+// v / 2^256 mod p for a number of 17 words
+__device__ __forceinline__ Fr reduce_words(const uint32_t (&v)[17]) {
+  Wide low;
+  Fr mid, top = Fr::zero();
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    low.v[k] = v[k];
+    low.v[k + 8] = 0;
+    mid.v[k] = v[k + 8];
+  }
+  top.v[0] = v[16];
+  return add(redc<FrParams>(low), add(mul(Fr::one(), mid), mul(Fr::r2(), top)));
+}
+
+// per: steps of a block; col_steps: steps of a column group, ceil(hi_n / 32); slots: as many as a column can have.
+__global__ void __launch_bounds__(kCtThreads, 2) k_from_right_bytes(const Fr* __restrict__ f, const Fr* __restrict__ eq, uint64_t lo_n,
+                                                                    uint64_t hi_n, uint32_t col_groups, uint32_t col_steps, uint64_t per,
+                                                                    uint32_t slots, Fr* partial) {
+  extern __shared__ uint4 ct_shared[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  uint4* stage = ct_shared + warp * kCtStages * 128;                                      // [slot][row][4 chunks], swizzled
+  uint32_t* frag = reinterpret_cast<uint32_t*>(ct_shared + kCtWarps * kCtStages * 128);   // [step of the chunk][lane][8]
+  const uint64_t all = (uint64_t)col_groups * col_steps, line0 = blockIdx.x * per, line1 = line0 + per < all ? line0 + per : all;
+  // this lane's part of a copy: chunk lane & 3 of rows lane / 4 + 8 i; a row's chunks sit permuted by its bit 1, so that the lanes'
+  // reads below meet no bank twice
+  const uint32_t to = (uint32_t)__cvta_generic_to_shared(stage + (lane >> 2) * 4 + ((lane & 3) ^ ((lane >> 2) & 2)));
+  const uint64_t row8 = lo_n * 8 * sizeof(Fr);
+  const int last_rows = (int)(hi_n - (uint64_t)(col_steps - 1) * kCtStep);
+  for (uint64_t line = line0; line < line1;) {
+    const uint32_t group = (uint32_t)(line / col_steps), step0 = (uint32_t)(line - (uint64_t)group * col_steps);
+    const uint32_t steps = (uint32_t)(line1 - line < col_steps - step0 ? line1 - line : col_steps - step0);
+    const uint64_t lo0 = ((uint64_t)group * kCtWarps + warp) * 2;
+    const bool in_columns = lo0 + ((lane & 3) >> 1) < lo_n;
+    const char* src = reinterpret_cast<const char*>(f + ((uint64_t)step0 * kCtStep + (lane >> 2)) * lo_n + lo0) + 16 * (lane & 3);
+    auto issue = [&](uint32_t step) {  // called for step 0, 1, ... in turn
+      if (step < steps) {
+        const uint32_t dst = to + (step % kCtStages) * 2048;
+        const int rows = step0 + step + 1 < col_steps ? kCtStep : last_rows;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const bool live = in_columns && (lane >> 2) + 8 * i < rows;
+          const uint32_t bytes = live ? 16u : 0u;  // 0: nothing is read, zeros are written
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + 512 * i), "l"(live ? src : (const char*)f), "r"(bytes) : "memory");
+          src += row8;
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // d[4 w + b][M]: byte b of word w of the lane columns' eight bytes against bytes 16 M .. 16 M + 15 of eq
+    uint32_t d[8][2][4];
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+#pragma unroll
+      for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) d[k][m][q] = 0;
+#pragma unroll
+    for (int k = 0; k < kCtStages - 1; k++) issue(k);
+    for (uint32_t step = 0; step < steps; step++) {
+      const uint32_t in_chunk = step % (kCtChunk / kCtStep);
+      if (in_chunk == 0) {
+        // the order of the rows of a step is free as long as both operands have the same: row 16 h + 4 q + t is byte q of word h of
+        // the lanes with that t
+        __syncthreads();
+        for (int k = threadIdx.x; k < kCtChunk * 2; k += kCtThreads) {
+          const int word = k & 7, ft = (k >> 3) & 3, fh = (k >> 5) & 1, fs = k >> 6;
+          uint32_t a[4], o[4];
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            const uint64_t h = (uint64_t)(step0 + step + fs) * kCtStep + 16 * fh + 4 * q + ft;
+            a[q] = h < hi_n ? __ldg(reinterpret_cast<const uint32_t*>(eq + h) + word) : 0u;
+          }
+          transpose_bytes(o, a[0], a[1], a[2], a[3]);
+#pragma unroll
+          for (int b = 0; b < 4; b++) {
+            const int j = 4 * word + b;
+            frag[(fs * 32 + 4 * (j & 7) + ft) * 8 + (j >> 3) * 2 + fh] = o[b];
+          }
+        }
+        __syncthreads();
+      }
+      asm volatile("cp.async.wait_group %0;" ::"n"(kCtStages - 2) : "memory");
+      __syncwarp();
+      issue(step + kCtStages - 1);  // into the slot that the warp read a step ago
+      const uint4* slot = stage + (step % kCtStages) * 128;
+      uint2 x[8];
+#pragma unroll
+      for (int r = 0; r < 8; r++) x[r] = reinterpret_cast<const uint2*>(slot + (4 * r + t) * 4 + ((g >> 1) ^ (t & 2)))[g & 1];
+      const uint4* fr = reinterpret_cast<const uint4*>(frag + (in_chunk * 32 + lane) * 8);
+      const uint4 e0 = fr[0], e1 = fr[1];  // bytes of eq: rows g and g + 8 of the first tile, then of the second
+#pragma unroll
+      for (int w = 0; w < 2; w++) {
+        uint32_t b0[4], b1[4];
+        if (w == 0) {
+          transpose_bytes(b0, x[0].x, x[1].x, x[2].x, x[3].x);
+          transpose_bytes(b1, x[4].x, x[5].x, x[6].x, x[7].x);
+        } else {
+          transpose_bytes(b0, x[0].y, x[1].y, x[2].y, x[3].y);
+          transpose_bytes(b1, x[4].y, x[5].y, x[6].y, x[7].y);
+        }
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+          mma_bytes(d[4 * w + b][0], e0.x, e0.z, e0.y, e0.w, b0[b], b1[b]);
+          mma_bytes(d[4 * w + b][1], e1.x, e1.z, e1.y, e1.w, b0[b], b1[b]);
+        }
+      }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    // The lane's sums: eight bytes each of columns n = 2 t and 2 t + 1 (n counts eight bytes along the two columns of f), against
+    // bytes g + 8 m of eq: u = sum over the column bytes, n - 2 t and m; it belongs at bytes g + 16 (t & 1) of column lo0 + (t >> 1).
+    unsigned long long u[11];
+#pragma unroll
+    for (int k = 0; k < 11; k++) u[k] = 0;
+#pragma unroll
+    for (int m = 0; m < 4; m++)
+#pragma unroll
+      for (int c = 0; c < 2; c++)
+#pragma unroll
+        for (int w = 0; w < 2; w++) {
+          unsigned long long s = 0;
+#pragma unroll
+          for (int b = 3; b >= 0; b--) s = (s << 8) + d[4 * w + b][m >> 1][2 * (m & 1) + c];
+          u[2 * (c + m) + w] += (uint32_t)s;
+          u[2 * (c + m) + w + 1] += s >> 32;
+        }
+    uint32_t v[12], z[17];
+    unsigned long long carry = 0;
+#pragma unroll
+    for (int k = 0; k < 11; k++) {
+      carry += u[k];
+      v[k] = (uint32_t)carry;
+      carry >>= 32;
+    }
+    v[11] = 0;  // below 2^(256 + 90)
+#pragma unroll
+    for (int k = 11; k > 0; k--) v[k] = __funnelshift_l(v[k - 1], v[k], 8 * (g & 3));
+    v[0] <<= 8 * (g & 3);
+#pragma unroll
+    for (int k = 0; k < 17; k++) z[k] = (k < 12) ? ((g & 4) ? (k > 0 ? v[k - 1] : 0u) : v[k]) : (k == 12 && (g & 4)) ? v[11] : 0u;
+    if (t & 1) {
+#pragma unroll
+      for (int k = 16; k >= 0; k--) z[k] = k >= 4 ? z[k - 4] : 0u;
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off = off == 4 ? 1 : off >> 1) {  // the eight g, and the two t of a column
+      carry = 0;
+#pragma unroll
+      for (int k = 0; k < 17; k++) {
+        carry += (unsigned long long)z[k] + __shfl_xor_sync(0xffffffffu, z[k], off);
+        z[k] = (uint32_t)carry;
+        carry >>= 32;
+      }
+    }
+    const Fr r = reduce_words(z);
+    const uint64_t lo = lo0 + (t >> 1);
+    if (g == 0 && (t & 1) == 0 && lo < lo_n) {
+      // the blocks that share a column are neighbours; the last of them clears the slots that are left over
+      uint32_t at = (uint32_t)(blockIdx.x - (uint64_t)group * col_steps / per);
+      st_fr_plain(partial + (uint64_t)at * lo_n + lo, r);
+      if (step0 + steps == col_steps)
+        for (at++; at < slots; at++) st_fr_plain(partial + (uint64_t)at * lo_n + lo, Fr::zero());
+    }
+    line += steps;
+  }
+}
+
 // out[lo] = sum_k partial[k * lo_n + lo].  A block takes 32 columns; its eight warps share the splits (warp g
 // sums splits g, g + 8, ...: a warp reads 1 KiB of one split at a time, and the loads of a thread do not wait
 // for one another), then the eight partial sums of a column are added through shared memory.
@@ -195,7 +387,30 @@ int launch_eq_table(const Fr* point_dev, uint32_t k, Fr* out, int sm_count, cuda
   return 1;
 }
 
+// Contractions of at least kCtRows rows go through the tensor cores.
+constexpr uint64_t kCtRows = 32;
+
+// How the steps of a contraction are cut (k_from_right_bytes).
+struct BytesPlan {
+  uint64_t groups, steps, per, blocks;
+  uint32_t slots;
+};
+static BytesPlan bytes_plan(uint64_t lo_n, uint64_t hi_n, int sm_count) {
+  BytesPlan p;
+  p.groups = (lo_n + kCtCols - 1) / kCtCols;
+  p.steps = (hi_n + kCtStep - 1) / kCtStep;
+  const uint64_t all = p.groups * p.steps, places = 2 * (uint64_t)sm_count;
+  p.per = (all + places - 1) / places;
+  // sums of 2^15 products of bytes stay below 2^31
+  if (p.per > 1024) p.per = 1024;
+  p.blocks = (all + p.per - 1) / p.per;
+  // a column that begins where a piece does has ceil(steps / per) of them; where all columns do, that is all
+  p.slots = (uint32_t)((p.steps + p.per - 1) / p.per + (p.per % p.steps == 0 || p.steps % p.per == 0 ? 0 : 1));
+  return p;
+}
+
 uint32_t from_right_splits(uint64_t lo_n, uint64_t hi_n, int sm_count) {
+  if (hi_n >= kCtRows) return bytes_plan(lo_n, hi_n, sm_count).slots;
   const uint64_t col_blocks = (lo_n + 255) / 256;
   uint64_t want = ((uint64_t)sm_count * 8 + col_blocks - 1) / col_blocks;  // about 8 blocks per SM
   if (want > hi_n) want = hi_n;
@@ -208,13 +423,16 @@ uint32_t from_right_splits(uint64_t lo_n, uint64_t hi_n, int sm_count) {
 int launch_from_right(const Fr* f, const Fr* eq, uint64_t lo_n, uint64_t hi_n, Fr* partial, Fr* out, int sm_count,
                       cudaStream_t s) {
   const uint32_t splits = from_right_splits(lo_n, hi_n, sm_count);
-  const uint64_t per = (hi_n + splits - 1) / splits;
-  dim3 grid((unsigned)((lo_n + 255) / 256), splits);
-  if (splits == 1) {
-    k_from_right<<<grid, 256, 0, s>>>(f, eq, lo_n, hi_n, per, out);
-    return 1;
+  Fr* dst = splits == 1 ? out : partial;
+  if (hi_n >= kCtRows) {
+    const BytesPlan p = bytes_plan(lo_n, hi_n, sm_count);
+    cudaFuncSetAttribute(k_from_right_bytes, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCtShared);
+    k_from_right_bytes<<<(unsigned)p.blocks, kCtThreads, kCtShared, s>>>(f, eq, lo_n, hi_n, (uint32_t)p.groups, (uint32_t)p.steps, p.per, p.slots, dst);
+  } else {
+    const uint64_t per = (hi_n + splits - 1) / splits;
+    k_from_right<<<dim3((unsigned)((lo_n + 255) / 256), splits), 256, 0, s>>>(f, eq, lo_n, hi_n, per, dst);
   }
-  k_from_right<<<grid, 256, 0, s>>>(f, eq, lo_n, hi_n, per, partial);
+  if (splits == 1) return 1;
   k_sum_splits<<<(unsigned)((lo_n + 31) / 32), 256, 0, s>>>(partial, lo_n, splits, out);
   return 2;
 }
