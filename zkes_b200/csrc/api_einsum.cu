@@ -9,7 +9,7 @@ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 }  // namespace
 
 namespace zk {
-int eq_table_device(zk_ctx* ctx, const uint64_t* point_host, uint32_t k, Fr* point_dev, Fr* table);
+int eq_table_device(zk_ctx* ctx, const uint64_t* point_host, uint32_t k, Fr* table, cudaStream_t on = nullptr);
 }
 
 extern "C" {
@@ -75,7 +75,7 @@ int zk_fix_variables_int(zk_ctx* ctx, uint32_t num_vars, const void* t, zk_mem t
   const size_t out_elems = out_mem == ZK_MEM_HOST ? m_cols : 0;
   const size_t part_elems = splits > 1 ? (size_t)splits * m_cols : 0;
   char* base = nullptr;
-  int rc = ctx->reserve_work(in_b + (n_rows + k + 16 + out_elems + part_elems) * sizeof(Fr) + 256, (void**)&base);
+  int rc = ctx->reserve_work(in_b + (n_rows + out_elems + part_elems) * sizeof(Fr) + 256, (void**)&base);
   if (rc) return rc;
   const void* d_t = t;
   if (t_mem == ZK_MEM_HOST) {
@@ -83,10 +83,9 @@ int zk_fix_variables_int(zk_ctx* ctx, uint32_t num_vars, const void* t, zk_mem t
     d_t = base;
   }
   Fr* eq = reinterpret_cast<Fr*>(base + in_b);
-  Fr* pt_dev = eq + n_rows;
-  Fr* d_out = out_mem == ZK_MEM_HOST ? pt_dev + k + 16 : reinterpret_cast<Fr*>(out);
-  Fr* partial = pt_dev + k + 16 + out_elems;
-  rc = eq_table_device(ctx, point, k, pt_dev, eq);
+  Fr* d_out = out_mem == ZK_MEM_HOST ? eq + n_rows : reinterpret_cast<Fr*>(out);
+  Fr* partial = eq + n_rows + out_elems;
+  rc = eq_table_device(ctx, point, k, eq);
   if (rc) return rc;
   ctx->prof_begin(ZK_PROF_OTHER, 16.0 * (double)(1ull << num_vars) + 32.0 * (double)m_cols, 1);
   ctx->launches += launch_int_fold(d_t, eq, n_rows, m_cols, partial, d_out, ctx->sm_count, s);

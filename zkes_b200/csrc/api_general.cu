@@ -8,7 +8,7 @@
 using namespace zk;
 
 namespace zk {
-int eq_table_device(zk_ctx* ctx, const uint64_t* point_host, uint32_t k, Fr* point_dev, Fr* table);
+int eq_table_device(zk_ctx* ctx, const uint64_t* point_host, uint32_t k, Fr* table, cudaStream_t on = nullptr);
 size_t keyset_scratch_bytes(uint32_t n_terms, uint32_t num_var);
 int keyset_order(zk_ctx* ctx, const uint64_t* positions_dev, const uint64_t* term_begin_dev, uint32_t n_terms, uint64_t total,
                  uint32_t num_var, void* scratch, uint32_t* keys_out, uint32_t bad_host[2]);
@@ -49,7 +49,7 @@ int sbool_prove(zk_ctx* ctx, zk_comm* comm, uint32_t num_var, uint32_t n_terms, 
   cudaStream_t s = ctx->stream;
   const uint64_t size = 1ull << num_var;
   char* base = nullptr;
-  size_t need = al((size + size / 2 + 8) * sizeof(Fr)) + al((size / 2 * 3 + 8) * sizeof(Fr)) + al((num_var + 8) * sizeof(Fr)) + 2 * (al((K + 1) * 4ull) + al((K + 1) * sizeof(Fr))) +
+  size_t need = al((size + size / 2 + 8) * sizeof(Fr)) + al((size / 2 * 3 + 8) * sizeof(Fr)) + 2 * (al((K + 1) * 4ull) + al((K + 1) * sizeof(Fr))) +
                 al((K / 256 + 2) * 4ull) + al((n_terms + 1) * sizeof(Fr)) + 4096;
   int rc = ctx->reserve_work(need, (void**)&base);
   if (rc) return rc;
@@ -58,7 +58,6 @@ int sbool_prove(zk_ctx* ctx, zk_comm* comm, uint32_t num_var, uint32_t n_terms, 
   Fr* eq0 = (Fr*)take((size + 1) * sizeof(Fr));
   Fr* eq1 = (Fr*)take((size / 2 + 1) * sizeof(Fr));
   Fr* eq_rec = (Fr*)take((size / 2 * 3 + 8) * sizeof(Fr));  // per-position records of the rounds after the first
-  Fr* pt_dev = (Fr*)take((num_var + 8) * sizeof(Fr));
   uint32_t* e_key[2] = {(uint32_t*)take((K + 1) * 4ull), (uint32_t*)take((K + 1) * 4ull)};
   Fr* e_val[2] = {(Fr*)take((K + 1) * sizeof(Fr)), (Fr*)take((K + 1) * sizeof(Fr))};
   uint32_t* block_counts = (uint32_t*)take((K / 256 + 2) * 4ull);
@@ -88,7 +87,7 @@ int sbool_prove(zk_ctx* ctx, zk_comm* comm, uint32_t num_var, uint32_t n_terms, 
     ctx->launches++;
   }
   // dense eq(eq_challenge, .) over the full hypercube (:509)
-  rc = eq_table_device(ctx, eq_point, num_var, pt_dev, eq0);
+  rc = eq_table_device(ctx, eq_point, num_var, eq0);
   if (rc) return rc;
   ZK_CUDA(cudaStreamSynchronize(s));  // keys / weights host buffers may go out of scope after this
 

@@ -18,7 +18,7 @@ int normalize_device(zk_ctx* ctx, const Jacobian* in, uint64_t n, Affine* out);
 size_t from_right_scratch_elems(zk_ctx* ctx, uint32_t n, uint32_t k);
 int fix_from_right_device(zk_ctx* ctx, uint32_t n, const Fr* f_dev, uint32_t k, const uint64_t* point_host, Fr* scratch,
                           Fr* out_dev);
-int eq_table_device(zk_ctx* ctx, const uint64_t* point_host, uint32_t k, Fr* point_dev, Fr* table);
+int eq_table_device(zk_ctx* ctx, const uint64_t* point_host, uint32_t k, Fr* table, cudaStream_t on = nullptr);
 }  // namespace zk
 
 namespace {
@@ -99,7 +99,7 @@ void pad_point(const uint64_t* point, uint32_t point_len, uint32_t n, std::vecto
 // sharded entry points; scratch is kzh3_tail_bytes() of device memory.
 size_t kzh3_tail_bytes(zk_ctx* ctx, const zk_kzh_srs* srs) {
   const uint64_t nx = 1ull << srs->x_log, ny = 1ull << srs->y_log, nz = 1ull << srs->z_log;
-  return al(nz * sizeof(Fr)) + al((nx + 8) * sizeof(Fr)) * 2 +
+  return al(nz * sizeof(Fr)) + al((nx + 8) * sizeof(Fr)) +
          al(from_right_scratch_elems(ctx, srs->y_log + srs->z_log, srs->y_log) * sizeof(Fr)) + al((nx + 2) * sizeof(Jacobian)) +
          al((ny + 2) * sizeof(Jacobian)) + al((nx + 1) * sizeof(Affine)) + 2048;
 }
@@ -115,7 +115,6 @@ int kzh3_open_tail(zk_ctx* ctx, const zk_kzh_srs* srs, const Fr* f_prime, const 
   auto take = [&](size_t bytes) { char* p = mem + off; off += al(bytes); return p; };
   Fr* f_star = (Fr*)take(nz * sizeof(Fr));
   Fr* eq_x = (Fr*)take((nx + 8) * sizeof(Fr));
-  Fr* pt_dev = (Fr*)take((nx + 8) * sizeof(Fr));
   Fr* scratch = (Fr*)take(from_right_scratch_elems(ctx, yl + zl, yl) * sizeof(Fr));
   Jacobian* d_dx = (Jacobian*)take((nx + 2) * sizeof(Jacobian));
   Jacobian* d_dy = (Jacobian*)take((ny + 2) * sizeof(Jacobian));
@@ -136,7 +135,7 @@ int kzh3_open_tail(zk_ctx* ctx, const zk_kzh_srs* srs, const Fr* f_prime, const 
   ZK_CUDA(cudaMemcpyAsync(d_dx, d_x_jac, nx * sizeof(Jacobian), cudaMemcpyHostToDevice, st));
   rc = normalize_device(ctx, d_dx, nx, d_aff);
   if (rc) return rc;
-  rc = eq_table_device(ctx, r_x, xl, pt_dev, eq_x);
+  rc = eq_table_device(ctx, r_x, xl, eq_x);
   if (rc) return rc;
   ctx->prof_begin(ZK_PROF_MSM, 0.0, 8);
   rc = msm_run(ctx, d_aff, nullptr, eq_x, nx, 1, d_dy + ny, &ctx->last_msm);
@@ -195,7 +194,7 @@ __global__ void __launch_bounds__(256) k_limbs_to_fr(const unsigned long long* _
 // f_prime (device, 2^(n - x_log) elements) of a sparse polynomial.  mem: sparse_contract_bytes() of device memory.
 size_t sparse_contract_bytes(const zk_kzh_srs* srs, uint64_t nnz, bool with_vals) {
   const uint64_t nx = 1ull << srs->x_log, lo_n = 1ull << (srs->n - srs->x_log);
-  return al(nnz * 8 + 8) + (with_vals ? al(nnz * sizeof(Fr) + 32) : 0) + al((nx + srs->x_log + 16) * sizeof(Fr)) + al(lo_n * 64) + 512;
+  return al(nnz * 8 + 8) + (with_vals ? al(nnz * sizeof(Fr) + 32) : 0) + al(nx * sizeof(Fr)) + al(lo_n * 64) + 512;
 }
 
 int sparse_contract_x(zk_ctx* ctx, const zk_kzh_srs* srs, uint64_t nnz, const uint64_t* indices, const uint64_t* vals,
@@ -207,14 +206,14 @@ int sparse_contract_x(zk_ctx* ctx, const zk_kzh_srs* srs, uint64_t nnz, const ui
   auto take = [&](size_t bytes) { char* p = mem + off; off += al(bytes); return p; };
   uint64_t* d_idx = (uint64_t*)take(nnz * 8 + 8);
   Fr* d_val = vals ? (Fr*)take(nnz * sizeof(Fr) + 32) : nullptr;
-  Fr* eq = (Fr*)take((nx + xl + 16) * sizeof(Fr));
+  Fr* eq = (Fr*)take(nx * sizeof(Fr));
   unsigned long long* limbs = (unsigned long long*)take(lo_n * 64);
   unsigned int* bad = ctx->rs.sink.counter + 16;
   if (nnz) {
     ZK_CUDA(cudaMemcpyAsync(d_idx, indices, nnz * 8, cudaMemcpyHostToDevice, st));
     if (vals) ZK_CUDA(cudaMemcpyAsync(d_val, vals, nnz * sizeof(Fr), cudaMemcpyHostToDevice, st));
   }
-  int rc = eq_table_device(ctx, r_x, xl, eq + nx, eq);
+  int rc = eq_table_device(ctx, r_x, xl, eq);
   if (rc) return rc;
   ZK_CUDA(cudaMemsetAsync(limbs, 0, lo_n * 64, st));
   ZK_CUDA(cudaMemsetAsync(bad, 0, 4, st));
@@ -471,13 +470,12 @@ static int kzh_open_sharded_impl(zk_ctx* ctx, zk_comm* comm, const zk_kzh_srs* s
   const uint64_t* r_x = pt.data() + (size_t)(n - xl) * 4;
   const uint32_t splits = from_right_splits(lo_n, hi_local, ctx->sm_count);
   char* base = nullptr;
-  size_t need = al((xl + 8) * sizeof(Fr)) + al(hi_n * sizeof(Fr)) + al((size_t)splits * lo_n * sizeof(Fr)) + al(lo_n * sizeof(Fr)) +
+  size_t need = al(hi_n * sizeof(Fr)) + al((size_t)splits * lo_n * sizeof(Fr)) + al(lo_n * sizeof(Fr)) +
                 (evals_mem == ZK_MEM_HOST ? al(slab * sizeof(Fr)) : 0) + (k3 ? kzh3_tail_bytes(ctx, srs) : 0) + 1024;
   int rc = ctx->reserve_work(need, (void**)&base);
   if (rc) return rc;
   size_t off = 0;
   auto take = [&](size_t bytes) { char* p = base + off; off += al(bytes); return p; };
-  Fr* pt_dev = (Fr*)take((xl + 8) * sizeof(Fr));
   Fr* eq = (Fr*)take(hi_n * sizeof(Fr));
   Fr* partial = (Fr*)take((size_t)splits * lo_n * sizeof(Fr));
   Fr* f_prime = (Fr*)take(lo_n * sizeof(Fr));
@@ -488,7 +486,7 @@ static int kzh_open_sharded_impl(zk_ctx* ctx, zk_comm* comm, const zk_kzh_srs* s
     f = p;
   }
   char* tail_mem = k3 ? take(kzh3_tail_bytes(ctx, srs)) : nullptr;
-  rc = eq_table_device(ctx, r_x, xl, pt_dev, eq);
+  rc = eq_table_device(ctx, r_x, xl, eq);
   if (rc) return rc;
   ctx->launches += launch_from_right(f, eq + hi_local * rank, lo_n, hi_local, partial, f_prime, ctx->sm_count, st);
   rc = comm_sum_fr_vec(ctx, comm, f_prime, lo_n);
@@ -532,7 +530,7 @@ int zk_kzh_verify_g1(zk_ctx* ctx, const zk_kzh_srs* srs, const uint64_t* point, 
   const uint64_t* r_x = pt.data() + (size_t)(k3 ? zl + yl : yl) * 4;
   const uint64_t n_big = nx > ny ? nx : ny;
   char* base = nullptr;
-  size_t need = al((n_big + 1) * sizeof(Jacobian)) + al((n_big + 1) * sizeof(Affine)) + al((n_big + 40) * sizeof(Fr)) * 2 +
+  size_t need = al((n_big + 1) * sizeof(Jacobian)) + al((n_big + 1) * sizeof(Affine)) + al((n_big + 40) * sizeof(Fr)) +
                 al(n_low * sizeof(Fr)) * 2 + al(8 * sizeof(Jacobian)) + al(8 * sizeof(Affine)) + 2048;
   int rc = ctx->reserve_work(need, (void**)&base);
   if (rc) return rc;
@@ -541,7 +539,6 @@ int zk_kzh_verify_g1(zk_ctx* ctx, const zk_kzh_srs* srs, const uint64_t* point, 
   Jacobian* d_jac = (Jacobian*)take((n_big + 1) * sizeof(Jacobian));
   Affine* d_aff = (Affine*)take((n_big + 1) * sizeof(Affine));
   Fr* eq = (Fr*)take((n_big + 40) * sizeof(Fr));
-  Fr* pt_dev = (Fr*)take((n_big + 40) * sizeof(Fr));
   Fr* d_fstar = (Fr*)take(n_low * sizeof(Fr));
   Fr* eq_low = (Fr*)take(n_low * sizeof(Fr));
   Jacobian* res = (Jacobian*)take(8 * sizeof(Jacobian));
@@ -551,7 +548,7 @@ int zk_kzh_verify_g1(zk_ctx* ctx, const zk_kzh_srs* srs, const uint64_t* point, 
   ZK_CUDA(cudaMemcpyAsync(d_jac, d_x_jac, nx * sizeof(Jacobian), cudaMemcpyHostToDevice, st));
   rc = normalize_device(ctx, d_jac, nx, d_aff);
   if (rc) return rc;
-  rc = eq_table_device(ctx, r_x, xl, pt_dev, eq);
+  rc = eq_table_device(ctx, r_x, xl, eq);
   if (rc) return rc;
   rc = msm_run(ctx, d_aff, nullptr, eq, nx, 1, res + 0, nullptr);
   if (rc) return rc;
@@ -563,7 +560,7 @@ int zk_kzh_verify_g1(zk_ctx* ctx, const zk_kzh_srs* srs, const uint64_t* point, 
     ZK_CUDA(cudaMemcpyAsync(d_jac, d_y_jac, ny * sizeof(Jacobian), cudaMemcpyHostToDevice, st));
     rc = normalize_device(ctx, d_jac, ny, d_aff);
     if (rc) return rc;
-    rc = eq_table_device(ctx, r_y3, yl, pt_dev, eq);
+    rc = eq_table_device(ctx, r_y3, yl, eq);
     if (rc) return rc;
     rc = msm_run(ctx, d_aff, nullptr, eq, ny, 1, res + 2, nullptr);
     if (rc) return rc;
@@ -571,7 +568,7 @@ int zk_kzh_verify_g1(zk_ctx* ctx, const zk_kzh_srs* srs, const uint64_t* point, 
   rc = normalize_device(ctx, res, k3 ? 3 : 2, res_aff);
   if (rc) return rc;
   // f_star(r_low)
-  rc = eq_table_device(ctx, r_low, low_log, pt_dev, eq_low);
+  rc = eq_table_device(ctx, r_low, low_log, eq_low);
   if (rc) return rc;
   RoundScratch sc = ctx->rs;
   sc.sink.pub_flag = nullptr;

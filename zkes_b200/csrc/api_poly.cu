@@ -5,29 +5,31 @@
 using namespace zk;
 
 namespace zk {
-// Builds eq(., point) in `table` (device, 2^k elements); `point_dev` is device scratch for k elements.
-int eq_table_device(zk_ctx* ctx, const uint64_t* point_host, uint32_t k, Fr* point_dev, Fr* table) {
-  cudaStream_t s = ctx->stream;
-  if (k) ZK_CUDA(cudaMemcpyAsync(point_dev, point_host, (size_t)k * sizeof(Fr), cudaMemcpyHostToDevice, s));
-  ctx->prof_begin(ZK_PROF_FROM_RIGHT, 32.0 * (double)(1ull << k), 1);  // every entry written once, nothing but the point read
-  ctx->launches += launch_eq_table(point_dev, k, table, ctx->sm_count, s);
-  ctx->prof_end();
+// Builds eq(., point) in `table` (device, 2^k elements), on the lane's stream or on another one of it.
+int eq_table_device(zk_ctx* ctx, const uint64_t* point_host, uint32_t k, Fr* table, cudaStream_t on = nullptr) {
+  if (k > kEqMax) return fail(ZK_ERR_ARG, "eq table: %u variables are too many", k);
+  cudaStream_t s = on ? on : ctx->stream;
+  EqPoint point;
+  if (k) memcpy(point.r, point_host, (size_t)k * sizeof(Fr));
+  memset(point.r + k, 0, (kEqMax - k) * sizeof(Fr));
+  if (s == ctx->stream) ctx->prof_begin(ZK_PROF_FROM_RIGHT, 32.0 * (double)(1ull << k), 1);  // every entry written once, nothing but the point read
+  ctx->launches += launch_eq_table(point, k, table, ctx->sm_count, s);
+  if (s == ctx->stream) ctx->prof_end();
   return ZK_OK;
 }
 
 // out_dev[lo] = sum_hi eq(point)[hi] f[hi * 2^(n-k) + lo]; f_dev holds 2^n elements on the device.
-// scratch must hold k + 2^k + splits * 2^(n-k) elements.
+// scratch must hold 2^k + splits * 2^(n-k) elements.
 size_t from_right_scratch_elems(zk_ctx* ctx, uint32_t n, uint32_t k) {
   const uint64_t lo_n = 1ull << (n - k), hi_n = 1ull << k;
-  return (size_t)k + 8 + hi_n + (size_t)from_right_splits(lo_n, hi_n, ctx->sm_count) * lo_n;
+  return hi_n + (size_t)from_right_splits(lo_n, hi_n, ctx->sm_count) * lo_n;
 }
 int fix_from_right_device(zk_ctx* ctx, uint32_t n, const Fr* f_dev, uint32_t k, const uint64_t* point_host, Fr* scratch,
                           Fr* out_dev) {
   const uint64_t lo_n = 1ull << (n - k), hi_n = 1ull << k;
-  Fr* point_dev = scratch;
-  Fr* eq = scratch + k + 8;
+  Fr* eq = scratch;
   Fr* partial = eq + hi_n;
-  int rc = eq_table_device(ctx, point_host, k, point_dev, eq);
+  int rc = eq_table_device(ctx, point_host, k, eq);
   if (rc) return rc;
   ctx->prof_begin(ZK_PROF_FROM_RIGHT, 32.0 * (double)((1ull << n) + lo_n), 1);
   ctx->launches += launch_from_right(f_dev, eq, lo_n, hi_n, partial, out_dev, ctx->sm_count, ctx->stream);
@@ -46,10 +48,10 @@ int zk_eq_table(zk_ctx* ctx, uint32_t k, const uint64_t* point, uint64_t* out, z
   ctx = lk.lane;
   const uint64_t size = 1ull << k;
   Fr* base = nullptr;
-  int rc = ctx->reserve_work((k + 8 + (out_mem == ZK_MEM_HOST ? size : 0)) * sizeof(Fr), (void**)&base);
+  int rc = ctx->reserve_work((out_mem == ZK_MEM_HOST ? size : 0) * sizeof(Fr) + 256, (void**)&base);
   if (rc) return rc;
-  Fr* table = out_mem == ZK_MEM_HOST ? base + k + 8 : reinterpret_cast<Fr*>(out);
-  rc = eq_table_device(ctx, point, k, base, table);
+  Fr* table = out_mem == ZK_MEM_HOST ? base : reinterpret_cast<Fr*>(out);
+  rc = eq_table_device(ctx, point, k, table);
   if (rc) return rc;
   ZK_CUDA(cudaGetLastError());
   if (out_mem == ZK_MEM_HOST) ZK_CUDA(cudaMemcpyAsync(out, table, size * sizeof(Fr), cudaMemcpyDeviceToHost, ctx->stream));
@@ -107,7 +109,7 @@ int zk_mle_eval(zk_ctx* ctx, uint32_t n, const uint64_t* evals, zk_mem evals_mem
     f = base;
   }
   Fr* eq = base + in_elems;
-  rc = eq_table_device(ctx, point, n, eq + size, eq);
+  rc = eq_table_device(ctx, point, n, eq);
   if (rc) return rc;
   RoundScratch sc = ctx->rs;
   sc.sink.pub_flag = nullptr;  // read back with a copy: nothing polls this result

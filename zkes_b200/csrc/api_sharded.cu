@@ -12,7 +12,7 @@ namespace zk {
 int comm_sum_points_n(zk_ctx* ctx, zk_comm* c, Jacobian* points, int n_points);
 int comm_sum_fr_vec(zk_ctx* ctx, zk_comm* c, Fr* vals, uint64_t n);
 int normalize_device(zk_ctx* ctx, const Jacobian* in, uint64_t n, Affine* out);
-int eq_table_device(zk_ctx* ctx, const uint64_t* point_host, uint32_t k, Fr* point_dev, Fr* table);
+int eq_table_device(zk_ctx* ctx, const uint64_t* point_host, uint32_t k, Fr* table, cudaStream_t on = nullptr);
 }  // namespace zk
 
 namespace {
@@ -133,13 +133,12 @@ static int fix_from_right_sharded_impl(zk_ctx* ctx, zk_comm* comm, uint32_t n, c
   const uint64_t lo_n = 1ull << (n - k), hi_n = 1ull << k, hi_local = hi_n / world, slab = hi_local * lo_n;
   const uint32_t splits = from_right_splits(lo_n, hi_local, ctx->sm_count);
   char* base = nullptr;
-  size_t need = al((k + 8) * sizeof(Fr)) + al(hi_n * sizeof(Fr)) + al((size_t)splits * lo_n * sizeof(Fr)) + al(lo_n * sizeof(Fr)) + 1024;
+  size_t need = al(hi_n * sizeof(Fr)) + al((size_t)splits * lo_n * sizeof(Fr)) + al(lo_n * sizeof(Fr)) + 1024;
   if (evals_mem == ZK_MEM_HOST) need += al(slab * sizeof(Fr));
   int rc = ctx->reserve_work(need, (void**)&base);
   if (rc) return rc;
   size_t off = 0;
   auto take = [&](size_t bytes) { char* p = base + off; off += al(bytes); return p; };
-  Fr* pt_dev = (Fr*)take((k + 8) * sizeof(Fr));
   Fr* eq = (Fr*)take(hi_n * sizeof(Fr));
   Fr* partial = (Fr*)take((size_t)splits * lo_n * sizeof(Fr));
   Fr* d_out = (Fr*)take(lo_n * sizeof(Fr));
@@ -149,7 +148,7 @@ static int fix_from_right_sharded_impl(zk_ctx* ctx, zk_comm* comm, uint32_t n, c
     ZK_CUDA(cudaMemcpyAsync(p, local_evals, slab * sizeof(Fr), cudaMemcpyHostToDevice, s));
     f = p;
   }
-  rc = eq_table_device(ctx, point, k, pt_dev, eq);
+  rc = eq_table_device(ctx, point, k, eq);
   if (rc) return rc;
   // this rank's share: sum over its hi range with the matching slice of the eq table
   ctx->launches += launch_from_right(f, eq + hi_local * rank, lo_n, hi_local, partial, d_out, ctx->sm_count, s);

@@ -25,74 +25,73 @@ __device__ __forceinline__ void st_fr_plain(Fr* p, const Fr& x) {
   reinterpret_cast<uint4*>(p)[1] = hi;
 }
 
-// The eq table in one launch, in stretches of 2^kEqBits consecutive entries that share their high bits; the factor of the
-// high bits is a product over the variables above kEqBits.  Launches and the multiplier tables that the host made for every
-// level were most of the time of a doubling level by level (2^17 entries: a head launch of 11 us and seven level launches of
-// 2.5 us each, with some 4 us of host work before each).
-//   One stretch a block (up to kEqWave blocks per SM): the factor seeds a doubling over the low variables in shared memory,
-//   a[x + cur] = r a[x], a[x] -= a[x + cur], whose last level goes to global memory; a chain of some twelve products.
-//   More: the doubling starts from one and makes the low table, and a block multiplies it by the factors of its stretches,
-//   one product an entry instead of a chain per stretch (2^21 entries: 54 us against 79 us with a chain for every stretch).
+// The eq table in one launch, in stretches of 2^kEqBits consecutive entries that share their high bits.  A stretch is the outer
+// product of two half tables over its low variables, the upper half times the factor of the high bits (a product over the variables
+// above kEqBits), so that an entry is some six dependent products deep, where doubling the table variable by variable is thirteen:
+// the products are few, and below 2^18 entries their latency is the whole time.
+//   One stretch a block (up to kEqWave blocks per SM): the seeded halves are multiplied out straight into global memory.
+//   More: the halves make the low table in shared memory, and a block multiplies it by the factors of its stretches, one product
+//   an entry instead of halves for every stretch (2^21 entries: 54 us against 79 us with a doubling for every stretch).
+// 2^12 entries take 6.8 us of kernel time, with a doubling 10.3; 2^17 7.3 and 12.4.
+// The point travels as a kernel argument: as a copy it was a call of its own before every table.
 constexpr int kEqBits = 10, kEqThreads = 512, kEqWave = 2;
 
-__device__ __forceinline__ Fr eq_factor(const Fr* __restrict__ point, uint64_t hi, int j) {
-  const Fr r = ldg_fr(point + j);
-  return ((hi >> j) & 1u) ? r : sub(Fr::one(), r);
+__device__ __forceinline__ Fr eq_factor(const EqPoint& point, uint64_t x, int j) {  // x: the entry's bits from variable 0 on
+  const Fr r = point.r[j];
+  return ((x >> j) & 1u) ? r : sub(Fr::one(), r);
+}
+// The factor of `bits` variables from `from` on for an entry with those bits `x`: two interleaved chains of products.
+__device__ __forceinline__ Fr eq_product(const EqPoint& point, int from, int bits, uint64_t x) {
+  Fr f = Fr::one(), g = Fr::one();
+  if (bits > 0) f = eq_factor(point, x << from, from);
+  if (bits > 1) g = eq_factor(point, x << from, from + 1);
+#pragma unroll 1
+  for (int j = 2; j < bits; j += 2) {
+    f = mul(f, eq_factor(point, x << from, from + j));
+    if (j + 1 < bits) g = mul(g, eq_factor(point, x << from, from + j + 1));
+  }
+  return bits > 1 ? mul(f, g) : f;
 }
 
-__global__ void __launch_bounds__(kEqThreads) k_eq_table(Fr* out, const Fr* __restrict__ point, int k) {
+__global__ void __launch_bounds__(kEqThreads) k_eq_table(Fr* out, const EqPoint point, int k) {
   __shared__ Fr sh[1 << kEqBits];
-  __shared__ Fr seeds[kEqThreads];
-  const int low = k < kEqBits ? k : kEqBits, high = k - low;
+  __shared__ Fr seeds[kEqThreads];  // the half tables, later the factors of the stretches
+  const int low = k < kEqBits ? k : kEqBits, high = k - low, low_a = low >> 1, low_b = low - low_a;
   const uint64_t n_hi = 1ull << high;
   const bool seeded = n_hi <= gridDim.x;  // one stretch per block
-  if (threadIdx.x < 32) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  Fr* half_a = seeds;
+  Fr* half_b = seeds + 32;
+  if (warp == 0 && lane < (1 << low_a)) half_a[lane] = eq_product(point, 0, low_a, lane);
+  if (warp == 1 && lane < (1 << low_b)) half_b[lane] = eq_product(point, low_a, low_b, lane);
+  if (warp == 2 && seeded) {
     Fr f = Fr::one();
-    if (seeded) {
-      if ((int)threadIdx.x < high) f = eq_factor(point + low, blockIdx.x, threadIdx.x);
-      int width = 1;
-      while (width < high) width <<= 1;
+    if (lane < high) f = eq_factor(point, (uint64_t)blockIdx.x << low, low + lane);
+    int width = 1;
+    while (width < high) width <<= 1;
 #pragma unroll 1
-      for (int off = width >> 1; off > 0; off >>= 1) {
-        Fr o;
+    for (int off = width >> 1; off > 0; off >>= 1) {
+      Fr o;
 #pragma unroll
-        for (int i = 0; i < 8; i++) o.v[i] = __shfl_down_sync(0xffffffffu, f.v[i], off);
-        f = mul(f, o);
-      }
+      for (int i = 0; i < 8; i++) o.v[i] = __shfl_down_sync(0xffffffffu, f.v[i], off);
+      f = mul(f, o);
     }
-    if (threadIdx.x == 0) {
-      if (low == 0) st_fr_plain(out, f); else sh[0] = f;
-    }
+    if (lane == 0) seeds[64] = f;
   }
   __syncthreads();
-  Fr* dst = out + ((uint64_t)blockIdx.x << low);
-#pragma unroll 1
-  for (int i = 0; i < low; i++) {
-    const uint32_t cur = 1u << i;
-    if (threadIdx.x < cur) {
-      const Fr r = ldg_fr(point + i);
-      const Fr v = sh[threadIdx.x];
-      const Fr hi = mul(r, v), lo = sub(v, hi);
-      if (seeded && i == low - 1) {
-        st_fr_plain(dst + threadIdx.x + cur, hi);
-        st_fr_plain(dst + threadIdx.x, lo);
-      } else {
-        sh[threadIdx.x + cur] = hi;
-        sh[threadIdx.x] = lo;
-      }
-    }
+  if (seeded) {
+    if (threadIdx.x < (1u << low_b)) half_b[threadIdx.x] = mul(half_b[threadIdx.x], seeds[64]);
     __syncthreads();
   }
+  Fr* dst = seeded ? out + ((uint64_t)blockIdx.x << low) : sh;
+#pragma unroll 1
+  for (uint32_t x = threadIdx.x; x < (1u << low); x += kEqThreads) st_fr_plain(dst + x, mul(half_a[x & ((1u << low_a) - 1u)], half_b[x >> low_a]));
   if (seeded) return;
+  __syncthreads();
   // this block's stretches are blockIdx.x, blockIdx.x + gridDim.x, ...: their factors kEqThreads at a time, then the products
   for (uint64_t first = blockIdx.x; first < n_hi; first += (uint64_t)kEqThreads * gridDim.x) {
     const uint64_t mine = first + (uint64_t)threadIdx.x * gridDim.x;
-    if (mine < n_hi) {
-      Fr f = eq_factor(point + low, mine, 0);
-#pragma unroll 1
-      for (int j = 1; j < high; j++) f = mul(f, eq_factor(point + low, mine, j));
-      seeds[threadIdx.x] = f;
-    }
+    if (mine < n_hi) seeds[threadIdx.x] = eq_product(point, low, high, mine);
     __syncthreads();
     for (uint32_t t = 0; t < kEqThreads; t++) {
       const uint64_t hi = first + (uint64_t)t * gridDim.x;
@@ -380,10 +379,10 @@ void launch_dot(const Fr* a, const Fr* b, uint64_t n, const RoundScratch& sc, cu
   k_dot<<<(unsigned)blocks, 256, 0, s>>>(a, b, n, sc.sink);
 }
 
-// out[0 .. 2^k) = eq(., point); point_dev holds the k coordinates on the device.  Returns launches.
-int launch_eq_table(const Fr* point_dev, uint32_t k, Fr* out, int sm_count, cudaStream_t s) {
+// out[0 .. 2^k) = eq(., point), k at most kEqMax.  Returns launches.
+int launch_eq_table(const EqPoint& point, uint32_t k, Fr* out, int sm_count, cudaStream_t s) {
   const uint64_t stretches = k > (uint32_t)kEqBits ? 1ull << (k - kEqBits) : 1, wave = (uint64_t)sm_count * kEqWave;
-  k_eq_table<<<(unsigned)(stretches < wave ? stretches : wave), kEqThreads, 0, s>>>(out, point_dev, (int)k);
+  k_eq_table<<<(unsigned)(stretches < wave ? stretches : wave), kEqThreads, 0, s>>>(out, point, (int)k);
   return 1;
 }
 

@@ -16,7 +16,7 @@
 using namespace zk;
 
 namespace zk {
-int eq_table_device(zk_ctx* ctx, const uint64_t* point_host, uint32_t k, Fr* point_dev, Fr* table);
+int eq_table_device(zk_ctx* ctx, const uint64_t* point_host, uint32_t k, Fr* table, cudaStream_t on = nullptr);
 }
 
 namespace {
@@ -141,14 +141,14 @@ int zk_range_aux_accumulate(zk_ctx* ctx, uint32_t k, const uint64_t* point, uint
   const uint64_t n_inputs = 1ull << k, n_table = 1ull << table_log;
   const bool host_idx = idx_mem == ZK_MEM_HOST, host_acc = acc_mem == ZK_MEM_HOST;
   char* base = nullptr;
-  size_t need = al((n_inputs + k + 16) * sizeof(Fr)) + al(n_table * 64) + 1024;
+  size_t need = al(n_inputs * sizeof(Fr)) + al(n_table * 64) + 1024;
   if (host_idx) need += 2 * al(n_sel * 8 + 8);
   if (host_acc) need += al(n_table * sizeof(Fr));
   int rc = ctx->reserve_work(need, (void**)&base);
   if (rc) return rc;
   size_t off = 0;
   auto take = [&](size_t bytes) { char* p = base + off; off += al(bytes); return p; };
-  Fr* eq = reinterpret_cast<Fr*>(take((n_inputs + k + 16) * sizeof(Fr)));
+  Fr* eq = reinterpret_cast<Fr*>(take(n_inputs * sizeof(Fr)));
   unsigned long long* limbs = reinterpret_cast<unsigned long long*>(take(n_table * 64));
   const uint64_t *d_in = input_idx, *d_tab = table_idx;
   if (host_idx && n_sel) {
@@ -164,7 +164,7 @@ int zk_range_aux_accumulate(zk_ctx* ctx, uint32_t k, const uint64_t* point, uint
     d_acc = reinterpret_cast<Fr*>(take(n_table * sizeof(Fr)));
     ZK_CUDA(cudaMemcpyAsync(d_acc, acc, n_table * sizeof(Fr), cudaMemcpyHostToDevice, s));
   }
-  rc = eq_table_device(ctx, point, k, eq + n_inputs, eq);
+  rc = eq_table_device(ctx, point, k, eq);
   if (rc) return rc;
   ZK_CUDA(cudaMemsetAsync(limbs, 0, n_table * 64, s));
   unsigned int* bad = ctx->rs.sink.counter + 14;  // spare word of the context's counter block
