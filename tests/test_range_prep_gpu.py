@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("k,table_log,n_sel", [(0, 0, 1), (1, 1, 2), (3, 2, 8), (6, 4, 64), (10, 8, 1024), (12, 8, 3000),
-                                               (9, 11, 512), (8, 3, 0)])
+                                               (9, 11, 512), (8, 3, 0), (7, 4, 31), (7, 4, 33), (7, 5, 33), (12, 4, 4095)])
 def test_aux_accumulate_matches_oracle(ctx, k, table_log, n_sel):
     rnd = random.Random(1000 * k + table_log)
     acc = DenseMLPoly.from_evaluations([0] * (1 << table_log))

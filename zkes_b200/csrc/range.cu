@@ -81,6 +81,54 @@ __global__ void __launch_bounds__(256) k_range_scatter_small(const uint64_t* __r
   }
 }
 
+// And for a table of at most kCopiesTable entries, where 32 lanes would meet on 16 counters: eight lanes take a pair, a limb each,
+// and add it into counters of their own, so that no addition is atomic before the block's copies are added up.  2^17 pairs on 16
+// entries take 6.9 us, by atomics on a block's one copy 21.6.  A block's copies are 32 KB for 16 entries, which double with the table
+// while the lanes of a warp meet half as often: larger tables stay with the atomics.
+constexpr uint32_t kCopiesTable = 16;
+constexpr int kCopiesThreads = 256, kCopies = kCopiesThreads / 8;
+__global__ void __launch_bounds__(kCopiesThreads) k_range_scatter_copies(const uint64_t* __restrict__ input_idx,
+                                                                         const uint64_t* __restrict__ table_idx, uint64_t n_sel,
+                                                                         const Fr* __restrict__ eq, uint64_t n_inputs, uint32_t n_table,
+                                                                         unsigned long long* limbs, unsigned int* bad) {
+  __shared__ unsigned long long copies[kCopies][kCopiesTable * 8];
+  const uint32_t lane = threadIdx.x & 31, limb = threadIdx.x & 7;
+  unsigned long long* mine = copies[threadIdx.x >> 3] + limb;
+#pragma unroll
+  for (uint32_t t = 0; t < kCopiesTable; t++) mine[t * 8] = 0;
+  const uint64_t warps = (uint64_t)gridDim.x * (kCopiesThreads / 32), warp = (uint64_t)blockIdx.x * (kCopiesThreads / 32) + (threadIdx.x >> 5);
+  for (uint64_t first = warp * 32; first < n_sel; first += warps * 32) {
+    uint32_t i = 0, t = kCopiesTable;  // kCopiesTable: no pair
+    if (first + lane < n_sel) {
+      const uint64_t in = input_idx[first + lane], to = table_idx[first + lane];
+      if (in < n_inputs && to < n_table) {
+        i = (uint32_t)in;
+        t = (uint32_t)to;
+      } else {
+        atomicExch(bad, 1u);
+      }
+    }
+    uint32_t word[8], at[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {  // the eight lanes of a copy take their eight pairs one after the other
+      const int from = (int)(lane & 24u) + k;
+      at[k] = __shfl_sync(0xffffffffu, t, from);
+      const uint32_t src = __shfl_sync(0xffffffffu, i, from);
+      word[k] = at[k] < kCopiesTable ? __ldg(reinterpret_cast<const uint32_t*>(eq + src) + limb) : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      if (at[k] < kCopiesTable) mine[at[k] * 8] += word[k];
+  }
+  __syncthreads();
+  for (uint32_t k = threadIdx.x; k < n_table * 8; k += kCopiesThreads) {
+    unsigned long long v = 0;
+#pragma unroll 8
+    for (int c = 0; c < kCopies; c++) v += copies[c][k];
+    if (v) atomicAdd(limbs + k, v);
+  }
+}
+
 // part[t] from its limb counters; acc[t] += beta_gamma * part[t]; sink.msg[0] = sum_t part[t] * t.
 __global__ void __launch_bounds__(256) k_range_finish(const unsigned long long* __restrict__ limbs, uint64_t n_table,
                                                       const FixedMul<FrParams> bg, Fr* acc, const MsgSink sink) {
@@ -141,7 +189,7 @@ int zk_range_aux_accumulate(zk_ctx* ctx, uint32_t k, const uint64_t* point, uint
   const uint64_t n_inputs = 1ull << k, n_table = 1ull << table_log;
   const bool host_idx = idx_mem == ZK_MEM_HOST, host_acc = acc_mem == ZK_MEM_HOST;
   char* base = nullptr;
-  size_t need = al(n_inputs * sizeof(Fr)) + al(n_table * 64) + 1024;
+  size_t need = al(n_inputs * sizeof(Fr)) + al(n_table * 64 + 8) + 1024;
   if (host_idx) need += 2 * al(n_sel * 8 + 8);
   if (host_acc) need += al(n_table * sizeof(Fr));
   int rc = ctx->reserve_work(need, (void**)&base);
@@ -149,7 +197,8 @@ int zk_range_aux_accumulate(zk_ctx* ctx, uint32_t k, const uint64_t* point, uint
   size_t off = 0;
   auto take = [&](size_t bytes) { char* p = base + off; off += al(bytes); return p; };
   Fr* eq = reinterpret_cast<Fr*>(take(n_inputs * sizeof(Fr)));
-  unsigned long long* limbs = reinterpret_cast<unsigned long long*>(take(n_table * 64));
+  unsigned long long* limbs = reinterpret_cast<unsigned long long*>(take(n_table * 64 + 8));
+  unsigned int* bad = reinterpret_cast<unsigned int*>(limbs + n_table * 8);  // cleared together with the counters
   const uint64_t *d_in = input_idx, *d_tab = table_idx;
   if (host_idx && n_sel) {
     uint64_t* a = reinterpret_cast<uint64_t*>(take(n_sel * 8 + 8));
@@ -166,13 +215,14 @@ int zk_range_aux_accumulate(zk_ctx* ctx, uint32_t k, const uint64_t* point, uint
   }
   rc = eq_table_device(ctx, point, k, eq);
   if (rc) return rc;
-  ZK_CUDA(cudaMemsetAsync(limbs, 0, n_table * 64, s));
-  unsigned int* bad = ctx->rs.sink.counter + 14;  // spare word of the context's counter block
-  ZK_CUDA(cudaMemsetAsync(bad, 0, 4, s));
+  ZK_CUDA(cudaMemsetAsync(limbs, 0, n_table * 64 + 8, s));
   if (n_sel) {
     uint64_t blocks = (n_sel + 255) / 256;
     if (blocks > (uint64_t)ctx->sm_count * 8) blocks = ctx->sm_count * 8;
-    if (n_table <= kSmallTable) {
+    if (n_table <= kCopiesTable) {
+      if (blocks > (uint64_t)ctx->sm_count) blocks = ctx->sm_count;
+      k_range_scatter_copies<<<(unsigned)blocks, kCopiesThreads, 0, s>>>(d_in, d_tab, n_sel, eq, n_inputs, (uint32_t)n_table, limbs, bad);
+    } else if (n_table <= kSmallTable) {
       if (blocks > (uint64_t)ctx->sm_count * 4) blocks = ctx->sm_count * 4;
       k_range_scatter_small<<<(unsigned)blocks, 256, n_table * 64, s>>>(d_in, d_tab, n_sel, eq, n_inputs, (uint32_t)n_table, limbs, bad);
     } else {
