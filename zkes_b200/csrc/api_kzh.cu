@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(256) k_sparse_contract(const uint64_t* __restr
                                                          uint64_t nnz, uint32_t low_bits, uint64_t limit,
                                                          const Fr* __restrict__ eq, unsigned long long* limbs, unsigned int* bad) {
   for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t i = idx[e];
+    const uint64_t i = idx[e];  // may be the caller's pinned list: read once
     if (i >= limit) {
       atomicExch(bad, 1u);
       continue;
@@ -191,14 +191,15 @@ __global__ void __launch_bounds__(256) k_limbs_to_fr(const unsigned long long* _
   }
 }
 
-// f_prime (device, 2^(n - x_log) elements) of a sparse polynomial.  mem: sparse_contract_bytes() of device memory.
+// f_prime (device, 2^(n - x_log) elements) of a sparse polynomial.  mem: sparse_contract_bytes() of device memory.  *bad_out: a
+// device word that is not zero afterwards when an index was outside the domain.
 size_t sparse_contract_bytes(const zk_kzh_srs* srs, uint64_t nnz, bool with_vals) {
   const uint64_t nx = 1ull << srs->x_log, lo_n = 1ull << (srs->n - srs->x_log);
-  return al(nnz * 8 + 8) + (with_vals ? al(nnz * sizeof(Fr) + 32) : 0) + al(nx * sizeof(Fr)) + al(lo_n * 64) + 512;
+  return al(nnz * 8 + 8) + (with_vals ? al(nnz * sizeof(Fr) + 32) : 0) + al(nx * sizeof(Fr)) + al(lo_n * 64 + 8) + 512;
 }
 
 int sparse_contract_x(zk_ctx* ctx, const zk_kzh_srs* srs, uint64_t nnz, const uint64_t* indices, const uint64_t* vals,
-                      const uint64_t* r_x, char* mem, Fr* f_prime) {
+                      const uint64_t* r_x, char* mem, Fr* f_prime, const unsigned int** bad_out) {
   cudaStream_t st = ctx->stream;
   const uint32_t xl = srs->x_log, low_bits = srs->n - xl;
   const uint64_t nx = 1ull << xl, lo_n = 1ull << low_bits;
@@ -207,20 +208,25 @@ int sparse_contract_x(zk_ctx* ctx, const zk_kzh_srs* srs, uint64_t nnz, const ui
   uint64_t* d_idx = (uint64_t*)take(nnz * 8 + 8);
   Fr* d_val = vals ? (Fr*)take(nnz * sizeof(Fr) + 32) : nullptr;
   Fr* eq = (Fr*)take(nx * sizeof(Fr));
-  unsigned long long* limbs = (unsigned long long*)take(lo_n * 64);
-  unsigned int* bad = ctx->rs.sink.counter + 16;
+  unsigned long long* limbs = (unsigned long long*)take(lo_n * 64 + 8);
+  unsigned int* bad = (unsigned int*)(limbs + lo_n * 8);  // an index outside the domain; cleared together with the counters
+  *bad_out = bad;
+  const uint64_t* from = d_idx;
   if (nnz) {
-    ZK_CUDA(cudaMemcpyAsync(d_idx, indices, nnz * 8, cudaMemcpyHostToDevice, st));
+    from = reinterpret_cast<const uint64_t*>(ctx->device_view(indices, nnz * 8));
+    if (!from) {
+      ZK_CUDA(cudaMemcpyAsync(d_idx, indices, nnz * 8, cudaMemcpyHostToDevice, st));
+      from = d_idx;
+    }
     if (vals) ZK_CUDA(cudaMemcpyAsync(d_val, vals, nnz * sizeof(Fr), cudaMemcpyHostToDevice, st));
   }
   int rc = eq_table_device(ctx, r_x, xl, eq);
   if (rc) return rc;
-  ZK_CUDA(cudaMemsetAsync(limbs, 0, lo_n * 64, st));
-  ZK_CUDA(cudaMemsetAsync(bad, 0, 4, st));
+  ZK_CUDA(cudaMemsetAsync(limbs, 0, lo_n * 64 + 8, st));
   if (nnz) {
     uint64_t blocks = (nnz + 255) / 256;
     if (blocks > (uint64_t)ctx->sm_count * 8) blocks = ctx->sm_count * 8;
-    k_sparse_contract<<<(unsigned)blocks, 256, 0, st>>>(d_idx, d_val, nnz, low_bits, 1ull << srs->n, eq, limbs, bad);
+    k_sparse_contract<<<(unsigned)blocks, 256, 0, st>>>(from, d_val, nnz, low_bits, 1ull << srs->n, eq, limbs, bad);
     ctx->launches++;
   }
   uint64_t blocks = (lo_n + 255) / 256;
@@ -612,11 +618,12 @@ int zk_sparse_kzh2_open(zk_ctx* ctx, const zk_kzh_srs* srs, uint64_t nnz, const 
   int rc = ctx->reserve_work(sparse_contract_bytes(srs, nnz, vals != nullptr) + al(ny * sizeof(Fr)) + 1024, (void**)&base);
   if (rc) return rc;
   Fr* f_star = reinterpret_cast<Fr*>(base);
-  rc = sparse_contract_x(ctx, srs, nnz, indices, vals, pt.data() + (size_t)srs->y_log * 4, base + al(ny * sizeof(Fr)), f_star);
+  const unsigned int* bad = nullptr;
+  rc = sparse_contract_x(ctx, srs, nnz, indices, vals, pt.data() + (size_t)srs->y_log * 4, base + al(ny * sizeof(Fr)), f_star, &bad);
   if (rc) return rc;
-  unsigned int* bad = ctx->rs.sink.counter + 16;
-  ZK_CUDA(cudaMemcpyAsync(f_star_out, f_star, ny * sizeof(Fr), cudaMemcpyDeviceToHost, st));
+  // the flag first: the copy into the caller's buffer, which is seldom pinned, returns when it is through
   ZK_CUDA(cudaMemcpyAsync(ctx->host_small, bad, 4, cudaMemcpyDeviceToHost, st));
+  ZK_CUDA(cudaMemcpyAsync(f_star_out, f_star, ny * sizeof(Fr), cudaMemcpyDeviceToHost, st));
   ZK_CUDA(cudaStreamSynchronize(st));
   if (*reinterpret_cast<const unsigned int*>(ctx->host_small)) return fail(ZK_ERR_ARG, "sparse_kzh2_open: an index is outside the SRS domain");
   return ZK_OK;
@@ -645,9 +652,9 @@ int zk_sparse_kzh3_open(zk_ctx* ctx, const zk_kzh_srs* srs, uint64_t nnz, const 
   Fr* f_prime = reinterpret_cast<Fr*>(base);
   char* tail_mem = base + al(nyz * sizeof(Fr));
   char* contract_mem = tail_mem + kzh3_tail_bytes(ctx, srs);
-  rc = sparse_contract_x(ctx, srs, nnz, indices, vals, pt.data() + (size_t)(srs->y_log + srs->z_log) * 4, contract_mem, f_prime);
+  const unsigned int* bad = nullptr;
+  rc = sparse_contract_x(ctx, srs, nnz, indices, vals, pt.data() + (size_t)(srs->y_log + srs->z_log) * 4, contract_mem, f_prime, &bad);
   if (rc) return rc;
-  unsigned int* bad = ctx->rs.sink.counter + 16;
   ZK_CUDA(cudaMemcpyAsync(ctx->host_small, bad, 4, cudaMemcpyDeviceToHost, st));
   ZK_CUDA(cudaStreamSynchronize(st));
   if (*reinterpret_cast<const unsigned int*>(ctx->host_small)) return fail(ZK_ERR_ARG, "sparse_kzh3_open: an index is outside the SRS domain");

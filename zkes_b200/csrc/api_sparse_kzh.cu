@@ -74,10 +74,14 @@ int zk_sparse_kzh_commit(zk_ctx* ctx, const zk_kzh_srs* srs, uint64_t nnz, const
     uint64_t* h_begin = reinterpret_cast<uint64_t*>(reinterpret_cast<char*>(ctx->host_small) + 2048);
     h_begin[0] = 0;
     h_begin[1] = nnz;
-    ZK_CUDA(cudaMemcpyAsync(d_idx, indices, nnz * 8, cudaMemcpyHostToDevice, st));
+    const uint64_t* from = reinterpret_cast<const uint64_t*>(ctx->device_view(indices, nnz * 8));
+    if (!from) {
+      ZK_CUDA(cudaMemcpyAsync(d_idx, indices, nnz * 8, cudaMemcpyHostToDevice, st));
+      from = d_idx;
+    }
     ZK_CUDA(cudaMemcpyAsync(d_begin, h_begin, 16, cudaMemcpyHostToDevice, st));
     uint32_t bad_keys[2] = {0, 0};
-    rc = keyset_order(ctx, d_idx, d_begin, 1, nnz, srs->n, ks, d_full, bad_keys);
+    rc = keyset_order(ctx, from, d_begin, 1, nnz, srs->n, ks, d_full, bad_keys);
     if (rc) return rc;
     if (bad_keys[0]) return fail(ZK_ERR_ARG, "sparse_kzh_commit: an index is outside the SRS domain");
     if (!bad_keys[1]) {

@@ -1,3 +1,4 @@
+#include <cuda.h>
 #include "ctx.hpp"
 
 using namespace zk;
@@ -144,6 +145,31 @@ int zk_ctx::reserve_cmp(size_t bytes, void** out) {
   if (rc) return rc;
   *out = cmp;
   return 0;
+}
+
+const void* zk_ctx::device_view(const void* host, size_t bytes) const {
+  typedef CUresult (*PointerAttribute)(void*, CUpointer_attribute, CUdeviceptr);
+  static const PointerAttribute attribute = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &f, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<PointerAttribute>(f);
+  }();
+  cudaPointerAttributes at;
+  if (!attribute || cudaPointerGetAttributes(&at, host) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (at.type != cudaMemoryTypeHost || !at.devicePointer) return nullptr;
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  const CUdeviceptr p = (CUdeviceptr)(uintptr_t)host;
+  if (attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, p) != CUDA_SUCCESS || attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, p) != CUDA_SUCCESS)
+    return nullptr;
+  return p >= start && p + bytes <= start + size ? at.devicePointer : nullptr;
 }
 
 int zk_ctx::reserve_work(size_t bytes, void** out) {
