@@ -64,32 +64,52 @@ int sbool_prove(zk_ctx* ctx, zk_comm* comm, uint32_t num_var, uint32_t n_terms, 
   Fr* d_w = (Fr*)take((n_terms + 1) * sizeof(Fr));
   uint32_t* counts = (uint32_t*)take(256);
 
+  char* ks = nullptr;
+  const size_t pos_bytes = al((size_t)K * 8), tb_bytes = al((size_t)(n_terms + 1) * 8);
   if (K) {
-    char* ks = nullptr;
-    const size_t pos_bytes = al((size_t)K * 8), tb_bytes = al((size_t)(n_terms + 1) * 8);
     rc = ctx->reserve_aux(pos_bytes + tb_bytes + keyset_scratch_bytes(n_terms, num_var), (void**)&ks);
     if (rc) return rc;
+  }
+  // What does not depend on the positions runs on the side stream while they cross the bus: the eq table over the full hypercube
+  // (:509), the entries' first values, the weights.  With the per-kernel profiler on it stays in line.
+  const bool beside = !ctx->prof_on;
+  cudaStream_t s2 = beside ? ctx->side_stream : s;
+  if (beside) {
+    ZK_CUDA(cudaEventRecord(ctx->ev_fork, s));
+    ZK_CUDA(cudaStreamWaitEvent(s2, ctx->ev_fork, 0));
+  }
+  auto prepare = [&]() -> int {
+    if (n_terms) ZK_CUDA(cudaMemcpyAsync(d_w, weights, (size_t)n_terms * sizeof(Fr), cudaMemcpyHostToDevice, s2));
+    ZK_CUDA(cudaMemsetAsync(counts, 0, 256, s2));
+    ZK_CUDA(cudaMemcpyAsync(counts, &K, 4, cudaMemcpyHostToDevice, s2));
+    if (K) {
+      launch_fill_ones(e_val[0], K, ctx->sm_count, s2);
+      ctx->launches++;
+    }
+    return eq_table_device(ctx, eq_point, num_var, eq0, s2);
+  };
+  auto order = [&](uint32_t (&bad)[2]) -> int {
     uint64_t* d_pos = reinterpret_cast<uint64_t*>(ks);
     uint64_t* d_tb = reinterpret_cast<uint64_t*>(ks + pos_bytes);
-    ZK_CUDA(cudaMemcpyAsync(d_pos, positions, (size_t)K * 8, cudaMemcpyHostToDevice, s));
+    const uint64_t* from = reinterpret_cast<const uint64_t*>(ctx->device_view(positions, (size_t)K * 8));
+    if (!from) {
+      ZK_CUDA(cudaMemcpyAsync(d_pos, positions, (size_t)K * 8, cudaMemcpyHostToDevice, s));
+      from = d_pos;
+    }
     ZK_CUDA(cudaMemcpyAsync(d_tb, term_begin.data(), (size_t)(n_terms + 1) * 8, cudaMemcpyHostToDevice, s));
-    uint32_t bad[2] = {0, 0};
-    rc = keyset_order(ctx, d_pos, d_tb, n_terms, K, num_var, ks + pos_bytes + tb_bytes, e_key[0], bad);
-    if (rc) return rc;
-    if (bad[0]) return fail(ZK_ERR_ARG, "sparse_bool_prove: position out of range in term %u", bad[0] - 1);
-    if (bad[1]) return fail(ZK_ERR_ARG, "sparse_bool_prove: duplicate position in term %u", bad[1] - 1);
+    return keyset_order(ctx, from, d_tb, n_terms, K, num_var, ks + pos_bytes + tb_bytes, e_key[0], bad);
+  };
+  rc = prepare();
+  uint32_t bad[2] = {0, 0};
+  if (!rc && K) rc = order(bad);
+  if (beside) {  // whatever happened, the stream that owns the scratch goes on after the side stream
+    ZK_CUDA(cudaEventRecord(ctx->ev_join, s2));
+    ZK_CUDA(cudaStreamWaitEvent(s, ctx->ev_join, 0));
   }
-  if (n_terms) ZK_CUDA(cudaMemcpyAsync(d_w, weights, (size_t)n_terms * sizeof(Fr), cudaMemcpyHostToDevice, s));
-  ZK_CUDA(cudaMemsetAsync(counts, 0, 256, s));
-  ZK_CUDA(cudaMemcpyAsync(counts, &K, 4, cudaMemcpyHostToDevice, s));
-  if (K) {
-    launch_fill_ones(e_val[0], K, ctx->sm_count, s);
-    ctx->launches++;
-  }
-  // dense eq(eq_challenge, .) over the full hypercube (:509)
-  rc = eq_table_device(ctx, eq_point, num_var, eq0);
   if (rc) return rc;
-  ZK_CUDA(cudaStreamSynchronize(s));  // keys / weights host buffers may go out of scope after this
+  if (bad[0]) return fail(ZK_ERR_ARG, "sparse_bool_prove: position out of range in term %u", bad[0] - 1);
+  if (bad[1]) return fail(ZK_ERR_ARG, "sparse_bool_prove: duplicate position in term %u", bad[1] - 1);
+  ZK_CUDA(cudaStreamSynchronize(s));  // the weights' host buffer may go out of scope after this
 
   const Fr* eq_cur = eq0;
   int e = 0;
@@ -103,16 +123,19 @@ int sbool_prove(zk_ctx* ctx, zk_comm* comm, uint32_t num_var, uint32_t n_terms, 
     launch_sbool_msg(e_key[e], e_val[e], counts + e, k_upper, round ? eq_rec : eq_cur, d_w, vars_left, round == 0,
                      ctx->next_msg_scratch(comm != nullptr), s);
     ctx->launches++;
+    // where the folded entries go depends on the positions alone: it is worked out while the host has the message
+    auto slots = [&] {
+      ctx->launches += launch_sparse_slots(e_key[e], counts + e, k_upper, block_counts, counts + (e ^ 1), s);
+    };
+    if (!comm) slots();
     rc = fs_round(ctx, comm, 4, round, fs, fs_user, tr, round_msgs, challenges, &challenge);
     if (rc) return rc;
     Fr* eq_next = (round & 1) ? eq0 : eq1;  // eq0 holds 2^n, eq1 2^(n-1); later rounds fit either
-    if (S >= 4)
-      launch_eq_fold_records(eq_cur, S / 4, challenge, eq_next, eq_rec, ctx->sm_count, s);
-    else
-      launch_fold(eq_cur, eq_next, challenge, S / 2, ctx->rs.max_blocks, s);
+    if (comm) slots();  // (there the exchange kernel is next on the stream)
+    launch_bool_fold(e_key[e], e_val[e], counts + e, k_upper, challenge, block_counts, e_key[e ^ 1], e_val[e ^ 1], eq_cur, S, eq_next, eq_rec,
+                     ctx->sm_count, s);
+    ctx->launches++;
     eq_cur = eq_next;
-    ctx->launches += 1 + launch_sparse_fold(e_key[e], e_val[e], counts + e, k_upper, challenge, block_counts, e_key[e ^ 1],
-                                            e_val[e ^ 1], counts + (e ^ 1), s);
     e ^= 1;
     // a term keeps at most one entry per remaining position: the bound the next round's grids are sized by
     const uint64_t cap = (uint64_t)n_terms * (S / 2);

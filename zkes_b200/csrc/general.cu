@@ -30,7 +30,7 @@ __device__ __forceinline__ Fr g_ld(const Fr* p) {
 // one entry in sixteen for the selection polynomials of the lookups; those entries are queued per warp and worked
 // off thirty-two at a time, so that the rare case does not cost every warp its products.
 //
-// The eq factors come from a per-position record built once per round (k_eq_fold_records; the table is far smaller than
+// The eq factors come from a per-position record built once per round (k_bool_fold; the table is far smaller than
 // the entry list, which repeats every position once per term): an even position holds {eq(0), eq(2), 2 eq(3)}, an
 // odd one {eq(1), 2 eq(2), 3 eq(3)}, so the entry's own factors are q - v, then q + v or 2q - v, then 2q + v or
 // 3q - v: sums of at most four field elements, formed without reduction (they stay below 2^256, which the second
@@ -42,28 +42,6 @@ __device__ __forceinline__ Fr g_ld(const Fr* p) {
 // ONES: the first round, where every value is one (the selection polynomials are 0/1): an entry alone gives
 // 2 eq(2) and 6 eq(3), a pair nothing; no value is read and nothing is multiplied but the weights.
 constexpr int kPairQueue = 64;  // per warp: a batch of 32 plus what one more sweep can add
-
-// Binds the eq table's lowest variable on the round's challenge and writes the next round's records in the same pass: the
-// folded table would only be read again for them (194 us for a 21-variable check; 157 us for the records and 80 us for the
-// folds as launches of their own).
-__global__ void __launch_bounds__(256) k_eq_fold_records(const Fr* __restrict__ eq, uint64_t pairs, const FixedMul<FrParams> r,
-                                                         Fr* __restrict__ next, Fr* __restrict__ rec) {
-  for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < pairs; j += (uint64_t)gridDim.x * blockDim.x) {
-    const Fr a0 = g_ld(eq + 4 * j), a1 = g_ld(eq + 4 * j + 1), b0 = g_ld(eq + 4 * j + 2), b1 = g_ld(eq + 4 * j + 3);
-    const Fr e0 = add(a0, mul_fixed(r, sub(a1, a0))), e1 = add(b0, mul_fixed(r, sub(b1, b0)));
-    next[2 * j] = e0;
-    next[2 * j + 1] = e1;
-    const Fr de = sub(e1, e0);
-    const Fr e2 = add(e1, de), e3 = add(e2, de);
-    Fr* out = rec + 6 * j;
-    out[0] = e0;
-    out[1] = e2;
-    out[2] = add(e3, e3);
-    out[3] = e1;
-    out[4] = add(e2, e2);
-    out[5] = add(add(e3, e3), e3);
-  }
-}
 
 template <bool ONES>
 __global__ void __launch_bounds__(kGThreads, 2) k_sbool_msg(const uint32_t* __restrict__ keys, const Fr* __restrict__ val,
@@ -232,17 +210,17 @@ __global__ void __launch_bounds__(kGThreads, 2) k_sbool_msg(const uint32_t* __re
 // final_evaluation (:644-655): eq[0] * sum_j w_j v_j (v_j - 1), v_j = the entry with key j.
 __global__ void k_sbool_final(const uint32_t* keys, const Fr* val, const uint32_t* count, const Fr* eq,
                               const Fr* weights, uint32_t n_terms, Fr* out) {
-  if (threadIdx.x || blockIdx.x) return;
   const uint32_t n = *count;
   const Fr one = Fr::one();
   Fr inner = Fr::zero();
-  for (uint32_t i = 0; i < n; i++) {
+  for (uint32_t i = threadIdx.x; i < n; i += 32) {  // one warp: the terms share the chain of products
     const uint32_t j = keys[i];
     if (j >= n_terms) continue;
     const Fr v = val[i];
     inner = add(inner, mul(weights[j], mul(v, sub(v, one))));
   }
-  out[0] = mul(eq[0], inner);
+  inner = warp_sum(inner);
+  if (threadIdx.x == 0) out[0] = mul(eq[0], inner);
 }
 
 __global__ void k_fill_ones(Fr* out, uint32_t n) {
@@ -339,11 +317,6 @@ void launch_sbool_msg(const uint32_t* keys, const Fr* val, const uint32_t* count
     cudaFuncSetAttribute(k_sbool_msg<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideBytes);
     k_sbool_msg<false><<<g_blocks(upper, sc), kGThreads, kWideBytes, s>>>(keys, val, count, eq, weights, vars_left, sc.sink);
   }
-}
-void launch_eq_fold_records(const Fr* eq, uint64_t pairs, const Fr& r, Fr* next, Fr* rec, int sm_count, cudaStream_t s) {
-  const uint64_t want = (pairs + 255) / 256;
-  const int blocks = (int)(want < (uint64_t)sm_count * 8 ? (want ? want : 1) : (uint64_t)sm_count * 8);
-  k_eq_fold_records<<<blocks, 256, 0, s>>>(eq, pairs, make_fixed_mul(r), next, rec);
 }
 void launch_sbool_final(const uint32_t* keys, const Fr* val, const uint32_t* count, const Fr* eq, const Fr* weights,
                         uint32_t n_terms, Fr* out, cudaStream_t s) {
