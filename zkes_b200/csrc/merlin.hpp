@@ -8,7 +8,33 @@
 
 namespace zk {
 
-inline uint64_t rotl64(uint64_t x, int n) { return n ? (x << n) | (x >> (64 - n)) : x; }
+template <int N>
+inline uint64_t turn(uint64_t x) {
+  return N ? (x << (N & 63)) | (x >> ((64 - N) & 63)) : x;
+}
+inline void chi(uint64_t* row, uint64_t x0, uint64_t x1, uint64_t x2, uint64_t x3, uint64_t x4) {
+  row[0] = x0 ^ (~x1 & x2);
+  row[1] = x1 ^ (~x2 & x3);
+  row[2] = x2 ^ (~x3 & x4);
+  row[3] = x3 ^ (~x4 & x0);
+  row[4] = x4 ^ (~x0 & x1);
+}
+
+// One round from a to b, every lane and rotation by name: lane (x, y) of the rho step, turned by its offset, is lane (y, 2x + 3y) of
+// the chi step.  A permutation takes a CPU core 0.35 us; with the lanes found by index arithmetic it was 3.3 us, most of a host-stepped
+// round's 7 us and 10 us of the start of a transcript.
+inline void keccak_round(const uint64_t* a, uint64_t* b, uint64_t constant) {
+  const uint64_t c0 = a[0] ^ a[5] ^ a[10] ^ a[15] ^ a[20], c1 = a[1] ^ a[6] ^ a[11] ^ a[16] ^ a[21];
+  const uint64_t c2 = a[2] ^ a[7] ^ a[12] ^ a[17] ^ a[22], c3 = a[3] ^ a[8] ^ a[13] ^ a[18] ^ a[23];
+  const uint64_t c4 = a[4] ^ a[9] ^ a[14] ^ a[19] ^ a[24];
+  const uint64_t d0 = c4 ^ turn<1>(c1), d1 = c0 ^ turn<1>(c2), d2 = c1 ^ turn<1>(c3), d3 = c2 ^ turn<1>(c4), d4 = c3 ^ turn<1>(c0);
+  chi(b + 0, turn<0>(a[0] ^ d0), turn<44>(a[6] ^ d1), turn<43>(a[12] ^ d2), turn<21>(a[18] ^ d3), turn<14>(a[24] ^ d4));
+  chi(b + 5, turn<28>(a[3] ^ d3), turn<20>(a[9] ^ d4), turn<3>(a[10] ^ d0), turn<45>(a[16] ^ d1), turn<61>(a[22] ^ d2));
+  chi(b + 10, turn<1>(a[1] ^ d1), turn<6>(a[7] ^ d2), turn<25>(a[13] ^ d3), turn<8>(a[19] ^ d4), turn<18>(a[20] ^ d0));
+  chi(b + 15, turn<27>(a[4] ^ d4), turn<36>(a[5] ^ d0), turn<10>(a[11] ^ d1), turn<15>(a[17] ^ d2), turn<56>(a[23] ^ d3));
+  chi(b + 20, turn<62>(a[2] ^ d2), turn<55>(a[8] ^ d3), turn<39>(a[14] ^ d4), turn<41>(a[15] ^ d0), turn<2>(a[21] ^ d1));
+  b[0] ^= constant;
+}
 
 inline void keccak_f1600(uint64_t a[25]) {
   static const uint64_t RC[24] = {
@@ -18,29 +44,10 @@ inline void keccak_f1600(uint64_t a[25]) {
       0x000000008000808Bull, 0x800000000000008Bull, 0x8000000000008089ull, 0x8000000000008003ull,
       0x8000000000008002ull, 0x8000000000000080ull, 0x000000000000800Aull, 0x800000008000000Aull,
       0x8000000080008081ull, 0x8000000000008080ull, 0x0000000080000001ull, 0x8000000080008008ull};
-  // rho offsets and pi destinations generated from the (x, y) -> (y, 2x + 3y) walk
-  for (int round = 0; round < 24; round++) {
-    uint64_t c[5], d[5];
-    for (int x = 0; x < 5; x++) c[x] = a[x] ^ a[x + 5] ^ a[x + 10] ^ a[x + 15] ^ a[x + 20];
-    for (int x = 0; x < 5; x++) d[x] = c[(x + 4) % 5] ^ rotl64(c[(x + 1) % 5], 1);
-    for (int i = 0; i < 25; i++) a[i] ^= d[i % 5];
-    // rho + pi: follow the single 24-cycle starting at (1, 0)
-    int x = 1, y = 0;
-    uint64_t cur = a[1];
-    for (int t = 0; t < 24; t++) {
-      const int nx = y, ny = (2 * x + 3 * y) % 5;
-      const uint64_t tmp = a[nx + 5 * ny];
-      a[nx + 5 * ny] = rotl64(cur, ((t + 1) * (t + 2) / 2) % 64);
-      cur = tmp;
-      x = nx;
-      y = ny;
-    }
-    for (int row = 0; row < 25; row += 5) {
-      uint64_t r[5];
-      for (int k = 0; k < 5; k++) r[k] = a[row + k];
-      for (int k = 0; k < 5; k++) a[row + k] = r[k] ^ (~r[(k + 1) % 5] & r[(k + 2) % 5]);
-    }
-    a[0] ^= RC[round];
+  uint64_t b[25];
+  for (int round = 0; round < 24; round += 2) {
+    keccak_round(a, b, RC[round]);
+    keccak_round(b, a, RC[round + 1]);
   }
 }
 
