@@ -1,10 +1,51 @@
 #include <cuda.h>
+
+#include <algorithm>
+#include <mutex>
+#include <vector>
+
 #include "ctx.hpp"
 
 using namespace zk;
 
+namespace zk {
+namespace {
+struct KernelShape {
+  const void* kernel;
+  int device, threads;
+  size_t shared;
+  int blocks;
+};
+std::mutex g_shapes_mu;
+std::vector<KernelShape> g_shapes;  // a line per kernel of this library and device
+}  // namespace
+
+int resident_blocks(const void* kernel, int threads, size_t shared) {
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) return 0;
+  std::lock_guard<std::mutex> lock(g_shapes_mu);
+  for (const KernelShape& k : g_shapes)
+    if (k.kernel == kernel && k.device == device && k.threads == threads && k.shared == shared) return k.blocks;
+  int blocks = 0;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, threads, shared) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;  // not kept: the next call asks again
+  }
+  g_shapes.push_back({kernel, device, threads, shared, blocks});
+  return blocks;
+}
+
+// A new context may follow a reset of its device, which takes the opt-ins back.
+static void forget_shapes(int device) {
+  std::lock_guard<std::mutex> lock(g_shapes_mu);
+  g_shapes.erase(std::remove_if(g_shapes.begin(), g_shapes.end(), [&](const KernelShape& k) { return k.device == device; }), g_shapes.end());
+}
+}  // namespace zk
+
 int zk_ctx::setup() {
   ZK_CUDA(cudaSetDevice(device));
+  forget_shapes(device);
   ZK_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
   ZK_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
   ZK_CUDA(cudaStreamCreateWithFlags(&side_stream, cudaStreamNonBlocking));

@@ -314,7 +314,7 @@ void launch_sbool_msg(const uint32_t* keys, const Fr* val, const uint32_t* count
   if (ones) {
     k_sbool_msg<true><<<g_blocks(upper, sc), kGThreads, 0, s>>>(keys, val, count, eq, weights, vars_left, sc.sink);
   } else {
-    cudaFuncSetAttribute(k_sbool_msg<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideBytes);
+    (void)resident_blocks((const void*)k_sbool_msg<false>, kGThreads, kWideBytes);
     k_sbool_msg<false><<<g_blocks(upper, sc), kGThreads, kWideBytes, s>>>(keys, val, count, eq, weights, vars_left, sc.sink);
   }
 }

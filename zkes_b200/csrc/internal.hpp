@@ -27,6 +27,11 @@ struct RoundScratch {
   int sm_count;
 };
 
+// ctx.cu: resident blocks per SM of a kernel on the current device, with its dynamic shared memory opted in; 0 when it cannot be
+// launched like that.  Asked of the runtime once per kernel and device: the two calls take some 3 us, of which a small prove made
+// one pair and an entry-form prove one a round.
+int resident_blocks(const void* kernel, int threads, size_t shared);
+
 // sumcheck.cu
 void launch_round(int num_poly, bool fold, const Fr* const* src, Fr* const* dst, const Fr& r, uint64_t pairs,
                   const RoundScratch& sc, cudaStream_t stream);

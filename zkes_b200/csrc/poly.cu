@@ -425,7 +425,7 @@ int launch_from_right(const Fr* f, const Fr* eq, uint64_t lo_n, uint64_t hi_n, F
   Fr* dst = splits == 1 ? out : partial;
   if (hi_n >= kCtRows) {
     const BytesPlan p = bytes_plan(lo_n, hi_n, sm_count);
-    cudaFuncSetAttribute(k_from_right_bytes, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCtShared);
+    (void)resident_blocks((const void*)k_from_right_bytes, kCtThreads, kCtShared);
     k_from_right_bytes<<<(unsigned)p.blocks, kCtThreads, kCtShared, s>>>(f, eq, lo_n, hi_n, (uint32_t)p.groups, (uint32_t)p.steps, p.per, p.slots, dst);
   } else {
     const uint64_t per = (hi_n + splits - 1) / splits;

@@ -641,9 +641,8 @@ int launch_resident_t(const Fr* const* src, Fr* const* ping, Fr* const* pong, ui
   }
   // the opt-in for more than 48 KB of dynamic shared memory is per device, and a process may hold contexts on several
   constexpr size_t kStageBytes = (size_t)kWarps * 2 * L * WarpTile<8>::kChunks * sizeof(uint4);
-  if (cudaFuncSetAttribute(k_resident<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageBytes) != cudaSuccess) return -2;
-  int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_resident<L>, kThreads, kStageBytes) != cudaSuccess || occ < 1) return -2;
+  const int occ = resident_blocks((const void*)k_resident<L>, kThreads, kStageBytes);
+  if (occ < 1) return -2;
   uint64_t grid = ((size >> 1) + 31) / 32;  // tiles of the first round, a warp each
   const uint64_t cap = (uint64_t)sm_count * occ < (uint64_t)max_blocks ? (uint64_t)sm_count * occ : (uint64_t)max_blocks;
   if (grid > cap) grid = cap;

@@ -372,9 +372,8 @@ static void launch_sparse_msg_t(uint32_t* idx, Fr* val, const uint32_t* count, u
                                 const FixedMul<FrParams>& pt, const FixedMul<FrParams>& bt, const RoundScratch& sc,
                                 cudaStream_t s, const PeerExchange& px, unsigned int xseq) {
   constexpr size_t smem = (size_t)2 * ((D ? 8 : 4) + 2) * kSpThreads * sizeof(uint4);
-  cudaFuncSetAttribute(k_sparse_msg<D, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_sparse_msg<D, F>, kSpThreads, smem) != cudaSuccess || occ < 1) occ = 1;
+  int occ = resident_blocks((const void*)k_sparse_msg<D, F>, kSpThreads, smem);
+  if (occ < 1) occ = 1;
   // one wave of resident blocks: every thread walks its entries through the copy pipeline
   int cap = sc.sm_count * occ;
   if (cap > sc.max_blocks) cap = sc.max_blocks;
