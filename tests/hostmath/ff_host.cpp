@@ -83,6 +83,18 @@ extern "C" void zkh_g1_jacobian(const uint32_t* a, uint32_t k, uint32_t* out) {
   memcpy(out, j.x.v, 32); memcpy(out + 8, j.y.v, 32); memcpy(out + 16, j.z.v, 32);
 }
 
+// ---- the split of a scalar by the endomorphism: two magnitudes of four words, then their signs
+#include "../../zkes_b200/csrc/glv.cuh"
+extern "C" void zkh_glv_split(const uint32_t* k, uint32_t* out) {
+  uint32_t words[8], m1[4], m2[4];
+  bool n1, n2;
+  memcpy(words, k, 32);
+  glv_split(words, m1, &n1, m2, &n2);
+  memcpy(out, m1, 16); memcpy(out + 4, m2, 16);
+  out[8] = n1; out[9] = n2;
+}
+extern "C" void zkh_glv_beta(uint32_t* out) { for (int i = 0; i < 8; i++) out[i] = Glv::beta(i); }
+
 // ---- device-form transcript (strobe_dev.cuh) driven from a raw 200-byte state
 #include "../../zkes_b200/csrc/strobe_dev.cuh"
 // state: 200 bytes + pos, pos_begin, cur_flags (3 x u32).  Appends n scalars (Montgomery) under

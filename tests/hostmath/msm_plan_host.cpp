@@ -29,6 +29,14 @@ extern "C" void zkp_rows(uint64_t n, uint32_t rows, uint32_t max_span, uint64_t 
   out[6] = (uint64_t)p.parts * rows * p.planes;
   out[7] = p.slab;
 }
+// out: window bits, windows, most points a row, most points a row of a split scalar
+extern "C" void zkp_merged(uint64_t n, uint64_t* out) {
+  const int w = merged_window(n);
+  out[0] = (uint64_t)w;
+  out[1] = (uint64_t)((kEndoMagnitude + 1 + w - 1) / w);
+  out[2] = kMergedMost;
+  out[3] = kEndoMost;
+}
 extern "C" uint32_t zkp_reduce_lanes(uint32_t n_items, uint32_t half, int sm) { return reduce_lanes(n_items, half, sm); }
 extern "C" int zkp_combine_by(uint32_t rows, int w, int k_windows, int sm) { return (int)combine_by(rows, w, k_windows, sm); }
 extern "C" uint32_t zkp_fixup_groups(uint32_t n_buckets, uint32_t n_chunks, uint64_t longest, uint32_t seg) {

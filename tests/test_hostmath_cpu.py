@@ -197,6 +197,30 @@ def test_device_rows(hm, name, p):
         assert val(out) == a * a * rinv % p
 
 
+def test_split_by_the_endomorphism(hm):
+    """k = k1 + k2 lambda with magnitudes of 126 bits, over the folded scalars' whole range (up to (r - 1) / 2), and beta the x factor
+    that belongs to that lambda."""
+    rnd = random.Random(15)
+    b = (ctypes.c_uint32 * 8)()
+    hm.zkh_glv_beta(b)
+    beta = val(b) * pow(R, -1, o.Q_MOD) % o.Q_MOD
+    assert beta != 1 and pow(beta, 3, o.Q_MOD) == 1
+    g = o.G1_GEN
+    image = (beta * g[0] % o.Q_MOD, g[1])
+    roots = [w for w in (pow(c, (o.R_MOD - 1) // 3, o.R_MOD) for c in (2, 3, 5, 7, 11)) if w != 1][:1]
+    lam = next(w for w in (roots[0], roots[0] ** 2 % o.R_MOD) if o.g1_mul(g, w) == image)
+    top = (o.R_MOD - 1) // 2
+    edge = [0, 1, 2, top, top - 1, 1 << 127, (1 << 126) - 1, 1 << 252, min(lam, o.R_MOD - lam), (1 << 64) - 1, 1 << 64]
+    for k in edge + [rnd.randrange(top + 1) for _ in range(5000)] + [rnd.randrange(1 << rnd.randrange(1, 253)) for _ in range(2000)]:
+        out = (ctypes.c_uint32 * 10)()
+        hm.zkh_glv_split(buf(k), out)
+        m1, m2 = val(out[0:4]), val(out[4:8])
+        assert max(m1, m2) < 1 << 126
+        assert ((-m1 if out[8] else m1) + (-m2 if out[9] else m2) * lam - k) % o.R_MOD == 0
+        if k < 1 << 60:
+            assert (m1, m2) == (k, 0)  # small scalars have no second half
+
+
 @pytest.mark.parametrize("name,p", [("fr", o.R_MOD), ("fq", o.Q_MOD)])
 def test_out_of_montgomery_form(hm, name, p):
     """The host's form and the reduction alone, which the device runs, over every value of eight limbs."""

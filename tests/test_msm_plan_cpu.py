@@ -20,6 +20,7 @@ def plan(tmp_path_factory):
     u64, u32, i = ctypes.c_uint64, ctypes.c_uint32, ctypes.c_int
     lib.zkp_buckets.argtypes = [u64, u32, i, i, i, ctypes.c_void_p]
     lib.zkp_windows.argtypes = [u64, u32, u32, ctypes.c_void_p]
+    lib.zkp_merged.argtypes = [u64, ctypes.c_void_p]
     lib.zkp_rows.argtypes = [u64, u32, u32, u64, i, i, i, u64, ctypes.c_void_p]
 
     lib.zkp_reduce_lanes.argtypes = [u32, u32, i]
@@ -74,6 +75,15 @@ def test_chains_cover_every_group(plan):
         assert group
         assert (groups - 1) * group < n <= groups * group
         assert (parts - 1) * seg < groups <= parts * seg
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 40, 2047, 2048, 1 << 14, (1 << 20) - 1, 1 << 20])
+def test_shared_buckets_hold_every_digit_and_entry(plan, n):
+    """Signed digits of 126 bits and a carry in the windows; a multiple's index beside the two flag bits of an entry."""
+    w, windows, most, split_most = plan("zkp_merged", 4, n)
+    assert w * windows >= 127 > w * (windows - 1)
+    assert n <= most and windows * n < 1 << 30 and split_most < 1 << 30
+    assert plan("zkp_buckets", 2, 2 * n * windows * 32, 32, w, 1, SM)[0] == 32 << (w - 1)
 
 
 # rows, columns, kind, share of zeros, subset sums: measured, both ways at least a tenth apart

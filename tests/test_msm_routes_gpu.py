@@ -144,6 +144,31 @@ def test_full_width_rows(ctx, multiples, rows, n):
         assert curve.jacobian_to_affine_py(out[r:r + 1])[0] == of_g(want), r
 
 
+@pytest.mark.parametrize("rows,n", [(31, 64), (32, 1), (32, 2), (32, 33), (33, 4097), (64, 128), (1500, 9)])
+def test_full_width_rows_that_share_buckets(ctx, multiples, rows, n):
+    """From 32 rows on the windows of a row share its buckets, over multiples of the bases; below they do not."""
+    test_full_width_rows(ctx, multiples, rows, n)
+
+
+@pytest.mark.parametrize("n", [1, 2, 5, 33, 1000])
+@pytest.mark.parametrize("rows", [1, 33])
+def test_scalars_at_the_ends_of_the_split(ctx, multiples, n, rows):
+    """Scalars whose halves are zero, one, or the largest that occur, beside ones of 160 and 161 bits, where the split begins."""
+    ks, pts = multiples
+    rnd = random.Random(n * rows)
+    lam = 0xb3c4d79d41a917585bfc41088d8daaa78b17ea66b99c90dd
+    assert (lam * lam + lam + 1) % o.R_MOD == 0
+    half = (o.R_MOD - 1) // 2
+    pool = [0, 1, o.R_MOD - 1, lam, o.R_MOD - lam, lam + 1, lam * lam % o.R_MOD, half, half + 1, (1 << 126) - 1, ((1 << 125) * lam) % o.R_MOD,
+            (1 << 160) - 1, 1 << 160, (1 << 161) - 1] + [(rnd.randrange(1 << 126) + rnd.randrange(1 << 125) * lam) % o.R_MOD for _ in range(20)]
+    mat = [[rnd.choice(pool) for _ in range(n)] for _ in range(rows)]
+    mat[0][0] = half
+    got = curve.msm_batched(ctx, curve.affine_to_array(pts[-n:] if n <= len(pts) else [pts[i % len(pts)] for i in range(n)]), mat)
+    use = ks[-n:] if n <= len(ks) else [ks[i % len(ks)] for i in range(n)]
+    for r in sorted({0, rows // 2, rows - 1}):
+        assert got[r] == of_g(sum(v * k for v, k in zip(mat[r], use))), r
+
+
 @pytest.mark.parametrize("rows,n", [(2, 30), (3, 100), (300, 130), (650, 255)])
 def test_full_width_rows_of_few_buckets(ctx, multiples, rows, n):
     """Fewer than 256 bases a row: windows of three bits, whose four buckets are one thread's."""

@@ -3,7 +3,10 @@
 //
 //   1. k_msm_bits     largest magnitude of the sign-folded scalars -> window width W, windows K
 //   2. k_msm_digits   signed W-bit digits; MODE 0 counts (row, window, bucket) keys, MODE 1
-//                     scatters point indices (sign in bit 31) to their bucket's slots
+//                     scatters point indices (sign in bit 31) to their bucket's slots.  Full-width scalars are split
+//                     into two halves by the curve's endomorphism (glv.cuh): the images of the bases (bit 30) are points of
+//                     their own, and there are half the windows.  Many rows of them share one set of buckets over all
+//                     windows (k_multiples): no step 6
 //   3. k_msm_accumulate  equal chunks of the sorted entry list are summed by one thread each with
 //                     mixed additions; a bucket inside one chunk is written directly, pieces of
 //                     buckets that cross chunk borders go to per-chunk head / tail slots
@@ -20,6 +23,7 @@
 #include "reduce.cuh"
 #include "batch_affine.cuh"
 #include "quad.cuh"
+#include "glv.cuh"
 
 namespace zk {
 namespace {
@@ -125,97 +129,131 @@ __device__ __forceinline__ bool load_mag(const Fr* __restrict__ scalars, const i
   }
 }
 
-// W-bit field of mag starting at bit `pos` (pos + W may run past 256: zeros).
-__device__ __forceinline__ uint32_t bit_field(const uint32_t (&mag)[8], int pos, int w) {
+// W-bit field of mag starting at bit `pos` (pos + W may run past its end: zeros).
+template <int N>
+__device__ __forceinline__ uint32_t bit_field(const uint32_t (&mag)[N], int pos, int w) {
   const int limb = pos >> 5, sh = pos & 31;
   uint64_t v = 0;
 #pragma unroll
-  for (int i = 0; i < 8; i++) {
+  for (int i = 0; i < N; i++) {
     if (i == limb) v |= (uint64_t)mag[i];
     if (i == limb + 1) v |= (uint64_t)mag[i] << 32;
   }
   return (uint32_t)(v >> sh) & ((1u << w) - 1u);
 }
 
-template <int MODE, bool COMPACT>  // MODE 0: count keys, 1: scatter entries
+// An entry of a bucket: the point's index, kEntryEndo for its image under the endomorphism, kEntryNeg for the negative.
+constexpr uint32_t kEntryNeg = 0x80000000u, kEntryEndo = 0x40000000u;
+
+// The signed digits of one magnitude that are not zero: use(window, |digit| - 1, digit negative).
+template <int N, class F>
+__device__ __forceinline__ void signed_digits(const uint32_t (&mag)[N], int w, int k_windows, F use) {
+  const uint32_t half = 1u << (w - 1);
+  uint32_t carry = 0;
+  for (int k = 0; k < k_windows; k++) {
+    uint32_t raw = bit_field(mag, k * w, w) + carry;
+    bool dneg = false;
+    if (raw > half) {
+      raw = (1u << w) - raw;
+      dneg = true;
+      carry = 1;
+    } else {
+      carry = 0;
+    }
+    if (raw) use((uint32_t)k, raw - 1, dneg);
+  }
+}
+
+enum ScalarForm : int {
+  kWide = 0,      // folded to a sign and a magnitude
+  kCompact = 1,   // the same from the compact form of small scalars
+  kEndo = 2       // split into two halves by the endomorphism
+};
+
+// The digits of scalar g: use(window, bucket of the window, flags of the entry).
+template <int FORM, class F>
+__device__ __forceinline__ void scalar_digits(const Fr* __restrict__ scalars, const int32_t* __restrict__ compact, uint64_t g, int w, int k_windows,
+                                              F use) {
+  uint32_t mag[8];
+  const bool negv = load_mag<FORM == kCompact>(scalars, compact, g, mag);
+  if constexpr (FORM == kEndo) {
+    uint32_t m[2][4];
+    bool n[2];
+    glv_split(mag, m[0], &n[0], m[1], &n[1]);
+#pragma unroll 1
+    for (int e = 0; e < 2; e++) {
+      uint32_t part[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) part[i] = e ? m[1][i] : m[0][i];
+      const bool neg = negv != (e ? n[1] : n[0]);
+      signed_digits(part, w, k_windows, [&](uint32_t k, uint32_t d, bool dneg) { use(k, d, (neg != dneg ? kEntryNeg : 0u) | (e ? kEntryEndo : 0u)); });
+    }
+  } else {
+    signed_digits(mag, w, k_windows, [&](uint32_t k, uint32_t d, bool dneg) { use(k, d, negv != dneg ? kEntryNeg : 0u); });
+  }
+}
+
+// table_step: not 0 where the windows of a row share its buckets, window k taking its points from `table_step` k on (k_multiples).
+template <int MODE, int FORM>  // MODE 0: count keys, 1: scatter entries
 __global__ void k_msm_digits(const Fr* __restrict__ scalars, const int32_t* __restrict__ compact,
                              const uint32_t* __restrict__ row_ids, uint64_t n, uint32_t rows,
-                             int w, int k_windows, uint32_t* counts_or_cursor, uint32_t* entries) {
+                             int w, int k_windows, uint32_t table_step, uint32_t* counts_or_cursor, uint32_t* entries) {
   const uint64_t total = row_ids ? n : n * rows;
-  const uint32_t half = 1u << (w - 1);
   for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < total; g += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t mag[8];
-    const bool negv = load_mag<COMPACT>(scalars, compact, g, mag);
     // dense rows: scalar g belongs to row g / n; listed rows: the caller names the row of every scalar
     const uint32_t row = row_ids ? row_ids[g] : (uint32_t)(g / n);
     const uint32_t col = row_ids ? (uint32_t)g : (uint32_t)(g - (uint64_t)row * n);
-    uint32_t carry = 0;
-    for (int k = 0; k < k_windows; k++) {
-      uint32_t raw = bit_field(mag, k * w, w) + carry;
-      bool dneg = false;
-      if (raw > half) {
-        raw = (1u << w) - raw;
-        dneg = true;
-        carry = 1;
-      } else {
-        carry = 0;
-      }
-      if (raw == 0) continue;
-      const uint32_t key = (row * (uint32_t)k_windows + (uint32_t)k) * half + (raw - 1);
+    scalar_digits<FORM>(scalars, compact, g, w, k_windows, [&](uint32_t k, uint32_t digit, uint32_t flags) {
+      const uint32_t key = ((table_step ? row : row * (uint32_t)k_windows + k) << (w - 1)) + digit;
       if (MODE == 0) {
         atomicAdd(counts_or_cursor + key, 1u);
       } else {
         const uint32_t slot = atomicAdd(counts_or_cursor + key, 1u);
-        entries[slot] = col | ((negv != dneg) ? 0x80000000u : 0u);
+        entries[slot] = (col + k * table_step) | flags;
       }
-    }
+    });
   }
 }
 
-// Same two passes for a small key space (at most kSmallKeys buckets in total): keys are counted in
+// Same two passes for a small key space (at most kSmallKeys buckets): keys are counted in
 // shared memory first, so the global counters see one atomic per (block, bucket) instead of
 // one per digit.  In scatter mode the block reserves a contiguous range per bucket.
+// row_blocks == 0: all buckets of the call are at most kSmallKeys.  Otherwise those of one row are, and row_blocks blocks take a row.
 constexpr uint32_t kSmallKeys = 4096;
 
-template <int MODE, bool COMPACT>
+template <int MODE, int FORM>
 __global__ void __launch_bounds__(256) k_msm_digits_small(const Fr* __restrict__ scalars, const int32_t* __restrict__ compact,
                                                           const uint32_t* __restrict__ row_ids,
-                                                          uint64_t n, uint32_t rows, int w, int k_windows, uint32_t n_keys,
-                                                          uint64_t per_block, uint32_t* counts_or_cursor, uint32_t* entries) {
+                                                          uint64_t n, uint32_t rows, int w, int k_windows, uint32_t table_step,
+                                                          uint32_t n_keys, uint64_t per_block, uint32_t row_blocks, uint32_t* counts_or_cursor,
+                                                          uint32_t* entries) {
   __shared__ uint32_t hist[kSmallKeys];
   __shared__ uint32_t basepos[kSmallKeys];
   const uint64_t total = row_ids ? n : n * rows;
-  const uint32_t half = 1u << (w - 1);
-  const uint64_t begin = (uint64_t)blockIdx.x * per_block;
-  const uint64_t end = begin + per_block < total ? begin + per_block : total;
+  uint64_t begin = (uint64_t)blockIdx.x * per_block, end = begin + per_block < total ? begin + per_block : total;
+  uint32_t row0 = 0;
+  if (row_blocks) {
+    row0 = blockIdx.x / row_blocks;
+    begin = row0 * n + (blockIdx.x - row0 * row_blocks) * per_block;
+    end = begin + per_block < (row0 + 1) * n ? begin + per_block : (row0 + 1) * n;
+    counts_or_cursor += (uint64_t)row0 * n_keys;
+  }
   for (uint32_t k = threadIdx.x; k < n_keys; k += blockDim.x) hist[k] = 0;
   __syncthreads();
   for (int pass = 0; pass < (MODE == 0 ? 1 : 2); pass++) {
     for (uint64_t g = begin + threadIdx.x; g < end; g += blockDim.x) {
-      uint32_t mag[8];
-      const bool negv = load_mag<COMPACT>(scalars, compact, g, mag);
-      const uint32_t row = row_ids ? row_ids[g] : (uint32_t)(g / n);
+      const uint32_t row = row_blocks ? row0 : row_ids ? row_ids[g] : (uint32_t)(g / n);
       const uint32_t col = row_ids ? (uint32_t)g : (uint32_t)(g - (uint64_t)row * n);
-      uint32_t carry = 0;
-      for (int k = 0; k < k_windows; k++) {
-        uint32_t raw = bit_field(mag, k * w, w) + carry;
-        bool dneg = false;
-        if (raw > half) {
-          raw = (1u << w) - raw;
-          dneg = true;
-          carry = 1;
-        } else {
-          carry = 0;
-        }
-        if (raw == 0) continue;
-        const uint32_t key = (row * (uint32_t)k_windows + (uint32_t)k) * half + (raw - 1);
+      scalar_digits<FORM>(scalars, compact, g, w, k_windows, [&](uint32_t k, uint32_t digit, uint32_t flags) {
+        const uint32_t item = table_step ? row - row0 : (row - row0) * (uint32_t)k_windows + k;
+        const uint32_t key = (item << (w - 1)) + digit;
         if (pass == 0) {
           atomicAdd(hist + key, 1u);
         } else {
           const uint32_t slot = basepos[key] + atomicAdd(hist + key, 1u);
-          entries[slot] = col | ((negv != dneg) ? 0x80000000u : 0u);
+          entries[slot] = (col + k * table_step) | flags;
         }
-      }
+      });
     }
     __syncthreads();
     if (pass == 0) {
@@ -231,6 +269,88 @@ __global__ void __launch_bounds__(256) k_msm_digits_small(const Fr* __restrict__
       __syncthreads();
     }
   }
+}
+
+__device__ __forceinline__ Fq ld_fq(const Fq* p) {
+  const uint4 a = __ldg(reinterpret_cast<const uint4*>(p)), b = __ldg(reinterpret_cast<const uint4*>(p) + 1);
+  Fq r;
+  r.v[0] = a.x; r.v[1] = a.y; r.v[2] = a.z; r.v[3] = a.w;
+  r.v[4] = b.x; r.v[5] = b.y; r.v[6] = b.z; r.v[7] = b.w;
+  return r;
+}
+__device__ __forceinline__ void st_fq(Fq* p, const Fq& x) {
+  reinterpret_cast<uint4*>(p)[0] = make_uint4(x.v[0], x.v[1], x.v[2], x.v[3]);
+  reinterpret_cast<uint4*>(p)[1] = make_uint4(x.v[4], x.v[5], x.v[6], x.v[7]);
+}
+
+// Many rows over the same bases: the multiples 2^(w k) of every base for all windows k, so that the digits of all windows of a row
+// fall into one set of buckets: the windows can be wider, there is one bucket sum per row instead of one per row and window, and no
+// Horner chain.  The chain of w (windows - 1) doublings is here instead, once per base; four lanes take a point (quad.cuh).
+// A latency chain (226 us for a hundred points, 555 for 2^14), beside the passes over the digits.  A KZH3 commitment and opening of
+// 2^22 values, half of them full width: accumulation 15 957 -> 13 315 us, bucket reduction 2 685 -> 1 327, Horner chains 1 120 -> 0, for
+// 935 us of multiples; 24 286 -> 19 126 us in all together with the split and with digits counted a row at a time.
+__global__ void __launch_bounds__(128) k_multiples(const Affine* __restrict__ bases, uint64_t n, int w, int k_windows, Xyzz* out) {
+  const uint64_t i = (uint64_t)blockIdx.x * 32 + (threadIdx.x >> 2);
+  const int role = threadIdx.x & 3;
+  const uint64_t at = i < n ? i : n - 1;
+  const Fq bx = ld_fq(&bases[at].x), by = ld_fq(&bases[at].y);
+  QuadXyzz p;
+  p.x = bx;
+  p.y = by;
+  p.z = bx.is_zero() && by.is_zero() ? Fq::zero() : Fq::one();
+  if (i < n) quad_store(out + i, p, role);
+#pragma unroll 1
+  for (int k = 1; k < k_windows; k++) {
+#pragma unroll 1
+    for (int j = 0; j < w; j++) p = quad_dbl(p, role);
+    if (i < n) quad_store(out + (uint64_t)k * n + i, p, role);
+  }
+}
+
+// Affine form of many points, kMultiplesPer a thread and inversion, and the x of their images under the endomorphism.
+constexpr int kMultiplesPer = 4;
+__global__ void __launch_bounds__(kBatchThreads, 4) k_multiples_affine(const Xyzz* __restrict__ points, uint64_t n, Affine* out, Fq* images) {
+  constexpr int kPer = kMultiplesPer;
+  __shared__ Fq sh[kBatchThreads];
+  const uint64_t t0 = (uint64_t)blockIdx.x * (kBatchThreads * kPer) + threadIdx.x;
+  Fq pre[kPer], run = Fq::one(), beta;
+#pragma unroll
+  for (int i = 0; i < 8; i++) beta.v[i] = Glv::beta(i);
+#pragma unroll 1
+  for (int j = 0; j < kPer; j++) {
+    const uint64_t t = t0 + (uint64_t)j * kBatchThreads;
+    if (t >= n) break;
+    const Fq z = ld_fq(&points[t].zzz);
+    pre[j] = run;
+    if (!z.is_zero()) run = fq_mul_fn(run, z);
+  }
+  Fq inv = block_inverse(run, sh);
+#pragma unroll 1
+  for (int j = kPer - 1; j >= 0; j--) {
+    const uint64_t t = t0 + (uint64_t)j * kBatchThreads;
+    if (t >= n) continue;
+    const Fq zzz = ld_fq(&points[t].zzz);
+    Fq x = Fq::zero(), y = Fq::zero();
+    if (!zzz.is_zero()) {
+      const Fq izzz = fq_mul_fn(inv, pre[j]);
+      inv = fq_mul_fn(inv, zzz);
+      const Fq iz = fq_mul_fn(izzz, ld_fq(&points[t].zz));  // 1 / zz = (zz / zzz)^2
+      x = fq_mul_fn(ld_fq(&points[t].x), fq_mul_fn(iz, iz));
+      y = fq_mul_fn(ld_fq(&points[t].y), izzz);
+    }
+    st_fq(&out[t].x, x);
+    st_fq(&out[t].y, y);
+    st_fq(images + t, fq_mul_fn(beta, x));
+  }
+}
+
+// images[i] = beta x of base i: the x of its image under the endomorphism (y is its own)
+__global__ void __launch_bounds__(256) k_endo_images(const Affine* __restrict__ bases, uint64_t n, Fq* images) {
+  Fq beta;
+#pragma unroll
+  for (int i = 0; i < 8; i++) beta.v[i] = Glv::beta(i);
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+    st_fq(images + i, mul(beta, ld_fq(&bases[i].x)));
 }
 
 __device__ __forceinline__ Affine ld_affine(const Affine* p) {
@@ -304,7 +424,7 @@ __device__ __forceinline__ Xyzz add_mixed_calls(const Xyzz& p, const Affine& q) 
 }
 
 __global__ void __launch_bounds__(128, kAccBlocks) k_msm_accumulate(const Affine* __restrict__ bases,
-                                                        const uint32_t* __restrict__ gather,
+                                                        const Fq* __restrict__ images, const uint32_t* __restrict__ gather,
                                                         const uint32_t* __restrict__ entries,
                                                         const uint32_t* __restrict__ offsets, uint32_t n_buckets,
                                                         uint32_t n_entries, uint32_t seg, uint32_t n_chunks,
@@ -325,9 +445,16 @@ __global__ void __launch_bounds__(128, kAccBlocks) k_msm_accumulate(const Affine
       do { b++; b_end = offsets[b + 1]; } while (b_end <= e);
     }
     const uint32_t ent = entries[e];
-    const uint32_t col = ent & 0x7fffffffu;
-    Affine pt = ld_affine(bases + (gather ? gather[col] : col));
-    if (ent & 0x80000000u) pt = neg(pt);
+    Affine pt;
+    if (images) {
+      const uint32_t col = ent & ~(kEntryNeg | kEntryEndo);
+      pt.x = ld_fq((ent & kEntryEndo) ? images + col : &bases[col].x);
+      pt.y = ld_fq(&bases[col].y);
+    } else {
+      const uint32_t col = ent & ~kEntryNeg;
+      pt = ld_affine(bases + (gather ? gather[col] : col));
+    }
+    if (ent & kEntryNeg) pt = neg(pt);
     acc = add_mixed(acc, pt);
   }
   // the bucket in progress at the end of the chunk
@@ -1038,10 +1165,28 @@ static int rows_run(zk_ctx* ctx, const Affine* bases, const int32_t* compact, ui
   return 0;
 }
 
+template <int MODE>
+static void launch_digits(ScalarForm form, uint32_t small_keys, uint32_t dig_blocks, uint64_t per_block, uint32_t row_blocks, int sm, const Fr* scalars, const int32_t* compact,
+                          const uint32_t* row_ids, uint64_t n, uint32_t rows, int w, int k_windows, uint32_t table_step,
+                          uint32_t* counts_or_cursor, uint32_t* entries, cudaStream_t s) {
+  auto launch = [&](auto small, auto large) {
+    if (small_keys)
+      small<<<dig_blocks, 256, 0, s>>>(scalars, compact, row_ids, n, rows, w, k_windows, table_step, small_keys, per_block, row_blocks, counts_or_cursor, entries);
+    else
+      large<<<sm * 8, 256, 0, s>>>(scalars, compact, row_ids, n, rows, w, k_windows, table_step, counts_or_cursor, entries);
+  };
+  switch (form) {
+    case kCompact: launch(k_msm_digits_small<MODE, kCompact>, k_msm_digits<MODE, kCompact>); break;
+    case kEndo: launch(k_msm_digits_small<MODE, kEndo>, k_msm_digits<MODE, kEndo>); break;
+    case kWide: launch(k_msm_digits_small<MODE, kWide>, k_msm_digits<MODE, kWide>); break;
+  }
+}
+
 // row_ids == nullptr: `rows` dense rows of n scalars each over the same n bases.  Otherwise: n scalars in
 // all, scalar i contributes scalars[i] * bases[gather ? gather[i] : i] to output row row_ids[i] < rows.
-int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const uint32_t* row_ids, const Fr* scalars,
-                 uint64_t n, uint32_t rows, Jacobian* out_dev, MsmStats* stats, MsmPrep* prep) {
+// plain: without what takes scratch beside the buckets, where there was no room for it.
+static int msm_run_impl(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const uint32_t* row_ids, const Fr* scalars,
+                        uint64_t n, uint32_t rows, Jacobian* out_dev, MsmStats* stats, MsmPrep* prep, bool plain) {
   cudaStream_t s = ctx->stream;
   const uint64_t total = row_ids ? n : n * rows;
   const int sm = ctx->sm_count;
@@ -1084,11 +1229,20 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
     ctx->launches++;
     return 0;
   }
-  const int w = pick_window(row_ids ? (n / rows ? n / rows : 1) : n, rows, (int)max_bits);
+  // Full-width scalars are split into two halves by the endomorphism: as many digits, half the windows (buckets, doublings).  100003
+  // points: kernels 752 -> 728 us (bucket reduction 153 -> 118), the chain of doublings on the host half as long, the call 929 -> 862 us.
+  // Scalars of up to 160 bits stay whole: they have fewer digits than 2 x 126 bits have.
+  const bool endo = !compact && !row_ids && !gather && max_bits > kEndoBits && n <= kEndoMost && !plain;
+  const int bits = endo ? kGlvBits : (int)max_bits;
+  const bool merged = endo && rows >= kMergedRows && n <= kMergedMost;
+  // Separate windows of several rows: a bit more than for whole scalars, as there are half as many (pick_window).
+  const int w = merged ? merged_window(n) : pick_window(row_ids ? (n / rows ? n / rows : 1) : n, rows, bits) + (endo && rows > 1 ? 1 : 0);
   // small scalars: the exact largest magnitude is known, which can save the window that would only
   // hold carries (int8 values reach 128 = one 8-bit signed digit)
-  const int k_windows = compact ? windows_for(prep->max_mag, w) : ((int)max_bits + 1 + w - 1) / w;
-  const BucketPlan plan = bucket_plan(total, rows, w, k_windows, sm);
+  const int digit_windows = compact ? windows_for(prep->max_mag, w) : (bits + 1 + w - 1) / w;
+  const int k_windows = merged ? 1 : digit_windows;  // with buckets of their own
+  const uint64_t digits = (uint64_t)digit_windows * (endo ? 2 : 1);  // of a scalar, at most
+  const BucketPlan plan = bucket_plan(endo ? (merged ? 2 * total * digit_windows : 2 * total) : total, rows, w, k_windows, sm);
   const uint32_t half = plan.half;
   const bool too_many = plan.n_buckets >= (1ull << 31);
   const uint32_t n_buckets = (uint32_t)plan.n_buckets;
@@ -1100,11 +1254,18 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
       if (rc != -2 /*ZK_ERR_OOM*/) return rc;  // no room for the tables: the buckets of a small call may still have it
     }
   }
+  auto plainly = [&] { return msm_run_impl(ctx, bases, gather, row_ids, scalars, n, rows, out_dev, stats, prep, true); };
+  if (too_many && endo) return plainly();
   if (too_many) return fail(-1, "msm: %llu buckets exceed the 32-bit key space; split the rows", (unsigned long long)plan.n_buckets);
 
   // ---- scratch layout (second scratch region of the context; the first holds caller data)
+  const uint64_t table_points = merged ? n * (uint64_t)digit_windows : 0;
+  const uint32_t table_step = merged ? (uint32_t)n : 0;
+  const size_t endo_bytes = (endo ? align256((merged ? table_points : n) * sizeof(Fq)) : 0) + align256(table_points * sizeof(Affine)) +
+                            align256(table_points * sizeof(Xyzz));
   char* base = nullptr;
-  int rc = ctx->reserve_aux(plan.scratch + scan_bytes, (void**)&base);
+  int rc = ctx->reserve_aux(plan.scratch + scan_bytes + endo_bytes, (void**)&base);
+  if (rc == -2 /*ZK_ERR_OOM*/ && endo) return plainly();
   if (rc) return rc;
   size_t off = 0;
   auto take = [&](size_t bytes) { char* p = base + off; off += align256(bytes); return p; };
@@ -1118,66 +1279,76 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
   Xyzz* tails = (Xyzz*)take((plan.chunks + 1) * sizeof(Xyzz));
   Xyzz* fix_part = (Xyzz*)take((size_t)kFixupPartials * sizeof(Xyzz));
   Xyzz* runs = (Xyzz*)take(plan.n_runs * sizeof(Xyzz));
-
+  Fq* images = endo ? (Fq*)take((merged ? table_points : n) * sizeof(Fq)) : nullptr;
+  Affine* table = (Affine*)take(table_points * sizeof(Affine));
+  Xyzz* multiples = (Xyzz*)take(table_points * sizeof(Xyzz));
   // ---- pass 2: count, scan, scatter
   ZK_CUDA(cudaMemsetAsync(offsets, 0, (n_buckets + 2) * 4ull, s));
-  const bool small_keys = n_buckets <= kSmallKeys;
-  // 4096 digits a block, not scalars: 1000 full-width scalars of 37 digits each were one block's work (638 us, 561 us with ten)
-  uint32_t dig_blocks = (uint32_t)std::min<uint64_t>((total * (uint64_t)k_windows + 4095) / 4096, 1u << 20);
-  if (dig_blocks > (uint32_t)sm * 8) dig_blocks = sm * 8;
-  const uint64_t per_block = (total + dig_blocks - 1) / dig_blocks;
-  if (small_keys) {
-    if (compact)
-      k_msm_digits_small<0, true><<<dig_blocks, 256, 0, s>>>(scalars, compact, row_ids, n, rows, w, k_windows, n_buckets, per_block, offsets, nullptr);
-    else
-      k_msm_digits_small<0, false><<<dig_blocks, 256, 0, s>>>(scalars, compact, row_ids, n, rows, w, k_windows, n_buckets, per_block, offsets, nullptr);
-  } else {
-    if (compact)
-      k_msm_digits<0, true><<<sm * 8, 256, 0, s>>>(scalars, compact, row_ids, n, rows, w, k_windows, offsets, nullptr);
-    else
-      k_msm_digits<0, false><<<sm * 8, 256, 0, s>>>(scalars, compact, row_ids, n, rows, w, k_windows, offsets, nullptr);
+  const ScalarForm form = compact ? kCompact : endo ? kEndo : kWide;
+  // The multiples are a chain of doublings that leaves most of the GPU idle: beside the digit passes, on the side stream.  With the
+  // per-kernel profiler on they stay in line.
+  const bool beside = merged && !ctx->prof_on;
+  if (merged) {
+    cudaStream_t s2 = beside ? ctx->side_stream : s;
+    if (beside) {
+      ZK_CUDA(cudaEventRecord(ctx->ev_fork, s));
+      ZK_CUDA(cudaStreamWaitEvent(s2, ctx->ev_fork, 0));
+    }
+    k_multiples<<<(unsigned)((n + 31) / 32), 128, 0, s2>>>(bases, n, w, digit_windows, multiples);
+    const uint64_t per = kBatchThreads * kMultiplesPer;
+    k_multiples_affine<<<(unsigned)((table_points + per - 1) / per), kBatchThreads, 0, s2>>>(multiples, table_points, table, images);
+    ctx->launches += 2;
+    if (beside) ZK_CUDA(cudaEventRecord(ctx->ev_join, s2));
+  } else if (endo) {
+    k_endo_images<<<(unsigned)std::min<uint64_t>((n + 255) / 256, (uint64_t)sm * 16), 256, 0, s>>>(bases, n, images);
+    ctx->launches++;
   }
+  // 4096 digits a block, not scalars: 1000 full-width scalars of 37 digits each were one block's work (638 us, 561 us with ten)
+  uint32_t dig_blocks = (uint32_t)std::min<uint64_t>((total * digits + 4095) / 4096, 1u << 20);
+  if (dig_blocks > (uint32_t)sm * 8) dig_blocks = sm * 8;
+  uint64_t per_block = (total + dig_blocks - 1) / dig_blocks;
+  // buckets that a block counts in shared memory: all of them, or those of a row (0: by global atomics).  A row's share of the blocks
+  // gets some 16384 digits each, four a bucket.
+  uint32_t small_keys = n_buckets <= kSmallKeys ? n_buckets : 0, row_blocks = 0;
+  if (!small_keys && !row_ids && n_buckets / rows <= kSmallKeys && n * digits >= 4ull * (n_buckets / rows)) {
+    small_keys = n_buckets / rows;
+    const uint64_t share = std::max<uint64_t>(1, std::min<uint64_t>(n * digits / (4ull * small_keys), ((uint64_t)sm * 16 + rows - 1) / rows));
+    row_blocks = (uint32_t)share;
+    per_block = (n + share - 1) / share;
+    dig_blocks = rows * row_blocks;
+  }
+  launch_digits<0>(form, small_keys, dig_blocks, per_block, row_blocks, sm, scalars, compact, row_ids, n, rows, w, digit_windows, table_step, offsets, nullptr, s);
   ctx->launches++;
   BucketCounts* d_counts = reinterpret_cast<BucketCounts*>(ctx->rs.sink.counter + 10);
   ZK_CUDA(cudaMemsetAsync(d_counts, 0, sizeof(BucketCounts), s));
-  const uint32_t chunk = chunk_entries((uint32_t)std::min<uint64_t>(prep->nonzero * (uint64_t)k_windows, 0xffffffffull), sm);  // or a little less
+  const uint32_t chunk = chunk_entries((uint32_t)std::min<uint64_t>(prep->nonzero * digits, 0xffffffffull), sm);  // or a little less
   k_total64<<<sm * 4, 256, 0, s>>>(offsets, n_buckets, kFewPieces * chunk, kManyPieces * chunk, d_counts);
   ctx->launches++;
   ZK_CUDA(cudaMemcpyAsync(ctx->host_small, d_counts, sizeof(BucketCounts), cudaMemcpyDeviceToHost, s));
   ZK_CUDA(cudaStreamSynchronize(s));
   BucketCounts counts;
   memcpy(&counts, ctx->host_small, sizeof(counts));
-  const unsigned long long total64 = counts.total;
-  if (total64 > 0xffffffffull) return fail(-1, "msm: %llu digit entries exceed 2^32 - 1; split the call", total64);
+  if (beside && counts.total > 0xffffffffull) ZK_CUDA(cudaStreamWaitEvent(s, ctx->ev_join, 0));
+  if (counts.total > 0xffffffffull && endo) return plainly();  // of other window widths, a few digits less
+  if (counts.total > 0xffffffffull) return fail(-1, "msm: %llu digit entries exceed 2^32 - 1; split the call", counts.total);
+  const uint32_t n_entries = (uint32_t)counts.total;
   ctx->launches += exclusive_scan_u32(offsets, n_buckets, scan_tmp, true, s);
   ZK_CUDA(cudaMemcpyAsync(cursor, offsets, (n_buckets + 1) * 4ull, cudaMemcpyDeviceToDevice, s));
-  if (small_keys) {
-    if (compact)
-      k_msm_digits_small<1, true><<<dig_blocks, 256, 0, s>>>(scalars, compact, row_ids, n, rows, w, k_windows, n_buckets, per_block, cursor, entries);
-    else
-      k_msm_digits_small<1, false><<<dig_blocks, 256, 0, s>>>(scalars, compact, row_ids, n, rows, w, k_windows, n_buckets, per_block, cursor, entries);
-  } else {
-    if (compact)
-      k_msm_digits<1, true><<<sm * 8, 256, 0, s>>>(scalars, compact, row_ids, n, rows, w, k_windows, cursor, entries);
-    else
-      k_msm_digits<1, false><<<sm * 8, 256, 0, s>>>(scalars, compact, row_ids, n, rows, w, k_windows, cursor, entries);
-  }
+  launch_digits<1>(form, small_keys, dig_blocks, per_block, row_blocks, sm, scalars, compact, row_ids, n, rows, w, digit_windows, table_step, cursor, entries, s);
   ctx->launches++;
-  ZK_CUDA(cudaMemcpyAsync(ctx->host_small, offsets + n_buckets, 4, cudaMemcpyDeviceToHost, s));
-  ZK_CUDA(cudaStreamSynchronize(s));
-  uint32_t n_entries = 0;
-  memcpy(&n_entries, ctx->host_small, 4);
 
   // ---- accumulate
+  if (beside) ZK_CUDA(cudaStreamWaitEvent(s, ctx->ev_join, 0));
   ZK_CUDA(cudaMemsetAsync(bucket_sums, 0, (size_t)n_buckets * sizeof(Xyzz), s));
   if (n_entries) {
     const uint32_t seg = chunk_entries(n_entries, sm);
     const uint32_t n_chunks = (n_entries + seg - 1) / seg;
-    k_msm_accumulate<<<(n_chunks + 127) / 128, 128, 0, s>>>(bases, gather, entries, offsets, n_buckets, n_entries, seg,
+    k_msm_accumulate<<<(n_chunks + 127) / 128, 128, 0, s>>>(merged ? table : bases, images, gather, entries, offsets, n_buckets, n_entries, seg,
                                                            n_chunks, bucket_sums, heads, tails);
     // cursor[] is free again after the scatter: it stands at the ends of the buckets
     if (n_buckets <= kFixupBuckets) {
-      const uint32_t groups = fixup_groups(n_buckets, n_chunks, row_ids ? n_entries : n, seg);
+      const uint64_t longest = row_ids ? n_entries : endo ? n * (merged ? digits : 2) : n;
+      const uint32_t groups = fixup_groups(n_buckets, n_chunks, longest, seg);
       k_msm_fixup_block<<<dim3(n_buckets, groups), 128, 0, s>>>(offsets, seg, groups, cursor, bucket_sums, heads, tails, fix_part);
     } else {
       uint32_t* listed = ctx->rs.sink.counter + 12;
@@ -1228,6 +1399,11 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
     stats->max_bits = (int)max_bits;
   }
   return 0;
+}
+
+int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const uint32_t* row_ids, const Fr* scalars,
+                 uint64_t n, uint32_t rows, Jacobian* out_dev, MsmStats* stats, MsmPrep* prep) {
+  return msm_run_impl(ctx, bases, gather, row_ids, scalars, n, rows, out_dev, stats, prep, false);
 }
 
 // C (out_dev[rows]) and d_x (out_dev[0 .. rows)) of a selection polynomial over n indices in non-decreasing order

@@ -8,6 +8,9 @@
 
 namespace zk {
 
+constexpr unsigned kEndoBits = 160;  // scalars of more bits are split by the endomorphism (glv.cuh)
+constexpr uint64_t kEndoMost = 1ull << 24;  // points a row: above, the buckets are few beside the points and their images are half a gigabyte
+constexpr int kEndoMagnitude = 126;  // into magnitudes of as many bits
 constexpr int kCompactBits = 30;  // magnitudes below 2^30 have a compact form (k_msm_bits)
 constexpr int kAccBlocks = 4;     // blocks of 128 threads per SM of the kernels that add points in chains (126 and 122 registers)
 constexpr uint32_t kReduceThreads = 128;   // threads of a block of the bucket reduction
@@ -35,6 +38,24 @@ inline int pick_window(uint64_t n, uint32_t rows, int max_bits) {
   // take 12000 points in 548 us where 10, which leave four, take 583.
   if (rows == 1 && w >= 14 && max_bits > kCompactBits && (max_bits + 1) - w * ((max_bits + w) / w - 1) < 4) w--;
   return w;
+}
+
+// Rows over the same bases whose windows share their buckets (k_multiples): from kMergedRows rows on.  Window width: a row adds
+// 2 n points a window and some three points a bucket.  Below 32 rows the multiples (a chain of 126 doublings, 0.2 to 0.6 ms) cost what
+// the shared buckets save.
+constexpr uint32_t kMergedRows = 32;
+constexpr uint64_t kMergedMost = 1ull << 20;  // points a row
+inline int merged_window(uint64_t n) {
+  int best = 4;
+  double least = 1e300;
+  for (int w = 4; w <= 16; w++) {
+    const double cost = 2.0 * (double)n * ((kEndoMagnitude + w) / w) + 3.0 * (double)(1u << (w - 1));
+    if (cost < least) {
+      least = cost;
+      best = w;
+    }
+  }
+  return best;
 }
 
 // Signed-digit windows needed for magnitudes up to max_mag: k digits in (-half, half] reach
