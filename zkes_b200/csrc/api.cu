@@ -4,6 +4,7 @@
 #include "ctx.hpp"
 #include "strobe_dev.cuh"
 
+#include <atomic>
 #include <chrono>
 #include <cstdio>
 #include <string>
@@ -25,6 +26,34 @@ int fail(int code, const char* fmt, ...) {
 }  // namespace zk
 
 namespace zk {
+// Until a word of pinned memory that a kernel of the stream sets is there, however long the stream takes.  *set is false, and that is
+// no error yet, where the stream came to its end without it.
+int wait_published(zk_ctx* ctx, const void* word, unsigned int want, bool* set) {
+  const volatile unsigned int* w = reinterpret_cast<const volatile unsigned int*>(word);
+  uint64_t spins = 0;
+  *set = true;
+  while (*w != want) {
+    if ((++spins & 0x3fff) == 0) {
+      const cudaError_t e = cudaStreamQuery(ctx->stream);
+      if (e != cudaSuccess && e != cudaErrorNotReady) return fail(ZK_ERR_CUDA, "kernel failed: %s", cudaGetErrorString(e));
+      if (e == cudaSuccess && *w != want) {
+        *set = false;
+        return ZK_OK;
+      }
+    }
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return ZK_OK;
+}
+
+// The values that the last next_msg_scratch(false) launch left in the mailbox, for calls that have nothing else to read back.
+int wait_result(zk_ctx* ctx) {
+  bool set = false;
+  const int rc = wait_published(ctx, reinterpret_cast<const char*>(ctx->mailbox) + 16 * sizeof(Fr), ctx->rs.sink.seq, &set);
+  if (rc) return rc;
+  return set ? ZK_OK : fail(ZK_ERR_TIMEOUT, "the stream drained without publishing its result");
+}
+
 // The kernel that completes a message publishes it to the host-mapped mailbox and then writes this launch's
 // sequence number: poll for it instead of synchronising the stream.  `exchanged`: the message went through the
 // ranks' exchange, whose kernel reports a wait that ran out in the word beside the sequence word.

@@ -111,14 +111,12 @@ int zk_mle_eval(zk_ctx* ctx, uint32_t n, const uint64_t* evals, zk_mem evals_mem
   Fr* eq = base + in_elems;
   rc = eq_table_device(ctx, point, n, eq);
   if (rc) return rc;
-  RoundScratch sc = ctx->rs;
-  sc.sink.pub_flag = nullptr;  // read back with a copy: nothing polls this result
-  launch_dot(f, eq, size, sc, s);
+  launch_dot(f, eq, size, ctx->next_msg_scratch(false), s);  // published to the polling host: no copy, no synchronisation
   ctx->launches++;
   ZK_CUDA(cudaGetLastError());
-  ZK_CUDA(cudaMemcpyAsync(ctx->host_small, ctx->rs.sink.msg, sizeof(Fr), cudaMemcpyDeviceToHost, s));
-  ZK_CUDA(cudaStreamSynchronize(s));
-  memcpy(out, ctx->host_small, sizeof(Fr));
+  rc = wait_result(ctx);
+  if (rc) return rc;
+  memcpy(out, ctx->mailbox, sizeof(Fr));
   return ZK_OK;
 }
 

@@ -158,6 +158,9 @@ struct zk_transcript {
 namespace zk {
 typedef int (*fs_round_fn_t)(void* user, const uint64_t* msgs, uint32_t n_msgs, uint64_t challenge_out[4]);
 bool comm_peer_args(const zk_ctx* ctx, const zk_comm* c, PeerExchange* out);
+// api.cu
+int wait_published(zk_ctx* ctx, const void* word, unsigned int want, bool* set);
+int wait_result(zk_ctx* ctx);  // until the last next_msg_scratch(false) launch has published
 void comm_peer_advance(zk_comm* c, unsigned int n);
 int comm_peer_gather(zk_ctx* ctx, zk_comm* c, int n_tables, const Fr* const* chunks, uint32_t m, unsigned int* error_word,
                      const Fr** tables_out);

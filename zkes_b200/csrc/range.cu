@@ -129,9 +129,10 @@ __global__ void __launch_bounds__(kCopiesThreads) k_range_scatter_copies(const u
   }
 }
 
-// part[t] from its limb counters; acc[t] += beta_gamma * part[t]; sink.msg[0] = sum_t part[t] * t.
+// part[t] from its limb counters; acc[t] += beta_gamma * part[t]; sink.msg[0] = sum_t part[t] * t, sink.msg[1] zero unless *bad is not.
 __global__ void __launch_bounds__(256) k_range_finish(const unsigned long long* __restrict__ limbs, uint64_t n_table,
-                                                      const FixedMul<FrParams> bg, Fr* acc, const MsgSink sink) {
+                                                      const unsigned int* __restrict__ bad, const FixedMul<FrParams> bg, Fr* acc,
+                                                      const MsgSink sink) {
   Fr mid = Fr::zero();
   for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n_table; t += (uint64_t)gridDim.x * blockDim.x) {
     // X = sum_j limbs[j] * 2^(32 j) < 2^288, as sixteen 32-bit limbs
@@ -156,8 +157,9 @@ __global__ void __launch_bounds__(256) k_range_finish(const unsigned long long* 
     mid = add(mid, mul(part, to_mont(tt)));
     acc[t] = add(acc[t], mul_fixed(bg, part));
   }
-  Fr s[1] = {mid};
-  grid_sum<1, 8>(s, sink);
+  Fr s[2] = {mid, Fr::zero()};
+  if (blockIdx.x == 0 && threadIdx.x == 0) s[1].v[0] = *bad != 0;
+  grid_sum<2, 8>(s, sink);
 }
 
 // out[i] = i + alpha
@@ -230,23 +232,22 @@ int zk_range_aux_accumulate(zk_ctx* ctx, uint32_t k, const uint64_t* point, uint
     }
     ctx->launches++;
   }
-  RoundScratch sc = ctx->rs;
-  sc.sink.pub_flag = nullptr;  // read back with a copy: nothing polls this result
+  const RoundScratch sc = ctx->next_msg_scratch(false);  // published to the polling host: no copy, no synchronisation
   uint64_t blocks = (n_table + 255) / 256;
   const uint64_t cap = (uint64_t)ctx->sm_count * 4 < (uint64_t)sc.max_blocks ? ctx->sm_count * 4 : sc.max_blocks;
   if (blocks > cap) blocks = cap;
-  k_range_finish<<<(unsigned)blocks, 256, 0, s>>>(limbs, n_table, make_fixed_mul(fr_load(beta_gamma)), d_acc, sc.sink);
+  k_range_finish<<<(unsigned)blocks, 256, 0, s>>>(limbs, n_table, bad, make_fixed_mul(fr_load(beta_gamma)), d_acc, sc.sink);
   ctx->launches++;
   ZK_CUDA(cudaGetLastError());
-  char* hs = reinterpret_cast<char*>(ctx->host_small);
-  ZK_CUDA(cudaMemcpyAsync(hs, ctx->rs.sink.msg, sizeof(Fr), cudaMemcpyDeviceToHost, s));
-  ZK_CUDA(cudaMemcpyAsync(hs + 64, bad, 4, cudaMemcpyDeviceToHost, s));
-  if (host_acc) ZK_CUDA(cudaMemcpyAsync(acc, d_acc, n_table * sizeof(Fr), cudaMemcpyDeviceToHost, s));
-  ZK_CUDA(cudaStreamSynchronize(s));
-  unsigned int was_bad = 0;
-  memcpy(&was_bad, hs + 64, 4);
-  if (was_bad) return fail(ZK_ERR_ARG, "range_aux_accumulate: a selection index is out of range");
-  memcpy(middle_claim_out, hs, sizeof(Fr));
+  if (host_acc) {
+    ZK_CUDA(cudaMemcpyAsync(acc, d_acc, n_table * sizeof(Fr), cudaMemcpyDeviceToHost, s));
+    ZK_CUDA(cudaStreamSynchronize(s));
+  }
+  rc = wait_result(ctx);  // every block's sums are in memory before the last one publishes
+  if (rc) return rc;
+  const Fr* found = reinterpret_cast<const Fr*>(ctx->mailbox);
+  if (!found[1].is_zero()) return fail(ZK_ERR_ARG, "range_aux_accumulate: a selection index is out of range");
+  memcpy(middle_claim_out, found, sizeof(Fr));
   return ZK_OK;
 }
 
