@@ -11,7 +11,7 @@ namespace zk {
 int eq_table_device(zk_ctx* ctx, const uint64_t* point_host, uint32_t k, Fr* table, cudaStream_t on = nullptr);
 size_t keyset_scratch_bytes(uint32_t n_terms, uint32_t num_var);
 int keyset_order(zk_ctx* ctx, const uint64_t* positions_dev, const uint64_t* term_begin_dev, uint32_t n_terms, uint64_t total,
-                 uint32_t num_var, void* scratch, uint32_t* keys_out, uint32_t bad_host[2]);
+                 uint32_t num_var, void* scratch, uint32_t* keys_out, uint32_t* bad_host, const uint32_t** bad_dev = nullptr);
 int comm_sum_fr_vec(zk_ctx* ctx, zk_comm* c, Fr* vals, uint64_t n);
 }
 

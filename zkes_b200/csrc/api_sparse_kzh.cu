@@ -14,7 +14,7 @@ int normalize_device(zk_ctx* ctx, const Jacobian* in, uint64_t n, Affine* out);
 // keyset.cu: distinct keys in increasing order through a bitmap of the domain
 size_t keyset_scratch_bytes(uint32_t n_terms, uint32_t num_var);
 int keyset_order(zk_ctx* ctx, const uint64_t* positions_dev, const uint64_t* term_begin_dev, uint32_t n_terms, uint64_t total,
-                 uint32_t num_var, void* scratch, uint32_t* keys_out, uint32_t bad_host[2]);
+                 uint32_t num_var, void* scratch, uint32_t* keys_out, uint32_t* bad_host, const uint32_t** bad_dev = nullptr);
 }
 
 namespace {
@@ -80,15 +80,19 @@ int zk_sparse_kzh_commit(zk_ctx* ctx, const zk_kzh_srs* srs, uint64_t nnz, const
       from = d_idx;
     }
     ZK_CUDA(cudaMemcpyAsync(d_begin, h_begin, 16, cudaMemcpyHostToDevice, st));
-    uint32_t bad_keys[2] = {0, 0};
-    rc = keyset_order(ctx, from, d_begin, 1, nnz, srs->n, ks, d_full, bad_keys);
+    const uint32_t* bad_keys = nullptr;
+    rc = keyset_order(ctx, from, d_begin, 1, nnz, srs->n, ks, d_full, nullptr, &bad_keys);
     if (rc) return rc;
-    if (bad_keys[0]) return fail(ZK_ERR_ARG, "sparse_kzh_commit: an index is outside the SRS domain");
-    if (!bad_keys[1]) {
-      rc = msm_select_sums(ctx, srs->h[0], srs->h[1], d_full, (uint32_t)nnz, low_bits, (uint32_t)rows, d_jac, d_sel);
-      if (rc) return rc;
-      Jacobian* h_c = reinterpret_cast<Jacobian*>(reinterpret_cast<char*>(ctx->host_small) + 4096);
-      ZK_CUDA(cudaMemcpyAsync(h_c, d_jac + rows, sizeof(Jacobian), cudaMemcpyDeviceToHost, st));
+    // the sums look at the list's error words themselves; the host sees them together with the result
+    rc = msm_select_sums(ctx, srs->h[0], srs->h[1], d_full, bad_keys, (uint32_t)nnz, low_bits, (uint32_t)rows, d_jac, d_sel);
+    if (rc) return rc;
+    Jacobian* h_c = reinterpret_cast<Jacobian*>(reinterpret_cast<char*>(ctx->host_small) + 4096);
+    const uint32_t* h_bad = reinterpret_cast<const uint32_t*>(ctx->host_small);
+    ZK_CUDA(cudaMemcpyAsync(ctx->host_small, bad_keys, 8, cudaMemcpyDeviceToHost, st));
+    ZK_CUDA(cudaMemcpyAsync(h_c, d_jac + rows, sizeof(Jacobian), cudaMemcpyDeviceToHost, st));
+    ZK_CUDA(cudaStreamSynchronize(st));
+    if (h_bad[0]) return fail(ZK_ERR_ARG, "sparse_kzh_commit: an index is outside the SRS domain");
+    if (!h_bad[1]) {
       ZK_CUDA(cudaMemcpyAsync(d_x_jac_out, d_jac, rows * sizeof(Jacobian), cudaMemcpyDeviceToHost, st));
       ZK_CUDA(cudaStreamSynchronize(st));
       const Affine c_aff = jacobian_to_affine_host(*h_c);

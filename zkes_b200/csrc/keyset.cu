@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(256) k_keyset_expand(const uint32_t* __restric
 // keys_out[0 .. total) <- the keys (term << num_var | position) in increasing order.  positions_dev: the terms'
 // position lists concatenated (device); term_begin_dev: n_terms + 1 prefix offsets (device).  scratch: at least
 // keyset_scratch_bytes(...) bytes of device memory.  *bad_host receives {term + 1 with a position out of range or
-// 0, term + 1 with a duplicate or 0}.  Synchronises the stream.
+// 0, term + 1 with a duplicate or 0} and the stream is synchronised; with bad_host null *bad_dev is where they lie on the device.
 size_t keyset_scratch_bytes(uint32_t n_terms, uint32_t num_var) {
   const uint64_t n_words = (((uint64_t)n_terms << num_var) + 31) / 32;
   const uint64_t n_blocks = (n_words + kWordsPerBlock - 1) / kWordsPerBlock;
@@ -102,7 +102,7 @@ size_t keyset_scratch_bytes(uint32_t n_terms, uint32_t num_var) {
 }
 
 int keyset_order(zk_ctx* ctx, const uint64_t* positions_dev, const uint64_t* term_begin_dev, uint32_t n_terms, uint64_t total,
-                 uint32_t num_var, void* scratch, uint32_t* keys_out, uint32_t bad_host[2]) {
+                 uint32_t num_var, void* scratch, uint32_t* keys_out, uint32_t* bad_host, const uint32_t** bad_dev) {
   cudaStream_t s = ctx->stream;
   const uint64_t n_words = (((uint64_t)n_terms << num_var) + 31) / 32;
   const uint64_t n_blocks = (n_words + kWordsPerBlock - 1) / kWordsPerBlock;
@@ -114,8 +114,7 @@ int keyset_order(zk_ctx* ctx, const uint64_t* positions_dev, const uint64_t* ter
   uint32_t* scan_tmp = reinterpret_cast<uint32_t*>(p);
   p += (scan_scratch_elems(n_blocks + 1) * 4 + 255) & ~(size_t)255;
   uint32_t* bad = reinterpret_cast<uint32_t*>(p);
-  ZK_CUDA(cudaMemsetAsync(bitmap, 0, n_words * 4, s));
-  ZK_CUDA(cudaMemsetAsync(bad, 0, 8, s));
+  ZK_CUDA(cudaMemsetAsync(bitmap, 0, (size_t)((char*)bad - (char*)bitmap) + 8, s));  // the counts and scan sums between are written before they are read
   if (total) {
     uint64_t blocks = (total + 255) / 256;
     if (blocks > (uint64_t)ctx->sm_count * 16) blocks = (uint64_t)ctx->sm_count * 16;
@@ -126,6 +125,8 @@ int keyset_order(zk_ctx* ctx, const uint64_t* positions_dev, const uint64_t* ter
     ctx->launches++;
   }
   ZK_CUDA(cudaGetLastError());
+  if (bad_dev) *bad_dev = bad;
+  if (!bad_host) return 0;
   ZK_CUDA(cudaMemcpyAsync(ctx->host_small, bad, 8, cudaMemcpyDeviceToHost, s));
   ZK_CUDA(cudaStreamSynchronize(s));
   memcpy(bad_host, ctx->host_small, 8);

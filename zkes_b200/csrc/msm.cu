@@ -875,37 +875,51 @@ __device__ __forceinline__ uint32_t sel_lower_bound(const uint32_t* __restrict__
   return lo;
 }
 
-__global__ void __launch_bounds__(128) k_select_sums(const Affine* __restrict__ full, const Affine* __restrict__ mid,
-                                                     const uint32_t* __restrict__ idx, uint32_t n, uint32_t low_bits,
-                                                     uint32_t rows, Jacobian* d_x, Xyzz* c_partial) {
-  const uint32_t group = (blockIdx.x * blockDim.x + threadIdx.x) / kSelLanes, gl = threadIdx.x % kSelLanes;
+// A block takes kSelRows rows; its first 128 threads add the rows' points from h_mid, the others the same entries' points from h_full,
+// so that a thread has one chain of additions (inlined, the next point on its way) and a scheduler four warps.  Bound by the chain and the
+// trees.  2^18 entries: 162 us; with both chains in one thread, called products and half the warps 177.
+constexpr int kSelRows = 128 / kSelLanes;
+__global__ void __launch_bounds__(256, 2) k_select_sums(const Affine* __restrict__ full, const Affine* __restrict__ mid,
+                                                     const uint32_t* __restrict__ idx, const uint32_t* __restrict__ bad, uint32_t n,
+                                                     uint32_t low_bits, uint32_t rows, Jacobian* d_x, Xyzz* c_partial) {
+  if (bad[0] | bad[1]) return;  // the list is not in order: the host finds the same and goes another way
+  const uint32_t slot = threadIdx.x & 127u, gl = slot % kSelLanes;
+  const uint32_t group = blockIdx.x * kSelRows + slot / kSelLanes;
+  const bool for_c = threadIdx.x >= 128;
   uint32_t lo = 0, hi = 0;
   if (group < rows) {
     lo = sel_lower_bound(idx, n, (uint64_t)group << low_bits);
     hi = sel_lower_bound(idx, n, ((uint64_t)group + 1) << low_bits);
   }
-  const uint32_t mask = low_bits >= 32 ? 0xffffffffu : (1u << low_bits) - 1u;
-  Xyzz acc_c = Xyzz::inf(), acc_r = Xyzz::inf();
-  for (uint32_t i = lo + gl; i < hi; i += kSelLanes) {
-    const uint32_t v = idx[i];
-    acc_c = add_mixed_calls(acc_c, ld_affine(full + v));
-    acc_r = add_mixed_calls(acc_r, ld_affine(mid + (v & mask)));
+  const uint32_t mask = for_c || low_bits >= 32 ? 0xffffffffu : (1u << low_bits) - 1u;
+  const Affine* bases = for_c ? full : mid;
+  Xyzz acc = Xyzz::inf();
+  uint32_t i = lo + gl;
+  if (i < hi) {
+    Affine next = ld_affine(bases + (idx[i] & mask));
+    uint32_t v = i + kSelLanes < hi ? idx[i + kSelLanes] : 0u;
+#pragma unroll 1
+    for (; i < hi; i += kSelLanes) {
+      const Affine pt = next;
+      if (i + kSelLanes < hi) next = ld_affine(bases + (v & mask));
+      if (i + 2 * kSelLanes < hi) v = idx[i + 2 * kSelLanes];
+      acc = add_mixed(acc, pt);
+    }
   }
   // The lanes' shares of a row: a tree through shared memory.  The time of this kernel follows the number of
   // warp-wide additions it issues, so the additions of a level are packed into as few warps as they fill: the row
   // sums' pairs take the first threads of the block, C's pairs the next, and whole warps sit a level out
   // (128, 64, 32 and 16 additions for the four levels, against two additions by every warp at every level).
-  // The last two levels of the rows and the levels of C across the rows have few additions: four lanes each (quad.cuh; this
+  // The last three levels of the rows and the levels of C across the rows have few additions: four lanes each (quad.cuh; this
   // kernel 210 -> 187 us and the total of the blocks 62 -> 37 us at 2^18 entries).
   __shared__ Xyzz sh[2 * 128];  // [0, 128): shares of the rows' sums; [128, 256): shares of C
-  sh[threadIdx.x] = acc_r;
-  sh[128 + threadIdx.x] = acc_c;
+  sh[threadIdx.x] = acc;
   __syncthreads();
-  constexpr int kRowsPerBlock = 128 / kSelLanes;
+  constexpr int kRowsPerBlock = kSelRows;
 #pragma unroll 1
   for (int off = kSelLanes / 2; off > 0; off >>= 1) {
     const int per_kind = kRowsPerBlock * off;  // additions of this level for one of the two sums
-    if (2 * per_kind > 32) {
+    if (2 * per_kind > 64) {
       if ((int)threadIdx.x < 2 * per_kind) {
         const int kind = (int)threadIdx.x / per_kind, t = (int)threadIdx.x % per_kind;
         Xyzz* at = sh + kind * 128 + (t / off) * kSelLanes + (t % off);
@@ -918,7 +932,7 @@ __global__ void __launch_bounds__(128) k_select_sums(const Affine* __restrict__ 
     }
     __syncthreads();
   }
-  if (group < rows && gl == 0) d_x[group] = to_jacobian(sh[threadIdx.x]);
+  if (group < rows && gl == 0 && !for_c) d_x[group] = to_jacobian(sh[threadIdx.x]);
   // the shares of C of the block's rows
   Xyzz* sh_c = sh + 128;
 #pragma unroll 1
@@ -932,16 +946,19 @@ __global__ void __launch_bounds__(128) k_select_sums(const Affine* __restrict__ 
 }
 
 // C = the sum of the blocks' shares (one block).
-__global__ void __launch_bounds__(256) k_select_total(const Xyzz* __restrict__ c_partial, uint32_t rows, Jacobian* c_out) {
+__global__ void __launch_bounds__(512) k_select_total(const Xyzz* __restrict__ c_partial, const uint32_t* __restrict__ bad, uint32_t rows, Jacobian* c_out) {
   __shared__ Xyzz sh[256];
+  if (bad[0] | bad[1]) return;
   Xyzz acc = Xyzz::inf();
-  for (uint32_t r = threadIdx.x; r < rows; r += blockDim.x) {
-    const Xyzz v = ld_xyzz(c_partial + r);
-    add_to(&acc, &v);
+  if (threadIdx.x < 256) {
+    for (uint32_t r = threadIdx.x; r < rows; r += 256) {
+      const Xyzz v = ld_xyzz(c_partial + r);
+      add_to(&acc, &v);
+    }
+    sh[threadIdx.x] = acc;
   }
-  sh[threadIdx.x] = acc;
   __syncthreads();
-  tree_sum(sh, 256);
+  tree_sum(sh, 256);  // 512 threads: four lanes for every addition
   if (threadIdx.x == 0) *c_out = to_jacobian(sh[0]);
 }
 
@@ -1407,15 +1424,15 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
 }
 
 // C (out_dev[rows]) and d_x (out_dev[0 .. rows)) of a selection polynomial over n indices in non-decreasing order
-// (device, 32-bit), below rows << low_bits.  scratch: rows Xyzz elements of device memory.
-int msm_select_sums(zk_ctx* ctx, const Affine* full, const Affine* mid, const uint32_t* idx_dev, uint32_t n, uint32_t low_bits,
-                    uint32_t rows, Jacobian* out_dev, void* scratch) {
+// (device, 32-bit), below rows << low_bits; nothing is read or written where one of the two words of bad (device) is not zero.
+// scratch: rows Xyzz elements of device memory.
+int msm_select_sums(zk_ctx* ctx, const Affine* full, const Affine* mid, const uint32_t* idx_dev, const uint32_t* bad, uint32_t n,
+                    uint32_t low_bits, uint32_t rows, Jacobian* out_dev, void* scratch) {
   cudaStream_t s = ctx->stream;
   Xyzz* partial = reinterpret_cast<Xyzz*>(scratch);
-  const uint32_t threads = rows * kSelLanes;
-  const uint32_t blocks = (threads + 127) / 128;
-  k_select_sums<<<blocks, 128, 0, s>>>(full, mid, idx_dev, n, low_bits, rows, out_dev, partial);
-  k_select_total<<<1, 256, 0, s>>>(partial, blocks, out_dev + rows);
+  const uint32_t blocks = (rows + kSelRows - 1) / kSelRows;
+  k_select_sums<<<blocks, 256, 0, s>>>(full, mid, idx_dev, bad, n, low_bits, rows, out_dev, partial);
+  k_select_total<<<1, 512, 0, s>>>(partial, bad, blocks, out_dev + rows);
   ctx->launches += 2;
   ctx->msm_calls += 2;
   ctx->msm_entries_sum += 2ull * n;

@@ -36,8 +36,8 @@ int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const
                  uint64_t n, uint32_t rows, Jacobian* out_dev, MsmStats* stats, MsmPrep* prep = nullptr);
 
 // Commitment of a selection polynomial (all listed entries one) without the digit / sort / bucket passes: msm.cu.
-int msm_select_sums(zk_ctx* ctx, const Affine* full, const Affine* mid, const uint32_t* idx_dev, uint32_t n, uint32_t low_bits,
-                    uint32_t rows, Jacobian* out_dev, void* scratch);
+int msm_select_sums(zk_ctx* ctx, const Affine* full, const Affine* mid, const uint32_t* idx_dev, const uint32_t* bad, uint32_t n,
+                    uint32_t low_bits, uint32_t rows, Jacobian* out_dev, void* scratch);
 
 // ---- Host-side inversion (0 maps to 0): the division steps of inverse(), 1.6 us of a CPU core.
 template <class P>
