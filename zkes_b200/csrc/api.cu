@@ -323,19 +323,23 @@ int linear_rounds(zk_ctx* ctx, zk_comm* comm, int L, uint32_t rounds, const Fr**
   // Reads back what the device-resident rounds left in ctx->tail_out: `left` messages and challenges
   // (rounds round_offset + first ...), the transcript state and the resident kernel's error word.
   // The first `canonical` of them are the multi-round kernel's, which writes canonical integers, not Montgomery form.
-  auto collect_device_rounds = [&](uint32_t first, uint32_t left, bool resident, uint32_t canonical) -> int {
+  // published: the kernel puts them into host memory itself, and whether it has.
+  auto collect_device_rounds = [&](uint32_t first, uint32_t left, bool resident, uint32_t canonical, const bool* published = nullptr) -> int {
     const size_t bytes = ((size_t)left * (L + 2)) * sizeof(Fr) + sizeof(StrobeState);
     static_assert(34 * (kMaxPolys + 2) * sizeof(Fr) + sizeof(StrobeState) <= kFinalHostOffset, "34 rounds fit before the final values");
     const unsigned int* h_flags = reinterpret_cast<const unsigned int*>(reinterpret_cast<const char*>(ctx->host_small) + kFlagsHostOffset);
     // the final values and the error word come back in the same copy (the kernels before this point have written them): three
     // copies of some 3 us each were most of what a small prove spent outside its kernel
     if (bytes > kFinalHostOffset) return fail(ZK_ERR_ARG, "device rounds: too many rounds");
-    ZK_CUDA(cudaMemcpyAsync(ctx->host_small, ctx->tail_out, resident ? kFlagsHostOffset + 16 : kFinalHostOffset + (kMaxPolys + 1) * sizeof(Fr),
-                            cudaMemcpyDeviceToHost, ctx->stream));
-    ZK_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (!published || !*published) {
+      ZK_CUDA(cudaMemcpyAsync(ctx->host_small, ctx->tail_out, resident ? kFlagsHostOffset + 16 : kFinalHostOffset + (kMaxPolys + 1) * sizeof(Fr),
+                              cudaMemcpyDeviceToHost, ctx->stream));
+      ZK_CUDA(cudaStreamSynchronize(ctx->stream));
+      if (resident && h_flags[2] >= 2) return fail(ZK_ERR_TIMEOUT, "sharded rounds: another rank's partial sums or table chunk did not arrive");
+      if (resident && h_flags[2] != 0) return fail(ZK_ERR_TIMEOUT, "resident round kernel: a wait for a challenge ran out");
+      if (published) return fail(ZK_ERR_TIMEOUT, "resident round kernel: the stream drained without its results");
+    }
     ctx->final_on_host = true;
-    if (resident && h_flags[2] >= 2) return fail(ZK_ERR_TIMEOUT, "sharded rounds: another rank's partial sums or table chunk did not arrive");
-    if (resident && h_flags[2] != 0) return fail(ZK_ERR_TIMEOUT, "resident round kernel: a wait for a challenge ran out");
     Fr* h_msgs = reinterpret_cast<Fr*>(ctx->host_small);
     Fr* h_chal = h_msgs + (size_t)left * (L + 1);
     const StrobeState* h_st = reinterpret_cast<const StrobeState*>(h_chal + left);
@@ -417,7 +421,7 @@ int linear_rounds(zk_ctx* ctx, zk_comm* comm, int L, uint32_t rounds, const Fr**
           }
           uint32_t ahead_from = 0;
           // message k of the rest is message R + k of the protocol: the kernel writes it at index k + 1
-          const ResidentToEnd te = {ctx->ahead_log, ctx->final_out, d_st, &ahead_from, true};
+          const ResidentToEnd te = {ctx->ahead_log, ctx->final_out, d_st, &ahead_from, true, nullptr, nullptr, nullptr, 0};
           if (launch_resident(L, gathered, tping, tpong, gathered_entries, gathered_log, st, ctx->rs.sink.partials,
                               ctx->rs.max_blocks, ctx->sm_count, sh, d_msgs + (size_t)(R - 1) * (L + 1), d_chal + (R - 1),
                               ctx->stream, nullptr, &te))
@@ -454,14 +458,24 @@ int linear_rounds(zk_ctx* ctx, zk_comm* comm, int L, uint32_t rounds, const Fr**
         // All rounds in one cooperative launch: in step while the tables are large, prepared ahead of their
         // challenges once they are small, final values included.
         uint32_t ahead_from = 0;
-        const ResidentToEnd te = {ctx->ahead_log, ctx->final_out, d_st, &ahead_from, false};
+        char* far = reinterpret_cast<char*>(ctx->host_small_dev);  // tail_out's mirror
+        auto mirror = [&](const void* p) { return far + (reinterpret_cast<const char*>(p) - reinterpret_cast<const char*>(ctx->tail_out)); };
+        const ResidentToEnd te = {ctx->ahead_log, reinterpret_cast<Fr*>(mirror(ctx->final_out)), reinterpret_cast<StrobeState*>(mirror(d_st)),
+                                  &ahead_from, false, reinterpret_cast<Fr*>(mirror(d_msgs)), reinterpret_cast<Fr*>(mirror(d_chal)),
+                                  reinterpret_cast<unsigned int*>(far + kDoneHostOffset), ++ctx->done_seq};
         ctx->prof_begin(ZK_PROF_ROUND, 64.0 * L * (double)(cur_size / 2) + 192.0 * L * (double)(cur_size / 2));
         const int lrc = launch_resident(L, cur, ping, pong, cur_size, rounds, st, ctx->rs.sink.partials, ctx->rs.max_blocks,
                                         ctx->sm_count, sh, d_msgs, d_chal, ctx->stream, nullptr, &te);
         ctx->prof_end();
         if (lrc == 0) {
           ctx->launches++;
-          int rc = collect_device_rounds(0, left, true, left);
+          ZK_CUDA(cudaGetLastError());
+          bool published = true;
+          for (uint32_t word = 0; word < 2 && published; word++) {
+            const int rc = wait_published(ctx, reinterpret_cast<const char*>(ctx->host_small) + kDoneHostOffset + 4 * word, ctx->done_seq, &published);
+            if (rc) return rc;
+          }
+          int rc = collect_device_rounds(0, left, true, left, &published);
           if (rc) return rc;
           *finals_done = true;
           return ZK_OK;

@@ -72,7 +72,9 @@ int zk_ctx::setup() {
   ZK_CUDA(cudaMemsetAsync(resident_sh, 0, 8192, stream));
   ZK_CUDA(cudaMalloc(&tail_buf, sizeof(Fr) * 64 * kMaxPolys * 4));
   ZK_CUDA(cudaHostAlloc(&host_points, kHostPointsBytes, cudaHostAllocDefault));
-  ZK_CUDA(cudaHostAlloc(&host_small, kFlagsHostOffset + 256, cudaHostAllocDefault));
+  ZK_CUDA(cudaHostAlloc(&host_small, kFlagsHostOffset + 256, cudaHostAllocMapped));
+  memset(host_small, 0, kFlagsHostOffset + 256);
+  ZK_CUDA(cudaHostGetDevicePointer(&host_small_dev, host_small, 0));
   ZK_CUDA(cudaStreamSynchronize(stream));
   return 0;
 }

@@ -59,6 +59,7 @@ struct zk_comm;
 // values, then the hand-over area of the resident kernel (host_small mirrors its first 16 bytes, the error word among them)
 constexpr size_t kFinalHostOffset = 7168;
 constexpr size_t kFlagsHostOffset = 8192;
+constexpr size_t kDoneHostOffset = kFlagsHostOffset + 64;  // two words that the resident kernel sets when its results are in host_small
 constexpr size_t kHostPointsBytes = 68 * 1024;  // zk_ctx::host_points
 
 struct zk_ctx {
@@ -74,6 +75,8 @@ struct zk_ctx {
   void* resident_sh = nullptr;   // zk::ResidentShared: hand-over area of the resident multi-round kernel (8 KiB, inside tail_out's block)
   zk::Fr* tail_buf = nullptr;    // sharded proves: gathered values and the last log2(world) rounds' tables
   void* host_small = nullptr;    // pinned, kFlagsHostOffset + 256 bytes: round messages and other tiny read-backs
+  void* host_small_dev = nullptr;  // its device view
+  unsigned int done_seq = 0;       // of the last launch that puts its results there itself
   void* mailbox = nullptr;       // pinned + mapped: message kernels publish here, the host polls
   void* work = nullptr;          // grow-only device scratch (copies of caller data, round buffers)
   size_t work_bytes = 0;

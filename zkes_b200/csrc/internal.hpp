@@ -173,6 +173,10 @@ struct ResidentToEnd {    // launch_resident runs to the end of the protocol
   bool pending;           // the tables still have to be bound on sh->challenge, left with the transcript state in sh->st by
                           // the launch before (which stopped early): log2(size) - 1 messages remain, all prepared ahead;
                           // message k of them goes to out_msgs[(k + 1) * (L + 1)], its challenge to out_chal[k + 1]
+  Fr* far_msgs;           // with `done` (not pending): host memory, device view, for all messages and challenges; out_final and
+  Fr* far_chal;           // out_st are host memory then, too
+  unsigned int* done;     // two words in host memory that become `seq` when everything is there; an error leaves them as they are
+  unsigned int seq;
 };
 // px != nullptr: the tables are this rank's chunks of a sharded instance; every round's message is the
 // sum over the ranks, exchanged through the peer boxes by the block that completes the local sums.
