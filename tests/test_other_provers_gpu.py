@@ -52,6 +52,22 @@ def test_sparse_bool_random(ctx, n, terms, k):
     assert res == pr.final_eval
 
 
+@pytest.mark.parametrize("share", [0.03, 0.5, 1.0])
+@pytest.mark.parametrize("n", [1, 2, 10, 11, 12])
+def test_sparse_bool_coordinates_on_the_cube(ctx, n, share):
+    """The eq factors of the bound variables are put back by the host (0 and 1 among the point's coordinates make them vanish), the tables
+    of the others are sums of the one before (1024 entries a block); lone entries only, pairs, and nothing but pairs."""
+    rnd = random.Random(n * 100 + int(share * 10))
+    pos = [rnd.sample(range(1 << n), max(1, int(share * (1 << n)))) for _ in range(2)]
+    w = [rnd.randrange(M) for _ in range(2)]
+    for pt in ([0] * n, [rnd.choice([0, 1, M - 1, rnd.randrange(M)]) for _ in range(n)]):
+        t, ot = Transcript(b"range"), o.Transcript(b"range")
+        p, op = SparseBoolSumcheckProver(n, t), o.SparseBoolSumcheckProver(n, ot)
+        pr, opr = p.prove(ctx, w, pos, pt, t), op.prove(w, pos, pt, ot)
+        assert pr.round_messages == opr.round_messages and p.challenges == op.challenges
+        assert pr.final_eval == opr.final_eval
+
+
 def test_sparse_bool_lookup_scale_verifies(ctx):
     """At the size of one of the trace's boolean checks (48 selection terms of 2^17 ones over 2^21 positions, 6.3
     million entries: every warp's span is thousands of entries long and crosses terms, the pair queue fills many

@@ -49,15 +49,13 @@ int sbool_prove(zk_ctx* ctx, zk_comm* comm, uint32_t num_var, uint32_t n_terms, 
   cudaStream_t s = ctx->stream;
   const uint64_t size = 1ull << num_var;
   char* base = nullptr;
-  size_t need = al((size + size / 2 + 8) * sizeof(Fr)) + al((size / 2 * 3 + 8) * sizeof(Fr)) + 2 * (al((K + 1) * 4ull) + al((K + 1) * sizeof(Fr))) +
+  size_t need = al((size + 1) * sizeof(Fr)) + 2 * (al((K + 1) * 4ull) + al((K + 1) * sizeof(Fr))) +
                 al((K / 256 + 2) * 4ull) + al((n_terms + 1) * sizeof(Fr)) + 4096;
   int rc = ctx->reserve_work(need, (void**)&base);
   if (rc) return rc;
   size_t o = 0;
   auto take = [&](size_t bytes) { char* p = base + o; o += al(bytes); return p; };
-  Fr* eq0 = (Fr*)take((size + 1) * sizeof(Fr));
-  Fr* eq1 = (Fr*)take((size / 2 + 1) * sizeof(Fr));
-  Fr* eq_rec = (Fr*)take((size / 2 * 3 + 8) * sizeof(Fr));  // per-position records of the rounds after the first
+  Fr* eqs = (Fr*)take((size + 1) * sizeof(Fr));  // the eq table of the variables after the round's own, one round after the other
   uint32_t* e_key[2] = {(uint32_t*)take((K + 1) * 4ull), (uint32_t*)take((K + 1) * 4ull)};
   Fr* e_val[2] = {(Fr*)take((K + 1) * sizeof(Fr)), (Fr*)take((K + 1) * sizeof(Fr))};
   uint32_t* block_counts = (uint32_t*)take((K / 256 + 2) * 4ull);
@@ -70,8 +68,8 @@ int sbool_prove(zk_ctx* ctx, zk_comm* comm, uint32_t num_var, uint32_t n_terms, 
     rc = ctx->reserve_aux(pos_bytes + tb_bytes + keyset_scratch_bytes(n_terms, num_var), (void**)&ks);
     if (rc) return rc;
   }
-  // What does not depend on the positions runs on the side stream while they cross the bus: the eq table over the full hypercube
-  // (:509), the entries' first values, the weights.  With the per-kernel profiler on it stays in line.
+  // What does not depend on the positions runs on the side stream while they cross the bus: the eq tables (:509), the
+  // entries' first values, the weights.  With the per-kernel profiler on it stays in line.
   const bool beside = !ctx->prof_on;
   cudaStream_t s2 = beside ? ctx->side_stream : s;
   if (beside) {
@@ -86,7 +84,10 @@ int sbool_prove(zk_ctx* ctx, zk_comm* comm, uint32_t num_var, uint32_t n_terms, 
       launch_fill_ones(e_val[0], K, ctx->sm_count, s2);
       ctx->launches++;
     }
-    return eq_table_device(ctx, eq_point, num_var, eq0, s2);
+    if (num_var == 0) return ZK_OK;
+    const int rc = eq_table_device(ctx, eq_point + 4, num_var - 1, eqs, s2);
+    if (!rc) ctx->launches += launch_eq_sums(eqs, size / 2, s2);
+    return rc;
   };
   auto order = [&](uint32_t (&bad)[2]) -> int {
     uint64_t* d_pos = reinterpret_cast<uint64_t*>(ks);
@@ -111,37 +112,41 @@ int sbool_prove(zk_ctx* ctx, zk_comm* comm, uint32_t num_var, uint32_t n_terms, 
   if (bad[1]) return fail(ZK_ERR_ARG, "sparse_bool_prove: duplicate position in term %u", bad[1] - 1);
   ZK_CUDA(cudaStreamSynchronize(s));  // the weights' host buffer may go out of scope after this
 
-  const Fr* eq_cur = eq0;
+  Fr bound = Fr::one();  // eq over the variables bound so far
   int e = 0;
   uint32_t k_upper = K;
   Fr challenge = Fr::zero();
   for (uint32_t round = 0; round < num_var; round++) {
     const uint32_t vars_left = num_var - round;
     const uint64_t S = 1ull << vars_left;
-    // every value is one in the first round (the fill above); later rounds read the eq factors from the records that the
-    // round before left
-    launch_sbool_msg(e_key[e], e_val[e], counts + e, k_upper, round ? eq_rec : eq_cur, d_w, vars_left, round == 0,
+    // every value is one in the first round (the fill above)
+    launch_sbool_msg(e_key[e], e_val[e], counts + e, k_upper, eqs + (size - S), d_w, vars_left, round == 0,
                      ctx->next_msg_scratch(comm != nullptr), s);
     ctx->launches++;
+    const Fr tau = fr_load(eq_point + 4 * (uint64_t)round);
+    Fr scale[4];  // eq over the variables bound so far and the round's own at c = 0..3
+    scale[1] = mul(bound, tau);
+    scale[0] = sub(bound, scale[1]);
+    const Fr slope = sub(scale[1], scale[0]);
+    scale[2] = add(scale[1], slope);
+    scale[3] = add(scale[2], slope);
     // where the folded entries go depends on the positions alone: it is worked out while the host has the message
     auto slots = [&] {
       ctx->launches += launch_sparse_slots(e_key[e], counts + e, k_upper, block_counts, counts + (e ^ 1), s);
     };
     if (!comm) slots();
-    rc = fs_round(ctx, comm, 4, round, fs, fs_user, tr, round_msgs, challenges, &challenge);
+    rc = fs_round(ctx, comm, 4, round, fs, fs_user, tr, round_msgs, challenges, &challenge, false, scale);
     if (rc) return rc;
-    Fr* eq_next = (round & 1) ? eq0 : eq1;  // eq0 holds 2^n, eq1 2^(n-1); later rounds fit either
     if (comm) slots();  // (there the exchange kernel is next on the stream)
-    launch_bool_fold(e_key[e], e_val[e], counts + e, k_upper, challenge, block_counts, e_key[e ^ 1], e_val[e ^ 1], eq_cur, S, eq_next, eq_rec,
-                     ctx->sm_count, s);
+    launch_bool_fold(e_key[e], e_val[e], counts + e, k_upper, challenge, block_counts, e_key[e ^ 1], e_val[e ^ 1], s);
     ctx->launches++;
-    eq_cur = eq_next;
+    bound = add(scale[0], mul(challenge, slope));
     e ^= 1;
     // a term keeps at most one entry per remaining position: the bound the next round's grids are sized by
     const uint64_t cap = (uint64_t)n_terms * (S / 2);
     if (cap < k_upper) k_upper = (uint32_t)cap;
   }
-  launch_sbool_final(e_key[e], e_val[e], counts + e, eq_cur, d_w, n_terms, ctx->final_out, s);
+  launch_sbool_final(e_key[e], e_val[e], counts + e, bound, d_w, n_terms, ctx->final_out, s);
   ctx->launches++;
   ZK_CUDA(cudaGetLastError());
   rc = comm_sum_fr_vec(ctx, comm, ctx->final_out, 1);  // the final value is a sum over terms too

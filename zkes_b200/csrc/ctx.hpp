@@ -169,7 +169,7 @@ int comm_peer_gather(zk_ctx* ctx, zk_comm* c, int n_tables, const Fr* const* chu
                      const Fr** tables_out);
 int fs_round(zk_ctx* ctx, zk_comm* comm, int n_msgs, uint32_t round, fs_round_fn_t fs, void* fs_user, zk_transcript* tr,
              uint64_t* round_msgs, uint64_t* challenges, Fr* challenge,
-             bool exchanged_by_kernel = false);
+             bool exchanged_by_kernel = false, const Fr* bool_scale = nullptr);
 int linear_rounds(zk_ctx* ctx, zk_comm* comm, int L, uint32_t rounds, const Fr** cur, Fr** ping, Fr** pong,
                   uint32_t round_offset, fs_round_fn_t fs, void* fs_user, zk_transcript* tr, uint64_t* round_msgs,
                   uint64_t* challenges, Fr* challenge, bool* finals_done);

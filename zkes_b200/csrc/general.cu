@@ -18,29 +18,26 @@ __device__ __forceinline__ Fr g_ld(const Fr* p) {
   return fr_from_chunks(lo, hi);
 }
 
-// T(c), c = 0..3, over the live entries (compute_round_message, :529-591): sum_j w_j sum_y aux(aux - 1) eq at the
-// point c, where aux(c) = v0 (1 - c) + v1 c for the pair (v0, v1) of an even / odd position.
+// The round message (compute_round_message, :529-591) is s(c) = sum_y eq(c, y) sum_j w_j aux(aux - 1), c = 0..3, with aux(c) =
+// v0 + c (v1 - v0) for the pair (v0, v1) of an even / odd position.  The variable of the round has the factor K eq(tau, c) in eq to itself,
+// K the same factor of the variables bound before, so that s(c) = K eq(tau, c) t(c) with t of degree two in c: the kernel sums
+//   t(0) = sum_y E (v0^2 - v0),   t(1) = sum_y E (v1^2 - v1),   and t's leading coefficient   sum_y E (v1 - v0)^2
+// (weights and terms understood), E the eq table of the variables still to come, and the host makes the four values of them
+// (bool_message).  E needs no folding: it is the sum over the lowest variable of the table before (k_eq_sums), whatever the challenges.
 //
-// Entry by entry instead of pair by pair: (a + b)^2 - (a + b) = (a^2 - a) + (b^2 - b) + 2 a b, so a pair is its two
-// entries taken alone plus the cross term 2 v0 v1 c (1 - c).  An entry alone (value v on side b, nothing on the
-// other side) gives, with q = v^2:
-//   c = b: q - v         c = 1 - b: 0         c = 2: b ? 4q - 2v : q + v         c = 3: b ? 9q - 3v : 4q + 2v
-// times eq(c): one square and three products per entry whatever its parity (no branch), against eight for a pair
-// formed first.  The cross term (-4 v0 v1 eq(2) and -12 v0 v1 eq(3)) exists only where both sides are present,
-// one entry in sixteen for the selection polynomials of the lookups; those entries are queued per warp and worked
-// off thirty-two at a time, so that the rare case does not cost every warp its products.
-//
-// The eq factors come from a per-position record built once per round (k_bool_fold; the table is far smaller than
-// the entry list, which repeats every position once per term): an even position holds {eq(0), eq(2), 2 eq(3)}, an
-// odd one {eq(1), 2 eq(2), 3 eq(3)}, so the entry's own factors are q - v, then q + v or 2q - v, then 2q + v or
-// 3q - v: sums of at most four field elements, formed without reduction (they stay below 2^256, which the second
-// operand of mul() may be).
+// Entry by entry instead of pair by pair: an entry alone (value v) is two products, u = E v and u v; a pair's cross term -2 E v0 v1
+// exists only where both sides are present, one entry in sixteen for the selection polynomials of the lookups; those entries are queued
+// per warp and worked off thirty-two at a time, so that the rare case does not cost every warp its products.
+// (With four values straight from records {eq(c), c = 0..3} of every position it was a square and three products an entry and 96 bytes
+// gathered for 32: 20 rounds over 16 x 2^17 entries in 1 242 us, now 789.)
 //
 // The entries are ordered by (term, position), so a warp that walks a contiguous span of them stays inside one term
 // for thousands of entries: the weight is taken out of the inner sum and multiplied in when a lane's term changes.
+// The gather of E depends on the position: the entry after the next is looked up, and the next one's value and E are on their way,
+// while an entry is computed.
 //
-// ONES: the first round, where every value is one (the selection polynomials are 0/1): an entry alone gives
-// 2 eq(2) and 6 eq(3), a pair nothing; no value is read and nothing is multiplied but the weights.
+// ONES: the first round, where every value is one (the selection polynomials are 0/1): t(0) = t(1) = 0, and an entry alone adds E to the
+// leading coefficient, a pair nothing; no value is read and nothing is multiplied but the weights.
 constexpr int kPairQueue = 64;  // per warp: a batch of 32 plus what one more sweep can add
 
 template <bool ONES>
@@ -51,48 +48,44 @@ __global__ void __launch_bounds__(kGThreads, 2) k_sbool_msg(const uint32_t* __re
   __shared__ uint32_t queue[ONES ? 1 : kGThreads / 32][ONES ? 1 : kPairQueue];
   const uint32_t n = *count;
   const uint32_t mask = (vars_left >= 32) ? 0xffffffffu : ((1u << vars_left) - 1u);
-  // the weighted sums over all terms are touched once per term: they live in shared memory, which leaves the
-  // registers to the four running sums and the products (no spills at two blocks per SM)
-  __shared__ Fr s_sm[4][kGThreads];
+  // the weighted sums over all terms are touched once per term: they live in shared memory
+  __shared__ Fr s_sm[3][kGThreads];
   auto s_add = [&](int c, const Fr& x, bool negate) {
     const Fr cur = s_sm[c][threadIdx.x];
     s_sm[c][threadIdx.x] = negate ? sub(cur, x) : add(cur, x);
   };
 #pragma unroll
-  for (int c = 0; c < 4; c++) s_sm[c][threadIdx.x] = Fr::zero();
-  // the sums over the term this lane is in, without its weight.  ONES: two field elements.  Otherwise unreduced 512-bit
-  // sums of products, which halves their multiply-adds (20 rounds over 16 x 2^17 entries: 1 347 -> 1 255 us); the sum for c = 0
-  // or c = 1 is picked by the entry's parity, so they live in shared memory (four 16-byte words per sum and thread, conflict
-  // free), trimmed below p 2^256 after every product.
-  Fr inner[2] = {Fr::zero(), Fr::zero()};
-  extern __shared__ uint4 s_wide[];  // [4][4][kGThreads]
-  auto wide_ld = [&](int c, Wide& w) {
+  for (int c = 0; c < 3; c++) s_sm[c][threadIdx.x] = Fr::zero();
+  // the sums over the term this lane is in, without its weight.  ONES: a field element.  Otherwise, for either parity, an unreduced
+  // 512-bit sum of the products u v and the sum of the u; picked by the entry's parity, so they live in shared memory (16-byte words
+  // kGThreads apart, conflict free), the products trimmed below p 2^256 one by one.
+  Fr inner = Fr::zero();
+  extern __shared__ uint4 s_sums[];  // [2][6][kGThreads]
+  auto wide_ld = [&](int b, Wide& w) {
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      const uint4 x = s_wide[(c * 4 + k) * kGThreads + threadIdx.x];
+      const uint4 x = s_sums[(b * 6 + k) * kGThreads + threadIdx.x];
       w.v[4 * k] = x.x;
       w.v[4 * k + 1] = x.y;
       w.v[4 * k + 2] = x.z;
       w.v[4 * k + 3] = x.w;
     }
   };
-  auto wide_st = [&](int c, const Wide& w) {
+  auto wide_st = [&](int b, const Wide& w) {
 #pragma unroll
     for (int k = 0; k < 4; k++)
-      s_wide[(c * 4 + k) * kGThreads + threadIdx.x] = make_uint4(w.v[4 * k], w.v[4 * k + 1], w.v[4 * k + 2], w.v[4 * k + 3]);
+      s_sums[(b * 6 + k) * kGThreads + threadIdx.x] = make_uint4(w.v[4 * k], w.v[4 * k + 1], w.v[4 * k + 2], w.v[4 * k + 3]);
   };
-  // sum c += a f for a < p and f < 4p (4 p^2 < p 2^256, so one product on top of a trimmed sum can be trimmed again)
-  auto wide_acc = [&](int c, const Fr& a, const Fr& f) {
-    Wide w, sum;
-    mul_wide(w, a.v, f.v);
-    wide_ld(c, sum);
-    wide_add(sum, w);
-    wide_trim<FrParams>(sum);
-    wide_st(c, sum);
+  auto lin_ld = [&](int b) { return fr_from_chunks(s_sums[(b * 6 + 4) * kGThreads + threadIdx.x], s_sums[(b * 6 + 5) * kGThreads + threadIdx.x]); };
+  auto lin_st = [&](int b, const Fr& x) {
+    uint4 lo, hi;
+    fr_to_chunks(x, lo, hi);
+    s_sums[(b * 6 + 4) * kGThreads + threadIdx.x] = lo;
+    s_sums[(b * 6 + 5) * kGThreads + threadIdx.x] = hi;
   };
   if constexpr (!ONES) {
 #pragma unroll
-    for (int k = 0; k < 16; k++) s_wide[k * kGThreads + threadIdx.x] = make_uint4(0, 0, 0, 0);
+    for (int k = 0; k < 12; k++) s_sums[k * kGThreads + threadIdx.x] = make_uint4(0, 0, 0, 0);
   }
   uint32_t cur_term = 0xffffffffu;
   const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -104,44 +97,54 @@ __global__ void __launch_bounds__(kGThreads, 2) k_sbool_msg(const uint32_t* __re
   auto flush = [&](uint32_t term) {
     const Fr w = g_ld(weights + term);
     if constexpr (ONES) {
-      const Fr t2 = add(inner[0], inner[0]), t3 = add(inner[1], inner[1]);
-      s_add(2, mul(w, t2), false);
-      s_add(3, mul(w, add(add(t3, t3), t3)), false);
-      inner[0] = inner[1] = Fr::zero();
+      s_add(2, mul(w, inner), false);
+      inner = Fr::zero();
     } else {
       Wide zero;
 #pragma unroll
       for (int k = 0; k < 16; k++) zero.v[k] = 0;
+      Fr all = Fr::zero();
 #pragma unroll 1
-      for (int c = 0; c < 4; c++) {
+      for (int b = 0; b < 2; b++) {
         Wide sum;
-        wide_ld(c, sum);
-        s_add(c, mul(w, redc<FrParams>(sum)), false);
-        wide_st(c, zero);
+        wide_ld(b, sum);
+        const Fr x = redc<FrParams>(sum);
+        s_add(b, mul(w, sub(x, lin_ld(b))), false);
+        all = add(all, x);
+        wide_st(b, zero);
+        lin_st(b, Fr::zero());
       }
+      s_add(2, mul(w, all), false);
     }
   };
-  // the cross terms of 32 queued pairs (or of what is left, at the end); the even position's record holds
-  // eq(2) and 2 eq(3)
+  // the cross terms of 32 queued pairs (or of what is left, at the end)
   auto work_off = [&](uint32_t cnt) {
     if (lane < cnt) {
       const uint32_t i = queue[ONES ? 0 : wib][ONES ? 0 : lane];
       const uint32_t key = keys[i];
-      const Fr* rec = eq + 3 * (uint64_t)(key & mask);
       const Fr w = g_ld(weights + (vars_left >= 32 ? 0 : (key >> vars_left)));
       const Fr wx = mul(w, mul(g_ld(val + i), g_ld(val + i + 1)));
-      const Fr a = mul(wx, g_ld(rec + 1)), b = mul(wx, g_ld(rec + 2));
-      const Fr a2 = add(a, a), b2 = add(b, b);
-      s_add(2, add(a2, a2), true);           // 4 v0 v1 eq(2)
-      s_add(3, add(add(b2, b2), b2), true);  // 12 v0 v1 eq(3)
+      const Fr a = mul(wx, g_ld(eq + ((key & mask) >> 1)));
+      s_add(2, add(a, a), true);
     }
   };
+  auto key_at = [&](uint64_t i) { return i < end ? keys[i] : 0u; };
+  uint32_t key = key_at(begin + lane), key_n = key_at(begin + lane + 32);
+  Fr v = Fr::zero(), ev = Fr::zero();
+  if (begin + lane < end) {
+    if (!ONES) v = g_ld(val + begin + lane);
+    ev = g_ld(eq + ((key & mask) >> 1));
+  }
   for (uint64_t base = begin; base < end; base += 32) {
     const uint64_t i = base + lane;
     const bool valid = i < end;
-    const uint32_t key = valid ? keys[i] : 0u;
+    const uint32_t key_nn = key_at(i + 64);
+    Fr v_n = v, e_n = ev;
+    if (i + 32 < end) {
+      if (!ONES) v_n = g_ld(val + i + 32);
+      e_n = g_ld(eq + ((key_n & mask) >> 1));
+    }
     const bool odd = key & 1u;
-    const uint32_t pos = key & mask;
     const uint32_t term = vars_left >= 32 ? 0 : (key >> vars_left);
     if (valid && term != cur_term) {
       if (cur_term != 0xffffffffu) flush(cur_term);
@@ -150,37 +153,18 @@ __global__ void __launch_bounds__(kGThreads, 2) k_sbool_msg(const uint32_t* __re
     if constexpr (ONES) {
       // alone unless the neighbour of the same pair is the next (previous) entry
       const bool lone = valid && (odd ? !(i > 0 && keys[i - 1] == key - 1) : !(i + 1 < n && keys[i + 1] == key + 1));
-      if (lone) {
-        const Fr e0 = g_ld(eq + (pos & ~1u)), e1 = g_ld(eq + (pos | 1u));
-        const Fr de = sub(e1, e0);
-        const Fr e2 = add(e1, de);
-        inner[0] = add(inner[0], e2);
-        inner[1] = add(inner[1], add(e2, de));
-      }
+      if (lone) inner = add(inner, ev);
     } else {
       if (valid) {
-        const Fr v = g_ld(val + i);
-        const Fr* rec = eq + 3 * (uint64_t)pos;
-        const Fr q = sqr(v);
-        uint32_t pm[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++) pm[k] = FrParams::mod(k);
-        Fr f0, f2, f3, sv, q2, q3, t2, t3;
-        sub_lazy(f0.v, q, v);                 // q - v (+ p)
-        (void)sub8(sv.v, pm, v.v);            // p - v
-        (void)add8(q2.v, q.v, q.v);           // 2q
-        (void)add8(q3.v, q2.v, q.v);          // 3q
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-          sv.v[k] = odd ? sv.v[k] : v.v[k];   // +v on the even side, -v on the odd one
-          t2.v[k] = odd ? q2.v[k] : q.v[k];
-          t3.v[k] = odd ? q3.v[k] : q2.v[k];
-        }
-        (void)add8(f2.v, t2.v, sv.v);         // q + v | 2q - v  (< 3p)
-        (void)add8(f3.v, t3.v, sv.v);         // 2q + v | 3q - v  (< 4p < 2^256)
-        wide_acc(odd ? 1 : 0, g_ld(rec), f0);
-        wide_acc(2, g_ld(rec + 1), f2);
-        wide_acc(3, g_ld(rec + 2), f3);
+        const Fr u = mul(ev, v);
+        const int b = odd ? 1 : 0;
+        Wide x, sum;
+        mul_wide(x, u.v, v.v);
+        wide_ld(b, sum);
+        wide_add(sum, x);
+        wide_trim<FrParams>(sum);
+        wide_st(b, sum);
+        lin_st(b, add(lin_ld(b), u));
       }
       // an even entry whose odd neighbour is present: queue the pair's cross term
       const bool pair = valid && !odd && i + 1 < n && keys[i + 1] == key + 1;
@@ -196,19 +180,53 @@ __global__ void __launch_bounds__(kGThreads, 2) k_sbool_msg(const uint32_t* __re
         __syncwarp();
       }
     }
+    key = key_n;
+    key_n = key_nn;
+    v = v_n;
+    ev = e_n;
   }
   if constexpr (!ONES) {
     if (queued) work_off(queued);
   }
   if (cur_term != 0xffffffffu) flush(cur_term);
-  Fr s[4];
+  Fr s[3];
 #pragma unroll
-  for (int c = 0; c < 4; c++) s[c] = s_sm[c][threadIdx.x];
-  grid_sum<4, kGThreads / 32>(s, sink);
+  for (int c = 0; c < 3; c++) s[c] = s_sm[c][threadIdx.x];
+  grid_sum<3, kGThreads / 32>(s, sink);
 }
 
-// final_evaluation (:644-655): eq[0] * sum_j w_j v_j (v_j - 1), v_j = the entry with key j.
-__global__ void k_sbool_final(const uint32_t* keys, const Fr* val, const uint32_t* count, const Fr* eq,
+// The eq tables of fewer and fewer variables: level l of a table of n entries (a power of two), at tab + 2 n - (2 n >> l), sums the
+// pairs of the level before (eq(tau, 0) + eq(tau, 1) = 1).  A block takes kSumBlock entries and the levels up to one entry of its own.
+constexpr uint32_t kSumBlock = 1024;
+__global__ void __launch_bounds__(256) k_eq_sums(Fr* tab, uint64_t n) {
+  __shared__ Fr sh[kSumBlock / 2];
+  uint32_t m = n < kSumBlock ? (uint32_t)n : kSumBlock;
+  const Fr* src = tab + (uint64_t)blockIdx.x * m;
+  for (int level = 1; m > 1; level++) {
+    m >>= 1;
+    Fr* out = tab + 2 * n - ((2 * n) >> level) + (uint64_t)blockIdx.x * m;
+    Fr r[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const uint32_t t = threadIdx.x + 256 * k;
+      if (t < m) r[k] = add(src[2 * t], src[2 * t + 1]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const uint32_t t = threadIdx.x + 256 * k;
+      if (t < m) {
+        sh[t] = r[k];
+        out[t] = r[k];
+      }
+    }
+    __syncthreads();
+    src = sh;
+  }
+}
+
+// final_evaluation (:644-655): eq * sum_j w_j v_j (v_j - 1), v_j = the entry with key j, eq at the challenges.
+__global__ void k_sbool_final(const uint32_t* keys, const Fr* val, const uint32_t* count, const Fr eq,
                               const Fr* weights, uint32_t n_terms, Fr* out) {
   const uint32_t n = *count;
   const Fr one = Fr::one();
@@ -220,7 +238,7 @@ __global__ void k_sbool_final(const uint32_t* keys, const Fr* val, const uint32_
     inner = add(inner, mul(weights[j], mul(v, sub(v, one))));
   }
   inner = warp_sum(inner);
-  if (threadIdx.x == 0) out[0] = mul(eq[0], inner);
+  if (threadIdx.x == 0) out[0] = mul(eq, inner);
 }
 
 __global__ void k_fill_ones(Fr* out, uint32_t n) {
@@ -306,19 +324,30 @@ inline int g_blocks(uint64_t n, const RoundScratch& sc) {
 
 }  // namespace
 
-// The unreduced sums of k_sbool_msg<false>: 64 KB beside its 36 KB of static shared memory, two blocks per SM.
-constexpr int kWideBytes = 16 * kGThreads * (int)sizeof(uint4);
+// The sums of k_sbool_msg<false>: 48 KB beside its 27 KB of static shared memory, two blocks per SM.
+constexpr int kSumBytes = 12 * kGThreads * (int)sizeof(uint4);
 
 void launch_sbool_msg(const uint32_t* keys, const Fr* val, const uint32_t* count, uint32_t upper, const Fr* eq,
                       const Fr* weights, uint32_t vars_left, bool ones, const RoundScratch& sc, cudaStream_t s) {
   if (ones) {
     k_sbool_msg<true><<<g_blocks(upper, sc), kGThreads, 0, s>>>(keys, val, count, eq, weights, vars_left, sc.sink);
   } else {
-    (void)resident_blocks((const void*)k_sbool_msg<false>, kGThreads, kWideBytes);
-    k_sbool_msg<false><<<g_blocks(upper, sc), kGThreads, kWideBytes, s>>>(keys, val, count, eq, weights, vars_left, sc.sink);
+    (void)resident_blocks((const void*)k_sbool_msg<false>, kGThreads, kSumBytes);
+    k_sbool_msg<false><<<g_blocks(upper, sc), kGThreads, kSumBytes, s>>>(keys, val, count, eq, weights, vars_left, sc.sink);
   }
 }
-void launch_sbool_final(const uint32_t* keys, const Fr* val, const uint32_t* count, const Fr* eq, const Fr* weights,
+int launch_eq_sums(Fr* tab, uint64_t n, cudaStream_t s) {
+  int launches = 0;
+  while (n > 1) {
+    const uint64_t blocks = n > kSumBlock ? n / kSumBlock : 1;
+    k_eq_sums<<<(unsigned)blocks, 256, 0, s>>>(tab, n);
+    launches++;
+    tab += 2 * n - 2 * blocks;  // the level of one entry a block
+    n = blocks;
+  }
+  return launches;
+}
+void launch_sbool_final(const uint32_t* keys, const Fr* val, const uint32_t* count, const Fr& eq, const Fr* weights,
                         uint32_t n_terms, Fr* out, cudaStream_t s) {
   k_sbool_final<<<1, 32, 0, s>>>(keys, val, count, eq, weights, n_terms, out);
 }

@@ -60,10 +60,12 @@ int launch_int_fold(const void* t, const Fr* eq, uint64_t n_rows, uint64_t m_col
                     cudaStream_t s);
 
 // general.cu
-// eq: the plain table when `ones` (first round, every value one), else the per-position records that launch_bool_fold leaves
+// eq: the table of the variables after the round's own; publishes t(0), t(1) and t's leading coefficient (bool_message)
 void launch_sbool_msg(const uint32_t* keys, const Fr* val, const uint32_t* count, uint32_t upper, const Fr* eq,
                       const Fr* weights, uint32_t vars_left, bool ones, const RoundScratch& sc, cudaStream_t s);
-void launch_sbool_final(const uint32_t* keys, const Fr* val, const uint32_t* count, const Fr* eq, const Fr* weights,
+// the sums over more and more of the lowest variables of an eq table of n entries, one after the other behind it (n - 1 entries more)
+int launch_eq_sums(Fr* tab, uint64_t n, cudaStream_t s);
+void launch_sbool_final(const uint32_t* keys, const Fr* val, const uint32_t* count, const Fr& eq, const Fr* weights,
                         uint32_t n_terms, Fr* out, cudaStream_t s);
 void launch_fill_ones(Fr* out, uint32_t n, int sm_count, cudaStream_t s);
 void launch_general_msg(const Fr* const* tables_dev, const Fr* scalars, const Fr* eq, uint32_t n_terms, uint32_t n_factors,
@@ -198,11 +200,9 @@ void launch_scatter_runs(const uint32_t* idx, const Fr* val, const uint32_t* cou
 // in all.  Depends on the positions alone, so it need not wait for the round's challenge.
 int launch_sparse_slots(const uint32_t* idx, const uint32_t* count, uint32_t upper, uint32_t* block_counts, uint32_t* count_out,
                         cudaStream_t s);
-// The entries bound on r at the slots that launch_sparse_slots made, and the eq table of eq_size entries: eq_out = eq bound on r; rec:
-// the records of its pairs, rec[3 p .. 3 p + 2] for every position p: {eq(0), eq(2), 2 eq(3)} (p even) or {eq(1), 2 eq(2), 3 eq(3)}
-// (p odd) of p's pair (none for eq_size 2).
+// The entries bound on r at the slots that launch_sparse_slots made.
 void launch_bool_fold(const uint32_t* idx, const Fr* val, const uint32_t* count, uint32_t upper, const Fr& r, const uint32_t* block_offsets,
-                      uint32_t* idx_out, Fr* val_out, const Fr* eq, uint64_t eq_size, Fr* eq_out, Fr* rec, int sm_count, cudaStream_t s);
+                      uint32_t* idx_out, Fr* val_out, cudaStream_t s);
 void launch_scatter(const uint32_t* idx, const Fr* val, const uint32_t* count, uint32_t upper, Fr* dense,
                     int sm_count, cudaStream_t s);
 void launch_check_sorted(const uint32_t* idx, uint32_t n, uint64_t limit, uint32_t* bad, int sm_count, cudaStream_t s);

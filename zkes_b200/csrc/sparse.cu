@@ -221,44 +221,13 @@ __global__ void __launch_bounds__(1024) k_scan_blocks(uint32_t* block_counts, ui
   if (threadIdx.x == 0) *count_out = carry;
 }
 
-// Pass 3, and the eq table's part of the same round of the boolean check (general.cu) in one launch, since neither needs the
-// other: the first eq_blocks blocks bind the table's lowest variable on the round's challenge and write the next round's records
-// (see k_sbool_msg) in the same pass (the folded table would only be read again for them), the others fold the entries' pairs, each
-// written at its compacted slot.  Both are bound by memory in the first rounds (16 x 2^17 entries: 124 us for what took 73 and 43 as
-// launches of their own) and by the launch in the last.
+// Pass 3: each pair folded and written at its compacted slot.
 __global__ void __launch_bounds__(kSpThreads) k_bool_fold(const uint32_t* __restrict__ idx, const Fr* __restrict__ val,
                                                           const uint32_t* __restrict__ count, const uint32_t* __restrict__ block_offsets,
-                                                          const FixedMul<FrParams> r, uint32_t* idx_out, Fr* val_out, const Fr* __restrict__ eq,
-                                                          uint64_t eq_pairs, Fr* __restrict__ eq_out, Fr* __restrict__ rec, uint32_t eq_blocks) {
-  if (blockIdx.x < eq_blocks) {
-    if (eq_pairs == 0) {  // the last variable: no round after it, no records
-      if (blockIdx.x == 0 && threadIdx.x == 0) {
-        const Fr a = ld_fr(eq);
-        st_fr(eq_out, add(a, mul_fixed(r, sub(ld_fr(eq + 1), a))));
-      }
-      return;
-    }
-    for (uint64_t j = blockIdx.x * (uint64_t)kSpThreads + threadIdx.x; j < eq_pairs; j += (uint64_t)eq_blocks * kSpThreads) {
-      const Fr a0 = ld_fr(eq + 4 * j), a1 = ld_fr(eq + 4 * j + 1), b0 = ld_fr(eq + 4 * j + 2), b1 = ld_fr(eq + 4 * j + 3);
-      const Fr e0 = add(a0, mul_fixed(r, sub(a1, a0))), e1 = add(b0, mul_fixed(r, sub(b1, b0)));
-      st_fr(eq_out + 2 * j, e0);
-      st_fr(eq_out + 2 * j + 1, e1);
-      const Fr de = sub(e1, e0);
-      const Fr e2 = add(e1, de), e3 = add(e2, de);
-      Fr* out = rec + 6 * j;
-      st_fr(out, e0);
-      st_fr(out + 1, e2);
-      st_fr(out + 2, add(e3, e3));
-      st_fr(out + 3, e1);
-      st_fr(out + 4, add(e2, e2));
-      st_fr(out + 5, add(add(e3, e3), e3));
-    }
-    return;
-  }
+                                                          const FixedMul<FrParams> r, uint32_t* idx_out, Fr* val_out) {
   __shared__ uint32_t warp_cnt[kSpThreads / 32];
-  const uint32_t block = blockIdx.x - eq_blocks;
   const uint32_t n = *count;
-  const uint32_t i = block * kSpThreads + threadIdx.x;
+  const uint32_t i = blockIdx.x * kSpThreads + threadIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t pos = 0;
   bool lead = false;
@@ -270,7 +239,7 @@ __global__ void __launch_bounds__(kSpThreads) k_bool_fold(const uint32_t* __rest
   if (lane == 0) warp_cnt[warp] = __popc(ballot);
   __syncthreads();
   if (!lead) return;
-  uint32_t slot = block_offsets[block] + __popc(ballot & ((1u << lane) - 1u));
+  uint32_t slot = block_offsets[blockIdx.x] + __popc(ballot & ((1u << lane) - 1u));
   for (int w = 0; w < warp; w++) slot += warp_cnt[w];
   Fr v0 = Fr::zero(), v1 = Fr::zero();
   if ((pos & 1u) == 0) {
@@ -422,11 +391,9 @@ int launch_sparse_slots(const uint32_t* idx, const uint32_t* count, uint32_t upp
 }
 
 void launch_bool_fold(const uint32_t* idx, const Fr* val, const uint32_t* count, uint32_t upper, const Fr& r, const uint32_t* block_offsets,
-                      uint32_t* idx_out, Fr* val_out, const Fr* eq, uint64_t eq_size, Fr* eq_out, Fr* rec, int sm_count, cudaStream_t s) {
+                      uint32_t* idx_out, Fr* val_out, cudaStream_t s) {
   const uint32_t blocks = upper ? (upper + kSpThreads - 1) / kSpThreads : 1;
-  const uint32_t eq_blocks = (uint32_t)blocks_for(eq_size / 4, kSpThreads, sm_count * 4);
-  k_bool_fold<<<eq_blocks + blocks, kSpThreads, 0, s>>>(idx, val, count, block_offsets, make_fixed_mul(r), idx_out, val_out, eq, eq_size / 4, eq_out,
-                                                       rec, eq_blocks);
+  k_bool_fold<<<blocks, kSpThreads, 0, s>>>(idx, val, count, block_offsets, make_fixed_mul(r), idx_out, val_out);
 }
 
 void launch_scatter(const uint32_t* idx, const Fr* val, const uint32_t* count, uint32_t upper, Fr* dense,
