@@ -215,38 +215,29 @@ __global__ void k_msm_digits(const Fr* __restrict__ scalars, const int32_t* __re
   }
 }
 
-// Same two passes for a small key space (at most kSmallKeys buckets): keys are counted in
+// Same two passes for a small key space (at most kSmallKeys buckets in total): keys are counted in
 // shared memory first, so the global counters see one atomic per (block, bucket) instead of
 // one per digit.  In scatter mode the block reserves a contiguous range per bucket.
-// row_blocks == 0: all buckets of the call are at most kSmallKeys.  Otherwise those of one row are, and row_blocks blocks take a row.
 constexpr uint32_t kSmallKeys = 4096;
 
 template <int MODE, int FORM>
 __global__ void __launch_bounds__(256) k_msm_digits_small(const Fr* __restrict__ scalars, const int32_t* __restrict__ compact,
                                                           const uint32_t* __restrict__ row_ids,
                                                           uint64_t n, uint32_t rows, int w, int k_windows, uint32_t table_step,
-                                                          uint32_t n_keys, uint64_t per_block, uint32_t row_blocks, uint32_t* counts_or_cursor,
-                                                          uint32_t* entries) {
+                                                          uint32_t n_keys, uint64_t per_block, uint32_t* counts_or_cursor, uint32_t* entries) {
   __shared__ uint32_t hist[kSmallKeys];
   __shared__ uint32_t basepos[kSmallKeys];
   const uint64_t total = row_ids ? n : n * rows;
-  uint64_t begin = (uint64_t)blockIdx.x * per_block, end = begin + per_block < total ? begin + per_block : total;
-  uint32_t row0 = 0;
-  if (row_blocks) {
-    row0 = blockIdx.x / row_blocks;
-    begin = row0 * n + (blockIdx.x - row0 * row_blocks) * per_block;
-    end = begin + per_block < (row0 + 1) * n ? begin + per_block : (row0 + 1) * n;
-    counts_or_cursor += (uint64_t)row0 * n_keys;
-  }
+  const uint64_t begin = (uint64_t)blockIdx.x * per_block;
+  const uint64_t end = begin + per_block < total ? begin + per_block : total;
   for (uint32_t k = threadIdx.x; k < n_keys; k += blockDim.x) hist[k] = 0;
   __syncthreads();
   for (int pass = 0; pass < (MODE == 0 ? 1 : 2); pass++) {
     for (uint64_t g = begin + threadIdx.x; g < end; g += blockDim.x) {
-      const uint32_t row = row_blocks ? row0 : row_ids ? row_ids[g] : (uint32_t)(g / n);
+      const uint32_t row = row_ids ? row_ids[g] : (uint32_t)(g / n);
       const uint32_t col = row_ids ? (uint32_t)g : (uint32_t)(g - (uint64_t)row * n);
       scalar_digits<FORM>(scalars, compact, g, w, k_windows, [&](uint32_t k, uint32_t digit, uint32_t flags) {
-        const uint32_t item = table_step ? row - row0 : (row - row0) * (uint32_t)k_windows + k;
-        const uint32_t key = (item << (w - 1)) + digit;
+        const uint32_t key = ((table_step ? row : row * (uint32_t)k_windows + k) << (w - 1)) + digit;
         if (pass == 0) {
           atomicAdd(hist + key, 1u);
         } else {
@@ -288,7 +279,8 @@ __device__ __forceinline__ void st_fq(Fq* p, const Fq& x) {
 // Horner chain.  The chain of w (windows - 1) doublings is here instead, once per base; four lanes take a point (quad.cuh).
 // A latency chain (226 us for a hundred points, 555 for 2^14), beside the passes over the digits.  A KZH3 commitment and opening of
 // 2^22 values, half of them full width: accumulation 15 957 -> 13 315 us, bucket reduction 2 685 -> 1 327, Horner chains 1 120 -> 0, for
-// 935 us of multiples; 24 286 -> 19 126 us in all together with the split and with digits counted a row at a time.
+// 935 us of multiples; 24 286 -> 19 108 us in all together with the split.  (Counting the buckets of a row in shared
+// memory instead of by global atomics made no difference.)
 __global__ void __launch_bounds__(128) k_multiples(const Affine* __restrict__ bases, uint64_t n, int w, int k_windows, Xyzz* out) {
   const uint64_t i = (uint64_t)blockIdx.x * 32 + (threadIdx.x >> 2);
   const int role = threadIdx.x & 3;
@@ -1183,12 +1175,12 @@ static int rows_run(zk_ctx* ctx, const Affine* bases, const int32_t* compact, ui
 }
 
 template <int MODE>
-static void launch_digits(ScalarForm form, uint32_t small_keys, uint32_t dig_blocks, uint64_t per_block, uint32_t row_blocks, int sm, const Fr* scalars, const int32_t* compact,
+static void launch_digits(ScalarForm form, uint32_t small_keys, uint32_t dig_blocks, uint64_t per_block, int sm, const Fr* scalars, const int32_t* compact,
                           const uint32_t* row_ids, uint64_t n, uint32_t rows, int w, int k_windows, uint32_t table_step,
                           uint32_t* counts_or_cursor, uint32_t* entries, cudaStream_t s) {
   auto launch = [&](auto small, auto large) {
     if (small_keys)
-      small<<<dig_blocks, 256, 0, s>>>(scalars, compact, row_ids, n, rows, w, k_windows, table_step, small_keys, per_block, row_blocks, counts_or_cursor, entries);
+      small<<<dig_blocks, 256, 0, s>>>(scalars, compact, row_ids, n, rows, w, k_windows, table_step, small_keys, per_block, counts_or_cursor, entries);
     else
       large<<<sm * 8, 256, 0, s>>>(scalars, compact, row_ids, n, rows, w, k_windows, table_step, counts_or_cursor, entries);
   };
@@ -1323,18 +1315,9 @@ static int msm_run_impl(zk_ctx* ctx, const Affine* bases, const uint32_t* gather
   // 4096 digits a block, not scalars: 1000 full-width scalars of 37 digits each were one block's work (638 us, 561 us with ten)
   uint32_t dig_blocks = (uint32_t)std::min<uint64_t>((total * digits + 4095) / 4096, 1u << 20);
   if (dig_blocks > (uint32_t)sm * 8) dig_blocks = sm * 8;
-  uint64_t per_block = (total + dig_blocks - 1) / dig_blocks;
-  // buckets that a block counts in shared memory: all of them, or those of a row (0: by global atomics).  A row's share of the blocks
-  // gets some 16384 digits each, four a bucket.
-  uint32_t small_keys = n_buckets <= kSmallKeys ? n_buckets : 0, row_blocks = 0;
-  if (!small_keys && !row_ids && n_buckets / rows <= kSmallKeys && n * digits >= 4ull * (n_buckets / rows)) {
-    small_keys = n_buckets / rows;
-    const uint64_t share = std::max<uint64_t>(1, std::min<uint64_t>(n * digits / (4ull * small_keys), ((uint64_t)sm * 16 + rows - 1) / rows));
-    row_blocks = (uint32_t)share;
-    per_block = (n + share - 1) / share;
-    dig_blocks = rows * row_blocks;
-  }
-  launch_digits<0>(form, small_keys, dig_blocks, per_block, row_blocks, sm, scalars, compact, row_ids, n, rows, w, digit_windows, table_step, offsets, nullptr, s);
+  const uint64_t per_block = (total + dig_blocks - 1) / dig_blocks;
+  const uint32_t small_keys = n_buckets <= kSmallKeys ? n_buckets : 0;  // counted in shared memory
+  launch_digits<0>(form, small_keys, dig_blocks, per_block, sm, scalars, compact, row_ids, n, rows, w, digit_windows, table_step, offsets, nullptr, s);
   ctx->launches++;
   BucketCounts* d_counts = reinterpret_cast<BucketCounts*>(ctx->rs.sink.counter + 10);
   ZK_CUDA(cudaMemsetAsync(d_counts, 0, sizeof(BucketCounts), s));
@@ -1351,7 +1334,7 @@ static int msm_run_impl(zk_ctx* ctx, const Affine* bases, const uint32_t* gather
   const uint32_t n_entries = (uint32_t)counts.total;
   ctx->launches += exclusive_scan_u32(offsets, n_buckets, scan_tmp, true, s);
   ZK_CUDA(cudaMemcpyAsync(cursor, offsets, (n_buckets + 1) * 4ull, cudaMemcpyDeviceToDevice, s));
-  launch_digits<1>(form, small_keys, dig_blocks, per_block, row_blocks, sm, scalars, compact, row_ids, n, rows, w, digit_windows, table_step, cursor, entries, s);
+  launch_digits<1>(form, small_keys, dig_blocks, per_block, sm, scalars, compact, row_ids, n, rows, w, digit_windows, table_step, cursor, entries, s);
   ctx->launches++;
 
   // ---- accumulate
