@@ -53,11 +53,11 @@ def test_from_right_random(ctx, n, k):
         assert o.evaluate_multilinear_extension(got, lowpt) == o.evaluate_multilinear_extension(f, lowpt + pt)
 
 
-@pytest.mark.parametrize("lo,hi", [(0, 4), (0, 5), (0, 11), (1, 5), (3, 6), (4, 5), (5, 8), (5, 9), (2, 10), (6, 4)])
+@pytest.mark.parametrize("lo,hi", [(0, 4), (0, 8), (0, 9), (0, 11), (1, 9), (3, 8), (4, 9), (5, 8), (5, 9), (2, 10), (6, 4)])
 @pytest.mark.parametrize("kind", ["largest", "random"])
 def test_weighted_fold_edges(ctx, lo, hi, kind):
-    """2^hi rows of 2^lo columns around the sizes where the byte products begin (32 rows), a block's columns (16) and the rows that
-    its weights are held for (256) end, with the largest bytes that an element can have (p - 1 in memory) and random ones."""
+    """2^hi rows of 2^lo columns around the sizes where the byte products begin (512 rows) and a block's columns (16) end, its weights being
+    held for 256 rows at a time, with the largest bytes that an element can have (p - 1 in memory) and random ones."""
     rnd = random.Random(100 * lo + hi)
     largest = (M - 1) * pow(1 << 256, -1, M) % M
     f = [largest if kind == "largest" else rnd.randrange(M) for _ in range(1 << (lo + hi))]
