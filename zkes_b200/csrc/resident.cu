@@ -450,6 +450,48 @@ __device__ __forceinline__ void ahead_rounds(const ResidentParams<L>& p, WarpStr
   if (p.done) publish(p.done + 1, p.seq, lane);
 }
 
+__device__ __forceinline__ Fr times(const Fr& x, int k) {  // small k, known when compiling
+  Fr sum = x;
+#pragma unroll
+  for (int bit = 16; bit > 0; bit >>= 1) {
+    if (k < 2 * bit && k >= bit) sum = x;  // the top bit
+    if (k >= 2 * bit) {
+      sum = add(sum, sum);
+      if (k & bit) sum = add(sum, x);
+    }
+  }
+  return sum;
+}
+
+// s(lane), lane = 0..L, from the values that a pass sums (round_pass_async); claim: s(0) + s(1), of no use in the first round.
+template <int L>
+__device__ __forceinline__ Fr round_value(const Fr* v, bool first, const Fr& claim, int lane) {
+  const Fr lead = v[first ? L : L - 1];
+  if constexpr (L == 1) {
+    const Fr s1 = first ? add(v[0], lead) : sub(claim, v[0]);
+    return lane == 0 ? v[0] : s1;
+  } else {
+    const Fr s1 = first ? v[1] : sub(claim, v[0]);
+    const auto at = [&](int k) { return k == 0 ? v[0] : k == 1 ? s1 : v[first ? k : k - 1]; };
+    constexpr int kFactorial = L == 2 ? 2 : L == 3 ? 6 : 24;
+    Fr top = times(lead, kFactorial);  // the L-th difference: sum_k (-1)^(L-k) C(L, k) s(k)
+    int choose = 1;
+#pragma unroll
+    for (int k = 0; k < L; k++) {
+      const Fr term = times(at(k), choose);
+      top = ((L - k) & 1) ? add(top, term) : sub(top, term);
+      choose = choose * (L - k) / (k + 1);
+    }
+    Fr out = top;
+#pragma unroll
+    for (int k = 0; k < L; k++) {
+      const Fr x = at(k);
+      if (lane == k) out = x;
+    }
+    return out;
+  }
+}
+
 template <int L>
 __global__ void __launch_bounds__(kThreads, (L <= 1 ? 3 : 2)) k_resident(const ResidentParams<L> p) {
   extern __shared__ uint4 resident_stage[];  // per warp: 2 stages x L tables of WarpTile<8>::kChunks slots
@@ -457,6 +499,8 @@ __global__ void __launch_bounds__(kThreads, (L <= 1 ? 3 : 2)) k_resident(const R
   __shared__ FixedMul<FrParams> r_tab;
   __shared__ Fr red[kWarps][L + 1];
   __shared__ Fr msg[L + 1];
+  __shared__ Fr said[L + 2];  // block 0: the message of the round before and its challenge
+  __shared__ Fr claim;        // its value there
   __shared__ __align__(16) uint8_t stream[WarpStrobe::round_stream_bytes<L>() + 15];
   __shared__ unsigned long long macc_sm[L + 1][8];
   __shared__ int flag, ok_flag, px_ok;
@@ -507,6 +551,33 @@ __global__ void __launch_bounds__(kThreads, (L <= 1 ? 3 : 2)) k_resident(const R
       for (int i = 0; i < L; i++) cur[i] = dst[i];
       cur_size >>= 1;
     }
+    const int n_sums = round == 0 ? round_values<L, false>() : round_values<L, true>();
+    if (round != 0 && blockIdx.x == 0 && warp == 1) {  // while the other blocks are at their tiles
+      const int j = lane % NV;
+      const Fr at = said[NV];
+      Fr x;
+#pragma unroll
+      for (int m = 0; m < L; m++) {  // the nodes other than j
+        Fr kk = Fr::zero();
+        kk.v[0] = (uint32_t)(m < j ? m : m + 1);
+        const Fr term = sub(at, kk);
+        x = m == 0 ? term : mul_call(x, term);
+      }
+      Fr kc = p.kconst[0];
+#pragma unroll
+      for (int k = 1; k < NV; k++)
+        if (j == k) kc = p.kconst[k];
+      x = mul_call(mul_call(x, said[j]), kc);  // L + 1 Montgomery products of integers
+      Fr sum = x;
+#pragma unroll
+      for (int k = 1; k < NV; k++) {
+        Fr y;
+#pragma unroll
+        for (int i = 0; i < 8; i++) y.v[i] = __shfl_sync(0xffffffffu, x.v[i], k);
+        sum = add(sum, y);
+      }
+      if (lane == 0) claim = sum;
+    }
     // Block total -> global: the warps' sums are added as plain 64-bit sums of their 32-bit limbs, and the blocks add
     // those to the round's accumulators by atomics, so nobody has to read a partial sum per block afterwards.
     const uint64_t tiles = ((cur_size >> 1) + 31) >> 5;  // cur_size: entries of the table the message is over
@@ -514,11 +585,12 @@ __global__ void __launch_bounds__(kThreads, (L <= 1 ? 3 : 2)) k_resident(const R
     if (blockIdx.x < tiles) {  // the others had no tile this round
 #pragma unroll
       for (int c = 0; c < NV; c++) {
+        if (c >= n_sums) break;
         const Fr t = warp_sum(s[c]);
         if (lane == 0) red[warp][c] = t;
       }
       __syncthreads();
-      if (threadIdx.x < NV * 8) {
+      if (threadIdx.x < n_sums * 8) {
         const int c = threadIdx.x >> 3, limb = threadIdx.x & 7;
         unsigned long long v = 0;
 #pragma unroll
@@ -542,12 +614,12 @@ __global__ void __launch_bounds__(kThreads, (L <= 1 ? 3 : 2)) k_resident(const R
       if (!ok_flag) return;
     }
     if (blockIdx.x == 0) {
-      if (threadIdx.x < NV * 8) {  // read, and cleared for the round after the next
+      if (threadIdx.x < n_sums * 8) {  // read, and cleared for the round after the next
         const int c = threadIdx.x >> 3, limb = threadIdx.x & 7;
         macc_sm[c][limb] = atomicExch(&p.sh->macc[mpar][c][limb], 0ull);
       }
       __syncthreads();
-      if (threadIdx.x < NV) {
+      if (threadIdx.x < n_sums) {
         Wide x;
 #pragma unroll
         for (int k = 0; k < 16; k++) x.v[k] = 0;
@@ -569,14 +641,15 @@ __global__ void __launch_bounds__(kThreads, (L <= 1 ? 3 : 2)) k_resident(const R
         // for the other ranks' shares in this rank's own box and add them in rank order, so every rank
         // absorbs the same message and derives the same challenge.
         const unsigned int xseq = p.px.xseq_base + round + 1;
-        if (!peer_exchange_sum(p.px, xseq, msg, NV, px_stage, &px_ok, threadIdx.x, kThreads)) {
+        if (!peer_exchange_sum(p.px, xseq, msg, n_sums, px_stage, &px_ok, threadIdx.x, kThreads)) {
           if (threadIdx.x == 0) atomicExch(&p.sh->error, 2u);  // a rank is missing: stops every block of this launch
           return;
         }
       }
       if (warp == 0) {
         if (lane <= L) {
-          const Fr canon = msg[lane];
+          const Fr canon = round_value<L>(msg, round == 0, claim, lane);
+          said[lane] = canon;
           p.out_msgs[(size_t)round * NV + lane] = canon;
           uint8_t* dst = WarpStrobe::round_stream_data(stream, lane);
 #pragma unroll
@@ -589,7 +662,10 @@ __global__ void __launch_bounds__(kThreads, (L <= 1 ? 3 : 2)) k_resident(const R
         ws.fs_round<L>(stream, lane, raw.v);
         const Fr r = reduce_256(raw);
         if (lane < 3) st_tagged_part(&p.sh->rplain[round & 1], r, round + 1, lane);  // the hand-over to every block
-        if (lane == 0) p.out_chal[round] = r;
+        if (lane == 0) {
+          p.out_chal[round] = r;
+          said[NV] = r;
+        }
         if (round + 1 == p.rounds) {  // for the kernel that goes on: challenge in Montgomery form, transcript state
           if (lane < 25) p.sh->st.lanes[lane] = ws.a;
           if (lane == 0) {
@@ -666,6 +742,25 @@ int launch_resident_t(const Fr* const* src, Fr* const* ping, Fr* const* pong, ui
   const uint64_t cap = (uint64_t)sm_count * occ < (uint64_t)max_blocks ? (uint64_t)sm_count * occ : (uint64_t)max_blocks;
   if (grid > cap) grid = cap;
   if (grid < 1) grid = 1;
+  // host field inversions are slow (hundreds of products each): once per process and L
+  struct Consts {
+    Fr k[L + 1];
+    Consts() {
+      for (int j = 0; j <= L; j++) {
+        Fr den = Fr::one();
+        for (int i = 0; i <= L; i++) {
+          if (i == j) continue;
+          const Fr d = j > i ? from_u32<FrParams>((uint32_t)(j - i)) : neg(from_u32<FrParams>((uint32_t)(i - j)));
+          den = mul(den, d);
+        }
+        Fr c = inverse(den);                          // R / den
+        for (int i = 0; i < L; i++) c = to_mont(c);   // R^(L+1) / den
+        k[j] = c;
+      }
+    }
+  };
+  static const Consts consts;
+  for (int j = 0; j <= L; j++) p.kconst[j] = consts.k[j];
   p.ahead_from = rounds;
   p.pending = 0;
   p.out_final = nullptr;
@@ -698,25 +793,6 @@ int launch_resident_t(const Fr* const* src, Fr* const* ping, Fr* const* pong, ui
       p.done = to_end->done;
       p.seq = to_end->seq;
     }
-    // host field inversions are slow (hundreds of products each): once per process and L
-    struct Consts {
-      Fr k[L + 1];
-      Consts() {
-        for (int j = 0; j <= L; j++) {
-          Fr den = Fr::one();
-          for (int i = 0; i <= L; i++) {
-            if (i == j) continue;
-            const Fr d = j > i ? from_u32<FrParams>((uint32_t)(j - i)) : neg(from_u32<FrParams>((uint32_t)(i - j)));
-            den = mul(den, d);
-          }
-          Fr c = inverse(den);                          // R / den
-          for (int i = 0; i < L; i++) c = to_mont(c);   // R^(L+1) / den
-          k[j] = c;
-        }
-      }
-    };
-    static const Consts consts;
-    for (int j = 0; j <= L; j++) p.kconst[j] = consts.k[j];
     *to_end->ahead_from = t;
   }
   void* args[] = {&p};

@@ -105,18 +105,40 @@ __device__ __forceinline__ void round_pass(const SrcPtr& src, const DstPtr& dst,
 // registers a block has few warps to hide that latency otherwise).  stage: this warp's 2 * L tiles of
 // WarpTile<8>::kChunks slots; a tile's own slots double as the staging of its folded output.  cp.async.cg reads
 // through L2, so tables written earlier in the same launch by other blocks are seen.
+//
+// What is summed is not the message itself: s(1) follows from s(0) and from what the round before says about s(0) + s(1), once there is
+// a round before (FOLD), and s(L) from the leading coefficient, the sum of the products of the differences, which costs no addition to
+// get at.  s[]: s(0), s(1) (without FOLD), s(2) .. s(L - 1), then for L >= 2 or without FOLD the leading coefficient: round_values().
+// Two tables of 2^20: 306 us for the prove, 310 with all L + 1 values summed.
+template <int L, bool FOLD>
+constexpr int round_values() { return FOLD ? L : L + 1; }
 template <int L, bool FOLD, class SrcPtr, class DstPtr>
 __device__ __forceinline__ void round_pass_async(const SrcPtr& src, const DstPtr& dst, const FixedMul<FrParams>& r,
                                                  uint64_t pairs, uint64_t warp_global, uint64_t warp_stride, uint4* stage,
                                                  int lane, Fr (&s)[L + 1]) {
+  constexpr int NE = round_values<L, FOLD>();
+  constexpr int kLast = !FOLD || L >= 3 ? L - 1 : 0;  // the last point that is summed
   constexpr int CH = FOLD ? 8 : 4;
   constexpr int kSlots = WarpTile<8>::kChunks;  // per table and stage, for either variant
   const uint64_t tiles = (pairs + 31) >> 5;
-  Wide acc[L + 1];
+  Wide acc[NE];
 #pragma unroll
-  for (int c = 0; c <= L; c++)
+  for (int c = 0; c < NE; c++)
 #pragma unroll
     for (int k = 0; k < 16; k++) acc[c].v[k] = 0;
+  auto product_to = [&](Wide& sum, const Fr (&x)[L]) {
+    Wide w;
+    if (L == 1) {
+      const Fr one = Fr::one();
+      mul_wide(w, x[0].v, one.v);
+    } else {
+      Fr prod = x[0];
+#pragma unroll
+      for (int i = 1; i < L - 1; i++) prod = mul(prod, x[i]);
+      mul_wide(w, prod.v, x[L - 1].v);
+    }
+    wide_add(sum, w);
+  };
   int pending = 0;
   auto valid_of = [&](uint64_t tile) { return (uint32_t)((pairs - (tile << 5)) < 32 ? (pairs - (tile << 5)) : 32); };
   auto prefetch = [&](uint64_t tile, int buf) {
@@ -163,31 +185,22 @@ __device__ __forceinline__ void round_pass_async(const SrcPtr& src, const DstPtr
     }
     // lanes past the end of the table hold zeros and add nothing
 #pragma unroll
-    for (int c = 0; c <= L; c++) {
-      Wide w;
-      if (L == 1) {
-        const Fr one = Fr::one();
-        mul_wide(w, u0[0].v, one.v);
-      } else {
-        Fr prod = u0[0];
-#pragma unroll
-        for (int i = 1; i < L - 1; i++) prod = mul(prod, u0[i]);
-        mul_wide(w, prod.v, u0[L - 1].v);
-      }
-      wide_add(acc[c], w);
-      if (c < L) {
+    for (int c = 0; c <= kLast; c++) {
+      if (!(FOLD && c == 1)) product_to(acc[FOLD && c >= 2 ? c - 1 : c], u0);
+      if (c < kLast) {
 #pragma unroll
         for (int i = 0; i < L; i++) u0[i] = add(u0[i], d[i]);
       }
     }
+    if constexpr (!(FOLD && L == 1)) product_to(acc[NE - 1], d);
     if (++pending == kLazyProducts) {
 #pragma unroll
-      for (int c = 0; c <= L; c++) wide_trim<FrParams>(acc[c]);
+      for (int c = 0; c < NE; c++) wide_trim<FrParams>(acc[c]);
       pending = 0;
     }
   }
 #pragma unroll
-  for (int c = 0; c <= L; c++) {
+  for (int c = 0; c < NE; c++) {
     wide_trim<FrParams>(acc[c]);
     s[c] = redc<FrParams>(acc[c]);
   }
