@@ -103,26 +103,13 @@ int exchange_counts(zk_ctx* ctx, zk_comm* comm, uint32_t mine, uint32_t* out) {
   return ZK_OK;
 }
 
-// The boolean check's message (k_sbool_msg): scale[c] t(c), c = 0..3, from t(0), t(1) and the leading coefficient of t.
-static void bool_message(const Fr* t, const Fr* scale, Fr* out) {
-  const Fr slope = sub(t[1], t[0]), lead2 = add(t[2], t[2]);
-  Fr at = t[1], step = add(slope, lead2);  // t(c + 1) - t(c) = slope + 2 c lead
-  out[0] = mul(scale[0], t[0]);
-  out[1] = mul(scale[1], t[1]);
-  for (int c = 2; c < 4; c++) {
-    at = add(at, step);
-    step = add(step, lead2);
-    out[c] = mul(scale[c], at);
-  }
-}
-
 // Reads the round message the last kernel left in rs.msg, records it, runs the Fiat-Shamir
 // step (callback or built-in transcript) and records the challenge.
 int fs_round(zk_ctx* ctx, zk_comm* comm, int n_msgs, uint32_t round, zk_fs_round_fn fs, void* fs_user, zk_transcript* tr,
-             uint64_t* round_msgs, uint64_t* challenges, Fr* challenge, bool exchanged_by_kernel, const Fr* bool_scale) {
+             uint64_t* round_msgs, uint64_t* challenges, Fr* challenge, bool exchanged_by_kernel, const RoundSums* sums) {
   ZK_CUDA(cudaGetLastError());
   if (comm && !exchanged_by_kernel) {  // every rank holds a partial message: sum them so all ranks absorb the same scalars
-    int rc = comm_sum_fr(ctx, comm, ctx->rs.sink.msg, bool_scale ? 3 : n_msgs);
+    int rc = comm_sum_fr(ctx, comm, ctx->rs.sink.msg, sums ? sums->n_sums : n_msgs);
     if (rc) return rc;
   }
   {
@@ -130,9 +117,9 @@ int fs_round(zk_ctx* ctx, zk_comm* comm, int n_msgs, uint32_t round, zk_fs_round
     if (rc) return rc;
   }
   const Fr* msg = reinterpret_cast<const Fr*>(ctx->mailbox);
-  Fr made[4];
-  if (bool_scale) {
-    bool_message(msg, bool_scale, made);
+  Fr made[kMaxPolys + 2];
+  if (sums) {
+    sums->make(sums->user, msg, made);
     msg = made;
   }
   uint64_t* out_msg = round_msgs + (uint64_t)round * n_msgs * 4;

@@ -21,6 +21,20 @@ inline size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
 
 namespace {
 
+// The boolean check's message (k_sbool_msg): scale[c] t(c), c = 0..3, from t(0), t(1) and the leading coefficient of t.
+void bool_message(void* user, const Fr* t, Fr* out) {
+  const Fr* scale = static_cast<const Fr*>(user);
+  const Fr slope = sub(t[1], t[0]), lead2 = add(t[2], t[2]);
+  Fr at = t[1], step = add(slope, lead2);  // t(c + 1) - t(c) = slope + 2 c lead
+  out[0] = mul(scale[0], t[0]);
+  out[1] = mul(scale[1], t[1]);
+  for (int c = 2; c < 4; c++) {
+    at = add(at, step);
+    step = add(step, lead2);
+    out[c] = mul(scale[c], at);
+  }
+}
+
 // The boolean-check prover; with a communicator the terms given are this rank's share of them (the sum over
 // terms is the only thing the ranks have in common: the partial messages and the partial final value are summed
 // across the ranks, everything else is local).
@@ -135,7 +149,8 @@ int sbool_prove(zk_ctx* ctx, zk_comm* comm, uint32_t num_var, uint32_t n_terms, 
       ctx->launches += launch_sparse_slots(e_key[e], counts + e, k_upper, block_counts, counts + (e ^ 1), s);
     };
     if (!comm) slots();
-    rc = fs_round(ctx, comm, 4, round, fs, fs_user, tr, round_msgs, challenges, &challenge, false, scale);
+    const RoundSums sums = {3, bool_message, scale};
+    rc = fs_round(ctx, comm, 4, round, fs, fs_user, tr, round_msgs, challenges, &challenge, false, &sums);
     if (rc) return rc;
     if (comm) slots();  // (there the exchange kernel is next on the stream)
     launch_bool_fold(e_key[e], e_val[e], counts + e, k_upper, challenge, block_counts, e_key[e ^ 1], e_val[e ^ 1], s);

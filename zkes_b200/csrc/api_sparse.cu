@@ -18,6 +18,27 @@ struct Arena {
     return p;
   }
 };
+
+// A quadratic round message from s(0) and the leading coefficient; s(1) is summed in the first round and afterwards what the round
+// before leaves for it.
+struct QuadForm {
+  bool first = true;
+  Fr claim = Fr::zero(), s0 = Fr::zero(), s1 = Fr::zero(), lead = Fr::zero();
+  void bind(const Fr& r) {
+    claim = add(s0, mul(r, add(sub(sub(s1, s0), lead), mul(r, lead))));
+    first = false;
+  }
+};
+void quad_message(void* user, const Fr* sums, Fr* msg) {
+  QuadForm& f = *static_cast<QuadForm*>(user);
+  f.s0 = sums[0];
+  f.s1 = f.first ? sums[1] : sub(f.claim, sums[0]);
+  f.lead = sums[f.first ? 2 : 1];
+  const Fr half = add(f.s1, f.lead);
+  msg[0] = f.s0;
+  msg[1] = f.s1;
+  msg[2] = sub(add(half, half), f.s0);
+}
 }  // namespace
 
 static int sparse_dense_impl(zk_ctx* ctx, zk_comm* comm, uint32_t total_var, uint64_t nnz, const uint64_t* idx,
@@ -120,6 +141,7 @@ static int sparse_dense_impl(zk_ctx* ctx, zk_comm* comm, uint32_t total_var, uin
   Fr e_r = Fr::zero();
   uint32_t k_upper = K;  // bound on the live entry count
   Fr challenge = Fr::zero();
+  QuadForm form;
   uint64_t S = size;
   bool finished = false;  // the dense phase ran to the end (final values are in ctx->final_out)
   bool dense_done = false;  // ... inside the device-resident rounds, which read the final values back with the rounds
@@ -168,8 +190,10 @@ static int sparse_dense_impl(zk_ctx* ctx, zk_comm* comm, uint32_t total_var, uin
     ctx->prof_end();
     ctx->launches++;
     if (fused) comm_peer_advance(comm, 1);
-    rc = fs_round(ctx, comm, 3, round, fs, fs_user, tr, round_msgs, challenges, &challenge, fused);
+    const RoundSums sums = {form.first ? 3 : 2, quad_message, &form};
+    rc = fs_round(ctx, comm, 3, round, fs, fs_user, tr, round_msgs, challenges, &challenge, fused, &sums);
     if (rc != ZK_OK) return rc;
+    form.bind(challenge);
     rc = check_bad(false);  // the message kernel ran after the copy of the flag
     if (rc != ZK_OK) return rc;
     // Fold of the dense table.  When the next round is still in entry form its message can fold

@@ -167,9 +167,15 @@ int wait_result(zk_ctx* ctx);  // until the last next_msg_scratch(false) launch 
 void comm_peer_advance(zk_comm* c, unsigned int n);
 int comm_peer_gather(zk_ctx* ctx, zk_comm* c, int n_tables, const Fr* const* chunks, uint32_t m, unsigned int* error_word,
                      const Fr** tables_out);
+// What a round's kernel sums where that is not the message itself: n_sums values, of which make() makes the n_msgs values.
+struct RoundSums {
+  int n_sums;
+  void (*make)(void* user, const Fr* sums, Fr* msg);
+  void* user;
+};
 int fs_round(zk_ctx* ctx, zk_comm* comm, int n_msgs, uint32_t round, fs_round_fn_t fs, void* fs_user, zk_transcript* tr,
              uint64_t* round_msgs, uint64_t* challenges, Fr* challenge,
-             bool exchanged_by_kernel = false, const Fr* bool_scale = nullptr);
+             bool exchanged_by_kernel = false, const RoundSums* sums = nullptr);
 int linear_rounds(zk_ctx* ctx, zk_comm* comm, int L, uint32_t rounds, const Fr** cur, Fr** ping, Fr** pong,
                   uint32_t round_offset, fs_round_fn_t fs, void* fs_user, zk_transcript* tr, uint64_t* round_msgs,
                   uint64_t* challenges, Fr* challenge, bool* finals_done);
