@@ -8,6 +8,7 @@ import pytest
 
 import pyoracle as o
 from zkes_b200 import DenseMLPoly, kzh
+from zkes_b200._lib import check, lib
 
 pytestmark = pytest.mark.gpu
 M = o.R_MOD
@@ -60,6 +61,27 @@ def test_kzh2_small_poly_and_short_point(ctx):
     pt = [rnd.randrange(M) for _ in range(4)]
     _, f_star = kzh.kzh2_open(ctx, srs, pt, com, poly)
     assert f_star == o.kzh2_open(osrs, pt, odx, f)[1]
+
+
+@pytest.mark.parametrize("span", [1, 127, 32000])
+@pytest.mark.parametrize("n", [2, 8, 11, 16])
+def test_commitment_rows_beside_and_after_c(ctx, n, span):
+    """Small values: the rows' sums run beside C on the side stream; with the profiler on they follow it.  In turn, each on scratch that
+    the other order has left."""
+    rnd = random.Random(n + span)
+    xl, yl = o.kzh2_degrees(n)
+    gk, tx, ty, rest = trapdoors(4, 1 << xl, 1 << yl)
+    srs = kzh.KZHSRS.setup(ctx, 2, n, o.G1_GEN, tx, ty, alpha=rest[0])
+    poly = DenseMLPoly.from_evaluations([o.fr_from_int(rnd.randrange(-span, span + 1)) for _ in range(1 << n)])
+    got = []
+    try:
+        for profiled in (0, 1, 0, 1, 0):
+            check(lib.zk_profile_enable(ctx.handle, profiled), "zk_profile_enable")
+            com = kzh.commit(ctx, srs, poly)
+            got.append((com.c, com.d_x))
+    finally:
+        check(lib.zk_profile_enable(ctx.handle, 0), "zk_profile_enable")
+    assert all(g == got[1] for g in got)
 
 
 @pytest.mark.parametrize("n,kind", [(3, "full"), (4, "int8"), (5, "full"), (7, "mixed")])

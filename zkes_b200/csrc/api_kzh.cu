@@ -366,14 +366,17 @@ int zk_kzh_commit(zk_ctx* ctx, const zk_kzh_srs* srs, uint32_t poly_n, const uin
   // C = sum_i f[i] h_full[i]   (kzh2.rs:636-647, kzh3.rs:662-673)
   MsmPrep prep;  // both MSMs run over the same scalars: one analysis pass serves the two
   ctx->prof_begin(ZK_PROF_MSM, 0.0, 8);
-  rc = msm_run(ctx, srs->h[0], nullptr, f, size, 1, d_jac + rows, &ctx->last_msm, &prep);
+  MsmRowsBeside beside = {srs->h[1], srs->count[1], (uint32_t)rows, d_jac};
+  rc = msm_run_commit(ctx, srs->h[0], f, size, d_jac + rows, &ctx->last_msm, &prep, &beside);
   ctx->prof_end();
   if (rc) return rc;
   // d_x[i] = sum_j f[i * 2^(n - x_log) + j] h_mid[j]   (kzh2.rs:653-660, kzh3.rs:680-687)
-  ctx->prof_begin(ZK_PROF_MSM, 0.0, 8);
-  rc = msm_run(ctx, srs->h[1], nullptr, f, srs->count[1], (uint32_t)rows, d_jac, nullptr, &prep);
-  ctx->prof_end();
-  if (rc) return rc;
+  if (!beside.done) {
+    ctx->prof_begin(ZK_PROF_MSM, 0.0, 8);
+    rc = msm_run(ctx, srs->h[1], nullptr, f, srs->count[1], (uint32_t)rows, d_jac, nullptr, &prep);
+    ctx->prof_end();
+    if (rc) return rc;
+  }
   Jacobian* h_c = reinterpret_cast<Jacobian*>(reinterpret_cast<char*>(ctx->host_small) + 4096);
   ZK_CUDA(cudaMemcpyAsync(h_c, d_jac + rows, sizeof(Jacobian), cudaMemcpyDeviceToHost, st));
   ZK_CUDA(cudaMemcpyAsync(d_x_jac_out, d_jac, rows * sizeof(Jacobian), cudaMemcpyDeviceToHost, st));

@@ -32,6 +32,17 @@ struct MsmPrep {
 int msm_run(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const Fr* scalars, uint64_t n, uint32_t rows,
             Jacobian* out_dev, MsmStats* stats, MsmPrep* prep = nullptr);
 
+// The same for one row, C of a commitment, and beside it the commitment's rows over the same scalars where that is of use (done).
+struct MsmRowsBeside {
+  const Affine* bases;
+  uint64_t n;     // a row
+  uint32_t rows;
+  Jacobian* out_dev;
+  bool done = false;
+};
+int msm_run_commit(zk_ctx* ctx, const Affine* bases, const Fr* scalars, uint64_t n, Jacobian* out_dev, MsmStats* stats, MsmPrep* prep,
+                   MsmRowsBeside* rows);
+
 int msm_run_rows(zk_ctx* ctx, const Affine* bases, const uint32_t* gather, const uint32_t* row_ids, const Fr* scalars,
                  uint64_t n, uint32_t rows, Jacobian* out_dev, MsmStats* stats, MsmPrep* prep = nullptr);
 
