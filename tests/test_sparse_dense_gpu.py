@@ -7,6 +7,7 @@ import pytest
 import pyoracle as o
 from zkes_b200 import DenseMLPoly, SparseDenseSumcheckProver, Transcript
 from zkes_b200._lib import ZkError
+from zkes_b200.field import to_mont_array
 
 pytestmark = pytest.mark.gpu
 
@@ -84,3 +85,49 @@ def test_rejects_unsorted_or_out_of_range(ctx):
         p = SparseDenseSumcheckProver(4, t)
         with pytest.raises(ZkError):
             p.prove(ctx, bad, [1, 1], dense, t)
+
+
+@pytest.mark.parametrize("vals_at", ["aligned", "eight bytes off", "pinned"])
+@pytest.mark.parametrize("n,nnz", [(5, 1), (12, 40), (14, 1000)])
+def test_device_inputs(ctx, n, nnz, vals_at):
+    """Values in device memory are taken over by the launch that narrows the indices; unaligned or in other memory, by a copy."""
+    import torch
+    rnd = random.Random(n + nnz)
+    idx = sorted(rnd.sample(range(1 << n), nnz))
+    vals = [rnd.randrange(o.R_MOD) for _ in idx]
+    dense = [rnd.randrange(o.R_MOD) for _ in range(1 << n)]
+
+    def words(a):
+        return torch.from_numpy(a.view("int64").reshape(-1).copy())
+
+    d = words(DenseMLPoly.from_evaluations(dense).mont).cuda()
+    i = torch.tensor(idx, dtype=torch.int64, device="cuda")
+    v = words(to_mont_array(vals))
+    off = 1 if vals_at == "eight bytes off" else 0
+    buf = torch.zeros(v.numel() + 2, dtype=torch.int64)
+    buf = buf.pin_memory() if vals_at == "pinned" else buf.cuda()
+    buf[off:off + v.numel()] = v
+    torch.cuda.synchronize()
+    t, ot = Transcript(b"sd"), o.Transcript(b"sd")
+    p = SparseDenseSumcheckProver(n, t)
+    proof = p.prove(ctx, None, None, DenseMLPoly(n, device_ptr=d.data_ptr()), t, device_ptrs=(i.data_ptr(), buf.data_ptr() + 8 * off, nnz))
+    _, oproof = o.sparse_dense_prove(n, idx, vals, dense, ot)
+    assert proof.round_messages == oproof.round_messages and proof.final_eval == oproof.final_eval
+
+
+def test_rejects_a_bad_order_on_the_device(ctx):
+    """The word that the launch writes into host memory, once set and once not."""
+    import torch
+    d = torch.zeros(4 << 6, dtype=torch.int64, device="cuda")
+    v = torch.zeros(8, dtype=torch.int64, device="cuda")
+    dense = DenseMLPoly(6, device_ptr=d.data_ptr())
+    for idx, ok in (([3, 2], False), ([2, 3], True), ([5, 5], False), ([5, 64], False), ([5, 1 << 40], False), ([5, 63], True)):
+        i = torch.tensor(idx, dtype=torch.int64, device="cuda")
+        torch.cuda.synchronize()
+        t = Transcript(b"sd")
+        p = SparseDenseSumcheckProver(6, t)
+        if ok:
+            assert p.prove(ctx, None, None, dense, t, device_ptrs=(i.data_ptr(), v.data_ptr(), 2)).final_eval == 0
+        else:
+            with pytest.raises(ZkError):
+                p.prove(ctx, None, None, dense, t, device_ptrs=(i.data_ptr(), v.data_ptr(), 2))

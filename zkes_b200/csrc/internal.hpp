@@ -194,8 +194,9 @@ void launch_sparse_msg(uint32_t* idx, Fr* val, const uint32_t* count, uint32_t u
                        const PeerExchange* exchange = nullptr, unsigned int xseq = 0);
 void launch_sparse_bind(uint32_t* idx, Fr* val, const uint32_t* count, uint32_t upper, const Fr& r, int sm_count,
                         cudaStream_t s);
+// bind: the entries still have to be bound on it; null: they are
 void launch_scatter_runs(const uint32_t* idx, const Fr* val, const uint32_t* count, uint32_t upper, Fr* dense,
-                         int sm_count, cudaStream_t s);
+                         const Fr* bind, int sm_count, cudaStream_t s);
 // Where the folded entries of a list go: the leaders of every block of 256 counted and summed up (block_counts), *count_out of them
 // in all.  Depends on the positions alone, so it need not wait for the round's challenge.
 int launch_sparse_slots(const uint32_t* idx, const uint32_t* count, uint32_t upper, uint32_t* block_counts, uint32_t* count_out,
@@ -205,7 +206,8 @@ void launch_bool_fold(const uint32_t* idx, const Fr* val, const uint32_t* count,
                       uint32_t* idx_out, Fr* val_out, cudaStream_t s);
 void launch_scatter(const uint32_t* idx, const Fr* val, const uint32_t* count, uint32_t upper, Fr* dense,
                     int sm_count, cudaStream_t s);
-void launch_check_sorted(const uint32_t* idx, uint32_t n, uint64_t limit, uint32_t* bad, int sm_count, cudaStream_t s);
+void launch_take_entries(const uint64_t* in, const Fr* vals, uint32_t n, uint64_t limit, uint32_t* out, Fr* vals_out, uint32_t* count, uint32_t* bad,
+                         int sm_count, cudaStream_t s);
 void launch_check_bound(const uint32_t* idx, uint32_t n, uint64_t limit, uint32_t* bad, int sm_count, cudaStream_t s);
 void launch_narrow_idx(const uint64_t* in, uint32_t n, uint32_t* out, uint32_t* bad, int sm_count, cudaStream_t s,
                        uint64_t clamp_below = 0);

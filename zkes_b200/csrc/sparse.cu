@@ -281,24 +281,46 @@ __global__ void k_sparse_bind(uint32_t* __restrict__ idx, Fr* __restrict__ val, 
 }
 
 // Dense table from a sorted entry list that may hold several entries per position: the first entry of a run adds
-// up its run (a run is at most 2^rounds long and short in practice) and writes the position.
+// up its run (a run is at most 2^rounds long and short in practice) and writes the position.  BIND: the entries still have to be bound on
+// a challenge (as k_sparse_msg<., true> does); a run is then the entries of a pair, and one product binds its two sums.
+template <bool BIND>
 __global__ void k_scatter_runs(const uint32_t* __restrict__ idx, const Fr* __restrict__ val,
-                               const uint32_t* __restrict__ count, Fr* dense) {
+                               const uint32_t* __restrict__ count, const FixedMul<FrParams> bind, Fr* dense) {
   const uint32_t n = *count;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint32_t pos = idx[i];
-    if (i && idx[i - 1] == pos) continue;
-    Fr s = ld_fr(val + i);
-    for (uint32_t j = i + 1; j < n && idx[j] == pos; j++) s = add(s, ld_fr(val + j));
-    st_fr(dense + pos, s);
+    uint32_t key = idx[i];
+    const uint32_t pos = BIND ? key >> 1 : key;
+    if (i && (BIND ? idx[i - 1] >> 1 : idx[i - 1]) == pos) continue;
+    Fr even = Fr::zero(), odd = Fr::zero();
+    uint32_t j = i;
+    do {
+      const Fr v = ld_fr(val + j);
+      if (BIND && (key & 1u))
+        odd = add(odd, v);
+      else
+        even = add(even, v);
+      if (++j == n) break;
+      key = idx[j];
+    } while ((BIND ? key >> 1 : key) == pos);
+    st_fr(dense + pos, BIND ? add(even, mul_fixed(bind, sub(odd, even))) : even);
   }
 }
 
-// 1 when idx[0..n) is strictly increasing and below `limit`, else 0.
-__global__ void k_check_sorted(const uint32_t* __restrict__ idx, uint32_t n, uint64_t limit, uint32_t* bad) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    if ((uint64_t)idx[i] >= limit || (i > 0 && idx[i - 1] >= idx[i])) *bad = 1;
+// The entries of a call as the rounds take them: indices of 32 bits, values copied (from `vals`, 16-byte aligned device memory, unless
+// null), their count.  *bad becomes 1 unless the indices are strictly increasing and below limit; one that is not below is stored as
+// limit - 1, so that the kernels after this one stay inside their tables whatever the caller passed (the host looks at the word later).
+__global__ void __launch_bounds__(256) k_take_entries(const uint64_t* __restrict__ in, const uint4* __restrict__ vals, uint32_t n, uint64_t limit,
+                                                      uint32_t* __restrict__ out, uint4* __restrict__ vals_out, uint32_t* count, uint32_t* bad) {
+  const uint64_t first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+  if (first == 0) *count = n;
+  for (uint64_t i = first; i < n; i += step) {
+    uint64_t v = in[i];
+    if (v >= limit || (i && in[i - 1] >= v)) *bad = 1;
+    if (v >= limit) v = limit - 1;
+    out[i] = (uint32_t)v;
   }
+  if (vals)
+    for (uint64_t i = first; i < 2 * (uint64_t)n; i += step) vals_out[i] = __ldg(vals + i);
 }
 
 // Flags any idx[i] >= limit.
@@ -386,8 +408,12 @@ void launch_sparse_bind(uint32_t* idx, Fr* val, const uint32_t* count, uint32_t 
 }
 
 void launch_scatter_runs(const uint32_t* idx, const Fr* val, const uint32_t* count, uint32_t upper, Fr* dense,
-                         int sm_count, cudaStream_t s) {
-  k_scatter_runs<<<blocks_for(upper, 256, sm_count * 8), 256, 0, s>>>(idx, val, count, dense);
+                         const Fr* bind, int sm_count, cudaStream_t s) {
+  const unsigned blocks = (unsigned)blocks_for(upper, 256, sm_count * 8);
+  if (bind)
+    k_scatter_runs<true><<<blocks, 256, 0, s>>>(idx, val, count, make_fixed_mul(*bind), dense);
+  else
+    k_scatter_runs<false><<<blocks, 256, 0, s>>>(idx, val, count, FixedMul<FrParams>(), dense);
 }
 
 int launch_sparse_slots(const uint32_t* idx, const uint32_t* count, uint32_t upper, uint32_t* block_counts, uint32_t* count_out,
@@ -409,8 +435,10 @@ void launch_scatter(const uint32_t* idx, const Fr* val, const uint32_t* count, u
   k_scatter<<<blocks_for(upper, 256, sm_count * 8), 256, 0, s>>>(idx, val, count, dense);
 }
 
-void launch_check_sorted(const uint32_t* idx, uint32_t n, uint64_t limit, uint32_t* bad, int sm_count, cudaStream_t s) {
-  k_check_sorted<<<blocks_for(n, 256, sm_count * 8), 256, 0, s>>>(idx, n, limit, bad);
+void launch_take_entries(const uint64_t* in, const Fr* vals, uint32_t n, uint64_t limit, uint32_t* out, Fr* vals_out, uint32_t* count, uint32_t* bad,
+                         int sm_count, cudaStream_t s) {
+  k_take_entries<<<blocks_for(2 * (uint64_t)n, 256, sm_count * 8), 256, 0, s>>>(in, reinterpret_cast<const uint4*>(vals), n, limit, out,
+                                                                                reinterpret_cast<uint4*>(vals_out), count, bad);
 }
 
 void launch_check_bound(const uint32_t* idx, uint32_t n, uint64_t limit, uint32_t* bad, int sm_count, cudaStream_t s) {
