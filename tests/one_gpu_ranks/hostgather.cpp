@@ -1,0 +1,95 @@
+// Stands in for libnccl.so.2 where the ranks are threads of one process on one GPU: an all-gather through host memory.  The threads
+// meet on the host with nothing of theirs left on the GPU, so no kernel waits for another rank's.  A rank that does not come within a
+// minute ends the wait with an error.  The first all-gather of a communicator delivers zeros: it carries the handles of the
+// ranks' exchange boxes, and zeros say that no rank could map any, so that the library stays with the all-gathers.
+#include <cuda_runtime_api.h>
+
+#include <chrono>
+#include <condition_variable>
+#include <cstring>
+#include <map>
+#include <mutex>
+#include <vector>
+
+namespace {
+struct Group {
+  std::mutex mu;
+  std::condition_variable cv;
+  int world = 0, arrived = 0;
+  unsigned turn = 0;
+  bool first = true, broken = false;
+  std::vector<std::vector<char>> shares;
+  // Until every rank has come; `last` is run by the one that comes last.
+  template <class F>
+  bool meet(F last) {
+    std::unique_lock<std::mutex> lock(mu);
+    if (broken) return false;
+    if (++arrived == world) {
+      arrived = 0;
+      last();
+      turn++;
+      cv.notify_all();
+      return true;
+    }
+    const unsigned mine = turn;
+    if (!cv.wait_for(lock, std::chrono::seconds(60), [&] { return turn != mine || broken; })) broken = true;
+    if (broken) cv.notify_all();
+    return !broken;
+  }
+};
+struct Rank {
+  Group* group;
+  int rank;
+};
+struct Id {
+  char internal[128];
+};
+std::mutex g_mu;
+unsigned long g_next = 1;
+std::map<unsigned long, Group*> g_groups;
+}  // namespace
+
+extern "C" {
+int ncclGetUniqueId(Id* id) {
+  std::lock_guard<std::mutex> lock(g_mu);
+  memset(id, 0, sizeof *id);
+  memcpy(id->internal, &g_next, sizeof g_next);
+  g_next++;
+  return 0;
+}
+int ncclCommInitRank(void** comm, int world, Id id, int rank) {
+  std::lock_guard<std::mutex> lock(g_mu);
+  unsigned long key = 0;
+  memcpy(&key, id.internal, sizeof key);
+  Group*& g = g_groups[key];
+  if (!g) {
+    g = new Group;
+    g->world = world;
+    g->shares.resize(world);
+  }
+  *comm = new Rank{g, rank};
+  return 0;
+}
+int ncclAllGather(const void* send, void* recv, size_t bytes, int, void* comm, cudaStream_t stream) {
+  Rank* me = static_cast<Rank*>(comm);
+  Group* g = me->group;
+  std::vector<char>& mine = g->shares[me->rank];
+  mine.resize(bytes);
+  if (cudaMemcpyAsync(mine.data(), send, bytes, cudaMemcpyDeviceToHost, stream) != cudaSuccess || cudaStreamSynchronize(stream) != cudaSuccess) return 1;
+  if (!g->meet([&] {
+        if (g->first)
+          for (auto& s : g->shares) std::fill(s.begin(), s.end(), 0);
+        g->first = false;
+      }))
+    return 1;
+  for (int r = 0; r < g->world; r++)
+    if (cudaMemcpyAsync(static_cast<char*>(recv) + r * bytes, g->shares[r].data(), bytes, cudaMemcpyHostToDevice, stream) != cudaSuccess) return 1;
+  if (cudaStreamSynchronize(stream) != cudaSuccess) return 1;
+  return g->meet([] {}) ? 0 : 1;
+}
+int ncclCommDestroy(void* comm) {
+  delete static_cast<Rank*>(comm);
+  return 0;
+}
+const char* ncclGetErrorString(int) { return "a rank did not come to the all-gather"; }
+}

@@ -313,8 +313,8 @@ namespace zk {
 // `rounds` rounds of the dense prover over device tables cur[i] of 2^rounds elements each; the
 // folded tables alternate between ping and pong.  On return cur[] points at the two-entry
 // tables the last challenge has not been bound on yet (or the inputs when rounds == 0), unless
-// *finals_done is set: then the single-block tail kernel ran the last rounds with the built-in
-// transcript on the device and ctx->final_out already holds the final values.
+// *finals_done is set: then the rounds ran to the end with the built-in transcript on the device and
+// the final values are where read_finals() finds them.
 int linear_rounds(zk_ctx* ctx, zk_comm* comm, int L, uint32_t rounds, const Fr** cur, Fr** ping, Fr** pong,
                   uint32_t round_offset, zk_fs_round_fn fs, void* fs_user, zk_transcript* tr, uint64_t* round_msgs,
                   uint64_t* challenges, Fr* challenge, bool* finals_done) {
@@ -586,6 +586,18 @@ int linear_rounds(zk_ctx* ctx, zk_comm* comm, int L, uint32_t rounds, const Fr**
   return ZK_OK;
 }
 
+// The n final values of a prove, in host memory: where its last rounds left them (final_on_host: the kernel of these rounds may have
+// written them there and nowhere else), or fetched from ctx->final_out, where launch_final and launch_sd_final put them.
+int read_finals(zk_ctx* ctx, int n, const Fr** values) {
+  ZK_CUDA(cudaGetLastError());
+  *values = reinterpret_cast<const Fr*>(reinterpret_cast<const char*>(ctx->host_small) + kFinalHostOffset);
+  if (ctx->final_on_host) return ZK_OK;
+  *values = reinterpret_cast<const Fr*>(ctx->host_small);
+  ZK_CUDA(cudaMemcpyAsync(ctx->host_small, ctx->final_out, n * sizeof(Fr), cudaMemcpyDeviceToHost, ctx->stream));
+  ZK_CUDA(cudaStreamSynchronize(ctx->stream));
+  return ZK_OK;
+}
+
 // Self-check of a sharded prove on the host, a few microseconds: every summed message must continue the
 // round before it, s_m(0) + s_m(1) = s_{m-1}(r_{m-1}) (the identity SumcheckVerifier checks, verifier.rs:
 // 7-70).  A share that was damaged on its way between the ranks breaks it on every rank alike, so all
@@ -622,7 +634,7 @@ int check_round_chain(const uint64_t* round_msgs, const uint64_t* challenges, ui
 
 // After the local rounds of a sharded prove: ctx->final_out[0..L) holds this rank's fully bound
 // value of each table.  Gathers them into L tables of `world` entries, runs the remaining
-// log2(world) rounds identically on every rank and leaves the final values in ctx->final_out.
+// log2(world) rounds identically on every rank and leaves the final values where read_finals() finds them.
 int sharded_tail(zk_ctx* ctx, zk_comm* comm, int L, uint32_t n_local, zk_fs_round_fn fs, void* fs_user,
                  zk_transcript* tr, uint64_t* round_msgs, uint64_t* challenges, Fr* challenge) {
   const int world = comm_world(comm);
@@ -715,13 +727,9 @@ int linear_prove_impl(zk_ctx* ctx, zk_comm* comm, uint32_t num_var, uint32_t num
     rc = sharded_tail(ctx, comm, L, n_local, fs, fs_user, tr, round_msgs, challenges, &challenge);
     if (rc) return rc;
   }
-  ZK_CUDA(cudaGetLastError());
-  const Fr* fin = reinterpret_cast<const Fr*>(reinterpret_cast<char*>(ctx->host_small) + kFinalHostOffset);
-  if (!(done && ctx->final_on_host && (world == 1 || ctx->sharded_finished))) {  // not read back with the rounds
-    fin = reinterpret_cast<const Fr*>(ctx->host_small);
-    ZK_CUDA(cudaMemcpyAsync(ctx->host_small, ctx->final_out, (L + 1) * sizeof(Fr), cudaMemcpyDeviceToHost, ctx->stream));
-    ZK_CUDA(cudaStreamSynchronize(ctx->stream));
-  }
+  const Fr* fin = nullptr;
+  rc = read_finals(ctx, L + 1, &fin);
+  if (rc) return rc;
   if (final_table0)
     for (int i = 0; i < L; i++) fr_store(final_table0 + 4 * i, fin[i]);
   fr_store(final_eval, fin[L]);

@@ -67,6 +67,7 @@ static int sparse_dense_impl(zk_ctx* ctx, zk_comm* comm, uint32_t total_var, uin
   // Sharded: every rank must leave the entry form at the same round (the dense rounds exchange
   // differently, and may gather the tables), so the rule below uses the largest entry count of any rank.
   ctx->time_mark();  // call entry
+  ctx->final_on_host = false;  // the dense rounds, if there are any, say so
   uint32_t K_rule = K;
   if (comm) {
     uint32_t all[16];
@@ -158,8 +159,7 @@ static int sparse_dense_impl(zk_ctx* ctx, zk_comm* comm, uint32_t total_var, uin
   Fr challenge = Fr::zero();
   QuadForm form;
   uint64_t S = size;
-  bool finished = false;  // the dense phase ran to the end (final values are in ctx->final_out)
-  bool dense_done = false;  // ... inside the device-resident rounds, which read the final values back with the rounds
+  bool finished = false;  // the dense phase ran to the end
   for (uint32_t round = 0; round < num_var; round++, S >>= 1) {
     if (K_rule && S <= dense_cap) {
       // hand over to the dense prover: scatter the entries into a table and run the remaining rounds
@@ -185,7 +185,6 @@ static int sparse_dense_impl(zk_ctx* ctx, zk_comm* comm, uint32_t total_var, uin
       rc = linear_rounds(ctx, comm, 2, num_var - round, d_cur, d_ping, d_pong, round, fs, fs_user, tr, round_msgs,
                          challenges, &challenge, &done);
       if (rc) return rc;
-      dense_done = done;
       ctx->time_mark();  // the dense rounds are back
       if (!done) {
         launch_final(2, true, d_cur, challenge, ctx->final_out, s);
@@ -269,13 +268,9 @@ static int sparse_dense_impl(zk_ctx* ctx, zk_comm* comm, uint32_t total_var, uin
     rc = sharded_tail(ctx, comm, 2, num_var, fs, fs_user, tr, round_msgs, challenges, &challenge);
     if (rc) return rc;
   }
-  ZK_CUDA(cudaGetLastError());
-  const Fr* fin = reinterpret_cast<const Fr*>(reinterpret_cast<char*>(ctx->host_small) + kFinalHostOffset);
-  if (!(dense_done && ctx->final_on_host && (!comm || ctx->sharded_finished))) {  // not read back with the dense rounds
-    fin = reinterpret_cast<const Fr*>(ctx->host_small);
-    ZK_CUDA(cudaMemcpyAsync(ctx->host_small, ctx->final_out, 3 * sizeof(Fr), cudaMemcpyDeviceToHost, s));
-    ZK_CUDA(cudaStreamSynchronize(s));
-  }
+  const Fr* fin = nullptr;
+  rc = read_finals(ctx, 3, &fin);
+  if (rc) return rc;
   if (final_table0) {
     fr_store(final_table0, fin[0]);
     fr_store(final_table0 + 4, fin[1]);

@@ -85,7 +85,7 @@ struct zk_ctx {
   void* cmp = nullptr;           // third grow-only scratch (compact small scalars of the MSM)
   size_t cmp_bytes = 0;
   uint64_t replicate_entries = zk::kReplicateEntries;  // sharded proves gather the tables at this many entries in all (0: never)
-  bool final_on_host = false;    // the dense round loop read final_out back together with its rounds (host_small + kFinalHostOffset)
+  bool final_on_host = false;    // the final values of this prove are in host memory (host_small + kFinalHostOffset), not in final_out
   bool sharded_finished = false; // set by the dense round loop of a sharded prove when it gathered the tables and ran to the end
   bool peer_exchange = true;     // sharded proves exchange round messages through peer memory when the ranks could map it
   uint32_t exchange_wait_ms = 16000;  // bound of a device-side wait for another rank's words (ZK_OPT_EXCHANGE_WAIT_MS)
@@ -164,6 +164,7 @@ bool comm_peer_args(const zk_ctx* ctx, const zk_comm* c, PeerExchange* out);
 // api.cu
 int wait_published(zk_ctx* ctx, const void* word, unsigned int want, bool* set);
 int wait_result(zk_ctx* ctx);  // until the last next_msg_scratch(false) launch has published
+int read_finals(zk_ctx* ctx, int n, const Fr** values);
 void comm_peer_advance(zk_comm* c, unsigned int n);
 int comm_peer_gather(zk_ctx* ctx, zk_comm* c, int n_tables, const Fr* const* chunks, uint32_t m, unsigned int* error_word,
                      const Fr** tables_out);
