@@ -69,6 +69,24 @@ def test_same_results(ctx, srs, count, before):
     del keep
 
 
+@pytest.mark.parametrize("off", [1, 4, 7])
+def test_lists_that_are_not_aligned_to_their_words(ctx, srs, off):
+    """Copied whatever their address, as from pageable memory: no kernel reads them in place."""
+    rnd = random.Random(off)
+    values = np.array(rnd.sample(range(1 << N), 100), dtype=np.uint64)
+    point, weights, counts = to_mont_array([rnd.randrange(o.R_MOD) for _ in range(N)]), to_mont_array([5]), np.array([100], dtype=np.uint64)
+    keep = torch.zeros(off + values.nbytes, dtype=torch.uint8, pin_memory=True)
+    keep[off:] = torch.from_numpy(values.view(np.uint8))
+    ptr = keep.data_ptr() + off
+    for call in (lambda p: opened(ctx, srs, p, 100, point), lambda p: committed(ctx, srs, p, 100),
+                 lambda p: checked(ctx, 1, p, counts, weights, point)):
+        rc, want = call(values.ctypes.data)
+        check(rc, "aligned")
+        rc, got = call(ptr)
+        check(rc, "not aligned")
+        assert np.array_equal(got, want)
+
+
 def test_refused_indices(ctx, srs):
     point, weights = to_mont_array([3] * N), to_mont_array([5])
     values = np.array([1, 2, 1 << N], dtype=np.uint64)

@@ -207,6 +207,7 @@ const void* zk_ctx::device_view(const void* host, size_t bytes) const {
     return nullptr;
   }
   if (at.type != cudaMemoryTypeHost || !at.devicePointer) return nullptr;
+  if (reinterpret_cast<uintptr_t>(at.devicePointer) % sizeof(uint64_t)) return nullptr;  // a kernel cannot load such a word, a copy can
   CUdeviceptr start = 0;
   size_t size = 0;
   const CUdeviceptr p = (CUdeviceptr)(uintptr_t)host;

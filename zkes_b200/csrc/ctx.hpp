@@ -147,9 +147,10 @@ struct zk_ctx {
   int reserve_work(size_t bytes, void** out);
   int reserve_aux(size_t bytes, void** out);
   int reserve_cmp(size_t bytes, void** out);
-  // The device's address of a caller's host buffer that is pinned and mapped over its whole length, or nullptr.  A list that a
-  // kernel reads once is read through it: the kernel's work goes on while the list crosses the bus instead of after it (2^18
-  // positions of a selection opening: the copy 41 us and the kernel 19, the kernel alone 45).
+  // The device's address of a caller's list of 64-bit words in host memory that is pinned and mapped over its whole length and
+  // aligned to its words, or nullptr: then the list has to be copied, which asks for no alignment.  A list that a kernel reads once is
+  // read through it: the kernel's work goes on while the list crosses the bus instead of after it (2^18 positions of a selection
+  // opening: the copy 41 us and the kernel 19, the kernel alone 45).
   const void* device_view(const void* host, size_t bytes) const;
 };
 
