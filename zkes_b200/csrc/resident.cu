@@ -212,6 +212,7 @@ __device__ __forceinline__ void ahead_rounds(const ResidentParams<L>& p, WarpStr
     if (!wait_tagged(&sh->rplain[(t0 - 1) & 1], true, t0, r, &sh->error, p.spin_limit)) return;
     const int j = lane % NV;
     if (p.done) {  // what this warp wrote in the rounds in step, while the workers tabulate the next message
+      __syncwarp();  // a lane reads what others have stored
       const uint4* from = reinterpret_cast<const uint4*>(p.out_msgs);
       for (uint32_t k = lane; k < 2 * t0 * NV; k += 32) reinterpret_cast<uint4*>(p.far_msgs)[k] = __ldcg(from + k);
       from = reinterpret_cast<const uint4*>(p.out_chal);
