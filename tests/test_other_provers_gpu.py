@@ -1,14 +1,17 @@
 """SparseBoolSumcheckProver and GeneralLinearSumcheckProver on the GPU against the oracle
 (src/crypto/sumcheck/linear_prover.rs:193-656), including the committed golden vectors."""
+import ctypes
 import json
 import os
 import random
 
+import numpy as np
 import pytest
 
 import pyoracle as o
 from zkes_b200 import DenseMLPoly, GeneralLinearSumcheckProver, SparseBoolSumcheckProver, Transcript
-from zkes_b200._lib import ZkError
+from zkes_b200._lib import ZK_ERR_ARG, ZkError, lib
+from zkes_b200.field import to_mont_array
 
 pytestmark = pytest.mark.gpu
 M = o.R_MOD
@@ -138,3 +141,21 @@ def test_general_linear(ctx, n, num_poly, terms):
     vt = o.Transcript(b"general")
     res, _ = o.SumcheckVerifier(n, num_poly, vt).verify(vt, pr.round_messages, claimed % M)
     assert res == pr.final_eval
+
+
+@pytest.mark.parametrize("positions", [[3, 3], [1, 1 << 24]])
+def test_refused_list_leaves_nothing_under_way(ctx, positions):
+    """A call that refuses its list does not return while work on the caller's weights, or on its own scratch, is still under way."""
+    import torch
+    n = 24
+    weights, flat, counts = to_mont_array([5]), np.array(positions, dtype=np.uint64), np.array([2], dtype=np.uint64)
+    point, msgs, chal, fin = to_mont_array([7] * n), np.zeros((n * 4, 4), dtype=np.uint64), np.zeros((n, 4), dtype=np.uint64), np.zeros((1, 4), dtype=np.uint64)
+    vp = ctypes.c_void_p
+    stream = torch.cuda.ExternalStream(lib.zk_stream(ctx.handle))
+    for _ in range(3):
+        tr = lib.zk_transcript_new(b"p", 1)
+        rc = lib.zk_sumcheck_sparse_bool_prove(ctx.handle, n, 1, vp(weights.ctypes.data), vp(flat.ctypes.data), vp(counts.ctypes.data),
+                                               vp(point.ctypes.data), None, None, tr, vp(msgs.ctypes.data), vp(chal.ctypes.data), vp(fin.ctypes.data))
+        idle = stream.query()
+        lib.zk_transcript_free(tr)
+        assert rc == ZK_ERR_ARG and idle

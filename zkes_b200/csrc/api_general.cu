@@ -121,10 +121,11 @@ int sbool_prove(zk_ctx* ctx, zk_comm* comm, uint32_t num_var, uint32_t n_terms, 
     ZK_CUDA(cudaEventRecord(ctx->ev_join, s2));
     ZK_CUDA(cudaStreamWaitEvent(s, ctx->ev_join, 0));
   }
+  const cudaError_t through = cudaStreamSynchronize(s);  // the weights, which a copy may still read, are the caller's again whatever we return
   if (rc) return rc;
+  ZK_CUDA(through);
   if (bad[0]) return fail(ZK_ERR_ARG, "sparse_bool_prove: position out of range in term %u", bad[0] - 1);
   if (bad[1]) return fail(ZK_ERR_ARG, "sparse_bool_prove: duplicate position in term %u", bad[1] - 1);
-  ZK_CUDA(cudaStreamSynchronize(s));  // the weights' host buffer may go out of scope after this
 
   Fr bound = Fr::one();  // eq over the variables bound so far
   int e = 0;
