@@ -37,6 +37,7 @@ extern "C" void zkp_merged(uint64_t n, uint64_t* out) {
   out[2] = kMergedMost;
   out[3] = kEndoMost;
 }
+extern "C" int zkp_merged_rows(uint64_t n, uint32_t rows) { return merged_rows(n, rows); }
 extern "C" uint32_t zkp_reduce_lanes(uint32_t n_items, uint32_t half, int sm) { return reduce_lanes(n_items, half, sm); }
 extern "C" int zkp_combine_by(uint32_t rows, int w, int k_windows, int sm) { return (int)combine_by(rows, w, k_windows, sm); }
 extern "C" uint32_t zkp_fixup_groups(uint32_t n_buckets, uint32_t n_chunks, uint64_t longest, uint32_t seg) {

@@ -21,6 +21,7 @@ def plan(tmp_path_factory):
     lib.zkp_buckets.argtypes = [u64, u32, i, i, i, ctypes.c_void_p]
     lib.zkp_windows.argtypes = [u64, u32, u32, ctypes.c_void_p]
     lib.zkp_merged.argtypes = [u64, ctypes.c_void_p]
+    lib.zkp_merged_rows.argtypes = [u64, u32]
     lib.zkp_rows.argtypes = [u64, u32, u32, u64, i, i, i, u64, ctypes.c_void_p]
 
     lib.zkp_reduce_lanes.argtypes = [u32, u32, i]
@@ -84,6 +85,17 @@ def test_shared_buckets_hold_every_digit_and_entry(plan, n):
     assert w * windows >= 127 > w * (windows - 1)
     assert n <= most and windows * n < 1 << 30 and split_most < 1 << 30
     assert plan("zkp_buckets", 2, 2 * n * windows * 32, 32, w, 1, SM)[0] == 32 << (w - 1)
+
+
+@pytest.mark.parametrize("n", [1, 1 << 14, 1 << 17, (1 << 18) - 1, 1 << 18, 1 << 19, 1 << 20, (1 << 20) + 1, 1 << 24, 1 << 40])
+@pytest.mark.parametrize("rows", [1, 31, 32, 1 << 12])
+def test_shared_buckets_have_bounded_tables(plan, n, rows):
+    """The multiples of a call's bases (an affine and an XYZZ point and a coordinate each) stay below half a gigabyte, whatever the rows."""
+    taken = bool(plan("zkp_merged_rows", 0, n, rows))
+    assert taken == (rows >= 32 and n <= 1 << 18)
+    if taken:
+        _, windows, _, _ = plan("zkp_merged", 4, n)
+        assert n * windows * (64 + 128 + 32) <= 512 << 20
 
 
 # rows, columns, kind, share of zeros, subset sums: measured, both ways at least a tenth apart

@@ -1252,7 +1252,7 @@ static int msm_run_impl(zk_ctx* ctx, const Affine* bases, const uint32_t* gather
   // Scalars of up to 160 bits stay whole: they have fewer digits than 2 x 126 bits have.
   const bool endo = !compact && !row_ids && !gather && max_bits > kEndoBits && n <= kEndoMost && !plain;
   const int bits = endo ? kGlvBits : (int)max_bits;
-  const bool merged = endo && rows >= kMergedRows && n <= kMergedMost;
+  const bool merged = endo && merged_rows(n, rows);
   // Separate windows of several rows: a bit more than for whole scalars, as there are half as many (pick_window).
   const int w = merged ? merged_window(n) : pick_window(row_ids ? (n / rows ? n / rows : 1) : n, rows, bits) + (endo && rows > 1 ? 1 : 0);
   // small scalars: the exact largest magnitude is known, which can save the window that would only
@@ -1281,6 +1281,7 @@ static int msm_run_impl(zk_ctx* ctx, const Affine* bases, const uint32_t* gather
   // ---- scratch layout (second scratch region of the context; the first holds caller data)
   const uint64_t table_points = merged ? n * (uint64_t)digit_windows : 0;
   const uint32_t table_step = merged ? (uint32_t)n : 0;
+  static_assert(sizeof(Affine) + sizeof(Xyzz) + sizeof(Fq) == kMultipleBytes, "what the plan counts for a multiple");
   const size_t endo_bytes = (endo ? align256((merged ? table_points : n) * sizeof(Fq)) : 0) + align256(table_points * sizeof(Affine)) +
                             align256(table_points * sizeof(Xyzz));
   RowsPlan also_plan;

@@ -43,8 +43,13 @@ inline int pick_window(uint64_t n, uint32_t rows, int max_bits) {
 // Rows over the same bases whose windows share their buckets (k_multiples): from kMergedRows rows on.  Window width: a row adds
 // 2 n points a window and some three points a bucket.  Below 32 rows the multiples (a chain of 126 doublings, 0.2 to 0.6 ms) cost what
 // the shared buckets save.
+// The tables of the multiples stay in the lane's scratch, so the route is bounded by their bytes: 2^18 points a row, 470 MB.  It
+// gains less with the points, too: 32 rows of 2^14 full-width scalars take 2.76 ms with shared buckets and 3.31 without, of 2^18 32.8 and
+// 34.4, of 2^19 63.9 and 59.1 (128 rows of 2^18: 111 and 137).
 constexpr uint32_t kMergedRows = 32;
-constexpr uint64_t kMergedMost = 1ull << 20;  // points a row
+constexpr uint64_t kMergedMost = 1ull << 20;  // points a row whose multiples' indices fit beside an entry's flags whatever the window
+constexpr size_t kMergedBytes = 512u << 20;
+constexpr size_t kMultipleBytes = 64 + 128 + 32;  // of a multiple: affine, XYZZ while they are made, the x of its image
 inline int merged_window(uint64_t n) {
   int best = 4;
   double least = 1e300;
@@ -56,6 +61,11 @@ inline int merged_window(uint64_t n) {
     }
   }
   return best;
+}
+inline bool merged_rows(uint64_t n, uint32_t rows) {
+  if (rows < kMergedRows || n > kMergedMost) return false;
+  const int w = merged_window(n);
+  return n * (uint64_t)((kEndoMagnitude + w) / w) * kMultipleBytes <= kMergedBytes;
 }
 
 // Signed-digit windows needed for magnitudes up to max_mag: k digits in (-half, half] reach
