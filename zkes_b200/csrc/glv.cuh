@@ -1,6 +1,6 @@
 // The endomorphism of the curve: BN254's G1 has phi(x, y) = (beta x, y) = lambda (x, y) with beta^3 = 1 mod q, lambda^3 = 1 mod r, and the
 // lattice of (u, v) with u + v lambda = 0 mod r has a basis v1 = (a1, b1), v2 = (a2, b2) of vectors of length about sqrt(r).  A scalar
-// k = k1 + k2 lambda with k1, k2 of 126 bits: (k1, k2) = (k, 0) - c1 v1 - c2 v2, c1 and c2 the nearest integers to b2 k / r and
+// k = k1 + k2 lambda with k1, k2 of 126 bits (kEndoMagnitude): (k1, k2) = (k, 0) - c1 v1 - c2 v2, c1 and c2 the nearest integers to b2 k / r and
 // -b1 k / r (Gallant, Lambert and Vanstone, "Faster point multiplication on elliptic curves with efficient endomorphisms", 2001; the
 // basis by the extended Euclidean algorithm on r and lambda, as there).  The rounded quotients come from products with 2^256 b2 / r and
 // 2^256 |b1| / r, whose own rounding adds k / 2^257 < 2^-4 to the half.
@@ -35,7 +35,6 @@ struct Glv {
     return m[i];
   }
 };
-constexpr int kGlvBits = 126;  // bits of a magnitude: (1/2 + 2^-4) (a1 + a2) is below 2^126
 
 // out = the NO low words of a b
 template <int NA, int NB, int NO>

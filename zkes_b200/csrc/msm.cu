@@ -1251,7 +1251,7 @@ static int msm_run_impl(zk_ctx* ctx, const Affine* bases, const uint32_t* gather
   // points: kernels 752 -> 728 us (bucket reduction 153 -> 118), the chain of doublings on the host half as long, the call 929 -> 862 us.
   // Scalars of up to 160 bits stay whole: they have fewer digits than 2 x 126 bits have.
   const bool endo = !compact && !row_ids && !gather && max_bits > kEndoBits && n <= kEndoMost && !plain;
-  const int bits = endo ? kGlvBits : (int)max_bits;
+  const int bits = endo ? kEndoMagnitude : (int)max_bits;
   const bool merged = endo && merged_rows(n, rows);
   // Separate windows of several rows: a bit more than for whole scalars, as there are half as many (pick_window).
   const int w = merged ? merged_window(n) : pick_window(row_ids ? (n / rows ? n / rows : 1) : n, rows, bits) + (endo && rows > 1 ? 1 : 0);

@@ -10,7 +10,7 @@ namespace zk {
 
 constexpr unsigned kEndoBits = 160;  // scalars of more bits are split by the endomorphism (glv.cuh)
 constexpr uint64_t kEndoMost = 1ull << 24;  // points a row: above, the buckets are few beside the points and their images are half a gigabyte
-constexpr int kEndoMagnitude = 126;  // into magnitudes of as many bits
+constexpr int kEndoMagnitude = 126;  // into magnitudes of as many bits: (1/2 + 2^-4) (a1 + a2) of glv.cuh is below 2^126
 constexpr int kCompactBits = 30;  // magnitudes below 2^30 have a compact form (k_msm_bits)
 constexpr int kAccBlocks = 4;     // blocks of 128 threads per SM of the kernels that add points in chains (126 and 122 registers)
 constexpr uint32_t kReduceThreads = 128;   // threads of a block of the bucket reduction
