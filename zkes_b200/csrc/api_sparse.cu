@@ -106,7 +106,7 @@ static int sparse_dense_impl(zk_ctx* ctx, zk_comm* comm, uint32_t total_var, uin
   uint32_t* e_idx[2] = {ar.take<uint32_t>(K + 1), ar.take<uint32_t>(K + 1)};
   Fr* e_val[2] = {ar.take<Fr>(K + 1), ar.take<Fr>(K + 1)};
   uint32_t* block_counts = ar.take<uint32_t>(K / 256 + 2);
-  uint32_t* counts = ar.take<uint32_t>(64);  // [0], [1]: entry counts (ping-pong); [2]: bad-input flag
+  uint32_t* counts = ar.take<uint32_t>(64);  // [0]: entry count
   Fr* a_dense = ar.take<Fr>(dense_cap + 1);
   Fr* d_ping[2] = {ar.take<Fr>(dense_cap / 2 + 1), ar.take<Fr>(dense_cap / 2 + 1)};
   Fr* d_pong[2] = {ar.take<Fr>(dense_cap / 4 + 1), ar.take<Fr>(dense_cap / 4 + 1)};
@@ -208,14 +208,15 @@ static int sparse_dense_impl(zk_ctx* ctx, zk_comm* comm, uint32_t total_var, uin
     rc = fs_round(ctx, comm, 3, round, fs, fs_user, tr, round_msgs, challenges, &challenge, fused, &sums);
     if (rc != ZK_OK) return rc;
     form.bind(challenge);
-    rc = check_bad(false);  // the message kernel ran after the copy of the flag
+    rc = check_bad(false);  // the message kernel ran after the launch that writes the word
     if (rc != ZK_OK) return rc;
     // Fold of the dense table.  When the next round is still in entry form its message can fold
     // the few values it needs on the fly, so this fold waits and is done together with the next
     // one in a single pass over the table (k_fold2).
     const bool next_sparse = round + 1 < num_var && (!K_rule || (S / 2) > dense_cap);
-    // The table fold goes to the side stream, which the next message waits for.  Nothing runs beside it since the message kernel
-    // binds the entries itself.  With the per-kernel profiler on it stays in line so that each span times one kernel alone.
+    // The table fold goes to the side stream.  Before another entry round the stream waits for it at once (the message kernel
+    // reads the folded table); the last one is joined by the hand-over, whose clearing and scattering of a_dense run beside it and
+    // touch nothing of the fold's.  With the per-kernel profiler on it stays in line so that each span times one kernel alone.
     const bool fold_now = pending || !next_sparse;
     const bool beside = fold_now && !ctx->prof_on;
     cudaStream_t fs_stream = beside ? ctx->side_stream : s;
@@ -256,11 +257,7 @@ static int sparse_dense_impl(zk_ctx* ctx, zk_comm* comm, uint32_t total_var, uin
   if (rc) return rc;
   rc = check_bad(true);
   if (rc != ZK_OK) return rc;
-  if (!finished && e_pending) {  // the entry form ran to the end (no entries anywhere): bind the last challenge
-    launch_sparse_bind(e_idx[e], e_val[e], counts + e, k_upper, e_r, ctx->sm_count, s);
-    ctx->launches++;
-  }
-  if (!finished) {  // no entries, or no variables: the entry form ran to the end
+  if (!finished) {  // no entries on any rank, or no variables: the entry form ran to the end
     launch_sd_final(e_idx[e], e_val[e], counts + e, b_cur, ctx->final_out, s);
     ctx->launches++;
   }

@@ -192,8 +192,6 @@ int launch_resident(int num_poly, const Fr* const* src, Fr* const* ping, Fr* con
 void launch_sparse_msg(uint32_t* idx, Fr* val, const uint32_t* count, uint32_t upper, const Fr* dense,
                        const Fr* pending, const Fr* bind, const RoundScratch& sc, cudaStream_t s,
                        const PeerExchange* exchange = nullptr, unsigned int xseq = 0);
-void launch_sparse_bind(uint32_t* idx, Fr* val, const uint32_t* count, uint32_t upper, const Fr& r, int sm_count,
-                        cudaStream_t s);
 // bind: the entries still have to be bound on it; null: they are
 void launch_scatter_runs(const uint32_t* idx, const Fr* val, const uint32_t* count, uint32_t upper, Fr* dense,
                          const Fr* bind, int sm_count, cudaStream_t s);
@@ -204,13 +202,10 @@ int launch_sparse_slots(const uint32_t* idx, const uint32_t* count, uint32_t upp
 // The entries bound on r at the slots that launch_sparse_slots made.
 void launch_bool_fold(const uint32_t* idx, const Fr* val, const uint32_t* count, uint32_t upper, const Fr& r, const uint32_t* block_offsets,
                       uint32_t* idx_out, Fr* val_out, cudaStream_t s);
-void launch_scatter(const uint32_t* idx, const Fr* val, const uint32_t* count, uint32_t upper, Fr* dense,
-                    int sm_count, cudaStream_t s);
 void launch_take_entries(const uint64_t* in, const Fr* vals, uint32_t n, uint64_t limit, uint32_t* out, Fr* vals_out, uint32_t* count, uint32_t* bad,
                          int sm_count, cudaStream_t s);
 void launch_check_bound(const uint32_t* idx, uint32_t n, uint64_t limit, uint32_t* bad, int sm_count, cudaStream_t s);
-void launch_narrow_idx(const uint64_t* in, uint32_t n, uint32_t* out, uint32_t* bad, int sm_count, cudaStream_t s,
-                       uint64_t clamp_below = 0);
+void launch_narrow_idx(const uint64_t* in, uint32_t n, uint32_t* out, uint32_t* bad, int sm_count, cudaStream_t s);
 void launch_sd_final(const uint32_t* idx, const Fr* val, const uint32_t* count, const Fr* dense, Fr* out,
                      cudaStream_t s);
 

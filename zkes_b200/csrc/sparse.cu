@@ -260,26 +260,6 @@ __global__ void __launch_bounds__(kSpThreads) k_bool_fold(const uint32_t* __rest
   st_fr(val_out + slot, add(v0, mul_fixed(r, sub(v1, v0))));
 }
 
-__global__ void k_scatter(const uint32_t* __restrict__ idx, const Fr* __restrict__ val,
-                          const uint32_t* __restrict__ count, Fr* dense) {
-  const uint32_t n = *count;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    st_fr(dense + idx[i], ld_fr(val + i));
-}
-
-// Entries bound by r in place (the step k_sparse_msg<., true> does on the fly), for the hand-over to the dense form.
-__global__ void k_sparse_bind(uint32_t* __restrict__ idx, Fr* __restrict__ val, const uint32_t* __restrict__ count,
-                              const FixedMul<FrParams> bind) {
-  const uint32_t n = *count;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint32_t pos = idx[i];
-    const Fr v = ld_fr(val + i);
-    const Fr t = mul_fixed(bind, v);
-    idx[i] = pos >> 1;
-    st_fr(val + i, (pos & 1u) ? t : sub(v, t));
-  }
-}
-
 // Dense table from a sorted entry list that may hold several entries per position: the first entry of a run adds
 // up its run (a run is at most 2^rounds long and short in practice) and writes the position.  BIND: the entries still have to be bound on
 // a challenge (as k_sparse_msg<., true> does); a run is then the entries of a pair, and one product binds its two sums.
@@ -330,16 +310,10 @@ __global__ void k_check_bound(const uint32_t* __restrict__ idx, uint32_t n, uint
 }
 
 // Narrow caller indices (u64) to the 32-bit form the kernels use; flags values >= 2^32.
-// With clamp_below > 0 a value at or above it is flagged and stored as clamp_below - 1, so that the kernels after
-// this one stay inside their tables whatever the caller passed (the host looks at the flag later).
-__global__ void k_narrow_idx(const uint64_t* __restrict__ in, uint32_t n, uint32_t* out, uint32_t* bad, uint64_t clamp_below) {
+__global__ void k_narrow_idx(const uint64_t* __restrict__ in, uint32_t n, uint32_t* out, uint32_t* bad) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    uint64_t v = in[i];
+    const uint64_t v = in[i];
     if (v >> 32) *bad = 1;
-    if (clamp_below && v >= clamp_below) {
-      *bad = 1;
-      v = clamp_below - 1;
-    }
     out[i] = (uint32_t)v;
   }
 }
@@ -402,11 +376,6 @@ void launch_sparse_msg(uint32_t* idx, Fr* val, const uint32_t* count, uint32_t u
     launch_sparse_msg_t<false, false>(idx, val, count, upper, dense, pt, bt, sc, s, px, xseq);
 }
 
-void launch_sparse_bind(uint32_t* idx, Fr* val, const uint32_t* count, uint32_t upper, const Fr& r, int sm_count,
-                        cudaStream_t s) {
-  k_sparse_bind<<<blocks_for(upper, 256, sm_count * 8), 256, 0, s>>>(idx, val, count, make_fixed_mul(r));
-}
-
 void launch_scatter_runs(const uint32_t* idx, const Fr* val, const uint32_t* count, uint32_t upper, Fr* dense,
                          const Fr* bind, int sm_count, cudaStream_t s) {
   const unsigned blocks = (unsigned)blocks_for(upper, 256, sm_count * 8);
@@ -430,11 +399,6 @@ void launch_bool_fold(const uint32_t* idx, const Fr* val, const uint32_t* count,
   k_bool_fold<<<blocks, kSpThreads, 0, s>>>(idx, val, count, block_offsets, make_fixed_mul(r), idx_out, val_out);
 }
 
-void launch_scatter(const uint32_t* idx, const Fr* val, const uint32_t* count, uint32_t upper, Fr* dense,
-                    int sm_count, cudaStream_t s) {
-  k_scatter<<<blocks_for(upper, 256, sm_count * 8), 256, 0, s>>>(idx, val, count, dense);
-}
-
 void launch_take_entries(const uint64_t* in, const Fr* vals, uint32_t n, uint64_t limit, uint32_t* out, Fr* vals_out, uint32_t* count, uint32_t* bad,
                          int sm_count, cudaStream_t s) {
   k_take_entries<<<blocks_for(2 * (uint64_t)n, 256, sm_count * 8), 256, 0, s>>>(in, reinterpret_cast<const uint4*>(vals), n, limit, out,
@@ -445,9 +409,8 @@ void launch_check_bound(const uint32_t* idx, uint32_t n, uint64_t limit, uint32_
   k_check_bound<<<blocks_for(n, 256, sm_count * 8), 256, 0, s>>>(idx, n, limit, bad);
 }
 
-void launch_narrow_idx(const uint64_t* in, uint32_t n, uint32_t* out, uint32_t* bad, int sm_count, cudaStream_t s,
-                       uint64_t clamp_below) {
-  k_narrow_idx<<<blocks_for(n, 256, sm_count * 8), 256, 0, s>>>(in, n, out, bad, clamp_below);
+void launch_narrow_idx(const uint64_t* in, uint32_t n, uint32_t* out, uint32_t* bad, int sm_count, cudaStream_t s) {
+  k_narrow_idx<<<blocks_for(n, 256, sm_count * 8), 256, 0, s>>>(in, n, out, bad);
 }
 
 void launch_sd_final(const uint32_t* idx, const Fr* val, const uint32_t* count, const Fr* dense, Fr* out,
