@@ -1,18 +1,18 @@
 """The sharded entry points with their ranks as threads of this process, a context each, on one GPU: argv[1] is the stand-in for NCCL
-(hostgather.cpp), argv[2] the number of ranks."""
+(hostgather.cpp), argv[2] the number of ranks; with argv[3] one share of an all-gather is damaged."""
 import ctypes
 import os
 import random
 import sys
 import threading
 
-ctypes.CDLL(sys.argv[1], mode=ctypes.RTLD_GLOBAL)  # before the library looks for libnccl.so.2, and torch stays out
+gather = ctypes.CDLL(sys.argv[1], mode=ctypes.RTLD_GLOBAL)  # before the library looks for libnccl.so.2, and torch stays out
 ROOT = os.path.dirname(os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 sys.path[:0] = [ROOT, os.path.join(ROOT, "oracle")]
 import pyoracle as o
 from zkes_b200 import Context, DenseMLPoly, Transcript
 from zkes_b200 import dist as zd
-from zkes_b200._lib import ZK_OPT_AHEAD_LOG, ZK_OPT_PEER_EXCHANGE, ZK_OPT_REPLICATE_LOG, check, lib
+from zkes_b200._lib import ZK_ERR_COMM, ZK_OPT_AHEAD_LOG, ZK_OPT_PEER_EXCHANGE, ZK_OPT_REPLICATE_LOG, ZkError, check, lib
 
 M = o.R_MOD
 WORLD = int(sys.argv[2])
@@ -92,17 +92,55 @@ def sparse(ranks, n, idx, vals, dense):
         assert tuple(got) == want, ("sparse", n, len(idx), r)
 
 
-ranks = start()
-rnd = random.Random(WORLD)
-for replicate_log, ahead_log in ((0, 14), (0, 0), (18, 14)):
-    for k in ranks:
-        k.ctx.set_option(ZK_OPT_REPLICATE_LOG, replicate_log)
-        k.ctx.set_option(ZK_OPT_AHEAD_LOG, ahead_log)
-    for n in (LOG, LOG + 1, LOG + 5):  # one entry of a table a rank, two, more
-        for L in (1, 2, 3, 4):
-            linear(ranks, n, [[rnd.randrange(M) for _ in range(1 << n)] for _ in range(L)])
-        dense = [rnd.randrange(M) for _ in range(1 << n)]
-        for nnz in (0, 1, min(1 << n, 40)):
-            idx = sorted(rnd.sample(range(1 << n), nnz))
-            sparse(ranks, n, idx, [rnd.randrange(M) for _ in idx], dense)
+def healthy():
+    ranks = start()
+    rnd = random.Random(WORLD)
+    for replicate_log, ahead_log in ((0, 14), (0, 0), (18, 14)):
+        for k in ranks:
+            k.ctx.set_option(ZK_OPT_REPLICATE_LOG, replicate_log)
+            k.ctx.set_option(ZK_OPT_AHEAD_LOG, ahead_log)
+        for n in (LOG, LOG + 1, LOG + 5):  # one entry of a table a rank, two, more
+            for L in (1, 2, 3, 4):
+                linear(ranks, n, [[rnd.randrange(M) for _ in range(1 << n)] for _ in range(L)])
+            dense = [rnd.randrange(M) for _ in range(1 << n)]
+            for nnz in (0, 1, min(1 << n, 40)):
+                idx = sorted(rnd.sample(range(1 << n), nnz))
+                sparse(ranks, n, idx, [rnd.randrange(M) for _ in idx], dense)
+
+
+def damaged():
+    """In the entry rounds s(1) is what the round before leaves for it, so a damaged share shows where the dense rounds begin and sum
+    s(0) and s(1) again: whichever all-gather it was, no rank returns a proof, and the communicator stays retired."""
+    rnd = random.Random(7)
+    n = LOG + 9
+    dense = [rnd.randrange(M) for _ in range(1 << n)]
+    idx = [r << 9 | j for r in range(WORLD) for j in (3, 4, 77, 200, 201, 300, 411, 500)]  # eight entries a rank: rounds of 2^9 to 2^5 in entry form
+    vals = [rnd.randrange(1, M) for _ in idx]
+    for replicate_log in (0, 18):
+        for first in (4, 5, 8, 9):  # two all-gathers of the start and one of the counts, then the rounds; 9: a round of the dense form or its table
+            gather.hostgather_damage(0)
+            ranks = start()
+            for k in ranks:
+                k.ctx.set_option(ZK_OPT_REPLICATE_LOG, replicate_log)
+
+            def prove(k):
+                t = Transcript(b"ranks")
+                t.append_u64(b"num_var", n)
+                t.append_u64(b"num_poly", 2)
+                li, lv = zd.shard_sparse(idx, vals, k.rank, WORLD, n)
+                try:
+                    zd.sharded_sparse_dense_prove(k.ctx, k, n, li, lv, DenseMLPoly.from_evaluations(zd.shard_dense(dense, k.rank, WORLD)), t)
+                except ZkError as e:
+                    return e.code
+                return 0
+
+            gather.hostgather_damage(first)
+            for again in range(2):
+                assert on_all(ranks, prove) == [ZK_ERR_COMM] * WORLD, (replicate_log, first, again)
+            for k in ranks:
+                lib.zk_comm_free(k.ctx.handle, k.handle)
+                k.ctx.close()
+
+
+damaged() if len(sys.argv) > 3 else healthy()
 print("ranks ok")

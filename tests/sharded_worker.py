@@ -179,8 +179,21 @@ class HostBox:
         return total
 
 
-def boxed_sharded_linear(box, tables, rank, world, label, fault=None):
-    """The sharded protocol over a HostBox.  fault = (kind, rank, round): "skip" (the rank never posts that
+def value_at(msg, r):
+    """The polynomial of degree len(msg) - 1 with the values msg at 0, 1, ..., at r."""
+    total = 0
+    for i, v in enumerate(msg):
+        num = den = 1
+        for j in range(len(msg)):
+            if j != i:
+                num, den = num * (r - j) % o.R_MOD, den * (i - j) % o.R_MOD
+        total += v * num * pow(den, -1, o.R_MOD)
+    return total % o.R_MOD
+
+
+def boxed_sharded_linear(box, tables, rank, world, label, fault=None, derive=False):
+    """The sharded protocol over a HostBox.  derive: after the first round the ranks do not exchange s(1), which follows from s(0) and the
+    round before, as in the library's resident rounds.  fault = (kind, rank, round): "skip" (the rank never posts that
     round's share), "damage" (its share arrives changed), "args" (it rejects its arguments before round 0).
     Returns ("OK", proof parts) or raises ExchangeError with the status the library would return."""
     from zkes_b200 import SumcheckVerifier, Transcript
@@ -203,7 +216,11 @@ def boxed_sharded_linear(box, tables, rank, world, label, fault=None):
             helper.a_arrays = local
             part = helper._round_message()
             hit = fault and fault[1] == rank and fault[2] == rnd_i
-            msg = box.exchange_sum(part, skip_post=bool(hit and fault[0] == "skip"), damage=bool(hit and fault[0] == "damage"))
+            known = derive and rnd_i > 0
+            msg = box.exchange_sum([part[0]] + part[2:] if known else part, skip_post=bool(hit and fault[0] == "skip"),
+                                   damage=bool(hit and fault[0] == "damage"))
+            if known:
+                msg.insert(1, (value_at(msgs[-1], chals[-1]) - msg[0]) % o.R_MOD)
             for m in msg:
                 tr.append_scalar(b"round_message", m)
             ch = tr.challenge_scalar(b"challenge")
@@ -244,9 +261,9 @@ def gloo_faults(rank, world):
     p = o.LinearSumcheckProver(n, 2, t)
     want = p.prove([dense, f], t)
 
-    def run(box, fault=None):
+    def run(box, fault=None, derive=False):
         try:
-            got = boxed_sharded_linear(box, [dense, f], rank, world, b"faults", fault)
+            got = boxed_sharded_linear(box, [dense, f], rank, world, b"faults", fault, derive)
             assert got[0] == want.round_messages and got[1] == p.challenges and got[2] == want.final_eval
             return "OK"
         except ExchangeError as e:
@@ -268,6 +285,10 @@ def gloo_faults(rank, world):
         dist.barrier()
         fresh = HostBox(store, f"case{case}-fresh", rank, world)
         assert run(fresh) == "OK"
+    for rnd_i in range(n - zd.log2_exact(world)):        # s(1) derived: damage in any round shows by the gathered rounds at the latest
+        box = HostBox(store, f"derived{rnd_i}", rank, world)
+        assert run(box, derive=True) == "OK"
+        assert run(box, ("damage", victim, rnd_i), derive=True) == "COMM"
 
 
 def nccl_faults(rank, world, local_rank):

@@ -18,8 +18,16 @@ def gather(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("world", [2, 4, 8])
-def test_sharded_provers(gather, world):
-    r = subprocess.run([sys.executable, os.path.join(HERE, "ranks.py"), gather, str(world)], capture_output=True, text=True, timeout=300)
+def run(*args):
+    r = subprocess.run([sys.executable, os.path.join(HERE, "ranks.py"), *args], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout[-1000:] + r.stderr[-3000:]
     assert "ranks ok" in r.stdout
+
+
+@pytest.mark.parametrize("world", [2, 4, 8])
+def test_sharded_provers(gather, world):
+    run(gather, str(world))
+
+
+def test_damaged_share(gather):
+    run(gather, "4", "damage")

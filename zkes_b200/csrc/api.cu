@@ -598,10 +598,13 @@ int read_finals(zk_ctx* ctx, int n, const Fr** values) {
   return ZK_OK;
 }
 
-// Self-check of a sharded prove on the host, a few microseconds: every summed message must continue the
+// Self-check of a sharded prove on the host, a few microseconds: every message must continue the
 // round before it, s_m(0) + s_m(1) = s_{m-1}(r_{m-1}) (the identity SumcheckVerifier checks, verifier.rs:
 // 7-70).  A share that was damaged on its way between the ranks breaks it on every rank alike, so all
-// ranks report ZK_ERR_COMM instead of returning a proof no verifier accepts.  n_msgs = degree + 1 values
+// ranks report ZK_ERR_COMM instead of returning a proof no verifier accepts.  In the rounds of the resident
+// launch and in the entry form, but for the first, s(1) is made from s(0) and this very identity, which then holds
+// whatever the shares: damage in them shows at the next message whose s(0) and s(1) are both summed.  There always is one,
+// as the rounds on the gathered tables and the first dense round after the entry form sum both.  n_msgs = degree + 1 values
 // per round at the points 0..degree; Lagrange form with the denominators cleared:
 //   degree! * s(r) = sum_i (-1)^(degree-i) C(degree, i) s(i) prod_{j != i} (r - j).
 int check_round_chain(const uint64_t* round_msgs, const uint64_t* challenges, uint32_t rounds, int n_msgs) {
@@ -627,7 +630,7 @@ int check_round_chain(const uint64_t* round_msgs, const uint64_t* challenges, ui
     }
     const Fr lhs = mul(fact_m, add(fr_load(cur), fr_load(cur + 4)));
     if (lhs != rhs)
-      return fail(ZK_ERR_COMM, "round %u: the summed message does not continue round %u (a rank's share was damaged in the exchange)", m, m - 1);
+      return fail(ZK_ERR_COMM, "round %u: the message does not continue the rounds before it (a rank's share was damaged in the exchange of this round or an earlier one)", m);
   }
   return ZK_OK;
 }
