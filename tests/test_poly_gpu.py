@@ -69,6 +69,31 @@ def test_weighted_fold_edges(ctx, lo, hi, kind):
     assert list(from_mont_array(out)) == [sum(w[h] * f[(h << lo) + c] for h in range(1 << hi)) % M for c in range(1 << lo)]
 
 
+@pytest.mark.parametrize("lo,hi", [(8, 13), (11, 9), (13, 9), (14, 9), (3, 16), (0, 19)])
+def test_weighted_fold_pieces(ctx, lo, hi):
+    """Shapes whose blocks take several steps of 32 rows, so that the sums go on from step to step, the slots of the stream and the weights'
+    256 rows are used again, and pieces end inside a column group, cross into the next, or are a column's only ones.  The table
+    has sixteen different elements, the largest (p - 1 in memory) and zero among them: out[c] = sum_e e sum_{h: f[h, c] = e} w[h], the
+    inner sums exact in double precision by 16-bit limbs."""
+    rnd = np.random.default_rng(100 * lo + hi)
+    largest = (M - 1) * pow(1 << 256, -1, M) % M
+    pool = [largest, 0] + [int.from_bytes(rnd.bytes(40), "little") % M for _ in range(14)]
+    w = [largest if h % 3 == 0 else int.from_bytes(rnd.bytes(40), "little") % M for h in range(1 << hi)]
+    which = rnd.integers(0, 16, size=(1 << hi, 1 << lo), dtype=np.uint8)
+    which[:, 0] = 0  # a column of nothing but the largest
+    f, wm, out = to_mont_array(pool)[which.reshape(-1)], to_mont_array(w), np.zeros((1 << lo, 4), dtype=np.uint64)
+    vp = ctypes.c_void_p
+    check(lib.zk_weighted_fold_from_right(ctx.handle, lo + hi, vp(f.ctypes.data), ZK_MEM_HOST, hi, vp(wm.ctypes.data), ZK_MEM_HOST,
+                                          vp(out.ctypes.data), ZK_MEM_HOST), "zk_weighted_fold_from_right")
+    limbs = np.frombuffer(b"".join(x.to_bytes(32, "little") for x in w), dtype="<u2").reshape(1 << hi, 16).astype(np.float64)
+    want = [0] * (1 << lo)
+    for e in range(16):
+        if pool[e]:
+            sums = (which == e).astype(np.float64).T @ limbs  # below 2^19 * 2^16
+            want = [a + pool[e] * sum(int(x) << (16 * k) for k, x in enumerate(row)) for a, row in zip(want, sums.tolist())]
+    assert list(from_mont_array(out)) == [x % M for x in want]
+
+
 @pytest.mark.parametrize("n", [0, 1, 3, 8, 11, 15])
 def test_evaluate_at_point(ctx, n):
     """DenseMLPoly::evaluate_at_point (poly.rs:788-791); test_kzh2.rs:149-175 relies on it."""

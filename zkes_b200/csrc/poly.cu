@@ -4,6 +4,7 @@
 #include "internal.hpp"
 #include "reduce.cuh"
 #include "byte_mma.cuh"
+#include "from_right_plan.hpp"
 
 namespace zk {
 namespace {
@@ -142,7 +143,7 @@ __global__ void __launch_bounds__(256) k_from_right(const Fr* __restrict__ f, co
 // 2^12 rows of 2^12 columns take 102 us (5.3 TB/s of the table's bytes), where the integer pipe took 171 with 64 multiply-adds an
 // element; cut by columns alone, 256 blocks for 296 places, it was 112 us.  What bounds it now is issue: some 100 instructions a warp
 // and step beside 16 of the tensor cores.
-constexpr int kCtThreads = 256, kCtWarps = kCtThreads / 32, kCtStages = 4, kCtChunk = 256, kCtStep = 32, kCtCols = 2 * kCtWarps;
+constexpr int kCtThreads = 32 * kCtWarps, kCtStages = 4, kCtChunk = 256;
 constexpr size_t kCtShared = (size_t)kCtWarps * kCtStages * 2048 + (size_t)kCtChunk * 32;
 
 // out[b] = bytes b of a0, a1, a2, a3
@@ -311,10 +312,9 @@ __global__ void __launch_bounds__(kCtThreads, 2) k_from_right_bytes(const Fr* __
     const Fr r = reduce_words(z);
     const uint64_t lo = lo0 + (t >> 1);
     if (g == 0 && (t & 1) == 0 && lo < lo_n) {
-      // the blocks that share a column are neighbours; the last of them clears the slots that are left over
-      uint32_t at = (uint32_t)(blockIdx.x - (uint64_t)group * col_steps / per);
+      uint32_t at = bytes_slot(blockIdx.x, group, col_steps, per);
       st_fr_plain(partial + (uint64_t)at * lo_n + lo, r);
-      if (step0 + steps == col_steps)
+      if (step0 + steps == col_steps)  // the column's last piece clears the slots that are left over
         for (at++; at < slots; at++) st_fr_plain(partial + (uint64_t)at * lo_n + lo, Fr::zero());
     }
     line += steps;
@@ -384,29 +384,6 @@ int launch_eq_table(const EqPoint& point, uint32_t k, Fr* out, int sm_count, cud
   const uint64_t stretches = k > (uint32_t)kEqBits ? 1ull << (k - kEqBits) : 1, wave = (uint64_t)sm_count * kEqWave;
   k_eq_table<<<(unsigned)(stretches < wave ? stretches : wave), kEqThreads, 0, s>>>(out, point, (int)k);
   return 1;
-}
-
-// Contractions of at least kCtRows rows go through the tensor cores.  A column's sums cost the same to put together whatever its rows:
-// 2^22 values take 212 us in 2^5 rows, 121 in 2^6, 73 in 2^7, 54 in 2^8, 43 in 2^10; on the integer pipe 60, 56, 54, 52 and 54.
-constexpr uint64_t kCtRows = 512;
-
-// How the steps of a contraction are cut (k_from_right_bytes).
-struct BytesPlan {
-  uint64_t groups, steps, per, blocks;
-  uint32_t slots;
-};
-static BytesPlan bytes_plan(uint64_t lo_n, uint64_t hi_n, int sm_count) {
-  BytesPlan p;
-  p.groups = (lo_n + kCtCols - 1) / kCtCols;
-  p.steps = (hi_n + kCtStep - 1) / kCtStep;
-  const uint64_t all = p.groups * p.steps, places = 2 * (uint64_t)sm_count;
-  p.per = (all + places - 1) / places;
-  // sums of 2^15 products of bytes stay below 2^31
-  if (p.per > 1024) p.per = 1024;
-  p.blocks = (all + p.per - 1) / p.per;
-  // a column that begins where a piece does has ceil(steps / per) of them; where all columns do, that is all
-  p.slots = (uint32_t)((p.steps + p.per - 1) / p.per + (p.per % p.steps == 0 || p.steps % p.per == 0 ? 0 : 1));
-  return p;
 }
 
 uint32_t from_right_splits(uint64_t lo_n, uint64_t hi_n, int sm_count) {
