@@ -1195,9 +1195,10 @@ static RowsPlan small_rows_plan(const MsmPrep& prep, uint64_t n, uint32_t rows, 
 }
 
 // The rows of a commitment beside its C, both over the same small scalars: the rows' tables and sums on the side stream while C sorts
-// its digits, whichever is done first leaving the GPU to the other.  Their scratch then lies beside C's; above kBesideMost the
-// two come one after the other, as the parts that leave the GPU idle are short beside the others then.  2^24 int8 values in 2^12 rows:
-// 5 759 us a commitment, one after the other 6 193.
+// its digits, whichever is done first leaving the GPU to the other.  A commitment of 2^24 int8 values in 2^12 rows takes 5 633 us, one after
+// the other 6 079; of 2^20 741 and 982, of 2^25 10 914 and 11 525; int16 942 and 1 289, 7 762 and 8 277, 14 949 and 15 655 (2^20, 2^24, 2^25).
+// Their scratch lies beside C's then and stays in the lane's: 153 MB for 2^24 int8 values, 357 MB for 2^25 of 24 bits.  kBesideMost bounds
+// that memory; every shape of up to 2^25 values is below it, and faster like this.
 constexpr size_t kBesideMost = 512u << 20;
 
 // row_ids == nullptr: `rows` dense rows of n scalars each over the same n bases.  Otherwise: n scalars in

@@ -83,8 +83,10 @@ __global__ void __launch_bounds__(256) k_range_scatter_small(const uint64_t* __r
 
 // And for a table of at most kCopiesTable entries, where 32 lanes would meet on 16 counters: eight lanes take a pair, a limb each,
 // and add it into counters of their own, so that no addition is atomic before the block's copies are added up.  2^17 pairs on 16
-// entries take 6.9 us, by atomics on a block's one copy 21.6.  A block's copies are 32 KB for 16 entries, which double with the table
-// while the lanes of a warp meet half as often: larger tables stay with the atomics.
+// entries take 6.9 us, by atomics on a block's one copy 21.6.  The line is where a block of 256 threads fills 32 KB of shared memory with
+// its copies.  Above it the lanes of a warp meet half as often with every doubling, and a block that keeps the 32 KB has half as many threads:
+// whole calls by copies in such blocks and by atomics take 40 and 50 us for 2^17 pairs on 32 entries, 46 and 50 on 64 (40 and 55 on 16),
+// 67 and 100, 70 and 93 (71 and 109) for 2^19, 36 and 40, 37 and 40 (36 and 42) for 2^12.  Blocks of other sizes are not built.
 constexpr uint32_t kCopiesTable = 16;
 constexpr int kCopiesThreads = 256, kCopies = kCopiesThreads / 8;
 __global__ void __launch_bounds__(kCopiesThreads) k_range_scatter_copies(const uint64_t* __restrict__ input_idx,
