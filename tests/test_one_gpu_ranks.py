@@ -1,5 +1,5 @@
 """The sharded entry points with several ranks on one GPU: the ranks are threads whose all-gathers go through host memory
-(tests/one_gpu_ranks), so that the code around the exchange runs as it is, with 4 and 8 ranks, where the box has one GPU."""
+(tests/one_gpu_ranks), so that the code around the exchange runs as it is, with 4 and 8 ranks, where the machine has one GPU."""
 import os
 import subprocess
 import sys
